@@ -88,6 +88,9 @@ cudaError_t ensure_smem_limit(const void* kernel, int bytes) {
         ++launches;                                                                \
     } while (0)
 
+// entries of the largest right block a plan hands to k_tiny_rref
+constexpr int64_t kTinyPlanBlock = 54000;
+
 // per-launch executed-K-step counters of a profiled run
 constexpr int kGemmProfileSlots = 4096;
 
@@ -202,11 +205,11 @@ struct Plan {
     int32_t np = 0;
     int64_t onnz = 0;
     uint32_t errbits = 0;
-    // small matrices: one-CTA echelon + compaction, no host round trip in a
+    // small matrices: one-cluster echelon + compaction, no host round trip in a
     // run; its checks, counts and timings are read when the answer is taken
     bool tiny = false;
-    int tiny_bytes = 0;
-    int64_t* tiny_counts = nullptr;  // [2]: rows, entries of the answer
+    int tiny_cl = 0;  // CTAs of its cluster
+    int64_t* tiny_counts = nullptr;  // [3]: rows, entries of the answer, verdict
     bool pending = false;            // a tiny run whose results are not read yet
     // answer streamed to host arrays during the run (gbgpu_plan_run_into_v)
     StreamOut* stream_req = nullptr;
@@ -327,13 +330,15 @@ static int plan_alloc(Plan* P) {
             A(losers, P->n_work);
         }
     }
-    if (P->mode == 0 && !P->blocked && P->n_work > 0 && P->ncr > 0)
-        P->tiny_bytes = tiny_rref_bytes(P->n_work, P->ncr, P->dev.smem_optin);
-    P->tiny = P->tiny_bytes > 0;
+    // small blocks; larger ones show the sparse-row form's own echelon
+    if (P->mode == 0 && !P->blocked && P->n_work > 0 && P->ncr > 0 &&
+        (int64_t)P->n_work * P->ncr <= kTinyPlanBlock)
+        P->tiny_cl = tiny_cluster(P->n_work, P->ncr, P->dev.smem_optin);
+    P->tiny = P->tiny_cl > 0;
     if (P->tiny) {
         // the answer has at most n_work rows of ncr entries
         const size_t cap = (size_t)P->n_work * P->ncr;
-        A(tiny_counts, 2);
+        A(tiny_counts, 3);
         A(out_cols, cap);
         A(out_vals, cap);
         P->out_cap = (int64_t)cap;
@@ -513,9 +518,9 @@ static int run_form(Plan* P, const F& f) {
 
     if (P->tiny) {
         // ---- small right block: echelon form and compaction in one CTA ------
-        GB_CALL(launch_tiny_rref(P->n_work, P->ncr, P->D, P->ld, P->lead, P->err, P->ncl,
+        GB_CALL(launch_tiny_rref(P->n_work, P->ncr, P->D, P->ld, P->err, P->ncl,
                                  P->offs, P->out_cols, P->out_vals, P->piv_of_col,
-                                 P->tiny_counts, P->tiny_bytes, s, f));
+                                 P->tiny_counts, P->tiny_cl, s, f));
         P->stats.echelon_rounds = 0;
         GB_CUDA(cudaEventRecord(P->ev[3], s));
         GB_CUDA(cudaEventRecord(P->ev[4], s));

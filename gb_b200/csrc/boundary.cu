@@ -655,7 +655,7 @@ static bool batch_small(const gbgpu_csr& m, const gbgpu_options* opt) {
     const int vb = m.val_bytes ? m.val_bytes : 4;
     if (!(vb == 1 || vb == 2 || vb == 4) || (vb < 4 && (int64_t)m.p >= ((int64_t)1 << (8 * vb))))
         return false;
-    return small_batch_bytes(m.nr, m.ncl, m.ncr, opt ? opt->device : 0) > 0;
+    return small_batchable(m.nr, m.ncl, m.ncr, opt ? opt->device : 0);
 }
 
 int gbgpu_reduce_batch(int32_t n, const gbgpu_csr* ms, const gbgpu_options* opt,

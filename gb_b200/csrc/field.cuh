@@ -20,6 +20,27 @@
 
 namespace gbgpu {
 
+// A sum of products in N independent chains (a dependent 64-bit multiply-add
+// takes 14 cycles): term k goes to chain k mod N.
+template <class F, int N = 4>
+struct ChainSum {
+    typename F::Sum s[N];
+    __device__ __forceinline__ ChainSum(const F& f) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) f.sum_init(s[k]);
+    }
+    __device__ __forceinline__ void add(const F& f, int k, uint32_t ep, uint32_t v) {
+        f.sum_add(s[k % N], ep, v);
+    }
+    __device__ __forceinline__ uint32_t mod(const F& f) {
+#pragma unroll
+        for (int w = N / 2; w > 0; w /= 2)
+#pragma unroll
+            for (int k = 0; k < w; ++k) s[k] = f.sum_join(s[k], s[k + w]);
+        return f.sum_mod(s[0]);
+    }
+};
+
 struct FieldSmall {
     uint32_t p;
     uint32_t mu;  // floor(2^32 / p)
@@ -57,6 +78,27 @@ struct FieldSmall {
         const uint32_t r = s - q * p;
         return r >= p ? r - p : r;
     }
+    // sums of at most 32 products prep(e) v (e, v < p), reduced once: below
+    // 2^37 = hi 2^32 + lo, hi < 32, and lo mod p + hi (2^32 mod p) < 2^22
+    using Sum = uint64_t;
+    __device__ __forceinline__ void sum_init(Sum& s) const { s = 0; }
+    __device__ __forceinline__ void sum_add(Sum& s, uint32_t ep, uint32_t v) const {
+        s += (uint64_t)ep * v;
+    }
+    __device__ __forceinline__ Sum sum_join(const Sum& a, const Sum& b) const { return a + b; }
+    // (right for any s < 2^46: hi < 2^14 and the sum below stays under 2^31)
+    __device__ __forceinline__ uint32_t sum_mod(const Sum& s) const {
+        const uint32_t lo = (uint32_t)s, hi = (uint32_t)(s >> 32);
+        const uint32_t t = lo - __umulhi(lo, mu) * p + hi * (0u - mu * p);
+        const uint32_t r = t - __umulhi(t, mu) * p;
+        return r >= p ? r - p : r;
+    }
+    // a residue with up to 2^14 products m v (m, v < p) added, not reduced
+    // (below 2^46), and its value
+    __device__ __forceinline__ uint64_t lazy_add(uint64_t t, uint32_t m, uint32_t v) const {
+        return t + (uint64_t)m * v;
+    }
+    __device__ __forceinline__ uint32_t lazy_mod(uint64_t t) const { return sum_mod(t); }
     // a^-1 = a^(p-2) mod p (0 < a < p), square and multiply
     __device__ __forceinline__ uint32_t inv(uint32_t a) const {
         uint32_t r = 1u, b = a;
@@ -113,6 +155,31 @@ struct FieldMont {
         const uint32_t r = (uint32_t)((T + (uint64_t)q * p) >> 32);
         return r >= p ? r - p : r;
     }
+    // sums of at most 32 products prep(e) v: v in 16-bit halves, so either sum
+    // is below 32 p 2^16 < p 2^32, the bound of redc
+    struct Sum {
+        uint64_t lo, hi;
+    };
+    __device__ __forceinline__ void sum_init(Sum& s) const { s.lo = s.hi = 0; }
+    __device__ __forceinline__ void sum_add(Sum& s, uint32_t ep, uint32_t v) const {
+        s.lo += (uint64_t)ep * (v & 0xFFFFu);
+        s.hi += (uint64_t)ep * (v >> 16);
+    }
+    __device__ __forceinline__ Sum sum_join(const Sum& a, const Sum& b) const {
+        return Sum{a.lo + b.lo, a.hi + b.hi};
+    }
+    __device__ __forceinline__ uint32_t sum_mod(const Sum& s) const {
+        const uint32_t r = redc(s.lo) + mulp(redc(s.hi), prep(65536u));
+        return r >= p ? r - p : r;
+    }
+    // a residue with products m v (m, v < p) added, kept below p^2 < 2^62, and
+    // its value (p^2 < p 2^32, the bound of redc)
+    __device__ __forceinline__ uint64_t lazy_add(uint64_t t, uint32_t m, uint32_t v) const {
+        const uint64_t p2 = (uint64_t)p * p;
+        t += (uint64_t)m * v;
+        return t >= p2 ? t - p2 : t;
+    }
+    __device__ __forceinline__ uint32_t lazy_mod(uint64_t t) const { return prep(redc(t)); }
     // a^-1 = a^(p-2) mod p (0 < a < p), square and multiply in Montgomery form
     __device__ __forceinline__ uint32_t inv(uint32_t a) const {
         uint32_t r = prep(1u), b = prep(a);

@@ -684,41 +684,75 @@ cudaError_t launch_promote(int grid, int threads, cudaStream_t s, const int32_t*
 // ---------------------------------------------------------------------------
 // Small matrices: the reduced row echelon form of the whole n x m block D'
 // (rows with lead < 0 are zero) and its compaction to CSR in the shared
-// memory of ONE CTA, in one launch instead of echelon rounds, back
-// substitution and compaction (which cost a host round trip each).  Row r
-// belongs to warp r % 32.  A step takes the non-pivot row with the smallest
-// (lead, row) as the pivot (the pivots of the column-by-column search),
-// normalises it (one inverse, lane 0 of its warp), and every warp clears the
-// pivot column from its other rows, pivots included (Gauss-Jordan),
-// recomputing the leads of the non-pivot rows it changed.  Output: the pivot
+// memory of one cluster, in one launch instead of echelon rounds, back
+// substitution and compaction (which cost a host round trip each); tiny.cuh has
+// the algorithm.  Output: the pivot
 // rows in descending pivot-column order as CSR (columns + col_shift), their
 // offsets, piv_of_col, and counts[0..1] = rows, entries.  When the input
 // checks flagged an error nothing is read and the answer is empty.
 template <class F>
-__global__ void __launch_bounds__(kTinyThreads)
+__global__ void __launch_bounds__(kTinyThreads, 1)
 k_tiny_rref(int32_t n, int32_t m, const uint32_t* __restrict__ D, int64_t ld,
-            const int32_t* __restrict__ lead_in, const uint32_t* err, TinyOut out, F f) {
-    extern __shared__ uint32_t tiny_smem[];
-    tiny_rref_body(n, m, D, ld, lead_in, err, out, f, tiny_smem);
+            const uint32_t* err, TinyOut out, F f) {
+    extern __shared__ __align__(16) uint32_t tiny_smem[];
+    const int CL = cluster_size(), rk = cluster_rank();
+    if (*err) {  // uniform over the cluster
+        if (rk == 0) {
+            if (out.piv_of_col)
+                for (int c = threadIdx.x; c < m; c += kTinyThreads) out.piv_of_col[c] = -1;
+            if (threadIdx.x == 0) {
+                out.offs[0] = 0;
+                out.counts[0] = 0;
+                out.counts[1] = 0;
+                out.counts[2] = (int64_t)*err;
+            }
+        }
+        return;
+    }
+    if (rk == 0 && threadIdx.x == 0) out.counts[2] = 0;
+    for (int t = rk; t * TP < m; t += CL)
+        for (int q = threadIdx.x; q < n * TP; q += kTinyThreads) {
+            const int r = q / TP, j = t * TP + q % TP;
+            tiny_smem[(t / CL) * n * TP + q] = j < m ? D[(size_t)r * ld + j] : 0u;
+        }
+    tiny_rref_body(n, m, tiny_smem, out, f);
 }
 
-// shared memory of k_tiny_rref for an n x m block (0: too large)
-int tiny_rref_bytes(int32_t n, int32_t m, int smem_optin) {
-    const int64_t mx = std::max(n, m);
-    const int64_t bytes = (int64_t)n * (m + 1) * 4 + (int64_t)n * 16 + (int64_t)m * 4 + mx * 8 + 64;
-    return bytes <= smem_optin - 4096 ? (int)bytes : 0;
+// CTAs of k_tiny_rref's cluster for an n x m block (0: too large)
+int tiny_cluster(int32_t n, int32_t m, int smem_optin) {
+    const int64_t room = smem_optin - 4096;
+    return tiny_layout(n, m, kTinyMaxCluster).words * 4 <= room ? kTinyMaxCluster : 0;
+}
+
+cudaError_t launch_cluster(const void* kernel, int grid, int cl, int threads, int bytes,
+                           cudaStream_t s, void** args) {
+    cudaError_t e = ensure_smem_limit(kernel, bytes);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)cl;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 template <class F>
 cudaError_t launch_tiny_rref(int32_t n, int32_t m, const uint32_t* D, int64_t ld,
-                             const int32_t* lead, const uint32_t* err, int32_t col_shift,
-                             int64_t* offs, int32_t* cols, int32_t* vals, int32_t* piv_of_col,
-                             int64_t* counts, int bytes, cudaStream_t s, const F& f) {
-    cudaError_t e = ensure_smem_limit((const void*)k_tiny_rref<F>, bytes);
-    if (e != cudaSuccess) return e;
-    const TinyOut o{col_shift, offs, cols, vals, piv_of_col, counts};
-    k_tiny_rref<F><<<1, kTinyThreads, bytes, s>>>(n, m, D, ld, lead, err, o, f);
-    return cudaGetLastError();
+                             const uint32_t* err, int32_t col_shift, int64_t* offs, int32_t* cols,
+                             int32_t* vals, int32_t* piv_of_col, int64_t* counts, int cl,
+                             cudaStream_t s, const F& f) {
+    TinyOut o{col_shift, offs, cols, vals, piv_of_col, counts};
+    F fv = f;
+    void* args[] = {&n, &m, &D, &ld, &err, &o, &fv};
+    return launch_cluster((const void*)k_tiny_rref<F>, cl, cl, kTinyThreads,
+                          (int)(tiny_layout(n, m, cl).words * 4), s, args);
 }
 
 #define GBGPU_INSTANTIATE(F)                                                                   \
@@ -733,9 +767,9 @@ cudaError_t launch_tiny_rref(int32_t n, int32_t m, const uint32_t* D, int64_t ld
                                            uint32_t*, int64_t, int32_t, int32_t*, int32_t*,    \
                                            const F&);                                          \
     template cudaError_t launch_tiny_rref<F>(int32_t, int32_t, const uint32_t*, int64_t,       \
-                                             const int32_t*, const uint32_t*, int32_t,         \
-                                             int64_t*, int32_t*, int32_t*, int32_t*, int64_t*, \
-                                             int, cudaStream_t, const F&);
+                                             const uint32_t*, int32_t, int64_t*, int32_t*,     \
+                                             int32_t*, int32_t*, int64_t*, int, cudaStream_t,  \
+                                             const F&);
 GBGPU_INSTANTIATE(FieldSmall)
 GBGPU_INSTANTIATE(FieldMont)
 #undef GBGPU_INSTANTIATE

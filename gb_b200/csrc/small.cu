@@ -1,5 +1,6 @@
-// small.cu -- one-pass reduction of small Macaulay matrices (the la calls of
-// the early F4 rounds and of small systems), built for latency.
+// small.cu -- one-launch reduction of small Macaulay matrices (the la calls of
+// the early F4 rounds, of small systems and of their prime images), built for
+// latency.
 //
 // A general plan (api.cu) creates a stream, allocates a dozen buffers, runs
 // ten or more launches and copies in and out through pageable memory; for a
@@ -9,17 +10,24 @@
 // mark and reused), and a call is
 //
 //   rows gathered into pinned staging  ->  one host-to-device copy
-//   k_small_prep      (1 CTA)   input checks, known pivots, ordered C|D row list
-//   k_reduce_rows_warp          one warp per C|D row, dense accumulator of the
-//                               row in shared memory, known pivots applied in
-//                               column order (src/la_ff_16.c:289-351 / :102-190)
-//   k_tiny_rref       (1 CTA)   reduced echelon form of the right block and its
-//                               compaction (plain.cu), written straight into
-//                               mapped host memory
-//   one 4-byte copy of the checks' verdict, one stream synchronisation.
+//   k_small   one thread-block cluster: input checks, known pivots and the
+//             C|D row list; a warp per C|D row reduces it by the known pivots
+//             (src/la_ff_16.c:289-351 / :102-190) in shared memory; the reduced
+//             echelon form of the right block and its compaction (tiny.cuh),
+//             written straight into mapped host memory with the checks' verdict
+//   one stream synchronisation.
 //
-// The answer is the canonical one of every other path (descending leads,
-// monic, columns ascending).
+// Measured on a B200, 441 x 491 matrix (141 x 191 block, p = 32003): 1425 us a
+// call with one CTA for the echelon and a launch per phase, 244 us now, of it
+// k_small 207 us (checks and diagonal blocks 22, rows 75, echelon 110; all three
+// are chains of dependent steps on a few SMs, not throughput); over 2^31 - 1,
+// 2430 and 276 us.  Matrices with more rows or a longer chain of left columns
+// run the three phases as launches of their own, the rows on the whole device
+// (kWideRows below).
+//
+// A batch's small matrices share one launch: the clusters take matrices from a
+// work queue.  The answer is the canonical one of every other path (descending
+// leads, monic, columns ascending).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,246 +46,10 @@
 
 namespace gbgpu {
 
-constexpr int kPrepThreads = 1024;
-constexpr int kSmallMaxLeft = 12288;  // left columns: the prep kernel's pivot table in smem
-constexpr int kRowWarpsMax = 16;      // warps (rows) per CTA of k_reduce_rows_warp
+constexpr int kSmallMaxLeft = 12288;  // left columns
+constexpr int LB = 32;                // left columns of a diagonal block (one per lane)
 
-// ---------------------------------------------------------------------------
-// kernels
-
-// Input checks (the contract k_check_rows enforces), the known pivot of every
-// left column (first row with that lead, src/la_ff_16.c:762-772), the check
-// that every left column has one, and the C|D rows in row order -- one CTA.
-__device__ void small_prep_body(int32_t nr, int32_t ncl, int32_t nc, uint32_t p,
-                                const int64_t* __restrict__ row_ptr,
-                                const int32_t* __restrict__ cols,
-                                const uint32_t* __restrict__ vals, int32_t* piv_row,
-                                int2* pext, int32_t* work, int32_t* n_work, uint32_t* err,
-                                int32_t* prep_tab /* smem [ncl] */) {
-    __shared__ uint32_t s_err;
-    __shared__ int s_warp[kPrepThreads / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = kPrepThreads / 32;
-    for (int c = tid; c < ncl; c += blockDim.x) prep_tab[c] = INT_MAX;
-    if (tid == 0) s_err = 0;
-    __syncthreads();
-    for (int i = warp; i < nr; i += NW) {
-        const int64_t b = row_ptr[i], e = row_ptr[i + 1];
-        uint32_t bad = 0;
-        if (e <= b) {
-            bad |= kErrEmptyRow;
-        } else {
-            const int32_t lead = cols[b];
-            if (lead < 0 || lead >= ncl) bad |= kErrLeadRange;
-            if (vals[b] != 1u) bad |= kErrNotMonic;
-            for (int64_t k = b + lane; k < e; k += 32) {
-                const int32_t c = cols[k];
-                const uint32_t v = vals[k];
-                if (c < lead || c >= nc || (k > b && c == lead)) bad |= kErrColRange;
-                if (v == 0u || v >= p) bad |= kErrCoefRange;
-            }
-            if (lane == 0 && lead >= 0 && lead < ncl) atomicMin(&prep_tab[lead], i);
-        }
-        for (int o = 16; o > 0; o >>= 1) bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-        if (lane == 0 && bad) atomicOr(&s_err, bad);
-    }
-    __syncthreads();
-    for (int c = tid; c < ncl; c += blockDim.x) {
-        const int32_t r = prep_tab[c];
-        if (r == INT_MAX) atomicOr(&s_err, kErrMissingPivot);
-        piv_row[c] = r;
-        // the pivot row's applied entries (its lead excluded), as 32-bit offsets
-        pext[c] = r == INT_MAX ? make_int2(0, 0)
-                               : make_int2((int)row_ptr[r] + 1, (int)row_ptr[r + 1]);
-    }
-    // rows that are not the known pivot of their lead, in row order
-    int base = 0;
-    for (int r0 = 0; r0 < nr; r0 += kPrepThreads) {
-        const int i = r0 + tid;
-        int f = 0;
-        if (i < nr) {
-            const int64_t b = row_ptr[i];
-            if (row_ptr[i + 1] > b) {
-                const int32_t lead = cols[b];
-                if (lead >= 0 && lead < ncl) f = prep_tab[lead] != i;
-            }
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) s_warp[warp] = __popc(bal);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int w = 0; w < NW; ++w) {
-            const int c = s_warp[w];
-            before += w < warp ? c : 0;
-            total += c;
-        }
-        if (f) work[base + before + __popc(bal & ((1u << lane) - 1u))] = i;
-        base += total;
-        __syncthreads();  // s_warp is rewritten by the next chunk
-    }
-    __syncthreads();
-    if (tid == 0) {
-        *n_work = base;
-        *err = s_err;
-    }
-}
-
-__global__ void __launch_bounds__(kPrepThreads)
-k_small_prep(int32_t nr, int32_t ncl, int32_t nc, uint32_t p, const int64_t* __restrict__ row_ptr,
-             const int32_t* __restrict__ cols, const uint32_t* __restrict__ vals,
-             int32_t* piv_row, int2* pext, int32_t* work, int32_t* n_work, uint32_t* err) {
-    extern __shared__ int32_t prep_smem[];  // [ncl]: first row of each lead
-    small_prep_body(nr, ncl, nc, p, row_ptr, cols, vals, piv_row, pext, work, n_work, err,
-                    prep_smem);
-}
-
-// One warp per C|D row: the row is scattered into a dense accumulator of nc
-// residues in shared memory, then the known pivots are applied in column
-// order -- the next column to clear is the first nonzero left column after
-// the last one cleared (a warp ballot over 32 columns at a time); the pivot
-// row (monic, its lead skipped) is applied by the 32 lanes in coalesced
-// strides (distinct columns, no conflicts).  The right block is written out
-// dense with its lead.  Nothing is read when the checks flagged the input.
-// rows w = w0, w0 + step, ... (< n_rows) by the calling warp, whose
-// accumulator is acc (stride entries, 16-byte aligned).  The pivot chain is
-// software-pipelined: before the current pivot row is applied, the warp
-// predicts the next pivot (the next nonzero column of the accumulator as it
-// stands) and loads that pivot row's first 128 entries, so that when the
-// prediction holds (the common case) the next step starts with its data in
-// registers; the pivot rows' extents come from a window of 32 consecutive
-// columns kept one per lane.
-template <class F>
-__device__ void rows_warp_body(int32_t n_rows, int w0, int step,
-                               const int32_t* __restrict__ work,
-                               const int64_t* __restrict__ row_ptr,
-                               const int32_t* __restrict__ cols,
-                               const uint32_t* __restrict__ vals,
-                               const int2* __restrict__ pext, int32_t ncl, int32_t nc,
-                               int32_t stride, uint32_t* out, int64_t ld, int32_t* out_lead,
-                               F f, uint32_t* acc) {
-    const int lane = threadIdx.x & 31;
-    const int32_t ncr = nc - ncl;
-    // first nonzero left column >= from (-1: none), the same for every lane
-    auto scan = [&](int from) -> int {
-        for (int base = from; base < ncl; base += 32) {
-            const int c = base + lane;
-            const unsigned bal = __ballot_sync(0xffffffffu, c < ncl && acc[c] != 0u);
-            if (bal) return base + __ffs(bal) - 1;
-        }
-        return -1;
-    };
-    int wbase = INT_MIN;  // extents window: lane l holds pext[wbase + l]
-    int2 wext = make_int2(0, 0);
-    auto extent = [&](int c) -> int2 {
-        if (c < wbase || c >= wbase + 32) {
-            wbase = c;
-            wext = c + lane < ncl ? pext[c + lane] : make_int2(0, 0);
-        }
-        const int l = c - wbase;
-        return make_int2(__shfl_sync(0xffffffffu, wext.x, l), __shfl_sync(0xffffffffu, wext.y, l));
-    };
-    // the first 128 entries of a pivot row, four per lane
-    auto fetch = [&](int2 e, int32_t (&c)[4], uint32_t (&v)[4]) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = e.x + lane + 32 * u;
-            c[u] = k < e.y ? cols[k] : -1;
-            v[u] = k < e.y ? vals[k] : 0u;
-        }
-    };
-    for (int w = w0; w < n_rows; w += step) {
-        const int32_t r = work[w];
-        const int64_t rb = row_ptr[r], re = row_ptr[r + 1];
-        const int32_t lead = cols[rb];
-        for (int c = (lead & ~3) + 4 * lane; c < stride; c += 128)
-            *(uint4*)(acc + c) = make_uint4(0u, 0u, 0u, 0u);
-        __syncwarp();
-        for (int64_t k = rb + lane; k < re; k += 32) acc[cols[k]] = vals[k];
-        __syncwarp();
-        int found = scan(lead);
-        if (found >= 0) {
-            int2 e = extent(found);
-            int32_t pc[4];
-            uint32_t pv[4];
-            fetch(e, pc, pv);
-            for (;;) {
-                const uint32_t m = f.prep(acc[found]);
-                // prediction: the next nonzero column before this update
-                const int spec = scan(found + 1);
-                int2 es = make_int2(0, 0);
-                int32_t sc[4];
-                uint32_t sv[4];
-                if (spec >= 0) {
-                    es = extent(spec);
-                    fetch(es, sc, sv);
-                }
-                // this pivot row: the first 128 entries from registers (distinct
-                // columns: all loads before the stores), the rest from memory
-                uint32_t y[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) y[u] = pc[u] >= 0 ? acc[pc[u]] : 0u;
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (pc[u] >= 0) acc[pc[u]] = f.mulsub(y[u], m, pv[u]);
-                for (int k = e.x + 128 + lane; k < e.y; k += 32) {
-                    const int32_t c = cols[k];
-                    acc[c] = f.mulsub(acc[c], m, vals[k]);
-                }
-                __syncwarp();
-                const int nxt = scan(found + 1);
-                if (nxt < 0) break;
-                if (nxt == spec) {
-                    e = es;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        pc[u] = sc[u];
-                        pv[u] = sv[u];
-                    }
-                } else {
-                    e = extent(nxt);
-                    fetch(e, pc, pv);
-                }
-                found = nxt;
-            }
-        }
-        uint32_t* o = out + (size_t)w * ld;
-        int first = -1;
-        for (int j0 = 0; j0 < ncr; j0 += 32) {
-            const int j = j0 + lane;
-            const uint32_t v = j < ncr ? acc[ncl + j] : 0u;
-            if (j < ncr) o[j] = v;
-            const unsigned bal = __ballot_sync(0xffffffffu, v != 0u);
-            if (first < 0 && bal) first = j0 + __ffs(bal) - 1;
-        }
-        if (lane == 0) out_lead[w] = first;
-        __syncwarp();
-    }
-}
-
-template <class F>
-__global__ void __launch_bounds__(kRowWarpsMax * 32)
-k_reduce_rows_warp(int32_t n_rows, const int32_t* __restrict__ work,
-                   const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
-                   const uint32_t* __restrict__ vals, const int2* __restrict__ pext,
-                   int32_t ncl, int32_t nc, int32_t stride, uint32_t* out, int64_t ld,
-                   int32_t* out_lead, const uint32_t* err, F f) {
-    extern __shared__ __align__(16) uint32_t rw_acc[];
-    if (*err) return;  // invalid input: nothing is read (uniform)
-    const int warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
-    rows_warp_body(n_rows, blockIdx.x * wpc + warp, gridDim.x * wpc, work, row_ptr, cols, vals,
-                   pext, ncl, nc, stride, out, ld, out_lead, f,
-                   rw_acc + (size_t)warp * stride);
-}
-
-
-// ---------------------------------------------------------------------------
-// batches: every small matrix of a batch in ONE launch.  Each CTA takes the
-// next matrix from a device work queue and runs the three phases above on it
-// (checks and classification, warp-per-row known-pivot reduction into its
-// scratch, one-CTA echelon and compaction into mapped host memory), so the
-// uneven small matrices of a batch share one persistent launch.
-
-struct BatchItem {
+struct SmallItem {
     int32_t p, nr, ncl, ncr;
     int64_t in_off, cols_off, vals_off;  // bytes into the input buffer
     int64_t scr_off;                     // bytes into the scratch buffer
@@ -286,27 +58,26 @@ struct BatchItem {
     FieldMont fm;
 };
 
-// scratch of one matrix: piv_row [ncl] | pivot extents [ncl] | work [nr] | n_work, err |
-// D [n_work][ld] | lead [n_work] | piv_of_col [ncr]
-struct ScrLayout {
-    int64_t piv, pext, work, cnt, D, lead, poc, bytes, ld;
-};
 __host__ __device__ inline int64_t rup(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
-__host__ __device__ inline ScrLayout scr_layout(int32_t nr, int32_t ncl, int32_t ncr) {
+// scratch of one matrix: pivot row of every left column [ncl] | its entries'
+// extent [ncl] | C|D rows [nr] | checks' verdict | diagonal blocks [ncl][LB]
+// | dense rows [n_work][ncr] of the three-launch form
+struct ScrLayout {
+    int64_t piv, pext, work, err, diag, D, bytes;
+};
+__host__ __device__ inline ScrLayout scr_layout(int32_t nr, int32_t ncl, int64_t dense = 0) {
     ScrLayout L;
-    const int64_t nw = nr - ncl > 0 ? nr - ncl : 1;
-    L.ld = rup(ncr > 0 ? ncr : 1, 4);
+    const int64_t n = ncl > 0 ? ncl : 1;
     L.piv = 0;
-    L.pext = rup(4 * (int64_t)(ncl > 0 ? ncl : 1), 256);
-    L.work = L.pext + rup(8 * (int64_t)(ncl > 0 ? ncl : 1), 256);
-    L.cnt = L.work + rup(4 * (int64_t)nr, 256);
-    L.D = L.cnt + 256;
-    L.lead = L.D + rup(4 * nw * L.ld, 256);
-    L.poc = L.lead + rup(4 * nw, 256);
-    L.bytes = L.poc + rup(4 * (int64_t)(ncr > 0 ? ncr : 1), 256);
+    L.pext = rup(4 * n, 256);
+    L.work = L.pext + rup(8 * n, 256);
+    L.err = L.work + rup(4 * (int64_t)nr, 256);
+    L.diag = L.err + 256;
+    L.D = rup(L.diag + 4 * LB * n, 256);
+    L.bytes = rup(L.D + 4 * dense, 256);
     return L;
 }
-// mapped output of one matrix: counts[2], err | offs [n_work + 1] | cols | vals
+// mapped output of one matrix: rows, entries, verdict | offs [n_work + 1] | cols | vals
 struct OutLayout {
     int64_t offs, cols, vals, bytes;
 };
@@ -321,67 +92,365 @@ __host__ __device__ inline OutLayout out_layout(int32_t nr, int32_t ncl, int32_t
     return L;
 }
 
-__global__ void __launch_bounds__(kPrepThreads)
-k_batch_small(int32_t n, const BatchItem* __restrict__ items, const uint8_t* __restrict__ in,
-              uint8_t* scr, uint8_t* out, int32_t* queue, int32_t smem_bytes) {
-    extern __shared__ __align__(16) uint8_t bt_smem[];
+// ---------------------------------------------------------------------------
+// kernel phases
+
+struct SmallMat {
+    int32_t p, nr, ncl, nc;
+    const int64_t* row_ptr;
+    const int32_t* cols;
+    const uint32_t* vals;
+    int32_t* piv_row;
+    int2* pext;
+    int32_t* work;
+    uint32_t* err;
+    uint32_t* diag;
+};
+
+__host__ __device__ inline SmallMat small_mat(const SmallItem& it, const uint8_t* in,
+                                               uint8_t* scr) {
+    uint8_t* sb = scr + it.scr_off;
+    const ScrLayout S = scr_layout(it.nr, it.ncl);
+    return SmallMat{it.p,
+                    it.nr,
+                    it.ncl,
+                    it.ncl + it.ncr,
+                    (const int64_t*)(in + it.in_off),
+                    (const int32_t*)(in + it.cols_off),
+                    (const uint32_t*)(in + it.vals_off),
+                    (int32_t*)(sb + S.piv),
+                    (int2*)(sb + S.pext),
+                    (int32_t*)(sb + S.work),
+                    (uint32_t*)(sb + S.err),
+                    (uint32_t*)(sb + S.diag)};
+}
+
+// Input checks (the contract k_check_rows enforces), the known pivot of every
+// left column (first row with that lead, src/la_ff_16.c:762-772), the check
+// that every left column has one, the C|D rows in row order, and, for the row
+// phase, every pivot row's extent and the negated inverse of every LB x LB
+// diagonal block of the known pivots (prep form).  Spread over the cluster;
+// ends with the verdict.
+template <class F>
+__device__ uint32_t small_prep(const SmallMat& a, uint32_t* smem, int smem_words, const F f) {
+    __shared__ int s_part[kTinyWarps];
+    const int CL = cluster_size(), rk = cluster_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gw = rk * kTinyWarps + warp, ngw = CL * kTinyWarps;
+    for (int c = rk * kTinyThreads + tid; c < a.ncl; c += CL * kTinyThreads) a.piv_row[c] = INT_MAX;
+    if (rk == 0 && tid == 0) *a.err = 0;
+    cluster_sync();
+    for (int i = gw; i < a.nr; i += ngw) {
+        const int64_t b = a.row_ptr[i], e = a.row_ptr[i + 1];
+        uint32_t bad = 0;
+        if (e <= b) {
+            bad |= kErrEmptyRow;
+        } else {
+            const int32_t lead = a.cols[b];
+            if (lead < 0 || lead >= a.ncl) bad |= kErrLeadRange;
+            if (a.vals[b] != 1u) bad |= kErrNotMonic;
+            for (int64_t k = b + lane; k < e; k += 32) {
+                const int32_t c = a.cols[k];
+                const uint32_t v = a.vals[k];
+                if (c < lead || c >= a.nc || (k > b && c == lead)) bad |= kErrColRange;
+                if (v == 0u || v >= (uint32_t)a.p) bad |= kErrCoefRange;
+            }
+            if (lane == 0 && lead >= 0 && lead < a.ncl) atomicMin(&a.piv_row[lead], i);
+        }
+        bad = __reduce_or_sync(0xffffffffu, bad);
+        if (lane == 0 && bad) atomicOr(a.err, bad);
+    }
+    cluster_sync();
+    const bool good = __ldcg(a.err) == 0;  // the rows may be walked
+    for (int c = gw; c < a.ncl; c += ngw) {
+        const int32_t r = __ldcg(a.piv_row + c);
+        if (r == INT_MAX) {
+            if (lane == 0) atomicOr(a.err, kErrMissingPivot);
+            continue;
+        }
+        if (!good) continue;
+        // the applied entries (the lead excluded), as 32-bit offsets
+        const int b = (int)a.row_ptr[r] + 1, e = (int)a.row_ptr[r + 1];
+        if (lane == 0) a.pext[c] = make_int2(b, e);
+        const int k0 = c & ~(LB - 1), k1 = min(k0 + LB, a.ncl);
+        uint32_t* d = a.diag + (size_t)c * LB;
+        d[lane] = 0u;
+        __syncwarp();
+        for (int k = b + lane; k < e; k += 32) {
+            const int32_t j = a.cols[k];
+            if (j >= k0 && j < k1) d[j - k0] = a.vals[k];
+        }
+    }
+    if (rk == 0 && good) {
+        // rows that are not the known pivot of their lead, in row order
+        int base = 0;
+        for (int r0 = 0; r0 < a.nr; r0 += kTinyThreads) {
+            const int i = r0 + tid;
+            const bool f = i < a.nr && __ldcg(a.piv_row + a.cols[a.row_ptr[i]]) != i;
+            const unsigned bal = __ballot_sync(0xffffffffu, f);
+            if (lane == 0) s_part[warp] = __popc(bal);
+            __syncthreads();
+            int before = 0, total = 0;
+            for (int w = 0; w < kTinyWarps; ++w) {
+                const int c = s_part[w];
+                before += w < warp ? c : 0;
+                total += c;
+            }
+            if (f) a.work[base + before + __popc(bal & ((1u << lane) - 1u))] = i;
+            base += total;
+            __syncthreads();  // s_part is rewritten by the next chunk
+        }
+    }
+    cluster_sync();
+    const uint32_t verdict = __ldcg(a.err);
+    if (verdict == 0) {
+        // a warp per block U (unit upper triangular), lane j column j of its
+        // inverse V, from the last row up: V[i] = e_i - sum_(k > i) U[i][k] V[k]
+        const int warps = min(kTinyWarps, smem_words / (2 * LB * LB));
+        uint32_t* U = smem + warp * 2 * LB * LB;
+        uint32_t* V = U + LB * LB;
+        const int nb = (a.ncl + LB - 1) / LB;
+        for (int b = rk + CL * warp; warp < warps && b < nb; b += CL * warps) {
+            uint32_t* d = a.diag + (size_t)b * LB * LB;
+            const int kb = min(LB, a.ncl - b * LB);
+#pragma unroll 8
+            for (int i = 0; i < LB; ++i) {
+                U[i * LB + lane] = i < kb ? __ldcg(d + i * LB + lane) : 0u;
+                V[i * LB + lane] = 0u;  // rows not there yet meet zeros of U
+            }
+            __syncwarp();
+            for (int i = LB - 1; i >= 0; --i) {
+                // terms up to the next multiple of four are zero in U
+                ChainSum<F> s(f);
+#pragma unroll 1
+                for (int k = (i + 1) & ~3; k < LB; k += 4) {
+                    const uint4 u = *(const uint4*)(U + i * LB + k);
+                    s.add(f, 0, u.x, V[k * LB + lane]);
+                    s.add(f, 1, u.y, V[(k + 1) * LB + lane]);
+                    s.add(f, 2, u.z, V[(k + 2) * LB + lane]);
+                    s.add(f, 3, u.w, V[(k + 3) * LB + lane]);
+                }
+                const uint32_t t = s.mod(f);  // V is kept in prep form
+                const uint32_t v = lane == i ? 1u : lane > i && t ? f.p - t : 0u;
+                V[i * LB + lane] = f.prep(v);
+                if (i < kb) d[i * LB + lane] = v ? f.prep(f.p - v) : 0u;
+                __syncwarp();
+            }
+        }
+    }
+    cluster_sync();
+    return verdict;
+}
+
+// C|D rows w0, w0 + step, ... by the calling warp, whose accumulator is acc (nc
+// sums of 64 bits in shared memory, reduced only when a column is read).  The
+// known pivots are applied in column order, LB left columns at a time: the LB
+// multipliers are the block's entries times the inverse of the pivots' diagonal
+// block (independent sums, one shuffle a term), and then the pivot rows whose
+// multiplier is not zero are added to the columns right of the block.  All of
+// a block's multipliers are known before the first of its rows is added, so the
+// rows' entries are loaded GRP rows at a time, no load waiting for an update.
+// The search for the next nonzero column after every update, with a dependent
+// load behind it, took 1200 cycles per pivot, and one reduction per entry.
+// out(w, j, value): right column j of row w.
+constexpr int GRP = 4;  // pivot rows whose first 2 x 32 entries are loaded together
+template <class T>
+__device__ __forceinline__ T pick(const T (&x)[GRP], int q) {
+    return q == 0 ? x[0] : q == 1 ? x[1] : q == 2 ? x[2] : x[3];
+}
+template <class F, class Out>
+__device__ void small_rows(const SmallMat& a, int n_work, int w0, int step, int out_cols,
+                           uint64_t* acc, const F f, const Out out) {
+    const int lane = threadIdx.x & 31;
+    const int32_t ncl = a.ncl, nc = a.nc;
+    for (int w = w0; w < n_work; w += step) {
+        const int32_t r = __ldcg(a.work + w);
+        const int rb = (int)a.row_ptr[r], re = (int)a.row_ptr[r + 1];
+        const int32_t lead = a.cols[rb];
+        for (int c = (lead & ~(LB - 1)) + lane; c < nc; c += 32) acc[c] = 0u;
+        __syncwarp();
+        for (int k = rb + lane; k < re; k += 32) acc[a.cols[k]] = a.vals[k];
+        __syncwarp();
+        for (int k0 = lead & ~(LB - 1); k0 < ncl; k0 += LB) {
+            const int kend = min(k0 + LB, ncl);
+            const bool left = k0 + lane < kend;
+            const uint32_t x0 = left ? f.lazy_mod(acc[k0 + lane]) : 0u;
+            if (!__any_sync(0xffffffffu, x0 != 0u)) continue;
+            const int2 ext = left ? a.pext[k0 + lane] : make_int2(0, 0);
+            uint32_t x;  // the negated multiplier of column k0 + lane
+            {
+                uint32_t d[LB];
+#pragma unroll
+                for (int i = 0; i < LB; ++i)
+                    d[i] = k0 + i < kend ? a.diag[(size_t)(k0 + i) * LB + lane] : 0u;
+                ChainSum<F> s(f);
+#pragma unroll
+                for (int i = 0; i < LB; ++i) s.add(f, i, d[i], __shfl_sync(0xffffffffu, x0, i));
+                x = s.mod(f);
+            }
+            unsigned todo = __ballot_sync(0xffffffffu, x != 0u);
+            // the next GRP pivot rows: extents, multipliers, first entries
+            int b[GRP], e[GRP], nb[GRP], ne[GRP];
+            uint32_t m[GRP], nm[GRP];
+            int32_t c[GRP][2], ncol[GRP][2];
+            uint32_t v[GRP][2], nv[GRP][2];
+            auto fetch = [&]() {
+#pragma unroll
+                for (int q = 0; q < GRP; ++q) {
+                    const int j = todo ? __ffs(todo) - 1 : 0;
+                    nb[q] = __shfl_sync(0xffffffffu, ext.x, j);
+                    ne[q] = todo ? __shfl_sync(0xffffffffu, ext.y, j) : nb[q];
+                    nm[q] = __shfl_sync(0xffffffffu, x, j);
+                    todo &= todo - 1u;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int k = nb[q] + 32 * u + lane;
+                        ncol[q][u] = k < ne[q] ? a.cols[k] : -1;
+                        nv[q][u] = k < ne[q] ? a.vals[k] : 0u;
+                    }
+                }
+            };
+            fetch();
+            for (bool more = true; more;) {
+#pragma unroll
+                for (int q = 0; q < GRP; ++q) {
+                    b[q] = nb[q];
+                    e[q] = ne[q];
+                    m[q] = nm[q];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        c[q][u] = ncol[q][u];
+                        v[q][u] = nv[q][u];
+                    }
+                }
+                more = todo != 0u;
+                if (more) fetch();  // in flight while these rows are added
+                int longest = 0;
+#pragma unroll
+                for (int q = 0; q < GRP; ++q) {
+                    longest = max(longest, e[q] - b[q]);
+                    uint64_t y[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) y[u] = c[q][u] >= kend ? acc[c[q][u]] : 0u;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        if (c[q][u] >= kend) acc[c[q][u]] = f.lazy_add(y[u], m[q], v[q][u]);
+                    __syncwarp();  // the next row may read what this one wrote
+                }
+                if (longest <= 64) continue;
+                // the rest of the long rows
+                for (int q = 0; q < GRP; ++q) {
+                    const int eq = pick(e, q);
+                    const uint32_t mq = pick(m, q);
+                    for (int k = pick(b, q) + 64 + lane; k < eq; k += 128) {
+                        int32_t cc[4];
+                        uint32_t vv[4];
+                        uint64_t yy[4];  // a pivot row's columns are distinct
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            cc[u] = k + 32 * u < eq ? a.cols[k + 32 * u] : -1;
+                            vv[u] = k + 32 * u < eq ? a.vals[k + 32 * u] : 0u;
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) yy[u] = cc[u] >= kend ? acc[cc[u]] : 0u;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (cc[u] >= kend) acc[cc[u]] = f.lazy_add(yy[u], mq, vv[u]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        for (int j = lane; j < out_cols; j += 32)
+            out(w, j, ncl + j < nc ? f.lazy_mod(acc[ncl + j]) : 0u);
+        __syncwarp();
+    }
+}
+
+// accumulators of the row phase that fit in `words` of shared memory
+__host__ __device__ inline int small_warps(int32_t nloc, int32_t nc, int64_t words) {
+    const int64_t fit = words / (2 * (int64_t)(nc > 0 ? nc : 1));
+    const int64_t w = fit < kTinyWarps ? fit : kTinyWarps;
+    return (int)(w < nloc ? w : nloc);
+}
+
+// one matrix by the calling cluster
+template <class F>
+__device__ void small_matrix(const SmallMat& a, int32_t ncr, const TinyOut& to, uint32_t* smem,
+                             int32_t smem_words, const F f) {
+    const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
+    const int n_work = a.nr - a.ncl, warp = threadIdx.x >> 5;
+    const uint32_t e = small_prep(a, smem, smem_words, f);
+    if (e == 0 && n_work > 0) {
+        const TinyLayout L = tiny_layout(n_work, ncr, CL);
+        const int warps = small_warps((n_work + CL - 1) / CL, a.nc, smem_words - L.words);
+        if (warp < warps)
+            // a row's right block to the CTAs that own its columns
+            small_rows(a, n_work, rk + CL * warp, CL * warps, L.panels * TP,
+                       (uint64_t*)(smem + L.words) + (size_t)warp * a.nc, f,
+                       [&](int w, int j, uint32_t v) {
+                           remote_st(remote_smem(smem + tiny_at(n_work, w, j, sh), (j / TP) & (CL - 1)),
+                                     v);
+                       });
+        tiny_rref_body(n_work, ncr, smem, to, f);
+    } else if (rk == 0 && threadIdx.x == 0) {
+        to.counts[0] = 0;
+        to.counts[1] = 0;
+        to.offs[0] = 0;
+    }
+    if (rk == 0 && threadIdx.x == 0) to.counts[2] = (int64_t)e;
+}
+
+// The three phases as launches of their own, for matrices whose rows want more
+// SMs than a cluster has: the row phase over the whole device, rows into D.
+template <class F>
+__global__ void __launch_bounds__(kTinyThreads)
+k_small_prep(const SmallMat a, int32_t smem_words, F f) {
+    extern __shared__ __align__(16) uint32_t sm_smem[];
+    small_prep(a, sm_smem, smem_words, f);
+}
+template <class F>
+__global__ void __launch_bounds__(kTinyThreads)
+k_small_rows(const SmallMat a, int32_t n_work, uint32_t* D, int64_t ld, F f) {
+    extern __shared__ __align__(16) uint32_t sm_smem[];
+    if (*a.err) return;  // invalid input: nothing is read (uniform)
+    const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    small_rows(a, n_work, blockIdx.x + gridDim.x * warp, gridDim.x * warps, a.nc - a.ncl,
+               (uint64_t*)sm_smem + (size_t)warp * a.nc, f,
+               [&](int w, int j, uint32_t v) { D[(size_t)w * ld + j] = v; });
+}
+
+// n matrices, items[0 .. n) from the queue, or the one in `one` (items null)
+__global__ void __launch_bounds__(kTinyThreads)
+k_small(int32_t n, const SmallItem one, const SmallItem* items, const uint8_t* in, uint8_t* scr,
+        uint8_t* out, int32_t* queue, int32_t smem_words) {
+    extern __shared__ __align__(16) uint32_t sm_smem[];
     __shared__ int s_item;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    for (;;) {
-        if (tid == 0) s_item = atomicAdd(queue, 1);
-        __syncthreads();
-        const int i = s_item;
-        __syncthreads();
-        if (i >= n) break;
-        const BatchItem it = items[i];
-        const int32_t nr = it.nr, ncl = it.ncl, ncr = it.ncr, nc = ncl + ncr;
-        const int64_t* row_ptr = (const int64_t*)(in + it.in_off);
-        const int32_t* cols = (const int32_t*)(in + it.cols_off);
-        const uint32_t* vals = (const uint32_t*)(in + it.vals_off);
-        const ScrLayout S = scr_layout(nr, ncl, ncr);
-        uint8_t* sb = scr + it.scr_off;
-        int32_t* piv = (int32_t*)(sb + S.piv);
-        int2* pext = (int2*)(sb + S.pext);
-        int32_t* work = (int32_t*)(sb + S.work);
-        int32_t* nwork = (int32_t*)(sb + S.cnt);
-        uint32_t* err = (uint32_t*)(sb + S.cnt + 16);
-        uint32_t* D = (uint32_t*)(sb + S.D);
-        int32_t* lead = (int32_t*)(sb + S.lead);
-        int32_t* poc = (int32_t*)(sb + S.poc);
+    const int CL = cluster_size(), rk = cluster_rank(), tid = threadIdx.x;
+    for (int pass = 0;; ++pass) {
+        if (items) {
+            if (rk == 0 && tid < 32) {
+                int i = 0;
+                if (tid == 0) i = atomicAdd(queue, 1);
+                i = __shfl_sync(0xffffffffu, i, 0);
+                if (tid < CL) remote_st(remote_smem(&s_item, tid), (uint32_t)i);
+            }
+            cluster_sync();
+            if (s_item >= n) break;
+        } else if (pass > 0) {
+            break;
+        }
+        const SmallItem it = items ? items[s_item] : one;
+        const int32_t nr = it.nr, ncl = it.ncl, ncr = it.ncr;
+        const SmallMat a = small_mat(it, in, scr);
         const OutLayout O = out_layout(nr, ncl, ncr);
         uint8_t* ob = out + it.out_off;
-        int64_t* counts = (int64_t*)ob;
-        small_prep_body(nr, ncl, nc, (uint32_t)it.p, row_ptr, cols, vals, piv, pext, work, nwork, err,
-                        (int32_t*)bt_smem);
-        __syncthreads();  // prep's global writes are visible to the block
-        const uint32_t e = *err;
-        const int32_t n_work = nr - ncl;
-        if (e == 0 && n_work > 0) {
-            const int32_t stride = (int32_t)rup(nc > 0 ? nc : 1, 4);
-            const int wpc = min(kPrepThreads / 32, smem_bytes / (stride * 4));
-            const TinyOut to{ncl, (int64_t*)(ob + O.offs), (int32_t*)(ob + O.cols),
-                             (int32_t*)(ob + O.vals), poc, counts};
-            uint32_t* acc = (uint32_t*)bt_smem + (size_t)warp * stride;
-            if ((uint32_t)it.p < 65536u) {
-                if (warp < wpc)
-                    rows_warp_body(n_work, warp, wpc, work, row_ptr, cols, vals, pext, ncl, nc,
-                                   stride, D, S.ld, lead, it.fs, acc);
-                __syncthreads();
-                tiny_rref_body(n_work, ncr, D, S.ld, lead, err, to, it.fs, (uint32_t*)bt_smem);
-            } else {
-                if (warp < wpc)
-                    rows_warp_body(n_work, warp, wpc, work, row_ptr, cols, vals, pext, ncl, nc,
-                                   stride, D, S.ld, lead, it.fm, acc);
-                __syncthreads();
-                tiny_rref_body(n_work, ncr, D, S.ld, lead, err, to, it.fm, (uint32_t*)bt_smem);
-            }
-        } else if (tid == 0) {
-            counts[0] = 0;
-            counts[1] = 0;
-            ((int64_t*)(ob + O.offs))[0] = 0;
-        }
-        if (tid == 0) counts[2] = (int64_t)e;
-        __syncthreads();  // the shared memory is reused by the next matrix
+        const TinyOut to{ncl, (int64_t*)(ob + O.offs), (int32_t*)(ob + O.cols),
+                         (int32_t*)(ob + O.vals), nullptr, (int64_t*)ob};
+        if ((uint32_t)it.p < 65536u)
+            small_matrix(a, ncr, to, sm_smem, smem_words, it.fs);
+        else
+            small_matrix(a, ncr, to, sm_smem, smem_words, it.fm);
     }
 }
 
@@ -399,7 +468,6 @@ struct Session {
     size_t hin_cap = 0;
     uint8_t* hout = nullptr;  // mapped pinned output
     size_t hout_cap = 0;
-    uint32_t* herr = nullptr;  // pinned: the checks' verdict
     ~Session() {
         // runs at thread exit; at process exit the runtime may already be
         // gone, which these calls tolerate
@@ -407,7 +475,6 @@ struct Session {
         if (dmem) cudaFree(dmem);
         if (hin) cudaFreeHost(hin);
         if (hout) cudaFreeHost(hout);
-        if (herr) cudaFreeHost(herr);
         if (s) cudaStreamDestroy(s);
     }
 };
@@ -473,8 +540,7 @@ int session_for(int device, Session** out) {
             delete n;
             return rc;
         }
-        if (cudaStreamCreateWithFlags(&n->s, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaHostAlloc((void**)&n->herr, 64, cudaHostAllocDefault) != cudaSuccess) {
+        if (cudaStreamCreateWithFlags(&n->s, cudaStreamNonBlocking) != cudaSuccess) {
             delete n;
             set_error("small-matrix session set-up failed");
             return GBGPU_ECUDA;
@@ -496,25 +562,80 @@ struct DeviceGuard {
     }
 };
 
-// rows (warps) per CTA of k_reduce_rows_warp and the accumulator stride
-int rows_warps(int32_t nc, const DeviceInfo& dev, int32_t* stride) {
-    *stride = (int32_t)round_up((size_t)std::max(nc, 1), 4);
-    const int per = *stride * 4;
-    const int fit = (dev.smem_optin - 2048) / per;
-    return std::min(kRowWarpsMax, fit);
+SmallItem small_item(int32_t p, int32_t nr, int32_t ncl, int32_t ncr) {
+    SmallItem it{};
+    it.p = p;
+    it.nr = nr;
+    it.ncl = ncl;
+    it.ncr = ncr;
+    it.fs = FieldSmall::make((uint32_t)std::max(p, 2));
+    it.fm = FieldMont::make((uint32_t)(p | 1));  // used only for odd p >= 2^16
+    return it;
+}
+
+// 32-bit words of shared memory a CTA of a cluster of cl needs for a matrix of
+// this shape: the echelon's, and an accumulator for every row of the CTA up to
+// one per warp (at least four, or one per row), or four blocks of the prep
+// phase; 0: does not fit
+int64_t small_words(int32_t nr, int32_t ncl, int32_t ncr, int cl, int smem_optin) {
+    const int64_t room = (smem_optin - 2048) / 4, least = 4 * 2 * LB * LB;
+    if (nr <= ncl) return least;
+    const TinyLayout L = tiny_layout(nr - ncl, ncr, cl);
+    const int32_t nc = ncl + ncr;
+    const int nloc = (nr - ncl + cl - 1) / cl;
+    const int w = L.words < room ? small_warps(nloc, nc, room - L.words) : 0;
+    if (w < std::min(4, nloc)) return 0;
+    return std::max<int64_t>(least, L.words + w * 2 * (int64_t)nc);
+}
+
+// The three-launch form takes matrices whose echelon fits a cluster and four of
+// whose accumulators fit an SM.
+bool small_wide(int32_t nr, int32_t ncl, int32_t ncr, int smem_optin) {
+    return nr > ncl && tiny_cluster(nr - ncl, ncr, smem_optin) > 0 &&
+           small_warps(4, ncl + ncr, (smem_optin - 2048) / 4) == 4;
+}
+
+// The three-launch form is the faster one where the cluster would take its rows
+// in several turns or the chain of left columns is long: measured for blocks of
+// 60 x 100, 141 x 191, 200 x 300 and 250 x 450 after 200, 300, 500 and 700 left
+// columns at 126 / 235 / 407 / 609 us a call against 113 / 225 / 443 / 738 us in
+// one launch, and 1032 against 1645 us for 120 x 400 after 3000.
+constexpr int kWideRows = 160, kWideLeft = 1024;
+
+// Blocks of more entries are faster in the blocked form (400 x 700: 1570 us here
+// against 1410 us; 300 x 600: 1100 against 1610 us).
+constexpr int64_t kSmallMaxBlock = 200000;
+
+bool small_shape(int32_t nr, int32_t ncl, int32_t ncr) {
+    return nr > 0 && ncl >= 0 && ncr > 0 && nr >= ncl && ncl <= kSmallMaxLeft &&
+           (int64_t)(nr - ncl) * ncr <= kSmallMaxBlock;
+}
+
+// CTAs per matrix: the most that leaves every one of n matrices its own
+// cluster on the device's SMs, and at least what the matrix needs
+int small_cluster(int32_t n, int sms) {
+    int cl = kTinyMaxCluster;
+    while (cl > 1 && (int64_t)n * cl > sms) cl /= 2;
+    return cl;
 }
 
 }  // namespace
 
 bool small_eligible(int32_t nr, int32_t ncl, int32_t ncr, int device) {
-    if (nr <= 0 || ncl < 0 || ncr <= 0 || nr < ncl || ncl > kSmallMaxLeft) return false;
+    if (!small_shape(nr, ncl, ncr)) return false;
     DeviceGuard guard;
     DeviceInfo dev{};
     if (device_init(device, &dev)) return false;
-    int32_t stride = 0;
-    if (rows_warps(ncl + ncr, dev, &stride) < 4) return false;
-    const int32_t n_work = nr - ncl;
-    return n_work == 0 || tiny_rref_bytes(n_work, ncr, dev.smem_optin) > 0;
+    return small_words(nr, ncl, ncr, kTinyMaxCluster, dev.smem_optin) > 0 ||
+           small_wide(nr, ncl, ncr, dev.smem_optin);
+}
+
+bool small_batchable(int32_t nr, int32_t ncl, int32_t ncr, int device) {
+    if (!small_shape(nr, ncl, ncr)) return false;
+    DeviceGuard guard;
+    DeviceInfo dev{};
+    if (device_init(device, &dev)) return false;
+    return small_words(nr, ncl, ncr, kTinyMaxCluster, dev.smem_optin) > 0;
 }
 
 int small_reduce(const SmallInput& in, SmallAnswer* ans) {
@@ -522,139 +643,91 @@ int small_reduce(const SmallInput& in, SmallAnswer* ans) {
     Session* S = nullptr;
     int rc = session_for(in.device, &S);
     if (rc) return rc;
-    const int32_t nr = in.nr, ncl = in.ncl, ncr = in.ncr, nc = ncl + ncr;
-    const int32_t n_work = nr - ncl;
+    const int32_t nr = in.nr, ncl = in.ncl, ncr = in.ncr;
     const int64_t nnz = in.nnz;
-    const int64_t ld = (int64_t)round_up((size_t)std::max(ncr, 1), 4);
     // pinned staging: row_ptr | cols | vals (copied to the arena's start)
-    const size_t b_ptr = sizeof(int64_t) * (size_t)(nr + 1);
-    const size_t o_cols = round_up(b_ptr, 16);
-    const size_t o_vals = round_up(o_cols + 4 * (size_t)nnz, 16);
-    const size_t in_bytes = round_up(o_vals + 4 * (size_t)nnz, 16);
-    if ((rc = grow_host(&S->hin, &S->hin_cap, in_bytes, cudaHostAllocDefault, S->s))) return rc;
+    SmallItem it = small_item(in.p, nr, ncl, ncr);
+    it.cols_off = rup((int64_t)sizeof(int64_t) * (nr + 1), 16);
+    it.vals_off = rup(it.cols_off + 4 * nnz, 16);
+    const int64_t in_bytes = rup(it.vals_off + 4 * nnz, 16);
+    if ((rc = grow_host(&S->hin, &S->hin_cap, (size_t)in_bytes, cudaHostAllocDefault, S->s)))
+        return rc;
     // every call ends with a synchronisation, so the staging is free to refill
-    in.fill(in.ctx, (int64_t*)S->hin, (int32_t*)(S->hin + o_cols), (uint32_t*)(S->hin + o_vals));
-    // device arena
-    const size_t o_piv = round_up(in_bytes, 256);
-    const size_t o_pext = round_up(o_piv + 4 * (size_t)std::max(ncl, 1), 256);
-    const size_t o_work = round_up(o_pext + 8 * (size_t)std::max(ncl, 1), 256);
-    const size_t o_cnt = round_up(o_work + 4 * (size_t)nr, 256);  // n_work, err
-    const size_t o_D = round_up(o_cnt + 64, 256);
-    const size_t o_lead = round_up(o_D + 4 * (size_t)std::max(n_work, 1) * ld, 256);
-    const size_t o_poc = round_up(o_lead + 4 * (size_t)std::max(n_work, 1), 256);
-    const size_t d_bytes = round_up(o_poc + 4 * (size_t)ncr, 256);
-    if ((rc = grow_device(*S, d_bytes))) return rc;
-    uint8_t* d = (uint8_t*)S->dmem;
-    const int64_t* d_ptr = (const int64_t*)d;
-    const int32_t* d_cols = (const int32_t*)(d + o_cols);
-    const uint32_t* d_vals = (const uint32_t*)(d + o_vals);
-    int32_t* d_piv = (int32_t*)(d + o_piv);
-    int2* d_pext = (int2*)(d + o_pext);
-    int32_t* d_work = (int32_t*)(d + o_work);
-    int32_t* d_nwork = (int32_t*)(d + o_cnt);
-    uint32_t* d_err = (uint32_t*)(d + o_cnt + 16);
-    uint32_t* d_D = (uint32_t*)(d + o_D);
-    int32_t* d_lead = (int32_t*)(d + o_lead);
-    int32_t* d_poc = (int32_t*)(d + o_poc);
-    // mapped output: counts | offs | cols | vals
-    const size_t cap = (size_t)std::max(n_work, 0) * ncr;
-    const size_t h_offs = 64;
-    const size_t h_cols = round_up(h_offs + 8 * (size_t)(std::max(n_work, 0) + 1), 16);
-    const size_t h_vals = round_up(h_cols + 4 * std::max<size_t>(cap, 1), 16);
-    const size_t out_bytes = round_up(h_vals + 4 * std::max<size_t>(cap, 1), 16);
-    if ((rc = grow_host(&S->hout, &S->hout_cap, out_bytes, cudaHostAllocMapped, S->s))) return rc;
+    in.fill(in.ctx, (int64_t*)S->hin, (int32_t*)(S->hin + it.cols_off),
+            (uint32_t*)(S->hin + it.vals_off));
+    it.scr_off = rup(in_bytes, 256);
+    const int optin = S->dev.smem_optin, cl = kTinyMaxCluster, n_work = nr - ncl;
+    int32_t words = (int32_t)small_words(nr, ncl, ncr, cl, optin);
+    const bool wide = small_wide(nr, ncl, ncr, optin) &&
+                      (words == 0 || n_work > kWideRows || ncl > kWideLeft);
+    const ScrLayout L = scr_layout(nr, ncl, wide ? (int64_t)n_work * ncr : 0);
+    if ((rc = grow_device(*S, (size_t)(it.scr_off + L.bytes)))) return rc;
+    const OutLayout O = out_layout(nr, ncl, ncr);
+    if ((rc = grow_host(&S->hout, &S->hout_cap, (size_t)O.bytes, cudaHostAllocMapped, S->s)))
+        return rc;
     uint8_t* hd = nullptr;
     if (cudaHostGetDevicePointer((void**)&hd, S->hout, 0) != cudaSuccess) {
         set_error("mapped output pointer unavailable");
         return GBGPU_ECUDA;
     }
-    int64_t* h_counts = (int64_t*)S->hout;
-    h_counts[0] = 0;
-    h_counts[1] = 0;
-
+    const int64_t* counts = (const int64_t*)S->hout;
     cudaStream_t s = S->s;
-    long long launches = 0;
-    if (cudaMemcpyAsync(d, S->hin, in_bytes, cudaMemcpyHostToDevice, s) != cudaSuccess) {
+    if (cudaMemcpyAsync(S->dmem, S->hin, (size_t)in_bytes, cudaMemcpyHostToDevice, s) !=
+        cudaSuccess) {
         set_error("small-matrix input copy failed");
         return GBGPU_ECUDA;
     }
-    const int prep_bytes = 4 * std::max(ncl, 1);
-    if (ensure_smem_limit((const void*)k_small_prep, prep_bytes) != cudaSuccess) {
-        set_error("prep kernel shared memory");
-        return GBGPU_ECUDA;
-    }
-    k_small_prep<<<1, kPrepThreads, prep_bytes, s>>>(nr, ncl, nc, (uint32_t)in.p, d_ptr, d_cols,
-                                                     d_vals, d_piv, d_pext, d_work, d_nwork,
-                                                     d_err);
-    ++launches;
-    if (n_work > 0) {
-        int32_t stride = 0;
-        const int wpc = rows_warps(nc, S->dev, &stride);
-        const int bytes = wpc * stride * 4;
-        const int grid = std::max(1, std::min((n_work + wpc - 1) / wpc, S->dev.sms * 4));
-        const int tb = tiny_rref_bytes(n_work, ncr, S->dev.smem_optin);
-        auto run = [&](auto f) -> int {
-            using Fd = decltype(f);
-            if (ensure_smem_limit((const void*)k_reduce_rows_warp<Fd>, bytes) != cudaSuccess) {
-                set_error("row kernel shared memory");
-                return GBGPU_ECUDA;
-            }
-            k_reduce_rows_warp<Fd><<<grid, wpc * 32, bytes, s>>>(
-                n_work, d_work, d_ptr, d_cols, d_vals, d_pext, ncl, nc, stride, d_D, ld, d_lead,
-                d_err, f);
-            ++launches;
-            cudaError_t e = launch_tiny_rref(n_work, ncr, d_D, ld, d_lead, d_err, ncl,
-                                             (int64_t*)(hd + h_offs), (int32_t*)(hd + h_cols),
-                                             (int32_t*)(hd + h_vals), d_poc, (int64_t*)hd, tb,
-                                             s, f);
-            ++launches;
-            if (e != cudaSuccess) {
-                set_error(std::string("small-matrix launch: ") + cudaGetErrorString(e));
-                return GBGPU_ECUDA;
-            }
-            return GBGPU_OK;
+    uint8_t* d = (uint8_t*)S->dmem;
+    cudaError_t e = cudaSuccess;
+    if (wide) {
+        SmallMat a = small_mat(it, d, d);
+        uint32_t* D = (uint32_t*)(d + it.scr_off + L.D);
+        int64_t ld = ncr;
+        const int wpr = small_warps(kTinyWarps, a.nc, (optin - 2048) / 4);
+        const int grid = std::min(n_work, S->dev.sms);
+        const int warps = std::min(wpr, (n_work + grid - 1) / grid);
+        auto run = [&](auto f) {
+            using F = decltype(f);
+            int32_t pw = 4 * 2 * LB * LB, nw = n_work;
+            void* prep[] = {&a, &pw, &f};
+            e = launch_cluster((const void*)k_small_prep<F>, cl, cl, kTinyThreads, pw * 4, s, prep);
+            void* rows[] = {&a, &nw, &D, &ld, &f};
+            if (e == cudaSuccess)
+                e = launch_cluster((const void*)k_small_rows<F>, grid, 1, 32 * warps,
+                                   warps * a.nc * 8, s, rows);
+            if (e == cudaSuccess)
+                e = launch_tiny_rref(n_work, ncr, D, ld, a.err, ncl, (int64_t*)(hd + O.offs),
+                                     (int32_t*)(hd + O.cols), (int32_t*)(hd + O.vals), nullptr,
+                                     (int64_t*)hd, tiny_cluster(n_work, ncr, optin), s, f);
         };
-        rc = (uint32_t)in.p < 65536u ? run(FieldSmall::make((uint32_t)in.p))
-                                     : run(FieldMont::make((uint32_t)in.p));
-        if (rc) return rc;
+        if ((uint32_t)in.p < 65536u) run(it.fs);
+        else run(it.fm);
+        count_launch(3);
     } else {
-        ((int64_t*)(S->hout + h_offs))[0] = 0;
+        int32_t n = 1;
+        const SmallItem* items = nullptr;
+        int32_t* queue = nullptr;
+        void* args[] = {&n, &it, &items, &d, &d, &hd, &queue, &words};
+        e = launch_cluster((const void*)k_small, cl, cl, kTinyThreads, words * 4, s, args);
+        count_launch(1);
     }
-    count_launch(launches);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(S->herr, d_err, 4, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         set_error(std::string("small-matrix run: ") + cudaGetErrorString(e));
         return GBGPU_ECUDA;
     }
-    if (*S->herr) {
+    if (counts[2]) {
         std::string msg;
-        rc = err_to_status(*S->herr, &msg);
+        rc = err_to_status((uint32_t)counts[2], &msg);
         set_error(msg);
         return rc;
     }
-    ans->np = n_work > 0 ? (int32_t)h_counts[0] : 0;
-    ans->nnz = n_work > 0 ? h_counts[1] : 0;
-    ans->offs = (const int64_t*)(S->hout + h_offs);
-    ans->cols = (const int32_t*)(S->hout + h_cols);
-    ans->vals = (const int32_t*)(S->hout + h_vals);
+    ans->np = (int32_t)counts[0];
+    ans->nnz = counts[1];
+    ans->offs = (const int64_t*)(S->hout + O.offs);
+    ans->cols = (const int32_t*)(S->hout + O.cols);
+    ans->vals = (const int32_t*)(S->hout + O.vals);
     return GBGPU_OK;
-}
-
-
-int small_batch_bytes(int32_t nr, int32_t ncl, int32_t ncr, int device) {
-    if (nr <= 0 || ncl < 0 || ncr <= 0 || nr < ncl || ncl > kSmallMaxLeft) return 0;
-    DeviceGuard guard;
-    DeviceInfo dev{};
-    if (device_init(device, &dev)) return 0;
-    const int64_t stride = rup(ncl + ncr, 4);
-    const int64_t rows = 4 * 4 * stride;  // at least four row warps
-    const int32_t n_work = nr - ncl;
-    const int64_t tiny = n_work > 0 ? tiny_rref_bytes(n_work, ncr, dev.smem_optin) : 1;
-    if (tiny <= 0) return 0;
-    const int64_t need = std::max<int64_t>({4 * (int64_t)std::max(ncl, 1), rows, tiny});
-    return need + 2048 <= dev.smem_optin ? (int)need : 0;
 }
 
 int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* outs,
@@ -664,32 +737,30 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
     DeviceInfo dev{};
     int rc = device_init(device, &dev);
     if (rc) return rc;
-    std::vector<BatchItem> items((size_t)n);
-    int64_t in_bytes = 0, scr_bytes = 0, out_bytes = 0;
-    int smem = 0;
+    std::vector<SmallItem> items((size_t)n);
+    int64_t in_bytes = 0, scr_bytes = 0, out_bytes = 0, words = 0;
+    int cl = small_cluster(n, dev.sms);
+    for (int32_t i = 0; i < n; ++i)
+        while (cl < kTinyMaxCluster &&
+               !small_words(ms[i]->nr, ms[i]->ncl, ms[i]->ncr, cl, dev.smem_optin))
+            cl *= 2;
     for (int32_t i = 0; i < n; ++i) {
         const gbgpu_csr* m = ms[i];
-        BatchItem& it = items[i];
-        it.p = m->p;
-        it.nr = m->nr;
-        it.ncl = m->ncl;
-        it.ncr = m->ncr;
+        SmallItem& it = items[i];
+        it = small_item(m->p, m->nr, m->ncl, m->ncr);
         const int64_t nnz = m->row_ptr[m->nr];
         it.in_off = in_bytes;
         it.cols_off = rup(it.in_off + 8 * (int64_t)(m->nr + 1), 16);
         it.vals_off = rup(it.cols_off + 4 * nnz, 16);
         in_bytes = rup(it.vals_off + 4 * nnz, 256);
         it.scr_off = scr_bytes;
-        scr_bytes += scr_layout(m->nr, m->ncl, m->ncr).bytes;
+        scr_bytes += scr_layout(m->nr, m->ncl).bytes;
         it.out_off = out_bytes;
         out_bytes += out_layout(m->nr, m->ncl, m->ncr).bytes;
-        it.fs = FieldSmall::make((uint32_t)std::max(m->p, 2));
-        it.fm = FieldMont::make((uint32_t)(m->p | 1));  // used only for odd p >= 2^16
-        smem = std::max(smem, small_batch_bytes(m->nr, m->ncl, m->ncr, device));
+        words = std::max(words, small_words(m->nr, m->ncl, m->ncr, cl, dev.smem_optin));
     }
-    smem = std::min(dev.smem_optin - 2048, std::max(smem, 4 * 4 * 1024));
     uint8_t *h_in = nullptr, *h_out = nullptr, *d_out = nullptr, *d_in = nullptr;
-    BatchItem* d_items = nullptr;
+    SmallItem* d_items = nullptr;
     int32_t* d_queue = nullptr;
     cudaStream_t s = nullptr;
     auto cleanup = [&]() {
@@ -701,7 +772,7 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
     };
     // device: input | scratch | items | queue
     const int64_t o_scr = rup(in_bytes, 256), o_items = rup(o_scr + scr_bytes, 256);
-    const int64_t o_queue = rup(o_items + (int64_t)sizeof(BatchItem) * n, 256);
+    const int64_t o_queue = rup(o_items + (int64_t)sizeof(SmallItem) * n, 256);
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
         cudaHostAlloc((void**)&h_in, (size_t)std::max<int64_t>(in_bytes, 16), 0) != cudaSuccess ||
         cudaHostAlloc((void**)&h_out, (size_t)std::max<int64_t>(out_bytes, 256),
@@ -718,20 +789,23 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
                            (int32_t*)(h_in + items[i].cols_off),
                            (uint32_t*)(h_in + items[i].vals_off));
     }
-    d_items = (BatchItem*)(d_in + o_items);
+    d_items = (SmallItem*)(d_in + o_items);
     d_queue = (int32_t*)(d_in + o_queue);
     cudaError_t e = cudaMemcpyAsync(d_in, h_in, (size_t)in_bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_items, items.data(), sizeof(BatchItem) * n, cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(d_items, items.data(), sizeof(SmallItem) * n, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_queue, 0, sizeof(int32_t), s);
-    if (e == cudaSuccess) e = ensure_smem_limit((const void*)k_batch_small, smem);
     if (e == cudaSuccess) {
-        const int per_sm = std::max(1, std::min(2, (dev.smem_optin - 1024) / (smem + 1024)));
-        const int grid = std::max(1, std::min(n, dev.sms * per_sm));
-        k_batch_small<<<grid, kPrepThreads, smem, s>>>(n, d_items, d_in, d_in + o_scr, d_out,
-                                                       d_queue, smem);
+        // as many clusters as the device holds at two CTAs per SM where they fit
+        const int per_sm = words * 4 + 1024 <= (dev.smem_optin - 1024) / 2 ? 2 : 1;
+        const int grid = cl * std::max(1, std::min(n, dev.sms * per_sm / cl));
+        SmallItem none{};
+        const SmallItem* its = d_items;
+        uint8_t* scr = d_in + o_scr;
+        int32_t w32 = (int32_t)words;
+        void* args[] = {&n, &none, &its, &d_in, &scr, &d_out, &d_queue, &w32};
+        e = launch_cluster((const void*)k_small, grid, cl, kTinyThreads, w32 * 4, s, args);
         count_launch(1);
-        e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {

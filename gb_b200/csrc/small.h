@@ -32,10 +32,10 @@ struct SmallAnswer {
 bool small_eligible(int32_t nr, int32_t ncl, int32_t ncr, int device);
 int small_reduce(const SmallInput& in, SmallAnswer* ans);
 
-// Batches: shared memory the one-launch batch kernel needs for a matrix of
-// this shape (0: not a batch-small matrix), and the batch itself -- every
-// matrix in one persistent launch, one status each (outs[i] malloc'ed rows).
-int small_batch_bytes(int32_t nr, int32_t ncl, int32_t ncr, int device);
+// True when the one-launch batch takes a matrix of this shape.
+bool small_batchable(int32_t nr, int32_t ncl, int32_t ncr, int device);
+// Batches: every matrix (all of them small_batchable) in one persistent launch,
+// one status each (outs[i] malloc'ed rows).
 int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* outs,
                 int32_t* status);
 // host CSR of a gbgpu_csr (values widened to u32) into three arrays

@@ -1,30 +1,68 @@
-// tiny.cuh -- the one-CTA reduced echelon form and compaction of a small
-// dense block (the body of plain.cu's k_tiny_rref, also run per matrix by the
-// batched small-matrix kernel of small.cu).  See plain.cu for the algorithm.
+// tiny.cuh -- the reduced echelon form and compaction of a small dense block in
+// the shared memory of one thread-block cluster (the body of plain.cu's
+// k_tiny_rref and the last phase of small.cu's k_small).
+//
+// What bounds it is the chain of pivots and the SMs' integer multipliers (a
+// 64-bit multiply-add takes about four issue cycles per warp: one SM alone
+// needs 130 us for the updates of a 141 x 191 block).  So the block is reduced
+// by panels of TP columns, and the work is split by how often it has to be
+// exchanged:
+//   * panel k (its TP columns of all rows) belongs to CTA k % CL.  Its owner
+//     copies it to every CTA, and every CTA finds the panel's pivots by itself;
+//   * the columns right of the panel are updated once per panel by their
+//     owners, with 64-bit sums of TP products and one reduction per entry.
+// One cluster barrier per panel, none per pivot.
+//
+// The panel's pivots come from TP rows at a time (the first row of every lead,
+// then any others): their TP x TP entries are brought to reduced echelon form,
+// a thread per entry, and every other row r is cleared at the pivots' columns c
+// at once, row_r -= sum_c row_r[c] (pivot row of c).  Rows that are still not
+// zero in the panel give the next TP (a dense panel is done after one turn).
+// The leads of some of the rows are leads of all of them, so every pivot found
+// this way is one of the reduced echelon form.  A step per pivot over all rows
+// of the panel took 1900 cycles per pivot.
+//
+// In the TP x TP echelon (pivot row i, column c, a = row_i[c]) every other row
+// with m = row_r[c] != 0 becomes a row_r - m row_i (no inverse on the chain),
+// and column c, which would be zero from here on, stores the coefficient of the
+// pivot row's old value: -m s_i, s_r being the product of the factors a that
+// row r took (s_i for the pivot row itself, whose own scale then is 0).  So
+// the TP columns hold both the reduced rows and the transformation F, in place;
+// the pivot rows are divided by their pivot entries at the end, in parallel.
 #pragma once
 #include <climits>
 #include <stdint.h>
 
+#include "cluster.cuh"
 #include "common.cuh"
 
 namespace gbgpu {
 
-constexpr int kTinyThreads = 1024;
-
-// in-place exclusive prefix sum of a[0..n) in shared memory; returns the total
-__device__ inline int tiny_exscan(int* a, int n, int* tmp) {
-    for (int off = 1; off < n; off <<= 1) {
-        for (int i = threadIdx.x; i < n; i += blockDim.x) tmp[i] = a[i] + (i >= off ? a[i - off] : 0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = tmp[i];
-        __syncthreads();
-    }
-    const int total = n > 0 ? a[n - 1] : 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) tmp[i] = i > 0 ? a[i - 1] : 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = tmp[i];
-    __syncthreads();
-    return total;
+constexpr int kTinyThreads = 512;
+constexpr int kTinyWarps = kTinyThreads / 32;
+constexpr int kTinyMaxCluster = 8;          // the portable limit
+constexpr int TP = 16;                      // panel columns
+// Shared memory of one CTA for an n x m block in a cluster of cl (offsets in
+// 32-bit words): its panels [panels / cl][n][TP], two copies of the current
+// panel [n][TP], the pivots' TP x TP blocks (F, the pivot rows in the panel, two
+// working blocks), arrays per row and per column.
+struct TinyLayout {
+    int32_t panels;  // of the block
+    int64_t pb, blk, rows, cols, words;
+};
+__host__ __device__ inline TinyLayout tiny_layout(int32_t n, int32_t m, int32_t cl) {
+    TinyLayout L;
+    L.panels = (m + TP - 1) / TP;
+    L.pb = (int64_t)((L.panels + cl - 1) / cl) * n * TP;
+    L.blk = L.pb + 2 * (int64_t)n * TP;
+    L.rows = L.blk + 4 * TP * TP;
+    L.cols = L.rows + (int64_t)n;
+    L.words = (L.cols + 3 * (int64_t)L.panels * TP + 3) & ~(int64_t)3;
+    return L;
+}
+// word offset of entry (r, j) in the CTA that owns it, (j / TP) % CL
+__device__ __forceinline__ int tiny_at(int n, int r, int j, int cl_shift) {
+    return (((j / TP) >> cl_shift) * n + r) * TP + j % TP;
 }
 
 struct TinyOut {
@@ -32,183 +70,366 @@ struct TinyOut {
     int64_t* offs;      // [rank + 1]
     int32_t* cols;      // [entries]
     int32_t* vals;      // [entries]
-    int32_t* piv_of_col;  // [m]
-    int64_t* counts;    // rows, entries
+    int32_t* piv_of_col;  // [m], or null
+    int64_t* counts;    // rows, entries; [2]: the input checks' verdict
 };
 
-template <class F>
-__device__ void tiny_rref_body(int32_t n, int32_t m, const uint32_t* __restrict__ D, int64_t ld,
-                               const int32_t* __restrict__ lead_in, const uint32_t* err,
-                               TinyOut out, F f, uint32_t* tiny_smem) {
-    const int tld = m + 1;
-    uint32_t* T = tiny_smem;                                 // [n][m + 1]
-    int32_t* lead = (int32_t*)(tiny_smem + (size_t)n * tld);  // [n]
-    int32_t* pcol = lead + n;                                // [n] pivot column of a pivot row, -1
-    int32_t* rcnt = pcol + n;                                // [n] entries of a pivot row
-    int32_t* prow = rcnt + n;                                // [m] pivot row of a column, -1
-    int32_t* rank = prow + m;                                // [max(n, m)] scan space
-    int32_t* tmp = rank + max(n, m);                         // [max(n, m)]
-    uint32_t* rinv = (uint32_t*)(tmp + max(n, m));           // [n] inverse of a row's lead entry
-    __shared__ int s_min[2][kTinyThreads / 32];
+// in-place exclusive prefix sum of a[0..n) in shared memory; returns the total.
+// Every thread sums a contiguous piece; `part` holds one int per warp.
+__device__ inline int tiny_exscan(int32_t* a, int n, int* part) {
+    const int per = (n + kTinyThreads - 1) / kTinyThreads;
+    const int b = min(n, (int)threadIdx.x * per), e = min(n, b + per);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int s = 0;
+    for (int i = b; i < e; ++i) s += a[i];
+    int inc = s;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) part[warp] = inc;
+    __syncthreads();
+    int before = inc - s, total = 0;
+    for (int w = 0; w < kTinyWarps; ++w) {
+        const int v = part[w];
+        before += w < warp ? v : 0;
+        total += v;
+    }
+    for (int i = b; i < e; ++i) {
+        const int v = a[i];
+        a[i] = before;
+        before += v;
+    }
+    __syncthreads();
+    return total;
+}
+
+// One turn's pivots of a panel (shared memory of the CTA).
+struct TinyTurn {
+    int first[TP];             // first row of every lead, INT_MAX
+    int sel[TP];               // the rows of the turn
+    int per_warp[kTinyWarps];
+    uint32_t scl2[TP];         // scales of the turn's rows (second buffer)
+    uint32_t mask;             // pivot columns found in this turn
+};
+
+// The rows of the next turn, the same in every CTA: the first row of every lead
+// in the panel, then the other nonzero rows in row order.  Returns their number
+// (uniform), 0 when no row but the pivots is nonzero.
+__device__ inline int tiny_select(const int n, const uint32_t* pb, const int32_t* pcol,
+                                  TinyTurn& S) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = kTinyThreads / 32;
-    static_assert(NW == 32, "one warp minimum per lane");
-    if (*err) {  // invalid input: nothing is read, the answer is empty (uniform)
-        for (int c = tid; c < m; c += blockDim.x) out.piv_of_col[c] = -1;
-        if (tid == 0) {
-            out.offs[0] = 0;
-            out.counts[0] = 0;
-            out.counts[1] = 0;
+    auto lead_of = [&](int r) {
+        int ld = INT_MAX;
+        if (r < n && pcol[r] < 0) {
+#pragma unroll
+            for (int q = TP / 4 - 1; q >= 0; --q) {
+                const uint4 x = *(const uint4*)(pb + r * TP + 4 * q);
+                const int f = x.x ? 0 : x.y ? 1 : x.z ? 2 : x.w ? 3 : 4;
+                if (f < 4) ld = 4 * q + f;
+            }
         }
-        return;
-    }
-    for (int c = tid; c < m; c += blockDim.x) prow[c] = -1;
-    for (int64_t t = tid; t < (int64_t)n * m; t += blockDim.x) {
-        const int r = (int)(t / m), c = (int)(t % m);
-        T[(size_t)r * tld + c] = D[(size_t)r * ld + c];
-    }
-    __syncthreads();  // the lead entries below were loaded by other threads
-    for (int r = tid; r < n; r += blockDim.x) {
-        const int l = lead_in[r] < 0 ? INT_MAX : lead_in[r];
-        lead[r] = l;
-        pcol[r] = -1;
-        // inverse of the row's lead entry, ready for the step that picks it
-        rinv[r] = l == INT_MAX ? 0u : f.inv(T[(size_t)r * tld + l]);
-    }
-    __syncthreads();
-    // Pivot rows are normalised at the end (the entry at a pivot column never
-    // changes afterwards, pivot columns only grow); a step clears the pivot
-    // column with row_r -= (row_r[c] / a_i) row_i, the inverse of a_i being
-    // ready since row i's lead was last set.  Every warp publishes the key of
-    // its rows right after its own updates: one barrier per pivot.
-    auto warp_key = [&]() {
-        int key = INT_MAX;
-        for (int r = warp + NW * lane; r < n; r += NW * 32)
-            if (pcol[r] < 0 && lead[r] != INT_MAX) key = min(key, lead[r] * n + r);
-        for (int o = 16; o > 0; o >>= 1) key = min(key, __shfl_xor_sync(0xffffffffu, key, o));
-        return key;
+        return ld;
     };
-    {
-        const int key = warp_key();
-        if (lane == 0) s_min[0][warp] = key;
+    if (tid < TP) S.first[tid] = INT_MAX;
+    __syncthreads();
+    const int ld0 = lead_of(tid);
+    if (ld0 != INT_MAX) atomicMin(&S.first[ld0], tid);
+    for (int r = tid + kTinyThreads; r < n; r += kTinyThreads) {
+        const int ld = lead_of(r);
+        if (ld != INT_MAX) atomicMin(&S.first[ld], r);
     }
     __syncthreads();
-    for (int step = 0; step < n; ++step) {
-        const int* sm = s_min[step & 1];
-        // the NW (= 32) warp minima: one read per lane, then a warp reduction
-        int best = sm[lane];
-        for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-        if (best == INT_MAX) break;  // uniform: rank reached
-        const int c = best / n, i = best % n;
-        const uint32_t* pr = T + (size_t)i * tld;
-        const uint32_t ainv = rinv[i];
-        if (warp == (i % NW) && lane == 0) {
-            pcol[i] = c;
-            prow[c] = i;
-        }
-        __syncwarp();  // the owner warp's lanes see pcol[i]
-        // clear column c from this warp's other rows, pivots included
-        for (int r = warp; r < n; r += NW) {
-            if (r == i) continue;
-            uint32_t* row = T + (size_t)r * tld;
-            const uint32_t mr = row[c];
-            if (mr == 0u) continue;  // uniform over the warp
-            const uint32_t mp = f.prep(f.mulmod(mr, ainv));
-            const bool track = pcol[r] < 0;  // its lead was c: find the next one
-            int nl = INT_MAX;
-            for (int j0 = c + 1; j0 < m; j0 += 32) {
-                const int j = j0 + lane;
-                uint32_t y = 0u;
-                if (j < m) {
-                    const uint32_t v = pr[j];
-                    y = row[j];
-                    if (v) {
-                        y = f.mulsub(y, mp, v);
-                        row[j] = y;
-                    }
-                }
-                if (track && nl == INT_MAX) {
-                    const unsigned bal = __ballot_sync(0xffffffffu, y != 0u);
-                    if (bal) nl = j0 + __ffs(bal) - 1;
-                }
-            }
-            __syncwarp();
-            if (lane == 0) {
-                row[c] = 0u;
-                if (track) {
-                    lead[r] = nl;
-                    rinv[r] = nl == INT_MAX ? 0u : f.inv(row[nl]);
-                }
-            }
-            __syncwarp();
-        }
-        const int key = warp_key();
-        if (lane == 0) s_min[(step + 1) & 1][warp] = key;
+    const int mine = lane < TP ? S.first[lane] : INT_MAX;
+    const unsigned leads = __ballot_sync(0xffffffffu, mine != INT_MAX);
+    int count = __popc(leads);
+    if (count == 0) {
+        __syncthreads();  // S.first is rewritten by the next call
+        return 0;
+    }
+    if (tid < TP && mine != INT_MAX) S.sel[__popc(leads & ((1u << lane) - 1u))] = mine;
+    for (int r0 = 0; r0 < n && count < TP; r0 += kTinyThreads) {
+        const int r = r0 + tid, ld = r0 ? lead_of(r) : ld0;
+        const bool other = ld != INT_MAX && S.first[ld] != r;
+        const unsigned bal = __ballot_sync(0xffffffffu, other);
+        if (lane == 0) S.per_warp[warp] = __popc(bal);
         __syncthreads();
-    }
-    // normalise the pivot rows
-    for (int r = warp; r < n; r += NW) {
-        const int c0 = pcol[r];
-        if (c0 < 0) continue;
-        uint32_t* row = T + (size_t)r * tld;
-        const uint32_t ip = f.prep(rinv[r]);
-        for (int j = c0 + 1 + lane; j < m; j += 32) {
-            const uint32_t v = row[j];
-            if (v) row[j] = f.mulp(v, ip);
+        int slot = count + __popc(bal & ((1u << lane) - 1u));
+        for (int w = 0; w < kTinyWarps; ++w) {
+            const int c = S.per_warp[w];
+            slot += w < warp ? c : 0;
+            count += c;
         }
-        __syncwarp();
-        if (lane == 0) row[c0] = 1u;
+        if (other && slot < TP) S.sel[slot] = r;
+        __syncthreads();  // per_warp is rewritten
     }
     __syncthreads();
-    // ---- compaction: pivot rows in descending pivot-column order ----
-    for (int r = warp; r < n; r += NW) {
-        const int c0 = pcol[r];
-        if (c0 < 0) continue;
-        const uint32_t* row = T + (size_t)r * tld;
-        int cnt = 0;
-        for (int j0 = c0; j0 < m; j0 += 32) {
-            const int j = j0 + lane;
-            cnt += __popc(__ballot_sync(0xffffffffu, j < m && row[j] != 0u));
+    return min(TP, count);
+}
+
+// The turn's rows: their pivots into pcol / prow / S.mask, and, by pivot column
+// c, F[c] (coefficients of the old pivot rows, prep form) and PP[c] (the new
+// pivot row in the panel); rows of F and PP without a pivot are 0.  One thread
+// per entry (threads 0 .. TP TP - 1, which alone call this), the entries
+// mirrored in two buffers of shared memory: one barrier per column, and a loop
+// short enough for the instruction cache (the same steps by one warp with the
+// entries in registers, unrolled, took 750 cycles per pivot).
+template <class F_>
+__device__ void tiny_turn(const int n_sel, const int c0, const uint32_t* pb, int32_t* pcol,
+                          int32_t* prow, uint32_t* Fm, uint32_t* PP, uint32_t* buf, TinyTurn& S,
+                          const F_ f) {
+    const int tid = threadIdx.x, lane = tid & 31, q = tid / TP, j = tid % TP;
+    const int row = q < n_sel ? S.sel[q] : -1;
+    uint32_t y = row >= 0 ? pb[row * TP + j] : 0u, scl = 1u, pval = 1u;
+    uint32_t pmask = 0u, done = 0u;  // pivot columns, rows that are pivots (uniform)
+    int my_col = -1, cur = 0;
+    uint32_t* s_scl = (uint32_t*)S.first;  // [TP], then the second buffer's
+    buf[tid] = y;
+    if (j == 0) s_scl[q] = 1u;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll 1
+    for (int c = 0; c < TP; ++c) {
+        const uint32_t* B = buf + cur * TP * TP;
+        const uint32_t col = B[(lane % TP) * TP + c];
+        const unsigned cand = __ballot_sync(0xffffffffu, col != 0u) & 0xFFFFu & ~done;
+        if (cand == 0u) continue;  // uniform
+        const int i = __ffs(cand) - 1;
+        const uint32_t a = B[i * TP + c], mr = B[q * TP + c], v = B[i * TP + j];
+        const uint32_t si = cur ? S.scl2[i] : s_scl[i];
+        pmask |= 1u << c;
+        done |= 1u << i;
+        if (q == i) {
+            if (j == c) y = scl;
+            scl = 0u;
+            pval = a;
+            my_col = c;
+        } else if (mr != 0u) {
+            const uint32_t ap = f.prep(a), mn = f.prep(f.p - mr);
+            y = j == c ? f.mulp(si, mn) : f.ffsub(y, ap, v, mn);
+            scl = f.mulp(scl, ap);
+            pval = f.mulp(pval, ap);
         }
-        if (lane == 0) rcnt[r] = cnt;
+        cur ^= 1;
+        buf[cur * TP * TP + tid] = y;
+        if (j == 0) (cur ? S.scl2 : s_scl)[q] = scl;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
     }
-    // rank of a pivot column = pivot columns to its right
-    for (int c = tid; c < m; c += blockDim.x) rank[c] = prow[m - 1 - c] >= 0 ? 1 : 0;
-    __syncthreads();
-    const int np = tiny_exscan(rank, m, tmp);  // rank[m-1-c] = pivots right of c
-    // entries per output row (rank order) -> offsets
-    for (int c = tid; c < m; c += blockDim.x) {
-        const int r = prow[c];
-        if (r >= 0) tmp[rank[m - 1 - c]] = rcnt[r];
+    if (!((pmask >> q) & 1u)) Fm[tid] = PP[tid] = 0u;  // no pivot in column q
+    if (my_col >= 0) {
+        const uint32_t z = f.mulp(y, f.prep(f.inv(pval)));
+        const bool pc = (pmask >> j) & 1u;
+        Fm[my_col * TP + j] = pc ? f.prep(z) : 0u;
+        PP[my_col * TP + j] = pc ? (j == my_col ? 1u : 0u) : z;
+        if (j == 0) {
+            pcol[row] = c0 + my_col;
+            prow[c0 + my_col] = row;
+        }
     }
-    __syncthreads();
-    for (int k = tid; k < np; k += blockDim.x) rcnt[k] = tmp[k];  // rcnt reused: [np]
-    __syncthreads();
-    const int nnz = tiny_exscan(rcnt, np, tmp);
-    for (int k = tid; k < np; k += blockDim.x) out.offs[k] = rcnt[k];
-    for (int c = tid; c < m; c += blockDim.x) out.piv_of_col[c] = prow[c];
-    if (tid == 0) {
-        out.offs[np] = nnz;
-        out.counts[0] = np;
-        out.counts[1] = nnz;
-    }
-    for (int r = warp; r < n; r += NW) {
-        const int c0 = pcol[r];
-        if (c0 < 0) continue;
-        const uint32_t* row = T + (size_t)r * tld;
-        int64_t pos = rcnt[rank[m - 1 - c0]];
-        for (int j0 = c0; j0 < m; j0 += 32) {
-            const int j = j0 + lane;
-            const uint32_t v = j < m ? row[j] : 0u;
-            const unsigned bal = __ballot_sync(0xffffffffu, v != 0u);
-            if (v) {
-                const int64_t q = pos + __popc(bal & ((1u << lane) - 1u));
-                out.cols[q] = j + out.col_shift;
-                out.vals[q] = (int32_t)v;
+    if (tid == 0) S.mask = pmask;
+}
+
+// G ([n][TP]) -= the turn's elimination: row r takes -= sum_c pb[r][c] P[c],
+// the turn's pivot rows become P[c]; P in v by pivot column (prep form), a lane
+// per column j, two rows per warp.  G may be pb itself.
+template <class F>
+__device__ __forceinline__ void tiny_update(const int n, const int c0, const uint32_t mask,
+                                            const uint32_t* pb, const int32_t* pcol,
+                                            const uint32_t (&v)[TP], uint32_t* G, const F f) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % TP;
+    constexpr int U = 2;  // rows in flight per lane
+#pragma unroll 1
+    for (int r0 = 2 * U * warp; r0 < n; r0 += 2 * U * kTinyWarps) {
+        uint4 e[U][TP / 4];
+        uint32_t g[U];
+        bool on[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + 2 * u + lane / TP;
+            const int k = r < n ? pcol[r] - c0 : 0;
+            on[u] = r < n && !(k >= 0 && k < TP && ((mask >> k) & 1u));
+#pragma unroll
+            for (int q = 0; q < TP / 4; ++q)
+                e[u][q] = on[u] ? *(const uint4*)(pb + r * TP + 4 * q) : make_uint4(0u, 0u, 0u, 0u);
+            g[u] = on[u] ? G[r * TP + j] : 0u;
+        }
+        __syncwarp();  // the rows are read before they are written (G = pb)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            uint32_t any = 0u;
+#pragma unroll
+            for (int q = 0; q < TP / 4; ++q) any |= e[u][q].x | e[u][q].y | e[u][q].z | e[u][q].w;
+            if (any == 0u) continue;
+            ChainSum<F> acc(f);
+#pragma unroll
+            for (int q = 0; q < TP / 4; ++q) {
+                acc.add(f, 0, e[u][q].x, v[4 * q]);
+                acc.add(f, 1, e[u][q].y, v[4 * q + 1]);
+                acc.add(f, 2, e[u][q].z, v[4 * q + 2]);
+                acc.add(f, 3, e[u][q].w, v[4 * q + 3]);
             }
-            pos += __popc(bal);
+            const uint32_t t = acc.mod(f);
+            G[(r0 + 2 * u + lane / TP) * TP + j] = g[u] >= t ? g[u] - t : g[u] + (f.p - t);
         }
     }
+}
+
+// The block is in the CTAs' panels (tiny_layout, columns past m zero) and
+// visible to the cluster.  Reached by every thread of every CTA of the
+// cluster, kTinyThreads a CTA.
+template <class F>
+__device__ void tiny_rref_body(const int32_t n, const int32_t m, uint32_t* smem, const TinyOut out,
+                               const F f) {
+    const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
+    const TinyLayout L = tiny_layout(n, m, CL);
+    uint32_t* T = smem;
+    uint32_t* Fm = smem + L.blk;                    // [TP][TP], see tiny_turn
+    uint32_t* PP = Fm + TP * TP;
+    uint32_t* NP = PP + TP * TP;  // the pivot rows in a panel right of it; [2][TP][TP]
+    int32_t* pcol = (int32_t*)(smem + L.rows);      // [n] pivot column of a pivot row, -1
+    int32_t* prow = (int32_t*)(smem + L.cols);      // [m] pivot row of a column, -1
+    int32_t* rank = prow + L.panels * TP;           // [m] pivots right of a column
+    int32_t* cnt = rank + L.panels * TP;            // [m] entries of the answer's rows
+    __shared__ int s_part[kTinyWarps];
+    __shared__ TinyTurn S;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the owner's panel k to every CTA's copy for panel k
+    auto push = [&](int k) {
+        const uint4* src = (const uint4*)(T + (k >> sh) * n * TP);
+        const uint32_t* dst = smem + L.pb + (k & 1) * n * TP;
+        for (int t = tid; t < n * (TP / 4) * CL; t += kTinyThreads) {
+            const int q = t >> sh, to = t & (CL - 1);
+            remote_st4(remote_smem(dst + 4 * q, to), src[q]);
+        }
+    };
+    for (int c = tid; c < L.panels * TP; c += kTinyThreads) prow[c] = -1;
+    for (int r = tid; r < n; r += kTinyThreads) pcol[r] = -1;
+    cluster_sync();  // every CTA has started, its panels are in place
+    if (rk == 0) push(0);
+    cluster_sync();
+    int found = 0;  // pivots so far (uniform over the cluster)
+    for (int k = 0; k < L.panels; ++k) {
+        uint32_t* pb = smem + L.pb + (k & 1) * n * TP;
+        const int c0 = k * TP, j = lane % TP;
+        uint32_t pmask = 0u;  // the panel's pivot columns so far (uniform)
+        while (pmask != (1u << TP) - 1u) {
+            const int n_sel = tiny_select(n, pb, pcol, S);
+            if (n_sel == 0) break;  // uniform over the cluster
+            if (tid < TP * TP) tiny_turn(n_sel, c0, pb, pcol, prow, Fm, PP, NP, S, f);
+            __syncthreads();
+            const uint32_t mask = S.mask;
+            pmask |= mask;
+            found += __popc(mask);
+            // this CTA's panels right of panel k
+            for (int t = k + 1; t < L.panels; ++t) {
+                if ((t & (CL - 1)) != rk) continue;
+                uint32_t* G = T + (t >> sh) * n * TP;
+                // the pivot rows there: F times their old values
+                const int c = tid / TP;
+                const bool piv = c < TP && ((mask >> c) & 1u);
+                uint32_t np = 0u;
+                if (piv) {
+                    uint32_t old[TP];
+#pragma unroll
+                    for (int q = 0; q < TP; ++q)
+                        old[q] = (mask >> q) & 1u ? G[prow[c0 + q] * TP + j] : 0u;
+                    ChainSum<F> acc(f);
+#pragma unroll
+                    for (int q = 0; q < TP; ++q) acc.add(f, q, Fm[c * TP + q], old[q]);
+                    np = acc.mod(f);
+                }
+                __syncthreads();  // every old value is read
+                if (c < TP) NP[tid] = piv ? f.prep(np) : 0u;
+                if (piv) G[prow[c0 + c] * TP + j] = np;
+                __syncthreads();
+                uint32_t v[TP];
+#pragma unroll
+                for (int q = 0; q < TP; ++q) v[q] = NP[q * TP + j];
+                tiny_update(n, c0, mask, pb, pcol, v, G, f);
+            }
+            if (pmask != (1u << TP) - 1u) {
+                // the panel itself, in every CTA's copy
+                __syncthreads();  // the updates above have read it
+                uint32_t v[TP];
+#pragma unroll
+                for (int q = 0; q < TP; ++q) v[q] = f.prep(PP[q * TP + j]);
+                tiny_update(n, c0, mask, pb, pcol, v, pb, f);
+                const int c = tid / TP;
+                if (c < TP && ((mask >> c) & 1u)) pb[prow[c0 + c] * TP + j] = PP[tid];
+            }
+            __syncthreads();
+        }
+        if (pmask != 0u && (k & (CL - 1)) == rk) {
+            // the owner's panel: the copy, or unit columns if all have a pivot
+            uint32_t* own = T + (k >> sh) * n * TP;
+            const bool full = pmask == (1u << TP) - 1u;
+            for (int t = tid; t < n * TP; t += kTinyThreads)
+                own[t] = full ? (pcol[t / TP] == c0 + t % TP ? 1u : 0u) : pb[t];
+        }
+        if (k + 1 == L.panels) break;
+        if (((k + 1) & (CL - 1)) == rk) push(k + 1);
+        cluster_sync();
+        if (found == n) break;
+    }
+    cluster_sync();
+    // ---- compaction: pivot rows in descending pivot-column order ----
+    // rank of a pivot column = pivot columns to its right
+    for (int c = tid; c < m; c += kTinyThreads) rank[c] = prow[m - 1 - c] >= 0 ? 1 : 0;
+    __syncthreads();
+    const int np = tiny_exscan(rank, m, s_part);  // rank[m-1-c] = pivots right of c
+    // four columns of a row per lane and pass, read from their owners
+    constexpr int CU = 4;
+    auto row_values = [&](int r, int j0, uint32_t (&v)[CU]) {
+#pragma unroll
+        for (int u = 0; u < CU; ++u) {
+            const int j = j0 + 32 * u + lane;
+            v[u] = j < m ? remote_ld(remote_smem(T + tiny_at(n, r, j, sh), (j / TP) & (CL - 1))) : 0u;
+        }
+    };
+    for (int r = rk + CL * warp; r < n; r += CL * kTinyWarps) {
+        const int p0 = pcol[r];
+        if (p0 < 0) continue;
+        int c = 0;
+        for (int j0 = p0; j0 < m; j0 += 32 * CU) {
+            uint32_t v[CU];
+            row_values(r, j0, v);
+#pragma unroll
+            for (int u = 0; u < CU; ++u) c += v[u] != 0u;
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane < CL) remote_st(remote_smem(cnt + rank[m - 1 - p0], lane), (uint32_t)c);
+    }
+    cluster_sync();
+    const int nnz = tiny_exscan(cnt, np, s_part);
+    if (rk == 0) {
+        for (int q = tid; q < np; q += kTinyThreads) out.offs[q] = cnt[q];
+        if (out.piv_of_col)
+            for (int c = tid; c < m; c += kTinyThreads) out.piv_of_col[c] = prow[c];
+        if (tid == 0) {
+            out.offs[np] = nnz;
+            out.counts[0] = np;
+            out.counts[1] = nnz;
+        }
+    }
+    for (int r = rk + CL * warp; r < n; r += CL * kTinyWarps) {
+        const int p0 = pcol[r];
+        if (p0 < 0) continue;
+        int64_t pos = cnt[rank[m - 1 - p0]];
+        for (int j0 = p0; j0 < m; j0 += 32 * CU) {
+            uint32_t v[CU];
+            row_values(r, j0, v);
+#pragma unroll
+            for (int u = 0; u < CU; ++u) {
+                const unsigned bal = __ballot_sync(0xffffffffu, v[u] != 0u);
+                if (v[u]) {
+                    const int64_t q = pos + __popc(bal & ((1u << lane) - 1u));
+                    out.cols[q] = j0 + 32 * u + lane + out.col_shift;
+                    out.vals[q] = (int32_t)v[u];
+                }
+                pos += __popc(bal);
+            }
+        }
+    }
+    cluster_sync();  // the other CTAs have read this one's panels
 }
 
 }  // namespace gbgpu
