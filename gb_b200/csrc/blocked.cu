@@ -84,15 +84,17 @@ __global__ void k_densify(int32_t n, const int32_t* __restrict__ rows,
 }
 
 // Dense rows from CSR without a separate clear: row i of out (i < n) receives
-// CSR row rows[i], columns [from_i, nc), from_i = (i / stride) stride (0 when
-// stride is 0); columns left of from_i are not written.  Each CTA assembles
+// CSR row rows[i], columns [from_i, nc + pad), from_i = (i / stride) stride (0
+// when stride is 0); columns left of from_i are not written.  Columns >= ncl
+// move right by pad (the right block starts on a 16-byte boundary; the pad
+// columns are zero).  Each CTA assembles
 // DS_COLS-column segments of a row in shared memory and writes them whole
 // with 16-byte stores (ld a multiple of 4, out 16-byte aligned).
 constexpr int DS_COLS = 16384;
 __global__ void __launch_bounds__(512)
 k_densify_seg(int32_t n, const int32_t* __restrict__ rows, const int64_t* __restrict__ row_ptr,
               const int32_t* __restrict__ cols, const uint32_t* __restrict__ vals, int32_t nc,
-              int32_t stride, uint32_t* out, int64_t ld) {
+              int32_t ncl, int32_t pad, int32_t stride, uint32_t* out, int64_t ld) {
     extern __shared__ uint4 ds_smem[];
     uint32_t* seg = (uint32_t*)ds_smem;
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
@@ -100,13 +102,13 @@ k_densify_seg(int32_t n, const int32_t* __restrict__ rows, const int64_t* __rest
         const int64_t b = row_ptr[r], e = row_ptr[r + 1];
         const int32_t from = stride ? (i / stride) * stride : 0;
         uint32_t* o = out + (size_t)i * ld;
-        for (int32_t s0 = from; s0 < nc; s0 += DS_COLS) {
-            const int32_t w = min(DS_COLS, nc - s0);
+        for (int32_t s0 = from; s0 < nc + pad; s0 += DS_COLS) {
+            const int32_t w = min(DS_COLS, nc + pad - s0);
             for (int j = threadIdx.x; j < (w + 3) / 4; j += blockDim.x)
                 ds_smem[j] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
             for (int64_t k = b + threadIdx.x; k < e; k += blockDim.x) {
-                const int32_t c = cols[k] - s0;
+                const int32_t cc = cols[k], c = cc + (cc >= ncl ? pad : 0) - s0;
                 if (c >= 0 && c < w) seg[c] = vals[k];
             }
             __syncthreads();
@@ -125,11 +127,12 @@ k_densify_seg(int32_t n, const int32_t* __restrict__ rows, const int64_t* __rest
 // later store of the CTA) and scatters the row's entries of the interval
 // straight into place.  Every entry is read once per interval.
 //
-// With split > 0 (the known pivots P = [A | B] of the tensor form, whose
-// readers need less) only two column intervals of row i are written:
-//   [from_i, e1), e1 = min(split, max(from_i + stride, span[i / stride] + 1)):
+// Columns >= ncl move right by pad, as in k_densify_seg.  With brange (the known
+// pivots P = [A | B] of the tensor form, whose readers need less) only two
+// column intervals of row i are written:
+//   [from_i, e1), e1 = min(ncl, max(from_i + stride, span[i / stride] + 1)):
 //       the diagonal block and the left columns the block's rows reach;
-//   [split + lo, split + hi): the right columns of row group i / 128, from
+//   [ncl + pad + lo, ncl + pad + hi): the right columns of row group i / 128, from
 //       brange[i / 128] = (first, last) nonzero right column of the group,
 //       widened to 64-column boundaries (the limb split reads whole
 //       64-column blocks); nothing when the group's right part is zero.
@@ -140,25 +143,26 @@ constexpr int DS_THREADS = 256;
 __global__ void __launch_bounds__(DS_THREADS)
 k_densify_direct(int32_t n, const int32_t* __restrict__ rows, const int64_t* __restrict__ row_ptr,
               const int32_t* __restrict__ cols, const uint32_t* __restrict__ vals, int32_t nc,
-              int32_t stride, uint32_t* out, int64_t ld, int32_t split = 0,
+              int32_t ncl, int32_t pad, int32_t stride, uint32_t* out, int64_t ld,
               const int32_t* __restrict__ span = nullptr,
               const int2* __restrict__ brange = nullptr) {
+    const int32_t split = ncl + pad;  // first right column
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const int32_t r = rows ? rows[i] : i;
         const int64_t b = row_ptr[r], e = row_ptr[r + 1];
         const int32_t from = stride ? (i / stride) * stride : 0;
         uint32_t* o = out + (size_t)i * ld;
         // the (one or two) intervals of this row
-        int32_t iv[2][2] = {{from, nc}, {0, 0}};
+        int32_t iv[2][2] = {{from, nc + pad}, {0, 0}};
         int n_iv = 1;
-        if (split > 0) {
-            int32_t e1 = split;
-            if (span && stride) e1 = min(split, max(from + stride, span[i / stride] + 1));
+        if (brange) {
+            int32_t e1 = ncl;
+            if (span && stride) e1 = min(ncl, max(from + stride, span[i / stride] + 1));
             iv[0][1] = e1;
             const int2 br = brange[i / 128];
             if (br.y >= br.x) {
                 const int32_t lo = split + (br.x / 64) * 64;
-                const int32_t hi = min(nc, split + (br.y / 64 + 1) * 64);
+                const int32_t hi = min(nc + pad, split + (br.y / 64 + 1) * 64);
                 const int32_t s = lo & ~3;
                 if (s <= e1) {
                     iv[0][1] = max(e1, hi);
@@ -177,7 +181,7 @@ k_densify_direct(int32_t n, const int32_t* __restrict__ rows, const int64_t* __r
             for (int32_t j = a0 + 4 * w4 + threadIdx.x; j < a1; j += blockDim.x) o[j] = 0u;
             __syncthreads();
             for (int64_t k = b + threadIdx.x; k < e; k += blockDim.x) {
-                const int32_t c = cols[k];
+                const int32_t cc = cols[k], c = cc + (cc >= ncl ? pad : 0);
                 if (c >= a0 && c < a1) o[c] = vals[k];
             }
         }
@@ -1290,7 +1294,9 @@ static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t*
     BL_CHECK(neg_inverse_big(c, f, Ublk, NB, (int64_t)NB * NB, nb, n_p - (nb - 1) * NB, NB, Ninv));
     for (int b = 0; b < nb; ++b) {
         const int kb = std::min(NB, n_p - b * NB);
-        const int32_t first_col = pc[b * NB];
+        // from the block's first pivot column, or up to three left of it for the
+        // GEMM's 16-byte accesses (the pivot rows are zero there)
+        const int32_t first_col = pc[b * NB] & ~3;
         BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)rows * kb), 256, 0, c.s>>>(
             rows, kb, M, ld, d_pc + b * NB, G, NB, t_rows));
         BL_CUDA(cudaMemsetAsync(X, 0, sizeof(uint32_t) * (size_t)rows * NB, c.s));
@@ -1313,7 +1319,9 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
 template <class F>
 static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const F& f) {
     const int32_t ncl = in.ncl, ncr = in.ncr, nc = ncl + ncr, t = in.n_work;
-    const int64_t ld = ((int64_t)nc + 3) & ~(int64_t)3;
+    // the right block starts on a 16-byte boundary (the GEMM's wide accesses of D)
+    const int32_t pad = -ncl & 3, nclp = ncl + pad;
+    const int64_t ld = ((int64_t)nc + pad + 3) & ~(int64_t)3;
     cudaStream_t s = c.s;
 
     // ---- 1. Schur complement ---------------------------------------------------
@@ -1335,7 +1343,7 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
         ++c.launches;
         BL_CUDA(ensure_smem_limit((const void*)k_densify_seg, DS_COLS * 4));
         BL_LAUNCH(k_densify_seg<<<std::min(t, 148 * 3), 512, DS_COLS * 4, s>>>(
-            t, work_sorted, in.row_ptr, in.cols, in.vals, nc, 0, W, ld));
+            t, work_sorted, in.row_ptr, in.cols, in.vals, nc, ncl, pad, 0, W, ld));
     }
     if (t > 0 && ncl > 0) {
         const int32_t NB = nb_for(ncl, 16 * KB);
@@ -1364,8 +1372,8 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
         // diagonal block on
         const bool banded = c.form != GBGPU_FORM_PLAIN;
         BL_LAUNCH(k_densify_direct<<<std::min(ncl, 148 * 8), DS_THREADS, 0, s>>>(
-            ncl, in.piv_row, in.row_ptr, in.cols, in.vals, nc, NB, P, ld, banded ? ncl : 0, span,
-            brange));
+            ncl, in.piv_row, in.row_ptr, in.cols, in.vals, nc, ncl, pad, NB, P, ld, span,
+            banded ? brange : nullptr));
         // -A_kk^-1 of every NB x NB diagonal block of A (read in place from P)
         BL_CHECK(neg_inverse_big(c, f, P, ld, (int64_t)NB * ld + NB, nbk, ncl - (nbk - 1) * NB, NB,
                                  Ninv));
@@ -1392,14 +1400,14 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
         // (b) D' = D - X B: one GEMM over the whole left block; the tile flags of
         //     the GEMM skip the zero tiles of the staircase X and of B
         {
-            TcGemmArgs g{c.p, t, ncr, ncl, W, ld, P + ncl, ld, W + ncl, ld};
+            TcGemmArgs g{c.p, t, ncr, ncl, W, ld, P + nclp, ld, W + nclp, ld};
             if (banded) g.b_nrange = brange;  // B is zero outside these columns
             BL_CHECK(gemm_args(c, g));
         }
     }
     if (out->ms_event_schur) BL_CUDA(cudaEventRecord(out->ms_event_schur, s));
-    BL_CHECK(echelon_rref(c, f, W + ncl, ld, t, ncr, out));
-    out->rows = W + ncl;
+    BL_CHECK(echelon_rref(c, f, W + nclp, ld, t, ncr, out));
+    out->rows = W + nclp;
     out->ld = ld;
     return GBGPU_OK;
 }
@@ -1733,12 +1741,12 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
             const int kb = std::min(NB, r - b * NB);
             const int32_t later = r - (b * NB + kb);
             const int32_t* rows_k = prow + b * NB;
-            const int32_t c0 = h_pc[b * NB];
+            const int32_t c0 = h_pc[b * NB] & ~3;  // zero left of the pivot column, as below
             if (later > 0) {
                 // E_k -= E_k[:, pc(>k)] R(>k)
                 BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * later), 256, 0, s>>>(
                     kb, later, Dp, ld, pc + b * NB + kb, G, later, rows_k));
-                const int32_t c_later = h_pc[b * NB + kb];
+                const int32_t c_later = h_pc[b * NB + kb] & ~3;
                 TcGemmArgs g{c.p, kb, ncr - c_later, later, G, later, Dp + c_later, ld,
                              Dp + c_later, ld};
                 g.b_rows = rows_k + kb;

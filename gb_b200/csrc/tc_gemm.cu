@@ -9,18 +9,29 @@
 // At most L limb pairs share a weight, each product is <= 255^2, so a K panel
 // of at most floor((2^31-1) / (L 255^2)) columns keeps every S_w below 2^31
 // (kPanelBytes below).  After each panel the epilogue folds the weights,
-//   v = sum_w REDC(S_w * (2^(8w) R mod p))   (Montgomery, R = 2^32),
+//   v = sum_w S_w * (2^(8w) R mod p)   (Montgomery, R = 2^32; one reduction of
+//       the 64-bit sum for up to three limbs, one per two weights for four),
 // and updates D <- D - v mod p in place, so no partial sum ever leaves [0, p).
 // The result is bit-identical to any exact evaluation of (D - A B) mod p.
 //
-// Pipeline (one CTA per 128 x BN output tile, 192 threads):
+// Pipeline (one CTA per 128 x BN output tile, 320 threads):
 //   warp 0      TMA producer: L A-limb tiles (128 x 128 B) and L B-limb tiles
 //               (BN x 128 B) per 128-byte K step into a STAGES-deep ring,
 //               128-byte swizzle (the canonical K-major UMMA layout);
 //   warp 1      TMEM allocation and MMA issue (one elected thread), stage
 //               release through tcgen05.commit;
-//   warps 2..5  epilogue: tcgen05.ld of the 2L-1 weight accumulators of its
+//   warps 2..9  epilogue: tcgen05.ld of the 2L-1 weight accumulators of its
 //               32-lane TMEM quarter, fold, read-modify-write of D.
+//
+// What bounds it (cycle counts in the roles, B200): an MMA 128 x BN x 32 takes
+// 184 / 80 / 53 cycles for BN = 256 / 128 / 64 (the rate cuBLAS's int8 product
+// reaches at BN = 256), so long K is bound by the MMAs, and short K by the
+// epilogue's path to D.  With the epilogue below, kernel and splits:
+// 8192^3, p = 251: 879 -> 613 us; 5000 x 8000 x 1024: 359 -> 159 us (p = 251),
+// 340 -> 301 us (p = 65521), 1013 -> 717 us (p = 2^31 - 1); 5000 x 20000 x 256:
+// 410 -> 327, 471 -> 350, 1418 -> 679 us.  CTA pairs (cta_group::2, 256-row tiles)
+// move a third less per flop but run their MMAs no faster: 914 us against 1048
+// on 8192^3, p = 251, before that epilogue, and equal or slower elsewhere.
 // Every mbarrier wait is bounded (clock64 budget); on expiry the CTA records
 // GBGPU_ETIMEDOUT in *err, drains its in-flight copies and frees its TMEM.
 // No cluster multicast is used anywhere.
@@ -100,21 +111,22 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint6
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// 32 consecutive TMEM columns of this warp's 32 lanes (one row per thread)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+// 16 consecutive TMEM columns of this warp's 32 lanes (one row per thread)
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
-        "[%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-          "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-          "=r"(r[31])
+          "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// the loads above have landed; `r` passes through so that no use moves before it
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                   "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 }
 
 // K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row
@@ -131,60 +143,49 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 
 // ---------------------------------------------------------------------------
 // Tile shapes (SHAPE):
-//   TC_BIG   long K: 128 x BN tiles, one CTA per SM; one- and two-limb shapes
-//            keep their accumulators twice (the next tile's MMAs run while the
-//            epilogue drains the last) when 2 x NW x BN fits the 512 TMEM
-//            columns: 128 x 256 for L = 1; L = 2 keeps 128 x 128 once (more
-//            reuse per operand byte), L = 3, 4 keep 128 x 64 once;
-//   TC_MID   two limbs, K up to 1536: 128 x 64 tiles, accumulators twice;
-//   TC_SMALL K <= 256, one or two limbs: 128 x 128/64 tiles, two CTAs per SM
-//            (TMEM <= 256 columns each), so one CTA's loads and MMAs overlap
-//            the other's epilogue.
-constexpr int TC_BIG = 0, TC_SMALL = 1, TC_MID = 2;
+//   TC_BIG   128 x BN tiles, one CTA per SM: 128 x 256 for L = 1, 128 x 128 for
+//            L = 2, 128 x 64 for L = 3, 4.  One limb keeps its accumulators twice
+//            (the next tile's MMAs run while the epilogue drains the last);
+//            2 x NW x BN does not fit the 512 TMEM columns of the others;
+//   TC_MID   one or two limbs, 128 x 64 tiles, accumulators twice: for products
+//            with fewer tiles than SMs, where a wide tile only lengthens the one
+//            tile of its SM (measured, L = 2: 512 x 512 x 128 6.4 us against 8.4,
+//            1024 x 1024 x 1024 11.7 against 14.0; with more tiles the wide one
+//            wins at every K: 500 x 3000 x 1024 14.6 against 19.0,
+//            5000 x 20000 x 256 302 against 316, 2000 x 9000 x 1024 91 against 125).
+constexpr int TC_BIG = 0, TC_MID = 2;
 
 template <int L, int SHAPE = TC_BIG>
 struct TcCfg {
-    static constexpr bool SMALL = SHAPE == TC_SMALL;
     static constexpr int BM = 128;
     static constexpr int BK = 128;  // bytes of K per stage (one swizzle row)
-    static constexpr int BN =
-        SMALL ? (L == 1 ? 128 : 64) : (L == 1 ? 256 : (L == 2 && SHAPE == TC_BIG ? 128 : 64));
+    static constexpr int BN = SHAPE == TC_MID ? 64 : (L == 1 ? 256 : (L == 2 ? 128 : 64));
     static constexpr int NW = 2 * L - 1;
     // accumulator sets in TMEM (see the shapes above)
-    static constexpr int ACC_BUFS = (!SMALL && 2 * (2 * L - 1) * BN <= 512) ? 2 : 1;
+    static constexpr int ACC_BUFS = 2 * (2 * L - 1) * BN <= 512 ? 2 : 1;
     static constexpr int A_BYTES = BM * BK;
     static constexpr int B_BYTES = BN * BK;
     static constexpr int STAGE_BYTES = L * (A_BYTES + B_BYTES);
-    static constexpr int STAGES = SMALL ? 1 : (L == 1 ? 4 : (L == 2 ? (BN == 128 ? 3 : 4) : 2));
+    static constexpr int STAGES = L == 1 ? 4 : (L == 2 ? (BN == 128 ? 3 : 4) : 2);
     static constexpr int ACC_COLS = ACC_BUFS * NW * BN;
     static constexpr int TMEM_COLS =
         ACC_COLS <= 64 ? 64 : (ACC_COLS <= 128 ? 128 : (ACC_COLS <= 256 ? 256 : 512));
-    // epilogue warps: two per TMEM lane quarter (each half of the columns) for
-    // the one-CTA-per-SM shapes with one or two limbs, one otherwise
-    static constexpr int EPI_WARPS = (!SMALL && L <= 2) ? 8 : 4;
+    // epilogue warps: two per TMEM lane quarter, each half of the columns
+    static constexpr int EPI_WARPS = 8;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-    // epilogue staging: a 32 x 32 block per epilogue warp (XOR-swizzled
-    // columns) and the D row indices of its 32 rows
+    static constexpr int COLS = BN / (EPI_WARPS / 4);  // columns of an epilogue warp
+    // epilogue staging: a 32 x 32 block per epilogue warp (XOR-swizzled columns)
     static constexpr int STG_BYTES = EPI_WARPS * 32 * 32 * 4;
-    // (64-bit pointers when there is room, 32-bit row indices otherwise)
-    static constexpr bool ROW_PTRS = EPI_WARPS == 4;
-    static constexpr int ROWP_BYTES = EPI_WARPS * 32 * (ROW_PTRS ? 8 : 4);
     static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
     static constexpr int STG_OFF = BAR_OFF + 256;
-    static constexpr int ROWP_OFF = STG_OFF + STG_BYTES;
-    static constexpr int USED_BYTES = ROWP_OFF + ROWP_BYTES + 1024 /*align*/;
-    // the small shape asks for enough shared memory that at most two CTAs
-    // share an SM (their TMEM allocations, 2 x 256 columns, then always fit)
-    static constexpr int SMEM_BYTES = SMALL && USED_BYTES < 100 * 1024 ? 100 * 1024 : USED_BYTES;
-    static constexpr int MIN_CTAS = SMALL ? 2 : 1;
+    static constexpr int USED_BYTES = STG_OFF + STG_BYTES + 1024 /*align*/;
+    static constexpr int SMEM_BYTES = USED_BYTES;
     // K bytes per panel: L * 255^2 * K < 2^31
     static constexpr int PANEL_KB = L == 1 ? 256 : (L == 2 ? 128 : (L == 3 ? 85 : 64));
     static constexpr uint32_t IDESC = (2u << 4)                      // D = s32
                                       | (0u << 7) | (0u << 10)       // A, B = u8
                                       | ((uint32_t)(BN >> 3) << 17)  // N
                                       | ((uint32_t)(BM >> 4) << 24); // M
-    static_assert(!SMALL || L <= 2, "small tiles for one or two limbs only");
-    static_assert(!SMALL || 2 * TMEM_COLS <= 512, "two small CTAs share the TMEM");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
     static_assert(ACC_COLS <= 512, "TMEM columns");
 };
@@ -214,8 +215,9 @@ struct TcParams {
     long long budget;
 };
 
-template <int L, int SHAPE>
-__global__ void __launch_bounds__(TcCfg<L, SHAPE>::THREADS, TcCfg<L, SHAPE>::MIN_CTAS)
+// VEC: D and its row and batch strides are 16-byte aligned
+template <int L, int SHAPE, bool VEC>
+__global__ void __launch_bounds__(TcCfg<L, SHAPE>::THREADS, 1)
 k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
             const TcParams prm) {
     using C = TcCfg<L, SHAPE>;
@@ -450,17 +452,21 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
         // Thread `lane` folds row q*32+lane of the tile; the 32 x 32 result
         // block goes through shared memory so that the read-modify-write of D
         // runs along rows (one 128-byte row segment per warp instruction).
+        //
+        // The D values of a warp's first two blocks are loaded before it waits for
+        // the accumulators, and those of a later one two blocks ahead: a load of D queues behind the operand ring's copies
+        // (up to 192 KB ahead of it, about 7000 cycles), so one that is only
+        // issued when its block is folded costs the epilogue more than the
+        // MMAs of the tile take (8192^3, p = 251: 25000 cycles per 32 x 32
+        // block, and the MMA warp waited 43% of its time for a free set of
+        // accumulators).
         const int e = warp - 2;
         const int q = warp & 3;
-        constexpr int HALVES = C::EPI_WARPS / 4;
-        constexpr int COLS = C::BN / HALVES;  // columns of this warp
-        const int cbeg = (e / 4) * COLS;
+        constexpr int NB = C::COLS / 32;  // blocks of this warp
+        const int cbeg = (e / 4) * C::COLS;
         const int row = q * 32 + lane;
         const uint32_t p = prm.p;
         uint32_t* stg = (uint32_t*)(gbase + C::STG_OFF + (size_t)e * 32 * 32 * 4);
-        uint8_t* rowb = gbase + C::ROWP_OFF + (size_t)e * 32 * (C::ROW_PTRS ? 8 : 4);
-        int32_t* rowi = (int32_t*)rowb;
-        uint32_t** rowp = (uint32_t**)rowb;
         int pc = 0;
         bool stop = false;
         for (int t = blockIdx.x; t < total && !stop; t += gridDim.x) {
@@ -474,49 +480,64 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
             const int m0 = mt * C::BM, n0 = nt * C::BN;
             const int gm = m0 + row;
             uint32_t* Dz = prm.D + (size_t)z * prm.sD;
-            bool rows_here;  // any of this warp's 32 rows is written
-            {
-                int32_t ri = -1;
-                if (gm < prm.M) ri = prm.d_rows ? prm.d_rows[(size_t)z * prm.sDr + gm] : gm;
-                __syncwarp();  // the previous tile's readers are done with the rows
-                if constexpr (C::ROW_PTRS)
-                    rowp[lane] = ri >= 0 ? Dz + (size_t)ri * prm.ldd : nullptr;
-                else
-                    rowi[lane] = ri;
-                rows_here = __any_sync(0xffffffffu, ri >= 0);
-                __syncwarp();  // the row table is visible to the whole warp
-            }
-            // row r of the tile in D (nullptr: not written)
-            auto drow = [&](int r) -> uint32_t* {
-                if constexpr (C::ROW_PTRS) {
-                    return rowp[r];
-                } else {
-                    const int32_t ri = rowi[r];
-                    return ri >= 0 ? Dz + (size_t)ri * prm.ldd : nullptr;
-                }
-            };
-            // D values of a 32 x 32 block (row r, this lane's column)
+            // row `lane` of the warp's 32 rows in D (< 0: not written)
+            int32_t ri = -1;
+            if (gm < prm.M) ri = prm.d_rows ? prm.d_rows[(size_t)z * prm.sDr + gm] : gm;
+            const bool rows_here = __any_sync(0xffffffffu, ri >= 0);
+            const int rows_q = prm.M - (m0 + q * 32);  // rows of the warp in the matrix
+            uint32_t* Dq = Dz + (size_t)(m0 + q * 32) * prm.ldd;
+            // A 32 x 32 block of D in registers.  VEC: entry 4 i + u of a lane is
+            // row 4 i + lane / 8, column 4 (lane % 8) + u (one 16-byte access per
+            // four entries); otherwise entry r is row r, column `lane`.
+            const int vr = lane / 8, vc = 4 * (lane % 8);
             auto load_d = [&](int c0, uint32_t (&dv)[32]) {
-                const int gn = n0 + c0 + lane;
-                const bool col_ok = gn < prm.N;
+                if constexpr (VEC) {
+                    const int gn = n0 + c0 + vc;
 #pragma unroll
-                for (int r = 0; r < 32; ++r) {
-                    const uint32_t* rp = drow(r);
-                    dv[r] = (rp && col_ok) ? rp[gn] : 0u;
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = 4 * i + vr;
+                        const int32_t rr = prm.d_rows ? __shfl_sync(0xffffffffu, ri, r)
+                                                      : (r < rows_q ? m0 + q * 32 + r : -1);
+                        const uint32_t* o = Dz + (size_t)(rr < 0 ? 0 : rr) * prm.ldd + gn;
+                        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                        if (rr >= 0 && gn + 4 <= prm.N) {
+                            x = *(const uint4*)o;
+                        } else if (rr >= 0) {
+                            if (gn < prm.N) x.x = o[0];
+                            if (gn + 1 < prm.N) x.y = o[1];
+                            if (gn + 2 < prm.N) x.z = o[2];
+                        }
+                        dv[4 * i] = x.x;
+                        dv[4 * i + 1] = x.y;
+                        dv[4 * i + 2] = x.z;
+                        dv[4 * i + 3] = x.w;
+                    }
+                } else {
+                    const int gn = n0 + c0 + lane;
+                    const bool col_ok = gn < prm.N;
+                    if (prm.d_rows) {
+#pragma unroll
+                        for (int r = 0; r < 32; ++r) {
+                            const int32_t rr = __shfl_sync(0xffffffffu, ri, r);
+                            dv[r] = (rr >= 0 && col_ok) ? Dz[(size_t)rr * prm.ldd + gn] : 0u;
+                        }
+                    } else {
+                        const uint32_t* o = Dq + gn;
+#pragma unroll
+                        for (int r = 0; r < 32; ++r, o += prm.ldd)
+                            dv[r] = (r < rows_q && col_ok) ? *o : 0u;
+                    }
                 }
             };
             for (int panel = 0; panel < npanels; ++panel, ++pc) {
                 const int ab = pc % C::ACC_BUFS, au = pc / C::ACC_BUFS;
                 const uint32_t acc_base = (uint32_t)(ab * C::NW * C::BN);
-                // the first block's D values do not depend on the accumulators:
-                // their loads are in flight while the MMAs finish (this lane
-                // wrote the same addresses in the previous panel, if any).
-                // Three and four limbs have no registers to spare for it; with
-                // two CTAs per SM the other CTA's epilogue covers the wait.
-                constexpr bool EARLY_D = L <= 2 && !C::SMALL;
-                uint32_t dv[32];
-                if constexpr (EARLY_D) {
-                    if (rows_here) load_d(cbeg, dv);
+                // (this lane wrote the same addresses in the previous panel, if any)
+                constexpr int PRE = NB > 1 ? 2 : 1;  // blocks in flight
+                uint32_t dv[PRE][32];
+                if (rows_here) {
+#pragma unroll
+                    for (int b = 0; b < PRE; ++b) load_d(cbeg + 32 * b, dv[b]);
                 }
                 bool ok = true;
                 if (lane == 0) ok = !*abort_flag && mbar_wait(tfull_bar(ab), au & 1, prm.budget);
@@ -529,74 +550,140 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                 tc_fence_after();
                 // a warp with no row to write keeps only its place in the
                 // accumulator handshake
-                for (int c0 = cbeg; rows_here && c0 < cbeg + COLS; c0 += 32) {
-                    const int gn = n0 + c0 + lane;
-                    const bool col_ok = gn < prm.N;
-                    // D values of the later blocks, issued before the fold
-                    if (!EARLY_D || c0 != cbeg) load_d(c0, dv);
+                if (!rows_here) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty_bar(ab));
+                    continue;
+                }
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const int c0 = cbeg + 32 * b;
+                    uint32_t(&d)[32] = dv[b % PRE];
                     uint32_t v[32];
                     if constexpr (L <= 3) {
                         // one Montgomery reduction of the weighted sum:
                         // T = sum_w S_w (2^(8w) R mod p) < (2L - 1) 2^31 p, so
-                        // (T + q p) / 2^32 < 2^32, then one Barrett step
-                        uint64_t T[32];
+                        // (T + q p) / 2^32 < 2^32, then one Barrett step; 16
+                        // columns at a time (registers)
 #pragma unroll
-                        for (int w = 0; w < C::NW; ++w) {
-                            uint32_t a[32];
-                            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
-                                          (uint32_t)(w * C::BN + c0),
-                                      a);
-                            const uint32_t cw = prm.cw[w];
+                        for (int h = 0; h < 32; h += 16) {
+                            uint32_t a[C::NW][16];
 #pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                T[j] = (w == 0 ? 0ull : T[j]) + (uint64_t)a[j] * cw;
-                        }
+                            for (int w = 0; w < C::NW; ++w)
+                                tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
+                                              (uint32_t)(w * C::BN + c0 + h),
+                                          a[w]);
+                            uint64_t T[16];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const uint32_t qq = (uint32_t)T[j] * prm.pneg_inv;
-                            const uint32_t t = (uint32_t)((T[j] + (uint64_t)qq * p) >> 32);
-                            const uint32_t r = t - __umulhi(t, prm.mu) * p;
-                            v[j] = r >= p ? r - p : r;
+                            for (int w = 0; w < C::NW; ++w) {
+                                tmem_wait(a[w]);
+                                const uint32_t cw = prm.cw[w];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    T[j] = (w == 0 ? 0ull : T[j]) + (uint64_t)a[w][j] * cw;
+                            }
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const uint32_t qq = (uint32_t)T[j] * prm.pneg_inv;
+                                const uint32_t t = (uint32_t)((T[j] + (uint64_t)qq * p) >> 32);
+                                const uint32_t r = t - __umulhi(t, prm.mu) * p;
+                                v[h + j] = r >= p ? r - p : r;
+                            }
                         }
                     } else {
+                        // two weights per reduction: T < 2 2^31 p, so
+                        // (T + q p) / 2^32 < 2 p
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = 0;
 #pragma unroll
-                        for (int w = 0; w < C::NW; ++w) {
-                            uint32_t a[32];
-                            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
-                                          (uint32_t)(w * C::BN + c0),
-                                      a);
-                            const uint32_t cw = prm.cw[w];
+                        for (int h = 0; h < 32; h += 16) {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                const uint64_t T = (uint64_t)a[j] * cw;
-                                const uint32_t qq = (uint32_t)T * prm.pneg_inv;
-                                uint32_t r = (uint32_t)((T + (uint64_t)qq * p) >> 32);
-                                r = r >= p ? r - p : r;
-                                const uint32_t sum = v[j] + r;
-                                v[j] = sum >= p ? sum - p : sum;
+                            for (int w = 0; w < C::NW; w += 2) {
+                                uint32_t a[16], a2[16];
+                                tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
+                                              (uint32_t)(w * C::BN + c0 + h),
+                                          a);
+                                if (w + 1 < C::NW)
+                                    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
+                                                  (uint32_t)((w + 1) * C::BN + c0 + h),
+                                              a2);
+                                tmem_wait(a);
+                                if (w + 1 < C::NW) tmem_wait(a2);
+                                const uint32_t cw = prm.cw[w], cw2 = prm.cw[w + 1 < C::NW ? w + 1 : w];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) {
+                                    uint64_t T = (uint64_t)a[j] * cw;
+                                    if (w + 1 < C::NW) T += (uint64_t)a2[j] * cw2;
+                                    const uint32_t qq = (uint32_t)T * prm.pneg_inv;
+                                    uint32_t r = (uint32_t)((T + (uint64_t)qq * p) >> 32);
+                                    r = r >= p ? r - p : r;
+                                    const uint32_t sum = v[h + j] + r;
+                                    v[h + j] = sum >= p ? sum - p : sum;
+                                }
                             }
                         }
                     }
-                    // stage (row lane, column j) at [lane][j ^ lane]
+                    if (b == NB - 1) {  // the accumulators are read: free for the next tile
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(tempty_bar(ab));
+                    }
+                    if constexpr (VEC) {
+                        // 16-byte group g of row `lane` at group g ^ (lane % 8)
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) stg[lane * 32 + (j ^ lane)] = v[j];
-                    __syncwarp();
+                        for (int g = 0; g < 8; ++g)
+                            *(uint4*)&stg[lane * 32 + ((g ^ (lane & 7)) << 2)] =
+                                make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+                        __syncwarp();
+                        const int gv = n0 + c0 + vc;
 #pragma unroll
-                    for (int r = 0; r < 32; ++r) {
-                        uint32_t* rp = drow(r);
-                        if (rp && col_ok) {
-                            const uint32_t vv = stg[r * 32 + (lane ^ r)];
-                            const uint32_t d = dv[r];
-                            rp[gn] = d >= vv ? d - vv : d + (p - vv);
+                        for (int i = 0; i < 8; ++i) {
+                            const int r = 4 * i + vr;
+                            uint4 x = *(const uint4*)&stg[r * 32 + (((lane & 7) ^ (r & 7)) << 2)];
+                            x.x = d[4 * i] >= x.x ? d[4 * i] - x.x : d[4 * i] + (p - x.x);
+                            x.y = d[4 * i + 1] >= x.y ? d[4 * i + 1] - x.y : d[4 * i + 1] + (p - x.y);
+                            x.z = d[4 * i + 2] >= x.z ? d[4 * i + 2] - x.z : d[4 * i + 2] + (p - x.z);
+                            x.w = d[4 * i + 3] >= x.w ? d[4 * i + 3] - x.w : d[4 * i + 3] + (p - x.w);
+                            const int32_t rr = prm.d_rows ? __shfl_sync(0xffffffffu, ri, r)
+                                                          : (r < rows_q ? m0 + q * 32 + r : -1);
+                            uint32_t* o = Dz + (size_t)(rr < 0 ? 0 : rr) * prm.ldd + gv;
+                            if (rr >= 0 && gv + 4 <= prm.N) {
+                                *(uint4*)o = x;
+                            } else if (rr >= 0) {
+                                if (gv < prm.N) o[0] = x.x;
+                                if (gv + 1 < prm.N) o[1] = x.y;
+                                if (gv + 2 < prm.N) o[2] = x.z;
+                            }
+                        }
+                    } else {
+                        // (row lane, column j) at [lane][j ^ lane]
+                        const int gn = n0 + c0 + lane;
+                        const bool col_ok = gn < prm.N;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) stg[lane * 32 + (j ^ lane)] = v[j];
+                        __syncwarp();
+#pragma unroll
+                        for (int r = 0; r < 32; ++r) {
+                            const uint32_t x = stg[r * 32 + (lane ^ r)];
+                            v[r] = d[r] >= x ? d[r] - x : d[r] + (p - x);
+                        }
+                        if (prm.d_rows) {
+#pragma unroll
+                            for (int r = 0; r < 32; ++r) {
+                                const int32_t rr = __shfl_sync(0xffffffffu, ri, r);
+                                if (rr >= 0 && col_ok) Dz[(size_t)rr * prm.ldd + gn] = v[r];
+                            }
+                        } else {
+                            uint32_t* o = Dq + gn;
+#pragma unroll
+                            for (int r = 0; r < 32; ++r, o += prm.ldd)
+                                if (r < rows_q && col_ok) *o = v[r];
                         }
                     }
+                    if (b + PRE < NB) load_d(cbeg + 32 * (b + PRE), d);
                     __syncwarp();
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty_bar(ab));
             }
         }
     }
@@ -1012,7 +1099,10 @@ static int tc_run(const TcGemmArgs& g, uint8_t* planes, cudaStream_t s, int32_t*
     }
     prm.err = err;
     prm.budget = 4000000000LL;  // about 2 s at 2 GHz per wait
-    cudaError_t e = ensure_smem_limit((const void*)k_tc_submul<L, SHAPE>, Cfg::SMEM_BYTES);
+    const bool vec = (uintptr_t)g.D % 16 == 0 && g.ldd % 4 == 0 && g.sD % 4 == 0;
+    const void* kernel = vec ? (const void*)k_tc_submul<L, SHAPE, true>
+                             : (const void*)k_tc_submul<L, SHAPE, false>;
+    cudaError_t e = ensure_smem_limit(kernel, Cfg::SMEM_BYTES);
     if (e != cudaSuccess) {
         set_error(std::string("tc smem attribute: ") + cudaGetErrorString(e));
         return GBGPU_ECUDA;
@@ -1020,7 +1110,7 @@ static int tc_run(const TcGemmArgs& g, uint8_t* planes, cudaStream_t s, int32_t*
     prm.batch = nb;
     const int64_t tiles = (int64_t)(Np / Cfg::BN) * (Mp / Cfg::BM) * nb;
     const dim3 grid((unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(tiles, (int64_t)num_sms() * Cfg::MIN_CTAS)));
+        1, std::min<int64_t>(tiles, (int64_t)num_sms())));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (prof) {
         const int slot = (int)prof->events.size();
@@ -1030,7 +1120,8 @@ static int tc_run(const TcGemmArgs& g, uint8_t* planes, cudaStream_t s, int32_t*
         cudaEventCreate(&e1);
         cudaEventRecord(e0, s);
     }
-    k_tc_submul<L, SHAPE><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, s>>>(ma, mb, prm);
+    void* args[] = {&ma, &mb, &prm};
+    e = cudaLaunchKernel(kernel, grid, dim3(Cfg::THREADS), args, Cfg::SMEM_BYTES, s);
     ++*launches;
     if (prof) {
         cudaEventRecord(e1, s);
@@ -1038,7 +1129,6 @@ static int tc_run(const TcGemmArgs& g, uint8_t* planes, cudaStream_t s, int32_t*
         // int8 MACs of one executed K step of one tile
         prof->macs_per_step.push_back((double)Cfg::BM * Cfg::BN * Cfg::BK * L * L);
     }
-    e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error(std::string("tc launch: ") + cudaGetErrorString(e));
         return GBGPU_ECUDA;
@@ -1070,24 +1160,25 @@ int tc_submul(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err
         set_error("tensor-core path needs an odd prime");
         return GBGPU_EINVAL;
     }
-    return tc_submul_shape(g, workspace, s, err, launches, tc_shape_for(limbs_for(g.p), g.K));
+    // fewer narrow tiles than SMs: the narrow shape (TC_MID)
+    const int64_t narrow = (int64_t)((g.M + 127) / 128) * ((g.N + 63) / 64) * g.batch;
+    const int shape = narrow <= num_sms() ? TC_MID : tc_shape_for(limbs_for(g.p), g.K);
+    return tc_submul_shape(g, workspace, s, err, launches, shape);
 }
 
-// the shapes: 0 big, 1 small (K <= 256, L <= 2), 2 mid (L = 2); any other
-// request falls back to the big shape
+// the shapes: 0 big, 2 mid (L <= 2); any other request falls back to big
 int tc_submul_shape(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err,
                     long long* launches, int shape) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.batch <= 0) return GBGPU_OK;
     uint8_t* planes = (uint8_t*)workspace;
-    const bool small = shape == 1 && g.K <= 256;
+    const bool mid = shape == TC_MID;
     switch (limbs_for(g.p)) {
         case 1:
-            return small ? tc_run<1, TC_SMALL>(g, planes, s, err, launches)
-                         : tc_run<1, TC_BIG>(g, planes, s, err, launches);
+            return mid ? tc_run<1, TC_MID>(g, planes, s, err, launches)
+                       : tc_run<1, TC_BIG>(g, planes, s, err, launches);
         case 2:
-            return small         ? tc_run<2, TC_SMALL>(g, planes, s, err, launches)
-                   : shape == 2  ? tc_run<2, TC_MID>(g, planes, s, err, launches)
-                                 : tc_run<2, TC_BIG>(g, planes, s, err, launches);
+            return mid ? tc_run<2, TC_MID>(g, planes, s, err, launches)
+                       : tc_run<2, TC_BIG>(g, planes, s, err, launches);
         case 3: return tc_run<3, TC_BIG>(g, planes, s, err, launches);
         default: return tc_run<4, TC_BIG>(g, planes, s, err, launches);
     }

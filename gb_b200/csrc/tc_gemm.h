@@ -58,7 +58,7 @@ size_t tc_workspace_bytes(uint32_t p, int32_t M, int32_t N, int32_t K, int32_t b
 // bounded wait expired
 int tc_submul(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err,
               long long* launches);
-// the same with an explicit tile shape (0 big, 1 small, 2 mid; tune.cu)
+// the same with an explicit tile shape (0 big, 2 mid; tune.cu)
 int tc_submul_shape(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err,
                     long long* launches, int shape);
 // the tile shape the autotuner's cache (or the built-in rule) picks for L, K

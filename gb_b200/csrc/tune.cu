@@ -1,13 +1,14 @@
 // tune.cu -- the autotuner of the tensor-core GEMM's tile shape.
 //
-// k_tc_submul has up to three tile shapes per limb count L (tc_gemm.cu:
-// big, mid, small), each best in a different range of the reduction depth K.
+// k_tc_submul has up to two tile shapes per limb count L (tc_gemm.cu: big and
+// mid); products with fewer tiles than SMs always take the mid one, the others
+// what is tuned here for their reduction depth K.
 // gbgpu_autotune times every candidate shape on this device for every
 // (L, K bucket) -- exact modular GEMMs on uniform residues, CUDA events, best
 // of three after a warm-up -- and writes the winners to a cache file:
 //
-//   # gbgpu GEMM tile shapes: limbs kmax shape (0 big, 1 small, 2 mid)
-//   2 256 1
+//   # gbgpu GEMM tile shapes: limbs kmax shape (0 big, 2 mid)
+//   2 256 0
 //   ...
 //
 // The library reads that file once per process (GBGPU_TUNE_FILE, else
@@ -35,7 +36,7 @@ namespace {
 
 constexpr int kBuckets = 7;
 constexpr int kKmax[kBuckets] = {128, 256, 512, 1024, 1536, 4096, 1 << 30};
-constexpr int kShapeBig = 0, kShapeSmall = 1, kShapeMid = 2;
+constexpr int kShapeBig = 0, kShapeMid = 2;
 
 std::mutex g_mu;
 bool g_loaded = false;
@@ -48,17 +49,10 @@ int bucket_of(int K) {
 }
 
 // the built-in rule (measured when the shapes were written)
-int default_shape(int L, int K) {
-    if (L == 1) return K <= 256 ? kShapeSmall : kShapeBig;
-    if (L == 2) return K <= 256 ? kShapeSmall : (K <= 1536 ? kShapeMid : kShapeBig);
-    return kShapeBig;
-}
+int default_shape(int, int) { return kShapeBig; }
 
-bool valid(int L, int kmax, int shape) {
-    if (shape == kShapeBig) return true;
-    if (shape == kShapeSmall) return L <= 2 && kmax <= 256;
-    if (shape == kShapeMid) return L == 2;
-    return false;
+bool valid(int L, int, int shape) {
+    return shape == kShapeBig || (shape == kShapeMid && L <= 2);
 }
 
 std::string default_path() {
@@ -154,7 +148,7 @@ extern "C" int gbgpu_autotune(int32_t device, const char* path) {
         set_error("gbgpu_autotune: status clear failed");
         return GBGPU_ECUDA;
     }
-    std::string text = "# gbgpu GEMM tile shapes: limbs kmax shape (0 big, 1 small, 2 mid)\n";
+    std::string text = "# gbgpu GEMM tile shapes: limbs kmax shape (0 big, 2 mid)\n";
     int table[5][kBuckets];
     for (auto& row : table)
         for (int& x : row) x = -1;
@@ -167,7 +161,7 @@ extern "C" int gbgpu_autotune(int32_t device, const char* path) {
         for (int b = 0; b < kBuckets; ++b) {
             const int K = std::min(kKmax[b], Kmax);
             int cands[3], nc = 0;
-            for (int sh : {kShapeBig, kShapeSmall, kShapeMid})
+            for (int sh : {kShapeBig, kShapeMid})
                 if (valid(L, kKmax[b], sh)) cands[nc++] = sh;
             if (nc < 2) continue;
             float best = 1e30f;
