@@ -144,11 +144,65 @@ int device_init(int device, DeviceInfo* info) {
 }
 
 // ---------------------------------------------------------------------------
+// Streams and events of finished plans, kept for the next ones: creating and
+// destroying a stream takes 0.1 to 0.5 ms, as long as the reduction of a small
+// matrix.  At most kMaxKits per device wait here (the rest are destroyed); a
+// plan holds its kit alone from plan_setup to its destructor, which returns it
+// with no work of its own pending.
+constexpr int kPlanEvents = 8;
+struct StreamKit {
+    cudaStream_t s = nullptr;
+    cudaEvent_t ev[kPlanEvents] = {};
+};
+constexpr int kMaxKits = 8;
+static std::mutex g_kit_mu;
+static std::vector<StreamKit>& kits_of(int device) {
+    static auto* kits = new std::map<int, std::vector<StreamKit>>();  // outlives every plan
+    return (*kits)[device];
+}
+static void kit_destroy(StreamKit& k) {
+    for (auto& e : k.ev)
+        if (e) cudaEventDestroy(e);
+    if (k.s) cudaStreamDestroy(k.s);
+    k = StreamKit{};
+}
+static cudaError_t kit_take(int device, StreamKit* out) {
+    {
+        std::lock_guard<std::mutex> lock(g_kit_mu);
+        auto& v = kits_of(device);
+        while (!v.empty()) {
+            *out = v.back();
+            v.pop_back();
+            if (cudaStreamQuery(out->s) == cudaSuccess) return cudaSuccess;
+            cudaGetLastError();  // a stream of a context that is gone: drop the handles
+        }
+    }
+    *out = StreamKit{};
+    cudaError_t e = cudaStreamCreateWithFlags(&out->s, cudaStreamNonBlocking);
+    for (auto& x : out->ev)
+        if (e == cudaSuccess) e = cudaEventCreate(&x);
+    if (e != cudaSuccess) kit_destroy(*out);
+    return e;
+}
+static void kit_return(int device, StreamKit& k) {
+    if (!k.s) return;
+    {
+        std::lock_guard<std::mutex> lock(g_kit_mu);
+        auto& v = kits_of(device);
+        if ((int)v.size() < kMaxKits && cudaStreamSynchronize(k.s) == cudaSuccess) {
+            v.push_back(k);
+            k = StreamKit{};
+            return;
+        }
+    }
+    kit_destroy(k);
+}
+
 struct Plan {
     int device = 0;
     DeviceInfo dev{};
     cudaStream_t stream = nullptr;
-    bool own_stream = false;
+    StreamKit kit;  // its events; its stream, unless the caller gave one
     int mode = 0;  // 0: linear_algebra, 1: interreduction
     int form = GBGPU_FORM_PLAIN;
     int requested_form = GBGPU_FORM_AUTO;
@@ -219,7 +273,7 @@ struct Plan {
     bool mapped = false;
     cudaStream_t s_out = nullptr;
     gbgpu_stats stats{};
-    cudaEvent_t ev[8] = {};
+    cudaEvent_t ev[kPlanEvents] = {};
     long long launches = 0;
 
     template <class T>
@@ -242,9 +296,7 @@ struct Plan {
         }
         for (void* q : bufs) cudaFreeAsync(q, stream);
         if (stream) cudaStreamSynchronize(stream);
-        for (auto& e : ev)
-            if (e) cudaEventDestroy(e);
-        if (own_stream && stream) cudaStreamDestroy(stream);
+        kit_return(device, kit);
     }
 };
 
@@ -271,13 +323,9 @@ static int plan_setup(Plan* P, const gbgpu_options* opt) {
     P->requested_form = o.form;
     P->profile = o.profile;
     P->check = 1;  // the contract check is cheap and guards every later index
-    if (o.stream) {
-        P->stream = (cudaStream_t)o.stream;
-    } else {
-        GB_CUDA(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking));
-        P->own_stream = true;
-    }
-    for (auto& e : P->ev) GB_CUDA(cudaEventCreate(&e));
+    GB_CUDA(kit_take(P->device, &P->kit));
+    P->stream = o.stream ? (cudaStream_t)o.stream : P->kit.s;
+    for (int k = 0; k < kPlanEvents; ++k) P->ev[k] = P->kit.ev[k];
     return GBGPU_OK;
 }
 

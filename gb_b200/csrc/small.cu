@@ -491,8 +491,6 @@ struct Sessions {
 };
 thread_local Sessions t_sessions;
 
-size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
-
 int grow_device(Session& S, size_t need) {
     if (need <= S.dcap) return GBGPU_OK;
     const size_t cap = std::max(need, S.dcap * 2);
@@ -525,6 +523,28 @@ int grow_host(uint8_t** buf, size_t* capv, size_t need, unsigned flags, cudaStre
     }
     *capv = cap;
     return GBGPU_OK;
+}
+
+// A session keeps at most this much of each buffer between calls; what one call
+// needed beyond it is given back when the call ends.
+constexpr size_t kKeepHost = (size_t)64 << 20, kKeepDevice = (size_t)256 << 20;
+
+void trim(Session& S) {
+    if (S.hin_cap > kKeepHost) {
+        cudaFreeHost(S.hin);
+        S.hin = nullptr;
+        S.hin_cap = 0;
+    }
+    if (S.hout_cap > kKeepHost) {
+        cudaFreeHost(S.hout);
+        S.hout = nullptr;
+        S.hout_cap = 0;
+    }
+    if (S.dcap > kKeepDevice) {
+        cudaFree(S.dmem);
+        S.dmem = nullptr;
+        S.dcap = 0;
+    }
 }
 
 int session_for(int device, Session** out) {
@@ -734,9 +754,19 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
                 int32_t* status) {
     if (n <= 0) return GBGPU_OK;
     DeviceGuard guard;
-    DeviceInfo dev{};
-    int rc = device_init(device, &dev);
+    Session* S = nullptr;
+    int rc = session_for(device, &S);
     if (rc) return rc;
+    const DeviceInfo& dev = S->dev;
+    // the thread's session buffers, given back down to their bound on every
+    // return: pinning and freeing the staging of one call took 4 to 20 ms
+    struct Trim {
+        Session* S;
+        ~Trim() {
+            cudaStreamSynchronize(S->s);
+            trim(*S);
+        }
+    } trimmer{S};
     std::vector<SmallItem> items((size_t)n);
     int64_t in_bytes = 0, scr_bytes = 0, out_bytes = 0, words = 0;
     int cl = small_cluster(n, dev.sms);
@@ -759,42 +789,33 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
         out_bytes += out_layout(m->nr, m->ncl, m->ncr).bytes;
         words = std::max(words, small_words(m->nr, m->ncl, m->ncr, cl, dev.smem_optin));
     }
-    uint8_t *h_in = nullptr, *h_out = nullptr, *d_out = nullptr, *d_in = nullptr;
-    SmallItem* d_items = nullptr;
-    int32_t* d_queue = nullptr;
-    cudaStream_t s = nullptr;
-    auto cleanup = [&]() {
-        if (s) cudaStreamSynchronize(s);
-        if (d_in) cudaFree(d_in);
-        if (h_in) cudaFreeHost(h_in);
-        if (h_out) cudaFreeHost(h_out);
-        if (s) cudaStreamDestroy(s);
-    };
-    // device: input | scratch | items | queue
-    const int64_t o_scr = rup(in_bytes, 256), o_items = rup(o_scr + scr_bytes, 256);
-    const int64_t o_queue = rup(o_items + (int64_t)sizeof(SmallItem) * n, 256);
-    if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaHostAlloc((void**)&h_in, (size_t)std::max<int64_t>(in_bytes, 16), 0) != cudaSuccess ||
-        cudaHostAlloc((void**)&h_out, (size_t)std::max<int64_t>(out_bytes, 256),
-                      cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&d_out, h_out, 0) != cudaSuccess ||
-        cudaMalloc((void**)&d_in, (size_t)(o_queue + 256)) != cudaSuccess) {
-        cleanup();
-        set_error("small-matrix batch: allocation failed");
-        return GBGPU_ENOMEM;
+    // device: input | items | queue | scratch (the first three in one copy)
+    const int64_t o_items = rup(in_bytes, 256);
+    const int64_t o_queue = o_items + rup((int64_t)sizeof(SmallItem) * n, 256);
+    const int64_t o_scr = o_queue + 256;
+    uint8_t* d_out = nullptr;
+    if ((rc = grow_host(&S->hin, &S->hin_cap, (size_t)o_scr, cudaHostAllocDefault, S->s)) ||
+        (rc = grow_host(&S->hout, &S->hout_cap, (size_t)std::max<int64_t>(out_bytes, 256),
+                        cudaHostAllocMapped, S->s)) ||
+        (rc = grow_device(*S, (size_t)(o_scr + scr_bytes))))
+        return rc;
+    if (cudaHostGetDevicePointer((void**)&d_out, S->hout, 0) != cudaSuccess) {
+        set_error("mapped output pointer unavailable");
+        return GBGPU_ECUDA;
     }
+    uint8_t *h_in = S->hin, *h_out = S->hout, *d_in = (uint8_t*)S->dmem;
+    cudaStream_t s = S->s;
     for (int32_t i = 0; i < n; ++i) {
         const gbgpu_csr* m = ms[i];
         fill_from_csr_vals((void*)m, (int64_t*)(h_in + items[i].in_off),
                            (int32_t*)(h_in + items[i].cols_off),
                            (uint32_t*)(h_in + items[i].vals_off));
     }
-    d_items = (SmallItem*)(d_in + o_items);
-    d_queue = (int32_t*)(d_in + o_queue);
-    cudaError_t e = cudaMemcpyAsync(d_in, h_in, (size_t)in_bytes, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_items, items.data(), sizeof(SmallItem) * n, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_queue, 0, sizeof(int32_t), s);
+    memcpy(h_in + o_items, items.data(), sizeof(SmallItem) * (size_t)n);
+    memset(h_in + o_queue, 0, 256);
+    SmallItem* d_items = (SmallItem*)(d_in + o_items);
+    int32_t* d_queue = (int32_t*)(d_in + o_queue);
+    cudaError_t e = cudaMemcpyAsync(d_in, h_in, (size_t)o_scr, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         // as many clusters as the device holds at two CTAs per SM where they fit
         const int per_sm = words * 4 + 1024 <= (dev.smem_optin - 1024) / 2 ? 2 : 1;
@@ -811,7 +832,6 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
     if (e != cudaSuccess) {
         set_error(std::string("small-matrix batch: ") + cudaGetErrorString(e));
         for (int32_t i = 0; i < n; ++i) status[i] = GBGPU_ECUDA;
-        cleanup();
         return GBGPU_OK;
     }
     for (int32_t i = 0; i < n; ++i) {
@@ -838,7 +858,6 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
         memcpy(r.vals, ob + O.vals, sizeof(int32_t) * (size_t)r.nnz);
         status[i] = GBGPU_OK;
     }
-    cleanup();
     return GBGPU_OK;
 }
 
