@@ -50,10 +50,12 @@
 #include "internal.h"
 #include "kernels.h"
 #include "tc_gemm.h"
+#include "tiny.cuh"
 
 namespace gbgpu {
 
-constexpr int KB = 128;  // pivots per elimination block
+constexpr int KB = 128;  // pivots per elimination block, columns of an echelon panel
+constexpr int PR = 256;  // candidate rows of a panel
 
 // per-round statistics of the echelon on stderr when GBGPU_DEBUG is set
 static bool trace_rounds() {
@@ -63,25 +65,6 @@ static bool trace_rounds() {
 
 // ---------------------------------------------------------------------------
 // kernels
-
-// scatter CSR rows rows[i] (i < n) into dense row i of out (columns
-// [col0, col0 + width) only), out already zeroed
-__global__ void k_densify(int32_t n, const int32_t* __restrict__ rows,
-                          const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ cols,
-                          const uint32_t* __restrict__ vals, int32_t col0, int32_t width,
-                          uint32_t* out, int64_t ld) {
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int i = warp; i < n; i += nwarps) {
-        const int32_t r = rows ? rows[i] : i;
-        uint32_t* o = out + (size_t)i * ld;
-        for (int64_t k = row_ptr[r] + lane; k < row_ptr[r + 1]; k += 32) {
-            const int32_t c = cols[k] - col0;
-            if (c >= 0 && c < width) o[c] = vals[k];
-        }
-    }
-}
 
 // Dense rows from CSR without a separate clear: row i of out (i < n) receives
 // CSR row rows[i], columns [from_i, nc + pad), from_i = (i / stride) stride (0
@@ -186,21 +169,6 @@ k_densify_direct(int32_t n, const int32_t* __restrict__ rows, const int64_t* __r
             }
         }
         __syncthreads();  // this row's stores are done before the CTA's next row
-    }
-}
-
-// dense known-pivot matrix: row c of out = the pivot row of lead c
-__global__ void k_densify_pivots(int32_t ncl, const int32_t* __restrict__ piv_row,
-                                 const int64_t* __restrict__ row_ptr,
-                                 const int32_t* __restrict__ cols,
-                                 const uint32_t* __restrict__ vals, uint32_t* out, int64_t ld) {
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int c = warp; c < ncl; c += nwarps) {
-        const int32_t r = piv_row[c];
-        uint32_t* o = out + (size_t)c * ld;
-        for (int64_t k = row_ptr[r] + lane; k < row_ptr[r + 1]; k += 32) o[cols[k]] = vals[k];
     }
 }
 
@@ -515,14 +483,6 @@ __global__ void k_compact_cols(int32_t n, const int32_t* __restrict__ flag,
 // ---------------------------------------------------------------------------
 // panel echelon
 
-// pending rows: nonzero and not yet pivots
-__global__ void k_collect_pending(int32_t t, const int32_t* __restrict__ lead,
-                                  const uint8_t* __restrict__ is_piv, int32_t* pend,
-                                  int32_t* n_pend) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < t; r += gridDim.x * blockDim.x)
-        if (lead[r] >= 0 && !is_piv[r]) pend[atomicAdd(n_pend, 1)] = r;
-}
-
 // the round's new pivots: count = last exclusive-scan position + last flag,
 // and their rows in ascending pivot-column order
 __global__ void k_new_pivots(int32_t ncr, const int32_t* __restrict__ wflag,
@@ -553,7 +513,7 @@ __global__ void k_panel_keys(int32_t n, const int32_t* __restrict__ pend,
     }
 }
 
-// rows sorted by (chunk slot, row): the first KB rows of every selected panel
+// rows sorted by (chunk slot, row): the first PR rows of every selected panel
 // fill its chunk in ascending row order; cursor = the panel's pending rows
 __global__ void k_bucket_sorted(int32_t n, const int32_t* __restrict__ key,
                                 const int32_t* __restrict__ rows, int32_t n_dirty,
@@ -568,7 +528,7 @@ __global__ void k_bucket_sorted(int32_t n, const int32_t* __restrict__ key,
             else hi = mid;
         }
         const int slot = q - lo;
-        if (slot < KB) chunk_rows[d * KB + slot] = rows[q];
+        if (slot < PR) chunk_rows[(size_t)d * PR + slot] = rows[q];
         if (q == n - 1 || key[q + 1] != d) cursor[d] = q - lo + 1;
     }
 }
@@ -597,7 +557,8 @@ __global__ void k_dirty_panels(const int32_t* __restrict__ n_dev, const int32_t*
 // rows of collision-free panels have leads of their own: they are pivots
 __global__ void k_claim_clean(const int32_t* __restrict__ n_dev, const int32_t* __restrict__ pend,
                               const int32_t* __restrict__ lead, const int32_t* __restrict__ pdirty,
-                              int32_t* piv_of_col, uint8_t* is_piv, int32_t* wflag) {
+                              int32_t* piv_of_col, uint8_t* is_piv, int32_t* wflag,
+                              int32_t* n_clean) {
     const int32_t n = *n_dev;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int32_t r = pend[i], l = lead[r];
@@ -605,51 +566,19 @@ __global__ void k_claim_clean(const int32_t* __restrict__ n_dev, const int32_t* 
             piv_of_col[l] = r;
             is_piv[r] = 1;
             wflag[l] = 1;
+            *n_clean = 1;
         }
-    }
-}
-
-// pending rows of the selected dirty panels (dslot[p] >= 0) into their
-// panel's chunk (at most KB rows; the others stay pending)
-__global__ void k_bucket_dirty(int32_t n, const int32_t* __restrict__ pend,
-                               const int32_t* __restrict__ lead, const int32_t* __restrict__ dslot,
-                               int32_t* cursor, int32_t* chunk_rows) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t r = pend[i];
-        const int32_t d = dslot[lead[r] / KB];
-        if (d < 0) continue;
-        const int32_t slot = atomicAdd(&cursor[d], 1);
-        if (slot < KB) chunk_rows[d * KB + slot] = r;
-    }
-}
-
-// row lists of the pivot rows of every chunk, packed to the front (the rest
-// -1): only the pivot rows take the panel transformation, as rows 0..n_piv of
-// the product -- D row k is the chunk row of pivot k, A row k the row of I - E
-// at that row's chunk position -- so that the GEMM's row quarters past n_piv
-// hold no row and skip their epilogue.  The other chunk rows are cleared later
-// by the round's elimination against all new pivots.
-__global__ void k_pivot_rowlist(const int32_t* __restrict__ n_piv, const int32_t* __restrict__ piv_pos,
-                                const int32_t* __restrict__ chunk_rows, int32_t* drows,
-                                int32_t* arows) {
-    const int d = blockIdx.x;
-    for (int k = threadIdx.x; k < n_piv[d]; k += blockDim.x) {
-        const int32_t pos = piv_pos[d * KB + k];
-        drows[d * KB + k] = chunk_rows[d * KB + pos];
-        arows[d * KB + k] = pos;
     }
 }
 
 // the factorized pivots of every chunk
 __global__ void k_register_chunks(const int32_t* __restrict__ n_piv,
-                                  const int32_t* __restrict__ piv_pos,
-                                  const int32_t* __restrict__ piv_col,
-                                  const int32_t* __restrict__ chunk_rows, int32_t* piv_of_col,
+                                  const int32_t* __restrict__ piv_rows,
+                                  const int32_t* __restrict__ piv_col, int32_t* piv_of_col,
                                   uint8_t* is_piv, int32_t* wflag) {
     const int d = blockIdx.x;
     for (int k = threadIdx.x; k < n_piv[d]; k += blockDim.x) {
-        const int32_t row = chunk_rows[d * KB + piv_pos[d * KB + k]];
-        const int32_t col = piv_col[d * KB + k];
+        const int32_t row = piv_rows[d * KB + k], col = piv_col[d * KB + k];
         piv_of_col[col] = row;
         is_piv[row] = 1;
         wflag[col] = 1;
@@ -691,180 +620,83 @@ __global__ void k_normalize_at(const int32_t* __restrict__ n_dev, const int32_t*
     }
 }
 
-// Row echelon of one panel (the 128 columns of panel dpanel[d], on the n <= KB
-// rows chunk_rows[d KB + i] of Dp) in shared memory, recording the
-// transformation E (E * old = rows whose panel part is in echelon form; the
-// rows that are not pivots become zero in the panel).  Writes I - E (KB x KB,
-// zero outside the leading n x n block), so that old - (I - E) old = E old is
-// one in-place GEMM update of the chunk rows, and the panel-local index and
-// column of every pivot, in increasing column order, and their count.
+// Reduced row echelon form of one panel (the 128 columns of panel dpanel[d], on
+// the n <= PR rows chunk_rows[d PR + i] of Dp) in the shared memory of one
+// cluster (tiny.cuh).  Its pivots, in ascending column order: piv_rows[d KB + k]
+// the row of Dp, piv_col[d KB + k] the column, n_piv[d] their number; and the
+// transformation: the reduced pivot row k (unit columns at the panel's pivots)
+// is sum_j F[d][k][j] (old pivot row j).  Rows of the chunk that are no pivots
+// have their panel part in the span of the pivots', so the round's elimination
+// clears them.
 //
-// Every row keeps its lead (first nonzero panel column) in registers of its
-// eight threads (adjacent lanes).  A step takes the non-pivot row with the
-// smallest (lead, index) as the next pivot -- the same pivot the column-by-
-// column search finds -- and updates exactly the other non-pivot rows with that
-// lead, fraction-free: row_r <- P[i][c] row_r - P[r][c] row_i on the columns
-// after c and on E (a nonzero multiple of the usual update: the same zero
-// pattern, hence the same leads and pivots, and no inverse on the sequential
-// path; each entry takes one reduction, f.ffsub).  On E only the columns in
-// the union of the two rows' supports are touched: every E row keeps its
-// support as a 128-bit mask (the chunk rows combined into it so far).
-// Pivot rows are not scaled (they are normalised after the round).
-// Column c is never read again, so it is not written; the pivot row is not
-// written in the step that chooses it, so the updates need no barrier of their
-// own.  The updated rows recompute their leads from the values they wrote and
-// publish their keys for the next step: one barrier per pivot.
-constexpr int PF_GROUPS = 8;     // threads (adjacent lanes) per row in k_panel_factor
-constexpr int PF_LD = KB + 8;    // row stride of P and E: conflict-free for 8 lanes per row
+// What bounds it is the chain of pivots (sixteen at a time, tiny.cuh).  A step
+// per pivot over all of the chunk's rows, with the transformation beside the
+// panel, took 191 us for 128 rows of a full panel on one SM; here one panel takes
+// 135 us with 256 candidate rows on eight SMs, and more candidates than pivots
+// keep a dense panel from running short of independent rows (an 8192 x 8192
+// block of rank 6144 takes 48 rounds instead of 76).
 
 template <class F>
-__global__ void __launch_bounds__(KB * PF_GROUPS)
+__global__ void __launch_bounds__(kTinyThreads, 1)
 k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __restrict__ chunk_rows,
-               const int32_t* __restrict__ dpanel, const int32_t* __restrict__ cursor, int32_t ncr,
-               uint32_t* ime_b, int32_t* piv_pos_b, int32_t* piv_col_b, int32_t* n_piv_b, F f) {
-    // chunk blockIdx.x: panel dpanel[d]
-    const int d = blockIdx.x;
-    const int32_t pj = dpanel[d] * KB;
-    const int32_t n = min(cursor[d], KB), bw = min(KB, ncr - pj), col0 = pj;
-    const int32_t* rows = chunk_rows + (size_t)d * KB;
-    uint32_t* ime = ime_b + (size_t)d * KB * KB;
-    int32_t* piv_pos = piv_pos_b + d * KB;
-    int32_t* piv_col = piv_col_b + d * KB;
-    int32_t* n_piv = n_piv_b + d;
+               const int32_t* __restrict__ dpanel, const int32_t* __restrict__ cursor,
+               int32_t max_rows, int32_t ncr, uint32_t* F_b, int32_t* piv_rows_b, int32_t* piv_col_b, int32_t* n_piv_b, F f) {
     extern __shared__ __align__(16) uint32_t pf_smem[];
-    uint32_t(*P)[PF_LD] = (uint32_t(*)[PF_LD])pf_smem;
-    uint32_t(*E)[PF_LD] = (uint32_t(*)[PF_LD])(pf_smem + KB * PF_LD);
-    __shared__ int s_min[2][KB * PF_GROUPS / 32];  // double-buffered block minimum
-    __shared__ uint32_t s_emask[KB][4];             // support of every E row
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int r = tid / PF_GROUPS, g = tid % PF_GROUPS;  // row and column group of this thread
-    const unsigned grp = 0xFFu << (lane & ~7);           // the row's eight lanes
-    for (int t = tid; t < KB * KB; t += nt) {
-        const int i = t / KB, c = t % KB;
-        P[i][c] = (i < n && c < bw) ? Dp[(size_t)rows[i] * ld + pj + c] : 0u;
-        E[i][c] = i == c ? 1u : 0u;
-    }
-    for (int t = tid; t < KB * 4; t += nt) {
-        const int i = t / 4, w = t % 4;
-        s_emask[i][w] = (i / 32 == w) ? 1u << (i % 32) : 0u;
+    const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
+    const int d = blockIdx.x / CL, tid = threadIdx.x;
+    const int32_t pj = dpanel[d] * KB, n = min(cursor[d], max_rows), bw = min(KB, ncr - pj);
+    const int32_t* rows = chunk_rows + (size_t)d * PR;
+    const TinyLayout L = tiny_layout(n, KB, CL);
+    for (int t = rk; t < KB / TP; t += CL)
+        for (int q = tid; q < n * TP; q += kTinyThreads) {
+            const int c = t * TP + q % TP;
+            pf_smem[(t >> sh) * n * TP + q] = c < bw ? Dp[(size_t)rows[q / TP] * ld + pj + c] : 0u;
+        }
+    const int np = tiny_echelon<true>(n, KB, pf_smem, f);
+    // pivots in column order: place of column c = pivot columns left of it
+    const int32_t* prow = (const int32_t*)(pf_smem + L.cols);
+    __shared__ int32_t s_col[KB];
+    if (tid < 32) {
+        int at = 0;
+        for (int c = tid; c < KB; c += 32) {
+            const unsigned bal = __ballot_sync(0xffffffffu, prow[c] >= 0);
+            if (prow[c] >= 0) s_col[at + __popc(bal & ((1u << tid) - 1u))] = c;
+            at += __popc(bal);
+        }
     }
     __syncthreads();
-    int my_lead = INT_MAX;  // this row's lead (INT_MAX: zero in the panel or not a row)
-    bool my_piv = false;
-    if (r < n)
-        for (int cc = g; cc < bw; cc += PF_GROUPS)
-            if (P[r][cc] != 0u) {
-                my_lead = cc;
-                break;
-            }
-    my_lead = min(my_lead, __shfl_xor_sync(0xffffffffu, my_lead, 1));
-    my_lead = min(my_lead, __shfl_xor_sync(0xffffffffu, my_lead, 2));
-    my_lead = min(my_lead, __shfl_xor_sync(0xffffffffu, my_lead, 4));
-    int k = 0;
-    for (int step = 0; step < KB; ++step) {
-        // warp minima by the warp-wide integer reduction (one redux.sync each)
-        const int key = __reduce_min_sync(
-            0xffffffffu, (g == 0 && !my_piv && my_lead != INT_MAX) ? my_lead * KB + r : INT_MAX);
-        int* sm = s_min[step & 1];
-        if (lane == 0) sm[warp] = key;
-        __syncthreads();  // also: the previous step's updates are visible
-        // the 32 warp minima: one read per lane, then a warp reduction
-        static_assert(KB * PF_GROUPS / 32 == 32, "one warp minimum per lane");
-        const int best = __reduce_min_sync(0xffffffffu, sm[lane]);
-        if (best == INT_MAX) break;  // uniform: no pivot left in the panel
-        const int c = best / KB, i = best % KB;
-        if (tid == 0) {
-            piv_pos[k] = i;
-            piv_col[k] = col0 + c;
+    if (rk == 0) {
+        if (tid == 0) n_piv_b[d] = np;
+        for (int k = tid; k < np; k += kTinyThreads) {
+            piv_rows_b[d * KB + k] = rows[prow[s_col[k]]];
+            piv_col_b[d * KB + k] = pj + s_col[k];
         }
-        if (r == i) my_piv = true;
-        if (!my_piv && my_lead == c) {
-            // row_r <- a row_r - m row_i, a = P[i][c], m = P[r][c], one
-            // reduction per entry (f.ffsub).  Lane g takes the 4-column groups
-            // 4 g + 32 t (16-byte shared-memory accesses).  Left of c both rows
-            // are zero and at c the result is zero, so whole groups are
-            // computed; groups entirely left of c are skipped.
-            const uint32_t ap = f.prep(P[i][c]);
-            const uint32_t mn = f.prep(f.p - P[r][c]);
-            int nl = INT_MAX;
-#pragma unroll
-            for (int t4 = 0; t4 < 4; ++t4) {
-                const int base = 32 * t4 + 4 * g;
-                if (base + 3 <= c || base >= bw) continue;
-                const uint4 x4 = *(const uint4*)&P[r][base];
-                const uint4 v4 = *(const uint4*)&P[i][base];
-                uint4 y;
-                y.x = f.ffsub(x4.x, ap, v4.x, mn);
-                y.y = f.ffsub(x4.y, ap, v4.y, mn);
-                y.z = f.ffsub(x4.z, ap, v4.z, mn);
-                y.w = f.ffsub(x4.w, ap, v4.w, mn);
-                *(uint4*)&P[r][base] = y;
-                const int first = y.x ? 0 : y.y ? 1 : y.z ? 2 : y.w ? 3 : 4;
-                if (first < 4) nl = min(nl, base + first);
-            }
-            // E: only the 4-column groups that meet the union of the two
-            // rows' supports (every E row keeps its support as a mask of the
-            // chunk rows combined into it so far)
-            uint32_t U[4];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) U[w] = s_emask[r][w] | s_emask[i][w];
-#pragma unroll
-            for (int t4 = 0; t4 < 4; ++t4) {
-                const int base = 32 * t4 + 4 * g;
-                if (base >= n || ((U[t4] >> (4 * g)) & 0xFu) == 0u) continue;
-                const uint4 x4 = *(const uint4*)&E[r][base];
-                const uint4 v4 = *(const uint4*)&E[i][base];
-                uint4 y;
-                y.x = f.ffsub(x4.x, ap, v4.x, mn);
-                y.y = f.ffsub(x4.y, ap, v4.y, mn);
-                y.z = f.ffsub(x4.z, ap, v4.z, mn);
-                y.w = f.ffsub(x4.w, ap, v4.w, mn);
-                *(uint4*)&E[r][base] = y;
-            }
-            __syncwarp(grp);  // the row's lanes have read its old support
-            if (g < 4) s_emask[r][g] = g == 0 ? U[0] : g == 1 ? U[1] : g == 2 ? U[2] : U[3];
-            // the row's eight lanes (all of them take this branch together)
-            my_lead = __reduce_min_sync(grp, nl);
-        }
-        ++k;
     }
-    for (int t = tid; t < KB * KB; t += nt) {
-        const int ii = t / KB, cc = t % KB;
-        uint32_t v = 0u;
-        if (ii < n && cc < n) {
-            const uint32_t e = E[ii][cc];
-            const uint32_t one = ii == cc ? 1u : 0u;
-            v = one >= e ? one - e : one + (f.p - e);
-        }
-        ime[t] = v;
+    uint32_t* Fo = F_b + (size_t)d * KB * KB;
+    for (int q = tid; q < np * np; q += kTinyThreads) {
+        const int k = q / np, c = s_col[q % np];
+        if (((c / TP) & (CL - 1)) == rk)
+            Fo[k * KB + q % np] = pf_smem[tiny_at(n, prow[s_col[k]], c, sh)];
     }
-    if (tid == 0) *n_piv = k;
 }
 
-
-
-
 // The panel transformation of every factorized chunk on CUDA cores: the pivot
-// rows of chunk d become E_d old over the columns from the first dirty panel
-// on, as  D[row of pivot k] = old[pos_k] - sum_j (I - E_d)[pos_k][j] old[j]
-// (ime = I - E_d from k_panel_factor; pos_k = the pivot's chunk position).
-// It is a small GEMM per chunk (np x n times n x width), done with register
-// tiles: a block owns tiles of 64 columns of one chunk; it stages the (I - E)
-// rows of its pivots transposed (A^T, n x 16 QC) once and, per tile, the old
-// values of the chunk's n rows (T, n x 64).  Every thread forms 4 pivots x QC
-// columns, one 16-byte read of A^T and QC reads of T per step of the sum; QC
-// (1, 2 or 4) is the smallest that covers the chunk's pivots in one pass
-// (16 QC pivots), so that every thread has work; chunks of more than 64
-// pivots take several passes.  64-bit sums without reduction (p < 2^16: each
-// product < 2^32, at most 128 of them; otherwise the column value in 16-bit
-// halves), one reduction per result.  A block reads all of a tile's columns
-// before it writes any (it owns them), so the update is in place.  Only pivot
-// rows are written.
+// rows of chunk d become F_d old over the columns from the first dirty panel on
+// (k_panel_factor), a small GEMM per chunk (np x np times np x width) done with
+// register tiles: a block owns tiles of 64 columns of one chunk; it stages the
+// rows of F transposed (A^T, np x 16 QC) once and, per tile, the old values of
+// the chunk's pivot rows (T, np x 64).  Every thread forms 4 pivots x QC columns,
+// one 16-byte read of A^T and QC reads of T per step of the sum; QC (1, 2 or 4)
+// is the smallest that covers the chunk's pivots in one pass (16 QC pivots), so
+// that every thread has work; chunks of more than 64 pivots take two passes.
+// 64-bit sums without reduction (p < 2^16: each product < 2^32, at most 128 of
+// them; otherwise the column value in 16-bit halves), one reduction per result.
+// A block reads all of a tile's columns before it writes any (it owns them), so
+// the update is in place.
 constexpr int PA_COLS = 64;
 constexpr int PA_THREADS = 256;
 constexpr int PA_PB = 64;            // most pivots per pass (QC = 4)
-constexpr int PA_SMALL_ROWS = 32;    // chunks up to this many rows: k_panel_apply_small
+constexpr int PA_SMALL_ROWS = 32;    // chunks up to this many pivots: k_panel_apply_small
 constexpr int PA_ALD = PA_PB + 4;    // row stride of A^T (16-byte aligned rows)
 constexpr int PA_SMEM = (KB * PA_COLS + KB * PA_ALD) * (int)sizeof(uint32_t);
 
@@ -874,8 +706,8 @@ constexpr int PA_SMEM = (KB * PA_COLS + KB * PA_ALD) * (int)sizeof(uint32_t);
 template <bool WIDE, int QC>
 __device__ __forceinline__ void pa_pass(uint32_t* Dp, int64_t ld, int32_t ncr, int c0, int n,
                                         int kp, int kn, const uint32_t (*T)[PA_COLS],
-                                        const uint32_t (*At)[PA_ALD], const int32_t* s_pos,
-                                        const int32_t* s_drow, uint32_t p, uint64_t m) {
+                                        const uint32_t (*At)[PA_ALD], const int32_t* s_rows,
+                                        uint32_t p, uint64_t m) {
     constexpr int CG = PA_COLS / QC;  // column groups
     const int cg = threadIdx.x % CG, pg = threadIdx.x / CG;
     if (4 * pg >= kn) return;
@@ -914,43 +746,37 @@ __device__ __forceinline__ void pa_pass(uint32_t* Dp, int64_t ld, int32_t ncr, i
     for (int q = 0; q < 4; ++q) {
         const int k = kp + 4 * pg + q;
         if (k >= kp + kn) break;
-        const int pos = s_pos[k];
-        uint32_t* out = Dp + (size_t)s_drow[k] * ld;
+        uint32_t* out = Dp + (size_t)s_rows[k] * ld;
 #pragma unroll
         for (int u = 0; u < QC; ++u) {
-            const int cc = cg + CG * u, col = c0 + cc;
-            if (col < ncr) {
-                const uint32_t s = WIDE ? fold_lohi(lo[q][u], hi[q][u], p, m) : mod64(lo[q][u], p, m);
-                const uint32_t old = T[pos][cc];
-                out[col] = old >= s ? old - s : old + (p - s);
-            }
+            const int col = c0 + cg + CG * u;
+            if (col < ncr)
+                out[col] = WIDE ? fold_lohi(lo[q][u], hi[q][u], p, m) : mod64(lo[q][u], p, m);
         }
     }
 }
 
-// Chunks of at most 32 rows: a warp per 32-column strip, the strip's old
-// values of the chunk's n rows in registers (one independent load each), the
-// chunk's transformation rows E (np x n, E = I - (I - E), so the pivot's own
-// old value is part of the sum) broadcast from shared memory.  No barrier
-// after the staging.  NJ >= n is the unrolled row count.
+// Chunks of at most 32 pivots: a warp per 32-column strip, the strip's old
+// values of the pivot rows in registers (one independent load each), the rows of
+// F broadcast from shared memory.  No barrier after the staging.  NJ >= np is
+// the unrolled row count.
 template <bool WIDE, int NJ>
 __device__ __forceinline__ void pa_small(uint32_t* Dp, int64_t ld, int32_t ncr, int c_lo,
-                                         int c_hi, int n, int np, const uint32_t* Es,
-                                         const int32_t* s_rows, const int32_t* s_drow,
-                                         uint32_t p, uint64_t m) {
+                                         int c_hi, int np, const uint32_t* Es,
+                                         const int32_t* s_rows, uint32_t p, uint64_t m) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int s0 = c_lo + 32 * warp; s0 < c_hi; s0 += 32 * (PA_THREADS / 32)) {
         const int col = s0 + lane;
         const bool ok = col < c_hi && col < ncr;
         uint32_t v[NJ];
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) v[j] = (ok && j < n) ? Dp[(size_t)s_rows[j] * ld + col] : 0u;
+        for (int j = 0; j < NJ; ++j) v[j] = (ok && j < np) ? Dp[(size_t)s_rows[j] * ld + col] : 0u;
         for (int k = 0; k < np; ++k) {
             const uint32_t* e = Es + k * 32;
             uint64_t lo = 0, hi = 0;
 #pragma unroll
             for (int j = 0; j < NJ; ++j) {
-                const uint32_t a = e[j];  // zero for j >= n
+                const uint32_t a = e[j];  // zero for j >= np
                 if (WIDE) {
                     lo += (uint64_t)a * (v[j] & 0xFFFFu);
                     hi += (uint64_t)a * (v[j] >> 16);
@@ -958,7 +784,7 @@ __device__ __forceinline__ void pa_small(uint32_t* Dp, int64_t ld, int32_t ncr, 
                     lo += (uint64_t)a * v[j];
                 }
             }
-            if (ok) Dp[(size_t)s_drow[k] * ld + col] = WIDE ? fold_lohi(lo, hi, p, m) : mod64(lo, p, m);
+            if (ok) Dp[(size_t)s_rows[k] * ld + col] = WIDE ? fold_lohi(lo, hi, p, m) : mod64(lo, p, m);
         }
     }
 }
@@ -966,16 +792,15 @@ __device__ __forceinline__ void pa_small(uint32_t* Dp, int64_t ld, int32_t ncr, 
 template <bool WIDE>
 __global__ void __launch_bounds__(PA_THREADS)
 k_panel_apply(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_per_block,
-              const int32_t* __restrict__ chunk_rows, const int32_t* __restrict__ dpanel,
-              const int32_t* __restrict__ cursor, const uint32_t* __restrict__ ime_b,
-              const int32_t* __restrict__ n_piv_b, const int32_t* __restrict__ arows_b,
-              const int32_t* __restrict__ drows_b, uint32_t p) {
+              const int32_t* __restrict__ dpanel, const uint32_t* __restrict__ F_b,
+              const int32_t* __restrict__ n_piv_b, const int32_t* __restrict__ piv_rows_b,
+              uint32_t p) {
     extern __shared__ __align__(16) uint32_t pa_smem[];
     uint32_t(*T)[PA_COLS] = (uint32_t(*)[PA_COLS])pa_smem;
     uint32_t(*At)[PA_ALD] = (uint32_t(*)[PA_ALD])(pa_smem + KB * PA_COLS);
-    __shared__ int32_t s_rows[KB], s_pos[KB], s_drow[KB];
+    __shared__ int32_t s_rows[KB];
     const int d = blockIdx.y;
-    const int n = min(cursor[d], KB), np = n_piv_b[d];
+    const int np = n_piv_b[d];
     const int pj = dpanel[d] * KB;
     // the block's tiles: [tile0, tile1), the first one right of the chunk's
     // panel start (the chunk rows are zero left of it)
@@ -984,23 +809,18 @@ k_panel_apply(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_p
     const int tile1 = min(ntiles, tile0 + tiles_per_block);
     tile0 = max(tile0, pj > j0 ? (pj - j0) / PA_COLS : 0);
     // uniform: nothing to do, or a chunk for k_panel_apply_small
-    if (np == 0 || tile0 >= tile1 || n <= PA_SMALL_ROWS) return;
-    for (int t = threadIdx.x; t < KB; t += PA_THREADS) {
-        s_rows[t] = t < n ? chunk_rows[(size_t)d * KB + t] : 0;
-        s_pos[t] = t < np ? arows_b[(size_t)d * KB + t] : 0;
-        s_drow[t] = t < np ? drows_b[(size_t)d * KB + t] : 0;
-    }
+    if (tile0 >= tile1 || np <= PA_SMALL_ROWS) return;
+    for (int t = threadIdx.x; t < np; t += PA_THREADS) s_rows[t] = piv_rows_b[(size_t)d * KB + t];
     __syncthreads();
-    const uint32_t* ime = ime_b + (size_t)d * KB * KB;
+    const uint32_t* F = F_b + (size_t)d * KB * KB;
     const uint64_t m = ~0ull / p;
-    // columns per thread and pivots per pass (uniform over the block)
-    const int qc = np <= 16 ? 1 : (np <= 32 ? 2 : 4);
-    const int pb = 16 * qc;
+    // pivots per pass (uniform over the block): np > 32 here
+    constexpr int pb = PA_PB;
     // A^T of pivots [kp, kp + kn)
     auto stage_a = [&](int kp, int kn) {
-        for (int t = threadIdx.x; t < kn * n; t += PA_THREADS) {
-            const int k = t / n, j = t % n;
-            At[j][k] = ime[(size_t)s_pos[kp + k] * KB + j];
+        for (int t = threadIdx.x; t < kn * np; t += PA_THREADS) {
+            const int k = t / np, j = t % np;
+            At[j][k] = F[(size_t)(kp + k) * KB + j];
         }
     };
     const bool one_pass = np <= pb;
@@ -1009,8 +829,8 @@ k_panel_apply(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_p
         const int c0 = j0 + tile * PA_COLS;
         __syncthreads();  // the last tile's readers of T are done
         {
-            // n x 64 old values, eight independent loads per thread at a time
-            const int total = n * PA_COLS;
+            // np x 64 old values, eight independent loads per thread at a time
+            const int total = np * PA_COLS;
             for (int t0 = threadIdx.x; t0 < total; t0 += 8 * PA_THREADS) {
                 uint32_t v[8];
 #pragma unroll
@@ -1033,60 +853,43 @@ k_panel_apply(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_p
                 stage_a(kp, kn);
             }
             __syncthreads();  // T and A^T are in place
-            if (qc == 1)
-                pa_pass<WIDE, 1>(Dp, ld, ncr, c0, n, kp, kn, T, At, s_pos, s_drow, p, m);
-            else if (qc == 2)
-                pa_pass<WIDE, 2>(Dp, ld, ncr, c0, n, kp, kn, T, At, s_pos, s_drow, p, m);
-            else
-                pa_pass<WIDE, 4>(Dp, ld, ncr, c0, n, kp, kn, T, At, s_pos, s_drow, p, m);
+            pa_pass<WIDE, 4>(Dp, ld, ncr, c0, np, kp, kn, T, At, s_rows, p, m);
         }
     }
 }
 
-// the chunks of k_panel_apply with at most PA_SMALL_ROWS rows (same grid)
+// the chunks of k_panel_apply with at most PA_SMALL_ROWS pivots
 template <bool WIDE>
 __global__ void __launch_bounds__(PA_THREADS)
 k_panel_apply_small(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_per_block,
-                    const int32_t* __restrict__ chunk_rows, const int32_t* __restrict__ dpanel,
-                    const int32_t* __restrict__ cursor, const uint32_t* __restrict__ ime_b,
-                    const int32_t* __restrict__ n_piv_b, const int32_t* __restrict__ arows_b,
-                    const int32_t* __restrict__ drows_b, uint32_t p) {
+                    const int32_t* __restrict__ dpanel, const uint32_t* __restrict__ F_b,
+                    const int32_t* __restrict__ n_piv_b, const int32_t* __restrict__ piv_rows_b,
+                    uint32_t p) {
     __shared__ uint32_t Es[PA_SMALL_ROWS * 32];
-    __shared__ int32_t s_rows[PA_SMALL_ROWS], s_drow[PA_SMALL_ROWS];
+    __shared__ int32_t s_rows[PA_SMALL_ROWS];
     const int d = blockIdx.y;
-    const int n = min(cursor[d], KB), np = n_piv_b[d];
+    const int np = n_piv_b[d];
     const int pj = dpanel[d] * KB;
     const int ntiles = (ncr - j0 + PA_COLS - 1) / PA_COLS;
     int tile0 = blockIdx.x * tiles_per_block;
     const int tile1 = min(ntiles, tile0 + tiles_per_block);
     tile0 = max(tile0, pj > j0 ? (pj - j0) / PA_COLS : 0);
-    if (np == 0 || tile0 >= tile1 || n > PA_SMALL_ROWS) return;  // uniform
-    for (int t = threadIdx.x; t < PA_SMALL_ROWS; t += PA_THREADS) {
-        s_rows[t] = t < n ? chunk_rows[(size_t)d * KB + t] : 0;
-        s_drow[t] = t < np ? drows_b[(size_t)d * KB + t] : 0;
-    }
-    // E rows of the pivots, 32 entries each (zero past n):
-    // E[k][j] = [j = pos_k] - (I - E)[pos_k][j] mod p
-    const uint32_t* ime = ime_b + (size_t)d * KB * KB;
-    for (int t = threadIdx.x; t < np * 32; t += PA_THREADS) {
-        const int k = t / 32, j = t % 32;
-        uint32_t e = 0u;
-        if (j < n) {
-            const int pos = arows_b[(size_t)d * KB + k];
-            const uint32_t a = ime[(size_t)pos * KB + j];
-            e = (j == pos) ? (a == 0u ? 1u : (1u + p - a) % p) : (a ? p - a : 0u);
-        }
-        Es[t] = e;
-    }
+    if (np == 0 || tile0 >= tile1 || np > PA_SMALL_ROWS) return;  // uniform
+    for (int t = threadIdx.x; t < PA_SMALL_ROWS; t += PA_THREADS)
+        s_rows[t] = t < np ? piv_rows_b[(size_t)d * KB + t] : 0;
+    // the rows of F, 32 entries each (zero past np)
+    const uint32_t* F = F_b + (size_t)d * KB * KB;
+    for (int t = threadIdx.x; t < np * 32; t += PA_THREADS)
+        Es[t] = t % 32 < np ? F[(size_t)(t / 32) * KB + t % 32] : 0u;
     __syncthreads();
     const uint64_t m = ~0ull / p;
     const int c_lo = j0 + tile0 * PA_COLS, c_hi = min(ncr, j0 + tile1 * PA_COLS);
-    if (n <= 8)
-        pa_small<WIDE, 8>(Dp, ld, ncr, c_lo, c_hi, n, np, Es, s_rows, s_drow, p, m);
-    else if (n <= 16)
-        pa_small<WIDE, 16>(Dp, ld, ncr, c_lo, c_hi, n, np, Es, s_rows, s_drow, p, m);
+    if (np <= 8)
+        pa_small<WIDE, 8>(Dp, ld, ncr, c_lo, c_hi, np, Es, s_rows, p, m);
+    else if (np <= 16)
+        pa_small<WIDE, 16>(Dp, ld, ncr, c_lo, c_hi, np, Es, s_rows, p, m);
     else
-        pa_small<WIDE, 32>(Dp, ld, ncr, c_lo, c_hi, n, np, Es, s_rows, s_drow, p, m);
+        pa_small<WIDE, 32>(Dp, ld, ncr, c_lo, c_hi, np, Es, s_rows, p, m);
 }
 
 // dst block b (NB x NB, leading dimension NB, block stride NB (NB + 1)) =
@@ -1272,12 +1075,23 @@ __global__ void k_offs_write(int32_t n, const int64_t* __restrict__ loc, int64_t
 //   T <- T - T[:, pc] (U[:, pc])^-1 U,
 // after which every T row is zero at every pivot column.  Blocks of NB
 // pivots, left to right; the rows are read and written in place through the
-// row lists (T and U rows are distinct).
+// row lists (T and U rows are distinct).  With `unit`, U[:, pc] is the identity.
 template <class F>
 static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t* t_rows,
                      int32_t rows, int32_t ncols, const int32_t* u_rows, int32_t n_p,
-                     const int32_t* d_pc, const std::vector<int32_t>& pc) {
+                     const int32_t* d_pc, const std::vector<int32_t>& pc, bool unit) {
     if (rows <= 0 || n_p <= 0) return GBGPU_OK;
+    if (unit) {  // U[:, pc] is the identity (at most KB pivots): T -= T[:, pc] U
+        uint32_t* G = c.alloc<uint32_t>((size_t)rows * KB);
+        if (!G) return GBGPU_ENOMEM;
+        const int32_t first_col = pc[0] & ~3;
+        BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)rows * n_p), 256, 0, c.s>>>(rows, n_p, M, ld, d_pc,
+                                                                              G, KB, t_rows));
+        TcGemmArgs g{c.p, rows, ncols - first_col, n_p, G, KB, M + first_col, ld, M + first_col, ld};
+        g.b_rows = u_rows;
+        g.d_rows = t_rows;
+        return gemm_args(c, g);
+    }
     const int32_t NB = nb_for(n_p);
     const int32_t nb = (n_p + NB - 1) / NB;
     const int64_t bstride = (int64_t)NB * (NB + 1);
@@ -1424,10 +1238,10 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
     // Every round looks at all pending rows (nonzero, not yet pivots) at once:
     //  * a 128-column panel in which no two pending rows share a lead is
     //    "clean": each of its rows has a lead of its own and becomes a pivot;
-    //  * every other ("dirty") panel gets up to KB of its pending rows
-    //    factorized in shared memory (k_panel_factor, one CTA per panel); the
-    //    recorded row transformation E is applied to their trailing columns
-    //    by one batched GEMM over all dirty panels;
+    //  * every other ("dirty") panel gets up to PR of its pending rows
+    //    factorized in shared memory (k_panel_factor, one cluster per panel); the
+    //    recorded transformation F of its pivot rows is applied to their
+    //    trailing columns (k_panel_apply);
     //  * the pending rows that did not become pivots are eliminated against
     //    all pivots of the round (eliminate), which leaves them zero at every
     //    pivot column, and the next round starts from their new leads.
@@ -1458,18 +1272,14 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
         BL_CUDA(cudaMemsetAsync(is_piv, 0, t, s));
         BL_LAUNCH(k_row_leads<<<grid_of((int64_t)t * 32), 256, 0, s>>>(t, nullptr, ncr, Dp, ld, lead));
     }
-    const int pf_bytes = 2 * KB * PF_LD * (int)sizeof(uint32_t);
-    BL_CUDA(ensure_smem_limit((const void*)k_panel_factor<F>, pf_bytes));
     // every dirty panel is factorized in the round that finds it (batch <= 4096)
     const int32_t max_dirty = std::max<int32_t>(1, std::min<int32_t>(npan, 4096));
-    int32_t* chunk_rows = c.alloc<int32_t>((size_t)max_dirty * KB);
+    int32_t* chunk_rows = c.alloc<int32_t>((size_t)max_dirty * PR);
     int32_t* cursor = c.alloc<int32_t>(max_dirty);
-    uint32_t* imeB = c.alloc<uint32_t>((size_t)max_dirty * KB * KB);
-    int32_t* piv_pos = c.alloc<int32_t>((size_t)max_dirty * KB);
+    uint32_t* panF = c.alloc<uint32_t>((size_t)max_dirty * KB * KB);
     int32_t* piv_colb = c.alloc<int32_t>((size_t)max_dirty * KB);
     int32_t* n_piv = c.alloc<int32_t>(max_dirty);
     int32_t* piv_rows = c.alloc<int32_t>((size_t)max_dirty * KB);
-    int32_t* piv_arows = c.alloc<int32_t>((size_t)max_dirty * KB);
     // ordered compaction of the pending rows and the stable (panel, row) sort
     // that fills the chunks: the same rows, in the same order, on every run
     uint8_t* pflag = c.alloc<uint8_t>(t);
@@ -1483,8 +1293,7 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                                     0, 32, s);
     void* sel_tmp = c.alloc<uint8_t>(sel_bytes);
     void* sort_tmp = c.alloc<uint8_t>(sort_bytes);
-    if (!chunk_rows || !cursor || !imeB || !piv_pos || !piv_colb || !n_piv || !piv_rows ||
-        !piv_arows || !pflag || !pkey || !pkey_sorted || !prow_sorted || !sel_tmp || !sort_tmp)
+    if (!chunk_rows || !cursor || !panF || !piv_colb || !n_piv || !piv_rows || !pflag || !pkey || !pkey_sorted || !prow_sorted || !sel_tmp || !sort_tmp)
         return GBGPU_ENOMEM;
     // pending rows (nonzero, not pivots) into pend[0 .. *count), ascending
     auto collect_pending = [&](int32_t* count) -> int {
@@ -1510,7 +1319,8 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
         BL_LAUNCH(k_lead_hist<<<grid_of(t), 256, 0, s>>>(counters, pend, lead, hist, pcnt));
         BL_LAUNCH(k_dirty_panels<<<grid_of(t), 256, 0, s>>>(counters, pend, lead, hist, pdirty));
         BL_LAUNCH(k_claim_clean<<<grid_of(t), 256, 0, s>>>(counters, pend, lead, pdirty,
-                                                            piv_of_col, is_piv, wflag));
+                                                            piv_of_col, is_piv, wflag,
+                                                            counters + 4));
         // dirty panels, leftmost first, at most max_dirty of them this round
         std::vector<int32_t> h_dirty(npan);
         BL_CUDA(cudaMemcpyAsync(&n_pend, counters, 4, cudaMemcpyDeviceToHost, s));
@@ -1536,8 +1346,6 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
             BL_CUDA(cudaMemcpyAsync(dpanel, h_dpanel.data(), sizeof(int32_t) * n_dirty,
                                     cudaMemcpyHostToDevice, s));
             BL_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * n_dirty, s));
-            BL_LAUNCH(k_fill_i32<<<grid_of((int64_t)n_dirty * KB), 256, 0, s>>>(
-                chunk_rows, n_dirty * KB, -1));
             BL_LAUNCH(k_panel_keys<<<grid_of(n_pend), 256, 0, s>>>(n_pend, pend, lead, dslot,
                                                                     n_dirty, pkey));
             {
@@ -1550,50 +1358,47 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
             }
             BL_LAUNCH(k_bucket_sorted<<<grid_of(n_pend), 256, 0, s>>>(
                 n_pend, pkey_sorted, prow_sorted, n_dirty, chunk_rows, cursor));
-            BL_LAUNCH(k_panel_factor<F><<<n_dirty, KB * PF_GROUPS, pf_bytes, s>>>(
-                Dp, ld, chunk_rows, dpanel, cursor, ncr, imeB, piv_pos, piv_colb, n_piv, f));
-            // pivot rows of every chunk (columns j0..) <- old - (I - E_d) old =
-            // E_d old, in place: the limb planes of `old` are cut before the
-            // product writes the rows.  The non-pivot chunk rows keep their
-            // values: their panel parts lie in the span of the pivot rows', so
-            // the elimination against the round's pivots below clears them.
-            BL_LAUNCH(k_fill_i32<<<grid_of((int64_t)n_dirty * KB), 256, 0, s>>>(
-                piv_rows, n_dirty * KB, -1));
-            BL_LAUNCH(k_fill_i32<<<grid_of((int64_t)n_dirty * KB), 256, 0, s>>>(
-                piv_arows, n_dirty * KB, -1));
-            BL_LAUNCH(k_pivot_rowlist<<<n_dirty, KB, 0, s>>>(n_piv, piv_pos, chunk_rows, piv_rows,
-                                                             piv_arows));
             {
-                // pivot rows of every chunk <- E_d old (CUDA cores, in place)
+                // CTAs per panel: as many as leave every panel its own SMs
+                int cl = kTinyMaxCluster;
+                while (cl > 1 && n_dirty * cl > 148) cl /= 2;
+                // many panels: the longest one sets the round's time
+                int32_t nc_ = ncr, rows_ = cl == 1 ? KB : PR;
+                int64_t ld_ = ld;
+                F fv = f;
+                void* args[] = {&Dp, &ld_, &chunk_rows, &dpanel, &cursor, &rows_, &nc_,
+                                &panF, &piv_rows, &piv_colb, &n_piv, &fv};
+                BL_LAUNCH(BL_CUDA(launch_cluster((const void*)k_panel_factor<F>, n_dirty * cl, cl,
+                                                 kTinyThreads,
+                                                 (int)tiny_layout(rows_, KB, cl).words * 4, s, args)));
+            }
+            {
+                // pivot rows of every chunk <- F_d old (CUDA cores, in place), columns j0..
                 const bool wide = c.p >= 65536u;
                 // tiles per block: enough blocks for about six per SM, at most 8
-                // tiles each (a block stages the (I - E) rows once for its tiles)
+                // tiles each (a block stages the rows of F once for its tiles)
                 const int tiles = (width + PA_COLS - 1) / PA_COLS;
                 const int tpb = (int)std::max<int64_t>(
                     1, std::min<int64_t>(8, (int64_t)tiles * n_dirty / (148 * 6)));
                 const dim3 grid((unsigned)((tiles + tpb - 1) / tpb), (unsigned)n_dirty);
-                // the chunks of more than 32 rows are few and long: one tile per block
+                // the chunks of more than 32 pivots are few and long: one tile per block
                 const dim3 grid1((unsigned)tiles, (unsigned)n_dirty);
                 if (wide) {
                     BL_CUDA(ensure_smem_limit((const void*)k_panel_apply<true>, PA_SMEM));
                     BL_LAUNCH(k_panel_apply_small<true><<<grid, PA_THREADS, 0, s>>>(
-                        Dp, ld, ncr, j0, tpb, chunk_rows, dpanel, cursor, imeB, n_piv, piv_arows,
-                        piv_rows, c.p));
+                        Dp, ld, ncr, j0, tpb, dpanel, panF, n_piv, piv_rows, c.p));
                     BL_LAUNCH(k_panel_apply<true><<<grid1, PA_THREADS, PA_SMEM, s>>>(
-                        Dp, ld, ncr, j0, 1, chunk_rows, dpanel, cursor, imeB, n_piv, piv_arows,
-                        piv_rows, c.p));
+                        Dp, ld, ncr, j0, 1, dpanel, panF, n_piv, piv_rows, c.p));
                 } else {
                     BL_CUDA(ensure_smem_limit((const void*)k_panel_apply<false>, PA_SMEM));
                     BL_LAUNCH(k_panel_apply_small<false><<<grid, PA_THREADS, 0, s>>>(
-                        Dp, ld, ncr, j0, tpb, chunk_rows, dpanel, cursor, imeB, n_piv, piv_arows,
-                        piv_rows, c.p));
+                        Dp, ld, ncr, j0, tpb, dpanel, panF, n_piv, piv_rows, c.p));
                     BL_LAUNCH(k_panel_apply<false><<<grid1, PA_THREADS, PA_SMEM, s>>>(
-                        Dp, ld, ncr, j0, 1, chunk_rows, dpanel, cursor, imeB, n_piv, piv_arows,
-                        piv_rows, c.p));
+                        Dp, ld, ncr, j0, 1, dpanel, panF, n_piv, piv_rows, c.p));
                 }
             }
-            BL_LAUNCH(k_register_chunks<<<n_dirty, KB, 0, s>>>(n_piv, piv_pos, piv_colb, chunk_rows,
-                                                                piv_of_col, is_piv, wflag));
+            BL_LAUNCH(k_register_chunks<<<n_dirty, KB, 0, s>>>(n_piv, piv_rows, piv_colb, piv_of_col,
+                                                                is_piv, wflag));
             if (trace_rounds()) {
                 std::vector<int32_t> h_cur(n_dirty), h_np(n_dirty);
                 BL_CUDA(cudaMemcpyAsync(h_cur.data(), cursor, 4 * n_dirty, cudaMemcpyDeviceToHost, s));
@@ -1602,7 +1407,7 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                 long long rows_in = 0, piv = 0;
                 int mx = 0;
                 for (int q = 0; q < n_dirty; ++q) {
-                    rows_in += std::min(h_cur[q], KB);
+                    rows_in += std::min(h_cur[q], PR);
                     piv += h_np[q];
                     mx = std::max(mx, h_cur[q]);
                 }
@@ -1623,16 +1428,18 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
         // the rest: eliminated against every pivot of the round; one host
         // round trip reads both counts and the pivot columns
         BL_CHECK(collect_pending(counters + 3));
-        int32_t cnt[2] = {0, 0};
+        int32_t cnt[3] = {0, 0, 0};
         std::vector<int32_t> h_pc((size_t)ncr);
-        BL_CUDA(cudaMemcpyAsync(cnt, counters + 2, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        BL_CUDA(cudaMemcpyAsync(cnt, counters + 2, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         BL_CUDA(cudaMemcpyAsync(h_pc.data(), pc, sizeof(int32_t) * ncr, cudaMemcpyDeviceToHost, s));
         BL_CUDA(cudaStreamSynchronize(s));
         const int32_t n_new = cnt[0], n_rest = cnt[1];
         if (trace_rounds()) fprintf(stderr, "gbgpu echelon round %d: new pivots %d\n", rounds, n_new);
         if (n_rest == 0) break;
         h_pc.resize((size_t)n_new);
-        BL_CHECK(eliminate(c, f, Dp, ld, pend, n_rest, ncr, prow, n_new, pc, h_pc));
+        // one panel alone: its pivot rows are reduced among themselves already
+        const bool unit = n_dirty == 1 && cnt[2] == 0;
+        BL_CHECK(eliminate(c, f, Dp, ld, pend, n_rest, ncr, prow, n_new, pc, h_pc, unit));
         BL_LAUNCH(k_row_leads<<<grid_of((int64_t)n_rest * 32), 256, 0, s>>>(n_rest, pend, ncr, Dp,
                                                                              ld, lead, 1));
     }

@@ -44,8 +44,8 @@ constexpr int kTinyMaxCluster = 8;          // the portable limit
 constexpr int TP = 16;                      // panel columns
 // Shared memory of one CTA for an n x m block in a cluster of cl (offsets in
 // 32-bit words): its panels [panels / cl][n][TP], two copies of the current
-// panel [n][TP], the pivots' TP x TP blocks (F, the pivot rows in the panel, two
-// working blocks), arrays per row and per column.
+// panel [n][TP], the pivots' TP x TP blocks (F, the pivot rows in the panel, and
+// eight working blocks), arrays per row and per column.
 struct TinyLayout {
     int32_t panels;  // of the block
     int64_t pb, blk, rows, cols, words;
@@ -55,7 +55,7 @@ __host__ __device__ inline TinyLayout tiny_layout(int32_t n, int32_t m, int32_t 
     L.panels = (m + TP - 1) / TP;
     L.pb = (int64_t)((L.panels + cl - 1) / cl) * n * TP;
     L.blk = L.pb + 2 * (int64_t)n * TP;
-    L.rows = L.blk + 4 * TP * TP;
+    L.rows = L.blk + (2 + 8) * TP * TP;
     L.cols = L.rows + (int64_t)n;
     L.words = (L.cols + 3 * (int64_t)L.panels * TP + 3) & ~(int64_t)3;
     return L;
@@ -114,8 +114,9 @@ struct TinyTurn {
 };
 
 // The rows of the next turn, the same in every CTA: the first row of every lead
-// in the panel, then the other nonzero rows in row order.  Returns their number
-// (uniform), 0 when no row but the pivots is nonzero.
+// in the panel, then the other nonzero rows in row order.  Returns the number of
+// nonzero rows that are no pivots, or TP + 1 if there are more than TP (uniform);
+// the turn takes at most TP of them.
 __device__ inline int tiny_select(const int n, const uint32_t* pb, const int32_t* pcol,
                                   TinyTurn& S) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -148,7 +149,7 @@ __device__ inline int tiny_select(const int n, const uint32_t* pb, const int32_t
         return 0;
     }
     if (tid < TP && mine != INT_MAX) S.sel[__popc(leads & ((1u << lane) - 1u))] = mine;
-    for (int r0 = 0; r0 < n && count < TP; r0 += kTinyThreads) {
+    for (int r0 = 0; r0 < n && count <= TP; r0 += kTinyThreads) {
         const int r = r0 + tid, ld = r0 ? lead_of(r) : ld0;
         const bool other = ld != INT_MAX && S.first[ld] != r;
         const unsigned bal = __ballot_sync(0xffffffffu, other);
@@ -164,7 +165,7 @@ __device__ inline int tiny_select(const int n, const uint32_t* pb, const int32_t
         __syncthreads();  // per_warp is rewritten
     }
     __syncthreads();
-    return min(TP, count);
+    return min(TP + 1, count);
 }
 
 // The turn's rows: their pivots into pcol / prow / S.mask, and, by pivot column
@@ -230,15 +231,17 @@ __device__ void tiny_turn(const int n_sel, const int c0, const uint32_t* pb, int
 
 // G ([n][TP]) -= the turn's elimination: row r takes -= sum_c pb[r][c] P[c],
 // the turn's pivot rows become P[c]; P in v by pivot column (prep form), a lane
-// per column j, two rows per warp.  G may be pb itself.
+// per column j, two rows per warp; by `parts` warps, this one the part-th.  G
+// may be pb itself.  The columns of `zero` count as zero before the update.
 template <class F>
 __device__ __forceinline__ void tiny_update(const int n, const int c0, const uint32_t mask,
                                             const uint32_t* pb, const int32_t* pcol,
-                                            const uint32_t (&v)[TP], uint32_t* G, const F f) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane % TP;
+                                            const uint32_t (&v)[TP], uint32_t* G, const int part,
+                                            const int parts, const F f, const uint32_t zero = 0u) {
+    const int lane = threadIdx.x & 31, j = lane % TP;
     constexpr int U = 2;  // rows in flight per lane
 #pragma unroll 1
-    for (int r0 = 2 * U * warp; r0 < n; r0 += 2 * U * kTinyWarps) {
+    for (int r0 = 2 * U * part; r0 < n; r0 += 2 * U * parts) {
         uint4 e[U][TP / 4];
         uint32_t g[U];
         bool on[U];
@@ -250,7 +253,7 @@ __device__ __forceinline__ void tiny_update(const int n, const int c0, const uin
 #pragma unroll
             for (int q = 0; q < TP / 4; ++q)
                 e[u][q] = on[u] ? *(const uint4*)(pb + r * TP + 4 * q) : make_uint4(0u, 0u, 0u, 0u);
-            g[u] = on[u] ? G[r * TP + j] : 0u;
+            g[u] = on[u] && !((zero >> j) & 1u) ? G[r * TP + j] : 0u;
         }
         __syncwarp();  // the rows are read before they are written (G = pb)
 #pragma unroll
@@ -273,25 +276,114 @@ __device__ __forceinline__ void tiny_update(const int n, const int c0, const uin
     }
 }
 
-// The block is in the CTAs' panels (tiny_layout, columns past m zero) and
-// visible to the cluster.  Reached by every thread of every CTA of the
-// cluster, kTinyThreads a CTA.
+// One turn on this CTA's panels g in [g0, g1) (panel g at T + g n TP), none of
+// them the current one (c0): the turn's pivot rows there are F times their old
+// values, every other row takes their multiples (see tiny_update).  Panel `own`
+// is the current one and keeps, in the turn's pivot columns, the coefficients of
+// the old pivot rows.  Up to TG panels at a time, so that a few rows still fill
+// the warps and the barriers are shared (a panel at a time, each turn of a
+// 33-row block of 8 panels took 40000 cycles).  Reached by the whole CTA; NP:
+// TG TP TP words of shared memory.
+constexpr int TG = 8;
+constexpr int kFewPivots = 6;
 template <class F>
-__device__ void tiny_rref_body(const int32_t n, const int32_t m, uint32_t* smem, const TinyOut out,
-                               const F f) {
+__device__ __forceinline__ void tiny_groups(const int n, const int c0, const uint32_t mask,
+                                            const uint32_t* pb, const int32_t* pcol,
+                                            const int32_t* prow, const uint32_t* Fm, uint32_t* NP,
+                                            uint32_t* T, const int g0, const int g1, const int own,
+                                            const F f) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER = TG * TP * TP / kTinyThreads;  // entries of new pivot rows per thread
+    const bool few = __popc(mask) <= kFewPivots;      // the sums skip the missing terms
+    for (int gb = g0; gb < g1; gb += TG) {
+        const int ng = min(TG, g1 - gb);
+        uint32_t np[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int e = tid + u * kTinyThreads, c = (e / TP) % TP, j = e % TP, g = e / (TP * TP);
+            np[u] = 0u;
+            if (g >= ng || !((mask >> c) & 1u)) continue;
+            const uint32_t* G = T + (size_t)(gb + g) * n * TP;
+            if (gb + g == own && ((mask >> j) & 1u)) {
+                np[u] = f.mulp(1u, Fm[c * TP + j]);
+                continue;
+            }
+            ChainSum<F> acc(f);
+            if (few) {
+                for (uint32_t b = mask; b; b &= b - 1u) {
+                    const int q = __ffs(b) - 1;
+                    acc.add(f, 0, Fm[c * TP + q], G[prow[c0 + q] * TP + j]);
+                }
+            } else {
+                uint32_t old[TP];
+#pragma unroll
+                for (int q = 0; q < TP; ++q)
+                    old[q] = (mask >> q) & 1u ? G[prow[c0 + q] * TP + j] : 0u;
+#pragma unroll
+                for (int q = 0; q < TP; ++q) acc.add(f, q, Fm[c * TP + q], old[q]);
+            }
+            np[u] = acc.mod(f);
+        }
+        __syncthreads();  // every old value is read, and the last panels' NP
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int e = tid + u * kTinyThreads, c = (e / TP) % TP, j = e % TP, g = e / (TP * TP);
+            if (g >= ng) continue;
+            NP[e] = f.prep(np[u]);
+            if ((mask >> c) & 1u) T[(size_t)(gb + g) * n * TP + prow[c0 + c] * TP + j] = np[u];
+        }
+        __syncthreads();
+        const int wpg = kTinyWarps / ng, g = warp / wpg;
+        if (g < ng && few) {
+            // few pivots: their values straight from shared memory
+            uint32_t* G = T + (size_t)(gb + g) * n * TP;
+            const int j = lane % TP;
+            const uint32_t* P = NP + g * TP * TP + j;
+            const bool zero = gb + g == own && ((mask >> j) & 1u);
+            for (int r = 2 * (warp % wpg) + lane / TP; r < n; r += 2 * wpg) {
+                const int k = pcol[r] - c0;
+                if (k >= 0 && k < TP && ((mask >> k) & 1u)) continue;
+                ChainSum<F, 2> acc(f);
+                uint32_t any = 0u;
+                for (uint32_t b = mask; b; b &= b - 1u) {
+                    const int q = __ffs(b) - 1;
+                    const uint32_t x = pb[r * TP + q];
+                    any |= x;
+                    acc.add(f, 0, x, P[q * TP]);
+                }
+                if (any == 0u) continue;
+                const uint32_t t = acc.mod(f), gv = zero ? 0u : G[r * TP + j];
+                G[r * TP + j] = gv >= t ? gv - t : gv + (f.p - t);
+            }
+        } else if (g < ng) {
+            uint32_t v[TP];
+#pragma unroll
+            for (int q = 0; q < TP; ++q) v[q] = NP[(g * TP + q) * TP + lane % TP];
+            tiny_update(n, c0, mask, pb, pcol, v, T + (size_t)(gb + g) * n * TP, warp % wpg, wpg, f,
+                        gb + g == own ? mask : 0u);
+        }
+    }
+}
+
+// The reduced echelon form of the block in the CTAs' panels (tiny_layout, columns
+// past m zero).  Reached by every thread of every CTA of the cluster,
+// kTinyThreads a CTA; on return pcol[row] and prow[column] hold the pivots
+// (the same in every CTA) and every CTA's panels are final and visible.  With
+// COEF the pivot columns hold, instead of unit vectors, the coefficients of the
+// old pivot rows: row r = sum over pivot columns c of T[r][c] old_(prow[c]).
+// Returns the rank.
+template <bool COEF, class F>
+__device__ int tiny_echelon(const int32_t n, const int32_t m, uint32_t* smem, const F f) {
     const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
     const TinyLayout L = tiny_layout(n, m, CL);
     uint32_t* T = smem;
     uint32_t* Fm = smem + L.blk;                    // [TP][TP], see tiny_turn
     uint32_t* PP = Fm + TP * TP;
-    uint32_t* NP = PP + TP * TP;  // the pivot rows in a panel right of it; [2][TP][TP]
+    uint32_t* NP = PP + TP * TP;  // the pivot rows in panels beside it; [TG][TP][TP]
     int32_t* pcol = (int32_t*)(smem + L.rows);      // [n] pivot column of a pivot row, -1
     int32_t* prow = (int32_t*)(smem + L.cols);      // [m] pivot row of a column, -1
-    int32_t* rank = prow + L.panels * TP;           // [m] pivots right of a column
-    int32_t* cnt = rank + L.panels * TP;            // [m] entries of the answer's rows
-    __shared__ int s_part[kTinyWarps];
     __shared__ TinyTurn S;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     // the owner's panel k to every CTA's copy for panel k
     auto push = [&](int k) {
         const uint4* src = (const uint4*)(T + (k >> sh) * n * TP);
@@ -306,64 +398,43 @@ __device__ void tiny_rref_body(const int32_t n, const int32_t m, uint32_t* smem,
     cluster_sync();  // every CTA has started, its panels are in place
     if (rk == 0) push(0);
     cluster_sync();
+    constexpr uint32_t kFull = (1u << TP) - 1u;
     int found = 0;  // pivots so far (uniform over the cluster)
     for (int k = 0; k < L.panels; ++k) {
         uint32_t* pb = smem + L.pb + (k & 1) * n * TP;
+        uint32_t* own = (k & (CL - 1)) == rk ? T + (k >> sh) * n * TP : nullptr;
         const int c0 = k * TP, j = lane % TP;
         uint32_t pmask = 0u;  // the panel's pivot columns so far (uniform)
-        while (pmask != (1u << TP) - 1u) {
-            const int n_sel = tiny_select(n, pb, pcol, S);
-            if (n_sel == 0) break;  // uniform over the cluster
-            if (tid < TP * TP) tiny_turn(n_sel, c0, pb, pcol, prow, Fm, PP, NP, S, f);
+        while (pmask != kFull) {
+            const int left = tiny_select(n, pb, pcol, S);
+            if (left == 0) break;  // uniform over the cluster
+            const bool last = left <= TP;  // every nonzero row is in this turn
+            if (tid < TP * TP) tiny_turn(min(left, TP), c0, pb, pcol, prow, Fm, PP, NP, S, f);
             __syncthreads();
             const uint32_t mask = S.mask;
             pmask |= mask;
             found += __popc(mask);
-            // this CTA's panels right of panel k
-            for (int t = k + 1; t < L.panels; ++t) {
-                if ((t & (CL - 1)) != rk) continue;
-                uint32_t* G = T + (t >> sh) * n * TP;
-                // the pivot rows there: F times their old values
-                const int c = tid / TP;
-                const bool piv = c < TP && ((mask >> c) & 1u);
-                uint32_t np = 0u;
-                if (piv) {
-                    uint32_t old[TP];
-#pragma unroll
-                    for (int q = 0; q < TP; ++q)
-                        old[q] = (mask >> q) & 1u ? G[prow[c0 + q] * TP + j] : 0u;
-                    ChainSum<F> acc(f);
-#pragma unroll
-                    for (int q = 0; q < TP; ++q) acc.add(f, q, Fm[c * TP + q], old[q]);
-                    np = acc.mod(f);
-                }
-                __syncthreads();  // every old value is read
-                if (c < TP) NP[tid] = piv ? f.prep(np) : 0u;
-                if (piv) G[prow[c0 + c] * TP + j] = np;
-                __syncthreads();
-                uint32_t v[TP];
-#pragma unroll
-                for (int q = 0; q < TP; ++q) v[q] = NP[q * TP + j];
-                tiny_update(n, c0, mask, pb, pcol, v, G, f);
-            }
-            if (pmask != (1u << TP) - 1u) {
+            // this CTA's panels right of panel k, with COEF all of them
+            tiny_groups(n, c0, mask, pb, pcol, prow, Fm, NP, T,
+                        COEF ? 0 : (k + CL - rk) / CL, (L.panels - rk + CL - 1) / CL,
+                        COEF && own ? k >> sh : -1, f);
+            if (pmask != kFull && (!last || (!COEF && own))) {
                 // the panel itself, in every CTA's copy
                 __syncthreads();  // the updates above have read it
                 uint32_t v[TP];
 #pragma unroll
                 for (int q = 0; q < TP; ++q) v[q] = f.prep(PP[q * TP + j]);
-                tiny_update(n, c0, mask, pb, pcol, v, pb, f);
+                tiny_update(n, c0, mask, pb, pcol, v, pb, tid >> 5, kTinyWarps, f);
                 const int c = tid / TP;
                 if (c < TP && ((mask >> c) & 1u)) pb[prow[c0 + c] * TP + j] = PP[tid];
             }
             __syncthreads();
+            if (last) break;
         }
-        if (pmask != 0u && (k & (CL - 1)) == rk) {
+        if (!COEF && pmask != 0u && own) {
             // the owner's panel: the copy, or unit columns if all have a pivot
-            uint32_t* own = T + (k >> sh) * n * TP;
-            const bool full = pmask == (1u << TP) - 1u;
             for (int t = tid; t < n * TP; t += kTinyThreads)
-                own[t] = full ? (pcol[t / TP] == c0 + t % TP ? 1u : 0u) : pb[t];
+                own[t] = pmask == kFull ? (pcol[t / TP] == c0 + t % TP ? 1u : 0u) : pb[t];
         }
         if (k + 1 == L.panels) break;
         if (((k + 1) & (CL - 1)) == rk) push(k + 1);
@@ -371,6 +442,23 @@ __device__ void tiny_rref_body(const int32_t n, const int32_t m, uint32_t* smem,
         if (found == n) break;
     }
     cluster_sync();
+    return found;
+}
+
+// tiny_echelon and the compaction of its pivot rows.
+template <class F>
+__device__ void tiny_rref_body(const int32_t n, const int32_t m, uint32_t* smem, const TinyOut out,
+                               const F f) {
+    const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
+    const TinyLayout L = tiny_layout(n, m, CL);
+    tiny_echelon<false>(n, m, smem, f);
+    const uint32_t* T = smem;
+    const int32_t* pcol = (const int32_t*)(smem + L.rows);
+    const int32_t* prow = (const int32_t*)(smem + L.cols);
+    int32_t* rank = (int32_t*)(smem + L.cols) + L.panels * TP;  // [m] pivots right of a column
+    int32_t* cnt = rank + L.panels * TP;                        // [m] entries of the answer's rows
+    __shared__ int s_part[kTinyWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // ---- compaction: pivot rows in descending pivot-column order ----
     // rank of a pivot column = pivot columns to its right
     for (int c = tid; c < m; c += kTinyThreads) rank[c] = prow[m - 1 - c] >= 0 ? 1 : 0;
