@@ -997,11 +997,36 @@ static int gemm(Ctx& c, uint32_t* D, int64_t ldd, const uint32_t* A, int64_t lda
     return gemm_args(c, g);
 }
 
-// batch of `batch` products D_z -= A_z B_z (element strides sA, sB, sD)
-static int gemm_batched(Ctx& c, uint32_t* D, int64_t ldd, int64_t sD, const uint32_t* A,
+// D <- -A B where D is A or B itself (unbatched).  The CUDA-core GEMM reads its
+// operands while it writes, so there the product goes through a copy.
+static int gemm_set_in_place(Ctx& c, TcGemmArgs g) {
+    if (g.M <= 0 || g.N <= 0 || g.K <= 0) return GBGPU_OK;
+    g.set = true;
+    if (c.form != GBGPU_FORM_PLAIN) return gemm_args(c, g);
+    uint32_t* D = g.D;
+    const int64_t ldd = g.ldd;
+    const int32_t* rows = g.d_rows;
+    uint32_t* T = c.alloc<uint32_t>((size_t)g.M * g.N);
+    if (!T) return GBGPU_ENOMEM;
+    g.D = T;
+    g.ldd = g.N;
+    g.d_rows = nullptr;
+    BL_CHECK(gemm_args(c, g));
+    if (rows)
+        BL_LAUNCH(k_scatter_rows_dense<<<grid_of((int64_t)g.M * g.N), 256, 0, c.s>>>(
+            g.M, rows, g.N, T, g.N, D, ldd));
+    else
+        BL_CUDA(cudaMemcpy2DAsync(D, ldd * 4, T, (size_t)g.N * 4, (size_t)g.N * 4, g.M,
+                                  cudaMemcpyDeviceToDevice, c.s));
+    return GBGPU_OK;
+}
+
+// batch of `batch` products D_z <- -A_z B_z (element strides sA, sB, sD)
+static int gemm_set_batched(Ctx& c, uint32_t* D, int64_t ldd, int64_t sD, const uint32_t* A,
                         int64_t lda, int64_t sA, const uint32_t* B, int64_t ldb, int64_t sB,
                         int32_t M, int32_t N, int32_t K, int32_t batch) {
     TcGemmArgs g{c.p, M, N, K, A, lda, B, ldb, D, ldd};
+    g.set = true;
     g.batch = batch;
     g.sA = sA;
     g.sB = sB;
@@ -1045,12 +1070,11 @@ static int neg_inverse_big(Ctx& c, const F& f, const uint32_t* src, int64_t lds,
         const int32_t items = n_blocks * (NB / (2 * sz));
         const int64_t istep = (int64_t)2 * sz * (NB + 1);
         const int64_t half = (int64_t)sz * (NB + 1);
-        BL_CUDA(cudaMemsetAsync(T, 0, sizeof(uint32_t) * (size_t)items * sz * sz, c.s));
-        // T = B C^-1 = 0 - B (-C^-1)
-        BL_CHECK(gemm_batched(c, T, sz, (int64_t)sz * sz, U + sz, NB, istep, out + half, NB, istep,
+        // T = B C^-1 = -(B (-C^-1))
+        BL_CHECK(gemm_set_batched(c, T, sz, (int64_t)sz * sz, U + sz, NB, istep, out + half, NB, istep,
                               sz, sz, sz, items));
-        // top right of -U^-1 = A^-1 B C^-1 = 0 - (-A^-1) T
-        BL_CHECK(gemm_batched(c, out + sz, NB, istep, out, NB, istep, T, sz, (int64_t)sz * sz, sz,
+        // top right of -U^-1 = A^-1 B C^-1 = -((-A^-1) T)
+        BL_CHECK(gemm_set_batched(c, out + sz, NB, istep, out, NB, istep, T, sz, (int64_t)sz * sz, sz,
                               sz, sz, items));
     }
     return GBGPU_OK;
@@ -1113,9 +1137,10 @@ static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t*
         const int32_t first_col = pc[b * NB] & ~3;
         BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)rows * kb), 256, 0, c.s>>>(
             rows, kb, M, ld, d_pc + b * NB, G, NB, t_rows));
-        BL_CUDA(cudaMemsetAsync(X, 0, sizeof(uint32_t) * (size_t)rows * NB, c.s));
-        // X = G * (U_kk)^-1 = 0 - G * (-(U_kk)^-1)
-        BL_CHECK(gemm(c, X, NB, G, NB, Ninv + (size_t)b * bstride, NB, rows, kb, kb));
+        // X = G * (U_kk)^-1 = -(G * (-(U_kk)^-1))
+        TcGemmArgs x{c.p, rows, kb, kb, G, NB, Ninv + (size_t)b * bstride, NB, X, NB};
+        x.set = true;
+        BL_CHECK(gemm_args(c, x));
         // T[:, first_col:] -= X * U_k[:, first_col:]
         TcGemmArgs g{c.p, rows, ncols - first_col, kb, X, NB, M + first_col, ld, M + first_col, ld};
         g.b_rows = u_rows + b * NB;
@@ -1165,12 +1190,11 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
         uint32_t* P = c.alloc<uint32_t>((size_t)ncl * ld);
         const int32_t nbk = (ncl + NB - 1) / NB;
         uint32_t* Ninv = c.alloc<uint32_t>((size_t)nbk * bstride);
-        uint32_t* X = c.alloc<uint32_t>((size_t)t * NB);
         int32_t* act = c.alloc<int32_t>(nbk);
         int32_t* span = c.alloc<int32_t>(nbk);
         const int32_t ngrp = (ncl + 127) / 128;
         int2* brange = c.alloc<int2>(ngrp);
-        if (!P || !Ninv || !X || !act || !span || !brange) return GBGPU_ENOMEM;
+        if (!P || !Ninv || !act || !span || !brange) return GBGPU_ENOMEM;
         // active rows of each block (rows sorted by lead), the last left
         // column the known pivots of each block touch, and the right columns
         // every 128 known pivots reach
@@ -1201,15 +1225,14 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
             const int32_t c0 = k * NB, kb = std::min(NB, ncl - c0), c1 = c0 + kb;
             const int32_t rows = h_act[k];
             if (rows <= 0) continue;
-            BL_CUDA(cudaMemsetAsync(X, 0, sizeof(uint32_t) * (size_t)rows * NB, s));
             // X_k = W[:, block] A_kk^-1
-            BL_CHECK(gemm(c, X, NB, W + c0, ld, Ninv + (size_t)k * bstride, NB, rows, kb, kb));
-            BL_CUDA(cudaMemcpy2DAsync(W + c0, ld * 4, X, NB * 4, (size_t)kb * 4, rows,
-                                      cudaMemcpyDeviceToDevice, s));
+            TcGemmArgs x{c.p, rows, kb, kb, W + c0, ld, Ninv + (size_t)k * bstride, NB, W + c0, ld};
+            BL_CHECK(gemm_set_in_place(c, x));
             // W[:, c1:e) -= X_k A[block rows, c1:e)
             const int32_t e = std::min(ncl, h_span[k] + 1);
             if (e > c1)
-                BL_CHECK(gemm(c, W + c1, ld, X, NB, P + (size_t)c0 * ld + c1, ld, rows, e - c1, kb));
+                BL_CHECK(gemm(c, W + c1, ld, W + c0, ld, P + (size_t)c0 * ld + c1, ld, rows, e - c1,
+                              kb));
         }
         // (b) D' = D - X B: one GEMM over the whole left block; the tile flags of
         //     the GEMM skip the zero tiles of the staircase X and of B
@@ -1536,8 +1559,7 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
         uint32_t* Ublk = c.alloc<uint32_t>((size_t)nb * NB * NB);
         uint32_t* Ninv = c.alloc<uint32_t>((size_t)nb * bstride);
         uint32_t* G = c.alloc<uint32_t>((size_t)NB * std::max(r, 1));
-        uint32_t* Y = c.alloc<uint32_t>((size_t)NB * ld);
-        if (!Ublk || !Ninv || !G || !Y) return GBGPU_ENOMEM;
+        if (!Ublk || !Ninv || !G) return GBGPU_ENOMEM;
         for (int b = 0; b < nb; ++b) {
             const int kb = std::min(NB, r - b * NB);
             BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * kb), 256, 0, s>>>(
@@ -1560,14 +1582,12 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                 g.d_rows = rows_k;
                 BL_CHECK(gemm_args(c, g));
             }
-            // E_k = (E_k[:, pc(k)])^-1 E_k, as Y = 0 - (-(U_kk)^-1) E_k, E_k = Y
-            BL_CUDA(cudaMemset2DAsync(Y + c0, ld * 4, 0, (size_t)(ncr - c0) * 4, kb, s));
-            TcGemmArgs g{c.p, kb, ncr - c0, kb, Ninv + (size_t)b * bstride, NB, Dp + c0, ld, Y + c0,
+            // E_k = (E_k[:, pc(k)])^-1 E_k = -((-(U_kk)^-1) E_k), in place
+            TcGemmArgs g{c.p, kb, ncr - c0, kb, Ninv + (size_t)b * bstride, NB, Dp + c0, ld, Dp + c0,
                          ld};
             g.b_rows = rows_k;
-            BL_CHECK(gemm_args(c, g));
-            BL_LAUNCH(k_scatter_rows_dense<<<grid_of((int64_t)kb * (ncr - c0)), 256, 0, s>>>(
-                kb, rows_k, ncr - c0, Y + c0, ld, Dp + c0, ld));
+            g.d_rows = rows_k;
+            BL_CHECK(gemm_set_in_place(c, g));
             if (so) BL_CHECK(send_block(b, kb));
         }
         if (blk_ev) cudaEventDestroy(blk_ev);

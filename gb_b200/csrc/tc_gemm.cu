@@ -211,6 +211,7 @@ struct TcParams {
     uint32_t p, pneg_inv;
     uint32_t mu;     // floor(2^32 / p)
     uint32_t cw[7];  // 2^(8w) R mod p
+    int32_t set;     // D <- -A B: D is not read
     int32_t* err;
     long long budget;
 };
@@ -475,7 +476,7 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
             const uint8_t *fa, *fb;
             flag_ptrs(z, mt, nt, fa, fb);
             const int n_it = live_steps(fa, fb);
-            if (n_it == 0) continue;  // A B is zero on this tile: D stays as it is
+            if (n_it == 0 && !prm.set) continue;  // A B is zero here: D stays as it is
             const int npanels = (n_it + C::PANEL_KB - 1) / C::PANEL_KB;
             const int m0 = mt * C::BM, n0 = nt * C::BN;
             const int gm = m0 + row;
@@ -529,15 +530,30 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                     }
                 }
             };
+            if (n_it == 0) {  // D <- 0
+                for (int r = 0; r < 32; ++r) {
+                    const int32_t rr = __shfl_sync(0xffffffffu, ri, r);
+                    for (int j = lane; j < C::COLS; j += 32)
+                        if (rr >= 0 && n0 + cbeg + j < prm.N)
+                            Dz[(size_t)rr * prm.ldd + n0 + cbeg + j] = 0u;
+                }
+                continue;
+            }
             for (int panel = 0; panel < npanels; ++panel, ++pc) {
                 const int ab = pc % C::ACC_BUFS, au = pc / C::ACC_BUFS;
                 const uint32_t acc_base = (uint32_t)(ab * C::NW * C::BN);
                 // (this lane wrote the same addresses in the previous panel, if any)
                 constexpr int PRE = NB > 1 ? 2 : 1;  // blocks in flight
+                const bool fresh = prm.set && panel == 0;  // nothing to read
                 uint32_t dv[PRE][32];
-                if (rows_here) {
 #pragma unroll
-                    for (int b = 0; b < PRE; ++b) load_d(cbeg + 32 * b, dv[b]);
+                for (int b = 0; b < PRE; ++b) {
+                    if (rows_here && !fresh) {
+                        load_d(cbeg + 32 * b, dv[b]);
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < 32; ++r) dv[b][r] = 0u;
+                    }
                 }
                 bool ok = true;
                 if (lane == 0) ok = !*abort_flag && mbar_wait(tfull_bar(ab), au & 1, prm.budget);
@@ -681,7 +697,7 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                                 if (r < rows_q && col_ok) *o = v[r];
                         }
                     }
-                    if (b + PRE < NB) load_d(cbeg + 32 * (b + PRE), d);
+                    if (b + PRE < NB && !fresh) load_d(cbeg + 32 * (b + PRE), d);
                     __syncwarp();
                 }
             }
@@ -868,6 +884,7 @@ __global__ void __launch_bounds__(256) k_split_ab(const SplitArgs a) {
 struct RowLists {
     const int32_t *a, *b, *d;
     int64_t sa, sb, sd;
+    int32_t set;  // D is not read
 };
 
 // ---------------------------------------------------------------------------
@@ -948,7 +965,7 @@ k_plain_submul(const uint32_t* __restrict__ A, int64_t lda, const uint32_t* __re
             if (n >= N) continue;
             const uint64_t h = (hi[i][j] % f.p) << 16;
             const uint32_t v = (uint32_t)((lo[i][j] % f.p + h % f.p) % f.p);
-            const uint32_t d = D[(size_t)rd * ldd + n];
+            const uint32_t d = rl.set ? 0u : D[(size_t)rd * ldd + n];
             D[(size_t)rd * ldd + n] = d >= v ? d - v : d + (f.p - v);
         }
     }
@@ -1108,6 +1125,7 @@ static int tc_run(const TcGemmArgs& g, uint8_t* planes, cudaStream_t s, int32_t*
         return GBGPU_ECUDA;
     }
     prm.batch = nb;
+    prm.set = g.set;
     const int64_t tiles = (int64_t)(Np / Cfg::BN) * (Mp / Cfg::BM) * nb;
     const dim3 grid((unsigned)std::max<int64_t>(
         1, std::min<int64_t>(tiles, (int64_t)num_sms())));
@@ -1189,7 +1207,7 @@ int plain_submul(const TcGemmArgs& g, cudaStream_t s, long long* launches) {
     dim3 grid((g.N + 63) / 64, (g.M + 63) / 64, g.batch);
     FieldMont f{};
     f.p = g.p;
-    const RowLists rl{g.a_rows, g.b_rows, g.d_rows, g.sAr, g.sBr, g.sDr};
+    const RowLists rl{g.a_rows, g.b_rows, g.d_rows, g.sAr, g.sBr, g.sDr, g.set};
     k_plain_submul<<<grid, 256, 0, s>>>(g.A, g.lda, g.B, g.ldb, g.D, g.ldd, g.M, g.N, g.K, g.sA,
                                         g.sB, g.sD, rl, f);
     ++*launches;

@@ -36,6 +36,10 @@ struct TcGemmArgs {
     // memory there is never read; between the two columns widened to
     // 64-column boundaries every entry must be valid.
     const int2* b_nrange = nullptr;
+    // D <- -A B mod p instead of D <- (D - A B) mod p: D is not read.  On the
+    // tensor cores D may then be A or B itself (their limb planes are cut before
+    // the product runs).
+    bool set = false;
 };
 
 // Optional per-thread profiling of the tensor-core GEMM launches: CUDA events
