@@ -198,6 +198,48 @@ static void kit_return(int device, StreamKit& k) {
     kit_destroy(k);
 }
 
+// mapped pages (internal.h): pinning one takes longer than a round of the echelon
+constexpr int kMaxPages = 8;
+static std::vector<MappedPage>& pages_of(int device) {
+    static auto* pages = new std::map<int, std::vector<MappedPage>>();
+    return (*pages)[device];
+}
+cudaError_t mapped_page_take(MappedPage* out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(g_kit_mu);
+        auto& v = pages_of(dev);
+        if (!v.empty()) {
+            *out = v.back();
+            v.pop_back();
+            return cudaSuccess;
+        }
+    }
+    MappedPage p;
+    p.device = dev;
+    e = cudaHostAlloc(&p.host, kMappedPageBytes, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&p.dev, p.host, 0);
+    if (e == cudaSuccess) *out = p;
+    else if (p.host) cudaFreeHost(p.host);
+    return e;
+}
+void mapped_page_return(MappedPage& p) {
+    if (!p.host) return;
+    {
+        std::lock_guard<std::mutex> lock(g_kit_mu);
+        auto& v = pages_of(p.device);
+        if ((int)v.size() < kMaxPages) {
+            v.push_back(p);
+            p = MappedPage{};
+            return;
+        }
+    }
+    cudaFreeHost(p.host);
+    p = MappedPage{};
+}
+
 struct Plan {
     int device = 0;
     DeviceInfo dev{};

@@ -32,8 +32,6 @@
 #include <cuda_runtime.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
-#include <cub/device/device_select.cuh>
-#include <cub/iterator/counting_input_iterator.cuh>
 
 #include <algorithm>
 #include <climits>
@@ -49,6 +47,7 @@
 #include "field.cuh"
 #include "internal.h"
 #include "kernels.h"
+#include "rounds.cuh"
 #include "tc_gemm.h"
 #include "tiny.cuh"
 
@@ -396,28 +395,6 @@ __global__ void k_gather_cols(int32_t rows, int32_t n, const uint32_t* __restric
     }
 }
 
-// dst row i = src row rows[i] (n columns; a negative index: a zero row)
-__global__ void k_gather_rows_dense(int32_t nrows, const int32_t* __restrict__ rows, int32_t n,
-                                    const uint32_t* __restrict__ src, int64_t lds, uint32_t* dst,
-                                    int64_t ldd) {
-    GB_WARP_ROWS(nrows, n) {
-        const int32_t r = rows[i];
-        const uint32_t* s = r >= 0 ? src + (size_t)r * lds : nullptr;
-        uint32_t* o = dst + (size_t)i * ldd;
-        for (int j0 = jb + lane; j0 < je; j0 += 128) {
-            uint32_t v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int jj = j0 + 32 * u;
-                v[u] = (s && jj < je) ? s[jj] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (j0 + 32 * u < je) o[j0 + 32 * u] = v[u];
-        }
-    }
-}
-
 // dst row rows[i] = src row i
 __global__ void k_scatter_rows_dense(int32_t nrows, const int32_t* __restrict__ rows, int32_t n,
                                      const uint32_t* __restrict__ src, int64_t lds,
@@ -472,119 +449,6 @@ __global__ void k_row_leads(int32_t rows, const int32_t* __restrict__ list, int3
     }
 }
 
-// columns with flag set, ascending, via a precomputed exclusive scan
-__global__ void k_compact_cols(int32_t n, const int32_t* __restrict__ flag,
-                               const int32_t* __restrict__ pos, int32_t* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        if (flag[i]) out[pos[i]] = i;
-}
-
-
-// ---------------------------------------------------------------------------
-// panel echelon
-
-// the round's new pivots: count = last exclusive-scan position + last flag,
-// and their rows in ascending pivot-column order
-__global__ void k_new_pivots(int32_t ncr, const int32_t* __restrict__ wflag,
-                             const int32_t* __restrict__ wpos, const int32_t* __restrict__ pc,
-                             const int32_t* __restrict__ piv_of_col, int32_t* n_new,
-                             int32_t* prow) {
-    const int32_t n = ncr > 0 ? wpos[ncr - 1] + wflag[ncr - 1] : 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        prow[i] = piv_of_col[pc[i]];
-    if (blockIdx.x == 0 && threadIdx.x == 0) *n_new = n;
-}
-
-// pending flags for an ordered compaction (rows in ascending order)
-__global__ void k_pending_flags(int32_t t, const int32_t* __restrict__ lead,
-                                const uint8_t* __restrict__ is_piv, uint8_t* flag) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < t; r += gridDim.x * blockDim.x)
-        flag[r] = (lead[r] >= 0 && !is_piv[r]) ? 1 : 0;
-}
-
-// chunk slot key of every pending row: its panel's slot, n_dirty for rows of
-// panels not factorized this round
-__global__ void k_panel_keys(int32_t n, const int32_t* __restrict__ pend,
-                             const int32_t* __restrict__ lead, const int32_t* __restrict__ dslot,
-                             int32_t n_dirty, int32_t* key) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t d = dslot[lead[pend[i]] / KB];
-        key[i] = d >= 0 ? d : n_dirty;
-    }
-}
-
-// rows sorted by (chunk slot, row): the first PR rows of every selected panel
-// fill its chunk in ascending row order; cursor = the panel's pending rows
-__global__ void k_bucket_sorted(int32_t n, const int32_t* __restrict__ key,
-                                const int32_t* __restrict__ rows, int32_t n_dirty,
-                                int32_t* chunk_rows, int32_t* cursor) {
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-        const int32_t d = key[q];
-        if (d >= n_dirty) continue;
-        int lo = 0, hi = q;  // first position of this run
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (key[mid] < d) lo = mid + 1;
-            else hi = mid;
-        }
-        const int slot = q - lo;
-        if (slot < PR) chunk_rows[(size_t)d * PR + slot] = rows[q];
-        if (q == n - 1 || key[q + 1] != d) cursor[d] = q - lo + 1;
-    }
-}
-
-// rows per lead column and per 128-column panel; a panel is "dirty" when
-// two pending rows share a lead in it
-__global__ void k_lead_hist(const int32_t* __restrict__ n_dev, const int32_t* __restrict__ pend,
-                            const int32_t* __restrict__ lead, int32_t* hist, int32_t* pcnt) {
-    const int32_t n = *n_dev;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t l = lead[pend[i]];
-        atomicAdd(&hist[l], 1);
-        atomicAdd(&pcnt[l / KB], 1);
-    }
-}
-__global__ void k_dirty_panels(const int32_t* __restrict__ n_dev, const int32_t* __restrict__ pend,
-                               const int32_t* __restrict__ lead, const int32_t* __restrict__ hist,
-                               int32_t* pdirty) {
-    const int32_t n = *n_dev;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t l = lead[pend[i]];
-        if (hist[l] > 1) pdirty[l / KB] = 1;
-    }
-}
-
-// rows of collision-free panels have leads of their own: they are pivots
-__global__ void k_claim_clean(const int32_t* __restrict__ n_dev, const int32_t* __restrict__ pend,
-                              const int32_t* __restrict__ lead, const int32_t* __restrict__ pdirty,
-                              int32_t* piv_of_col, uint8_t* is_piv, int32_t* wflag,
-                              int32_t* n_clean) {
-    const int32_t n = *n_dev;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t r = pend[i], l = lead[r];
-        if (!pdirty[l / KB]) {
-            piv_of_col[l] = r;
-            is_piv[r] = 1;
-            wflag[l] = 1;
-            *n_clean = 1;
-        }
-    }
-}
-
-// the factorized pivots of every chunk
-__global__ void k_register_chunks(const int32_t* __restrict__ n_piv,
-                                  const int32_t* __restrict__ piv_rows,
-                                  const int32_t* __restrict__ piv_col, int32_t* piv_of_col,
-                                  uint8_t* is_piv, int32_t* wflag) {
-    const int d = blockIdx.x;
-    for (int k = threadIdx.x; k < n_piv[d]; k += blockDim.x) {
-        const int32_t row = piv_rows[d * KB + k], col = piv_col[d * KB + k];
-        piv_of_col[col] = row;
-        is_piv[row] = 1;
-        wflag[col] = 1;
-    }
-}
-
 // scale row rows[i] by the inverse of its entry at column cols[i] (one CTA
 // per row; NORM_U independent loads per thread and pass)
 constexpr int NORM_U = 8;
@@ -622,9 +486,9 @@ __global__ void k_normalize_at(const int32_t* __restrict__ n_dev, const int32_t*
 
 // Reduced row echelon form of one panel (the 128 columns of panel dpanel[d], on
 // the n <= PR rows chunk_rows[d PR + i] of Dp) in the shared memory of one
-// cluster (tiny.cuh).  Its pivots, in ascending column order: piv_rows[d KB + k]
-// the row of Dp, piv_col[d KB + k] the column, n_piv[d] their number; and the
-// transformation: the reduced pivot row k (unit columns at the panel's pivots)
+// cluster (tiny.cuh).  Its pivots are registered (piv_of_col, is_piv, wflag);
+// piv_rows[d KB + k]: their rows in ascending column order, n_piv[d] of them; and
+// the transformation: the reduced pivot row k (unit columns at the panel's pivots)
 // is sum_j F[d][k][j] (old pivot row j).  Rows of the chunk that are no pivots
 // have their panel part in the span of the pivots', so the round's elimination
 // clears them.
@@ -640,7 +504,8 @@ template <class F>
 __global__ void __launch_bounds__(kTinyThreads, 1)
 k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __restrict__ chunk_rows,
                const int32_t* __restrict__ dpanel, const int32_t* __restrict__ cursor,
-               int32_t max_rows, int32_t ncr, uint32_t* F_b, int32_t* piv_rows_b, int32_t* piv_col_b, int32_t* n_piv_b, F f) {
+               int32_t max_rows, int32_t ncr, uint32_t* F_b, int32_t* piv_rows_b, int32_t* n_piv_b,
+               int32_t* piv_of_col, uint8_t* is_piv, int32_t* wflag, F f) {
     extern __shared__ __align__(16) uint32_t pf_smem[];
     const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
     const int d = blockIdx.x / CL, tid = threadIdx.x;
@@ -668,8 +533,11 @@ k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __res
     if (rk == 0) {
         if (tid == 0) n_piv_b[d] = np;
         for (int k = tid; k < np; k += kTinyThreads) {
-            piv_rows_b[d * KB + k] = rows[prow[s_col[k]]];
-            piv_col_b[d * KB + k] = pj + s_col[k];
+            const int32_t row = rows[prow[s_col[k]]], col = pj + s_col[k];
+            piv_rows_b[d * KB + k] = row;
+            piv_of_col[col] = row;
+            is_piv[row] = 1;
+            wflag[col] = 1;
         }
     }
     uint32_t* Fo = F_b + (size_t)d * KB * KB;
@@ -1093,9 +961,43 @@ __global__ void k_offs_write(int32_t n, const int64_t* __restrict__ loc, int64_t
         offs[k] = base + loc[k];
 }
 
+// Mapped host memory for one user at a time, from the pool of internal.h.
+struct InfoPage {
+    MappedPage p;
+    cudaStream_t s;
+    void *host = nullptr, *dev = nullptr;
+    InfoPage(cudaStream_t s_, size_t bytes) : s(s_) {
+        if (bytes <= kMappedPageBytes && mapped_page_take(&p) == cudaSuccess) {
+            host = p.host;
+            dev = p.dev;
+        } else {
+            set_error("mapped host page allocation failed");
+        }
+    }
+    ~InfoPage() {
+        cudaStreamSynchronize(s);  // an early return may leave a writer running
+        mapped_page_return(p);
+    }
+};
+
+// the columns of pivots 0, KB, 2 KB, ... (the last k_round_finish's)
+static int first_columns(Ctx& c, const volatile RoundInfo* info, const int32_t* d_pc, int32_t n,
+                         std::vector<int32_t>* out) {
+    const int32_t nb = (n + KB - 1) / KB;
+    out->resize((size_t)nb);
+    if (nb <= kInfoFirst) {
+        for (int32_t q = 0; q < nb; ++q) (*out)[q] = info->first[q];
+        return GBGPU_OK;
+    }
+    BL_CUDA(cudaMemcpy2DAsync(out->data(), 4, d_pc, 4 * KB, 4, nb, cudaMemcpyDeviceToHost, c.s));
+    BL_CUDA(cudaStreamSynchronize(c.s));
+    return GBGPU_OK;
+}
+
 // Rows t_rows[0 .. rows) of M (leading dimension ld, ncols columns) are
 // reduced by the pivot rows u_rows[0 .. n_p) of M (sorted by lead, monic,
-// zero left of their leads, pivot columns pc ascending):
+// zero left of their leads, pivot columns d_pc ascending, h_first[q] = that of
+// pivot q KB):
 //   T <- T - T[:, pc] (U[:, pc])^-1 U,
 // after which every T row is zero at every pivot column.  Blocks of NB
 // pivots, left to right; the rows are read and written in place through the
@@ -1103,12 +1005,12 @@ __global__ void k_offs_write(int32_t n, const int64_t* __restrict__ loc, int64_t
 template <class F>
 static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t* t_rows,
                      int32_t rows, int32_t ncols, const int32_t* u_rows, int32_t n_p,
-                     const int32_t* d_pc, const std::vector<int32_t>& pc, bool unit) {
+                     const int32_t* d_pc, const std::vector<int32_t>& h_first, bool unit) {
     if (rows <= 0 || n_p <= 0) return GBGPU_OK;
     if (unit) {  // U[:, pc] is the identity (at most KB pivots): T -= T[:, pc] U
         uint32_t* G = c.alloc<uint32_t>((size_t)rows * KB);
         if (!G) return GBGPU_ENOMEM;
-        const int32_t first_col = pc[0] & ~3;
+        const int32_t first_col = h_first[0] & ~3;
         BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)rows * n_p), 256, 0, c.s>>>(rows, n_p, M, ld, d_pc,
                                                                               G, KB, t_rows));
         TcGemmArgs g{c.p, rows, ncols - first_col, n_p, G, KB, M + first_col, ld, M + first_col, ld};
@@ -1134,7 +1036,7 @@ static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t*
         const int kb = std::min(NB, n_p - b * NB);
         // from the block's first pivot column, or up to three left of it for the
         // GEMM's 16-byte accesses (the pivot rows are zero there)
-        const int32_t first_col = pc[b * NB] & ~3;
+        const int32_t first_col = h_first[b * (NB / KB)] & ~3;
         BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)rows * kb), 256, 0, c.s>>>(
             rows, kb, M, ld, d_pc + b * NB, G, NB, t_rows));
         // X = G * (U_kk)^-1 = -(G * (-(U_kk)^-1))
@@ -1272,115 +1174,60 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
     int32_t* lead = c.alloc<int32_t>(t);
     uint8_t* is_piv = c.alloc<uint8_t>(t);
     int32_t* piv_of_col = out->piv_of_col;  // [ncr], -1 if none
-    int32_t* wflag = c.alloc<int32_t>(ncr);
-    int32_t* wpos = c.alloc<int32_t>(ncr);
-    int32_t* pend = c.alloc<int32_t>(t);
     int32_t* counters = c.alloc<int32_t>(8);
-    int32_t* pc = c.alloc<int32_t>(ncr);      // pivot columns
-    int32_t* prow = c.alloc<int32_t>(ncr);    // their rows
-    int32_t* hist = c.alloc<int32_t>(ncr);
-    int32_t* pcnt = c.alloc<int32_t>(npan);
-    int32_t* pdirty = c.alloc<int32_t>(npan);
-    int32_t* dslot = c.alloc<int32_t>(npan);
-    int32_t* dpanel = c.alloc<int32_t>(npan);
-    if (!lead || !is_piv || !wflag || !wpos || !pend || !counters || !pc || !prow || !hist ||
-        !pcnt || !pdirty || !dslot || !dpanel)
+    // every dirty panel is factorized in the round that finds it (batch <= 4096)
+    const int32_t max_dirty = std::max<int32_t>(1, std::min<int32_t>(npan, 4096));
+    RoundState rs{};
+    rs.t = t;
+    rs.ncr = ncr;
+    rs.npan = npan;
+    rs.max_dirty = max_dirty;
+    rs.lead = lead;
+    rs.is_piv = is_piv;
+    rs.piv_of_col = piv_of_col;
+    rs.wflag = c.alloc<int32_t>(ncr);
+    rs.hist = c.alloc<int32_t>(ncr);
+    rs.pdirty = c.alloc<int32_t>(npan);
+    rs.dslot = c.alloc<int32_t>(npan);
+    rs.dpanel = c.alloc<int32_t>(max_dirty);
+    rs.cursor = c.alloc<int32_t>(max_dirty);
+    rs.chunk_rows = c.alloc<int32_t>((size_t)max_dirty * PR);
+    rs.per_warp = c.alloc<int32_t>((size_t)RD_WARPS * max_dirty);
+    rs.pc = c.alloc<int32_t>(ncr);    // pivot columns
+    rs.prow = c.alloc<int32_t>(ncr);  // their rows
+    rs.pend = c.alloc<int32_t>(t);
+    rs.n_new = counters;
+    int32_t *pc = rs.pc, *prow = rs.prow, *pend = rs.pend;
+    uint32_t* panF = c.alloc<uint32_t>((size_t)max_dirty * KB * KB);
+    int32_t* n_piv = c.alloc<int32_t>(max_dirty);
+    int32_t* piv_rows = c.alloc<int32_t>((size_t)max_dirty * KB);
+    if (!lead || !is_piv || !counters || !rs.wflag || !rs.hist || !rs.pdirty || !rs.dslot ||
+        !rs.dpanel || !rs.cursor || !rs.chunk_rows || !rs.per_warp || !pc || !prow || !pend ||
+        !panF || !n_piv || !piv_rows)
         return GBGPU_ENOMEM;
-    size_t scan_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, wflag, wpos, ncr, s);
-    void* scan_tmp = c.alloc<uint8_t>(scan_bytes);
-    if (!scan_tmp) return GBGPU_ENOMEM;
+    // the counts the host sizes launches from
+    InfoPage page(s, sizeof(RoundInfo));
+    const volatile RoundInfo* info = (const volatile RoundInfo*)page.host;
+    rs.info = (RoundInfo*)page.dev;
+    if (!info) return GBGPU_ENOMEM;
     BL_LAUNCH(k_fill_i32<<<grid_of(ncr), 256, 0, s>>>(piv_of_col, ncr, -1));
     if (t > 0 && ncr > 0) {
         BL_CUDA(cudaMemsetAsync(is_piv, 0, t, s));
         BL_LAUNCH(k_row_leads<<<grid_of((int64_t)t * 32), 256, 0, s>>>(t, nullptr, ncr, Dp, ld, lead));
     }
-    // every dirty panel is factorized in the round that finds it (batch <= 4096)
-    const int32_t max_dirty = std::max<int32_t>(1, std::min<int32_t>(npan, 4096));
-    int32_t* chunk_rows = c.alloc<int32_t>((size_t)max_dirty * PR);
-    int32_t* cursor = c.alloc<int32_t>(max_dirty);
-    uint32_t* panF = c.alloc<uint32_t>((size_t)max_dirty * KB * KB);
-    int32_t* piv_colb = c.alloc<int32_t>((size_t)max_dirty * KB);
-    int32_t* n_piv = c.alloc<int32_t>(max_dirty);
-    int32_t* piv_rows = c.alloc<int32_t>((size_t)max_dirty * KB);
-    // ordered compaction of the pending rows and the stable (panel, row) sort
-    // that fills the chunks: the same rows, in the same order, on every run
-    uint8_t* pflag = c.alloc<uint8_t>(t);
-    int32_t* pkey = c.alloc<int32_t>(t);
-    int32_t* pkey_sorted = c.alloc<int32_t>(t);
-    int32_t* prow_sorted = c.alloc<int32_t>(t);
-    size_t sel_bytes = 0, sort_bytes = 0;
-    cub::CountingInputIterator<int32_t> row_ids(0);
-    cub::DeviceSelect::Flagged(nullptr, sel_bytes, row_ids, pflag, pend, counters, t, s);
-    cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, pkey, pkey_sorted, pend, prow_sorted, t,
-                                    0, 32, s);
-    void* sel_tmp = c.alloc<uint8_t>(sel_bytes);
-    void* sort_tmp = c.alloc<uint8_t>(sort_bytes);
-    if (!chunk_rows || !cursor || !panF || !piv_colb || !n_piv || !piv_rows || !pflag || !pkey || !pkey_sorted || !prow_sorted || !sel_tmp || !sort_tmp)
-        return GBGPU_ENOMEM;
-    // pending rows (nonzero, not pivots) into pend[0 .. *count), ascending
-    auto collect_pending = [&](int32_t* count) -> int {
-        BL_LAUNCH(k_pending_flags<<<grid_of(t), 256, 0, s>>>(t, lead, is_piv, pflag));
-        size_t bytes = sel_bytes;
-        BL_CUDA(cub::DeviceSelect::Flagged(sel_tmp, bytes, row_ids, pflag, pend, count, t, s));
-        ++c.launches;
-        return GBGPU_OK;
-    };
     int rounds = 0;
     bool first = true;
     while (t > 0 && ncr > 0) {
-        // pending rows, lead histogram, clean panels claimed, dirty panels
-        // flagged -- all sized on the device; one host round trip reads the
-        // count and the dirty flags
-        int32_t n_pend = 0;
-        BL_CUDA(cudaMemsetAsync(counters, 0, 8 * sizeof(int32_t), s));
-        BL_CHECK(collect_pending(counters));
-        BL_CUDA(cudaMemsetAsync(hist, 0, sizeof(int32_t) * ncr, s));
-        BL_CUDA(cudaMemsetAsync(pcnt, 0, sizeof(int32_t) * npan, s));
-        BL_CUDA(cudaMemsetAsync(pdirty, 0, sizeof(int32_t) * npan, s));
-        BL_CUDA(cudaMemsetAsync(wflag, 0, sizeof(int32_t) * ncr, s));
-        BL_LAUNCH(k_lead_hist<<<grid_of(t), 256, 0, s>>>(counters, pend, lead, hist, pcnt));
-        BL_LAUNCH(k_dirty_panels<<<grid_of(t), 256, 0, s>>>(counters, pend, lead, hist, pdirty));
-        BL_LAUNCH(k_claim_clean<<<grid_of(t), 256, 0, s>>>(counters, pend, lead, pdirty,
-                                                            piv_of_col, is_piv, wflag,
-                                                            counters + 4));
-        // dirty panels, leftmost first, at most max_dirty of them this round
-        std::vector<int32_t> h_dirty(npan);
-        BL_CUDA(cudaMemcpyAsync(&n_pend, counters, 4, cudaMemcpyDeviceToHost, s));
-        BL_CUDA(cudaMemcpyAsync(h_dirty.data(), pdirty, sizeof(int32_t) * npan,
-                                cudaMemcpyDeviceToHost, s));
+        // pending rows, clean panels claimed, the dirty panels and their chunks
+        BL_LAUNCH(k_round_plan<<<1, RD_THREADS, 0, s>>>(rs, KB, PR));
         BL_CUDA(cudaStreamSynchronize(s));
+        const int32_t n_pend = info->n_pend, n_dirty = info->n_dirty, n_clean = info->n_clean;
         if (first) out->dense_rows = n_pend;
         first = false;
         if (n_pend == 0) break;
         ++rounds;
-        std::vector<int32_t> h_dpanel, h_dslot(npan, -1);
-        for (int32_t p = 0; p < npan && (int32_t)h_dpanel.size() < max_dirty; ++p) {
-            if (h_dirty[p]) {
-                h_dslot[p] = (int32_t)h_dpanel.size();
-                h_dpanel.push_back(p);
-            }
-        }
-        const int32_t n_dirty = (int32_t)h_dpanel.size();
         if (n_dirty > 0) {
-            const int32_t j0 = h_dpanel[0] * KB, width = ncr - j0;
-            BL_CUDA(cudaMemcpyAsync(dslot, h_dslot.data(), sizeof(int32_t) * npan,
-                                    cudaMemcpyHostToDevice, s));
-            BL_CUDA(cudaMemcpyAsync(dpanel, h_dpanel.data(), sizeof(int32_t) * n_dirty,
-                                    cudaMemcpyHostToDevice, s));
-            BL_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * n_dirty, s));
-            BL_LAUNCH(k_panel_keys<<<grid_of(n_pend), 256, 0, s>>>(n_pend, pend, lead, dslot,
-                                                                    n_dirty, pkey));
-            {
-                int bits = 1;
-                while ((1 << bits) <= n_dirty) ++bits;
-                size_t bytes = sort_bytes;
-                BL_CUDA(cub::DeviceRadixSort::SortPairs(sort_tmp, bytes, pkey, pkey_sorted, pend,
-                                                        prow_sorted, n_pend, 0, bits, s));
-                ++c.launches;
-            }
-            BL_LAUNCH(k_bucket_sorted<<<grid_of(n_pend), 256, 0, s>>>(
-                n_pend, pkey_sorted, prow_sorted, n_dirty, chunk_rows, cursor));
+            const int32_t j0 = info->first_panel * KB, width = ncr - j0;
             {
                 // CTAs per panel: as many as leave every panel its own SMs
                 int cl = kTinyMaxCluster;
@@ -1389,8 +1236,8 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                 int32_t nc_ = ncr, rows_ = cl == 1 ? KB : PR;
                 int64_t ld_ = ld;
                 F fv = f;
-                void* args[] = {&Dp, &ld_, &chunk_rows, &dpanel, &cursor, &rows_, &nc_,
-                                &panF, &piv_rows, &piv_colb, &n_piv, &fv};
+                void* args[] = {&Dp, &ld_, &rs.chunk_rows, &rs.dpanel, &rs.cursor, &rows_, &nc_, &panF,
+                                &piv_rows, &n_piv, &piv_of_col, &is_piv, &rs.wflag, &fv};
                 BL_LAUNCH(BL_CUDA(launch_cluster((const void*)k_panel_factor<F>, n_dirty * cl, cl,
                                                  kTinyThreads,
                                                  (int)tiny_layout(rows_, KB, cl).words * 4, s, args)));
@@ -1409,22 +1256,20 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                 if (wide) {
                     BL_CUDA(ensure_smem_limit((const void*)k_panel_apply<true>, PA_SMEM));
                     BL_LAUNCH(k_panel_apply_small<true><<<grid, PA_THREADS, 0, s>>>(
-                        Dp, ld, ncr, j0, tpb, dpanel, panF, n_piv, piv_rows, c.p));
+                        Dp, ld, ncr, j0, tpb, rs.dpanel, panF, n_piv, piv_rows, c.p));
                     BL_LAUNCH(k_panel_apply<true><<<grid1, PA_THREADS, PA_SMEM, s>>>(
-                        Dp, ld, ncr, j0, 1, dpanel, panF, n_piv, piv_rows, c.p));
+                        Dp, ld, ncr, j0, 1, rs.dpanel, panF, n_piv, piv_rows, c.p));
                 } else {
                     BL_CUDA(ensure_smem_limit((const void*)k_panel_apply<false>, PA_SMEM));
                     BL_LAUNCH(k_panel_apply_small<false><<<grid, PA_THREADS, 0, s>>>(
-                        Dp, ld, ncr, j0, tpb, dpanel, panF, n_piv, piv_rows, c.p));
+                        Dp, ld, ncr, j0, tpb, rs.dpanel, panF, n_piv, piv_rows, c.p));
                     BL_LAUNCH(k_panel_apply<false><<<grid1, PA_THREADS, PA_SMEM, s>>>(
-                        Dp, ld, ncr, j0, 1, dpanel, panF, n_piv, piv_rows, c.p));
+                        Dp, ld, ncr, j0, 1, rs.dpanel, panF, n_piv, piv_rows, c.p));
                 }
             }
-            BL_LAUNCH(k_register_chunks<<<n_dirty, KB, 0, s>>>(n_piv, piv_rows, piv_colb, piv_of_col,
-                                                                is_piv, wflag));
             if (trace_rounds()) {
                 std::vector<int32_t> h_cur(n_dirty), h_np(n_dirty);
-                BL_CUDA(cudaMemcpyAsync(h_cur.data(), cursor, 4 * n_dirty, cudaMemcpyDeviceToHost, s));
+                BL_CUDA(cudaMemcpyAsync(h_cur.data(), rs.cursor, 4 * n_dirty, cudaMemcpyDeviceToHost, s));
                 BL_CUDA(cudaMemcpyAsync(h_np.data(), n_piv, 4 * n_dirty, cudaMemcpyDeviceToHost, s));
                 BL_CUDA(cudaStreamSynchronize(s));
                 long long rows_in = 0, piv = 0;
@@ -1440,29 +1285,22 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                         rounds, n_pend, n_dirty, j0 / KB, rows_in, mx, piv);
             }
         }
-        // all pivots of the round, ascending columns; normalise
-        BL_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, wflag, wpos, ncr, s));
-        ++c.launches;
-        BL_LAUNCH(k_compact_cols<<<grid_of(ncr), 256, 0, s>>>(ncr, wflag, wpos, pc));
-        BL_LAUNCH(k_new_pivots<<<grid_of(ncr), 256, 0, s>>>(ncr, wflag, wpos, pc, piv_of_col,
-                                                           counters + 2, prow));
-        BL_LAUNCH(k_normalize_at<F><<<std::min(t, 148 * 8), 256, 0, s>>>(counters + 2, prow, pc,
-                                                                         ncr, Dp, ld, f));
-        // the rest: eliminated against every pivot of the round; one host
-        // round trip reads both counts and the pivot columns
-        BL_CHECK(collect_pending(counters + 3));
-        int32_t cnt[3] = {0, 0, 0};
-        std::vector<int32_t> h_pc((size_t)ncr);
-        BL_CUDA(cudaMemcpyAsync(cnt, counters + 2, 3 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-        BL_CUDA(cudaMemcpyAsync(h_pc.data(), pc, sizeof(int32_t) * ncr, cudaMemcpyDeviceToHost, s));
+        // all pivots of the round, ascending columns, and the rows left; the
+        // panels' pivots are normalised already
+        BL_LAUNCH(k_round_finish<<<1, RD_THREADS, 0, s>>>(rs, KB, 0));
+        if (n_clean > 0)
+            BL_LAUNCH(k_normalize_at<F><<<std::min(t, 148 * 8), 256, 0, s>>>(counters, prow, pc, ncr,
+                                                                             Dp, ld, f));
         BL_CUDA(cudaStreamSynchronize(s));
-        const int32_t n_new = cnt[0], n_rest = cnt[1];
+        const int32_t n_new = info->n_new, n_rest = info->n_rest;
         if (trace_rounds()) fprintf(stderr, "gbgpu echelon round %d: new pivots %d\n", rounds, n_new);
         if (n_rest == 0) break;
-        h_pc.resize((size_t)n_new);
+        // the first pivot column of every block of KB pivots
+        std::vector<int32_t> h_first;
+        BL_CHECK(first_columns(c, info, pc, n_new, &h_first));
         // one panel alone: its pivot rows are reduced among themselves already
-        const bool unit = n_dirty == 1 && cnt[2] == 0;
-        BL_CHECK(eliminate(c, f, Dp, ld, pend, n_rest, ncr, prow, n_new, pc, h_pc, unit));
+        const bool unit = n_dirty == 1 && n_clean == 0;
+        BL_CHECK(eliminate(c, f, Dp, ld, pend, n_rest, ncr, prow, n_new, pc, h_first, unit));
         BL_LAUNCH(k_row_leads<<<grid_of((int64_t)n_rest * 32), 256, 0, s>>>(n_rest, pend, ncr, Dp,
                                                                              ld, lead, 1));
     }
@@ -1472,24 +1310,15 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
 
     // ---- 3. back substitution --------------------------------------------------
     // all pivots in ascending column order
-    BL_LAUNCH(k_pivot_flags<<<grid_of(ncr), 256, 0, s>>>(ncr, piv_of_col, 0, wflag));
-    BL_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, wflag, wpos, ncr, s));
-    ++c.launches;
-    BL_LAUNCH(k_compact_cols<<<grid_of(ncr), 256, 0, s>>>(ncr, wflag, wpos, pc));
-    int32_t r = 0;
-    if (ncr > 0) {
-        int32_t last_pos = 0, last_flag = 0;
-        BL_CUDA(cudaMemcpyAsync(&last_pos, wpos + ncr - 1, 4, cudaMemcpyDeviceToHost, s));
-        BL_CUDA(cudaMemcpyAsync(&last_flag, wflag + ncr - 1, 4, cudaMemcpyDeviceToHost, s));
-        BL_CUDA(cudaStreamSynchronize(s));
-        r = last_pos + last_flag;
-    }
+    BL_LAUNCH(k_round_finish<<<1, RD_THREADS, 0, s>>>(rs, KB, 1));
+    BL_CUDA(cudaStreamSynchronize(s));
+    const int32_t r = info->n_new;
     out->rank = r;
+    out->pivot_cols = pc;
+    out->pivot_rows = prow;
     if (r > 0) {
-        std::vector<int32_t> h_pc(r);
-        BL_CUDA(cudaMemcpyAsync(h_pc.data(), pc, sizeof(int32_t) * r, cudaMemcpyDeviceToHost, s));
-        BL_CUDA(cudaStreamSynchronize(s));
-        BL_LAUNCH(k_gather_rows<<<grid_of(r), 256, 0, s>>>(r, pc, piv_of_col, prow, counters + 2));
+        std::vector<int32_t> h_first;
+        BL_CHECK(first_columns(c, info, pc, r, &h_first));
         // echelon rows prow[0 .. r), ascending lead, reduced in place
         StreamOut* so = out->stream_out;
         int32_t* pcd = nullptr;          // pivot columns, descending (the answer's order)
@@ -1570,12 +1399,12 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
             const int kb = std::min(NB, r - b * NB);
             const int32_t later = r - (b * NB + kb);
             const int32_t* rows_k = prow + b * NB;
-            const int32_t c0 = h_pc[b * NB] & ~3;  // zero left of the pivot column, as below
+            const int32_t c0 = h_first[b * (NB / KB)] & ~3;  // zero left of the pivot column, as below
             if (later > 0) {
                 // E_k -= E_k[:, pc(>k)] R(>k)
                 BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * later), 256, 0, s>>>(
                     kb, later, Dp, ld, pc + b * NB + kb, G, later, rows_k));
-                const int32_t c_later = h_pc[b * NB + kb] & ~3;
+                const int32_t c_later = h_first[(b + 1) * (NB / KB)] & ~3;
                 TcGemmArgs g{c.p, kb, ncr - c_later, later, G, later, Dp + c_later, ld,
                              Dp + c_later, ld};
                 g.b_rows = rows_k + kb;
@@ -1638,23 +1467,13 @@ static int dense_rref_run(const DenseRrefInput& in, int32_t* rank, Ctx& c, const
     const int32_t r = (int32_t)out.rank;
     *rank = r;
     // pivot rows in ascending pivot order into the first r rows, zeros after
-    int32_t* flag = c.alloc<int32_t>(in.cols);
-    int32_t* pos = c.alloc<int32_t>(in.cols);
-    int32_t* order = c.alloc<int32_t>(std::max(r, 1));
-    int32_t* cnt = c.alloc<int32_t>(1);
     uint32_t* tmp = c.alloc<uint32_t>((size_t)in.rows * in.ld);
-    if (!flag || !pos || !order || !cnt || !tmp) return GBGPU_ENOMEM;
-    size_t bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, bytes, flag, pos, in.cols, c.s);
-    void* scan_tmp = c.alloc<uint8_t>(bytes);
-    if (!scan_tmp) return GBGPU_ENOMEM;
-    BL_LAUNCH(k_pivot_flags<<<grid_of(in.cols), 256, 0, c.s>>>(in.cols, piv_of_col, 0, flag));
-    BL_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, bytes, flag, pos, in.cols, c.s));
-    BL_LAUNCH(k_compact_cols<<<grid_of(in.cols), 256, 0, c.s>>>(in.cols, flag, pos, in.piv_cols));
+    if (!tmp) return GBGPU_ENOMEM;
     if (r > 0)
-        BL_LAUNCH(k_gather_rows<<<grid_of(r), 256, 0, c.s>>>(r, in.piv_cols, piv_of_col, order, cnt));
+        BL_CUDA(cudaMemcpyAsync(in.piv_cols, out.pivot_cols, sizeof(int32_t) * (size_t)r,
+                                cudaMemcpyDeviceToDevice, c.s));
     BL_LAUNCH(k_order_rows<<<grid_of((int64_t)in.rows * in.cols), 256, 0, c.s>>>(
-        r, in.rows, order, in.cols, in.D, in.ld, tmp, in.ld));
+        r, in.rows, out.pivot_rows, in.cols, in.D, in.ld, tmp, in.ld));
     BL_CUDA(cudaMemcpy2DAsync(in.D, in.ld * 4, tmp, in.ld * 4, (size_t)in.cols * 4, in.rows,
                               cudaMemcpyDeviceToDevice, c.s));
     return GBGPU_OK;

@@ -43,6 +43,8 @@ struct BlockedOutput {
     int32_t* piv_of_col = nullptr;  // [ncr], filled: reduced row of each pivot column or -1
     uint32_t* rows = nullptr;       // reduced rows (row piv_of_col[c] of `rows`), ld below
     int64_t ld = 0;
+    // pivot columns ascending and their rows of `rows` (device, alive like `keep`)
+    const int32_t *pivot_cols = nullptr, *pivot_rows = nullptr;
     int64_t rank = 0, dense_rows = 0, echelon_rounds = 0;
     cudaEvent_t ms_event_schur = nullptr, ms_event_echelon = nullptr;
     std::vector<void*>* keep = nullptr;  // device buffers alive until blocked_release

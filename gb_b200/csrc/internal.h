@@ -22,6 +22,17 @@ void count_launch(long long n);
 // so a launch in one host thread never sees another thread lower it.
 cudaError_t ensure_smem_limit(const void* kernel, int bytes);
 int device_init(int device, DeviceInfo* info);
+// Small pages of mapped host memory on the current device, for kernels that
+// report counts to the host: a bounded pool shared by all threads (api.cu).  The
+// user returns the page with no kernel left that writes it.
+constexpr size_t kMappedPageBytes = 65536;
+struct MappedPage {
+    int device = -1;
+    void* host = nullptr;
+    void* dev = nullptr;
+};
+cudaError_t mapped_page_take(MappedPage* out);
+void mapped_page_return(MappedPage& p);
 // The C-ABI entry points leave the caller's current device as they found it:
 // the scope notes it on entry (and makes `device` current when >= 0) and
 // restores it on exit.
