@@ -244,8 +244,6 @@ __device__ __forceinline__ uint32_t mod64(uint64_t x, uint32_t p, uint64_t m) {
     return (uint32_t)r;
 }
 
-constexpr int INV_THREADS = 1024;  // threads of k_neg_inverse
-
 // sum of u_k v_k mod p for u_k, v_k < p < 2^31, from 16-bit halves of v
 // accumulated without reduction (each product < 2^47, at most 128 terms)
 __device__ __forceinline__ uint32_t fold_lohi(uint64_t lo, uint64_t hi, uint32_t p, uint64_t m) {
@@ -253,106 +251,141 @@ __device__ __forceinline__ uint32_t fold_lohi(uint64_t lo, uint64_t hi, uint32_t
     return mod64((uint64_t)mod64(lo, p, m) + ((uint64_t)hr << 16), p, m);
 }
 
-// sum_{k in [k0, k1)} a[k sa] b[k sb] mod p (residues < p < 2^31), two
-// independent 16-bit-split accumulator pairs
-__device__ __forceinline__ uint32_t dot_lohi(const uint32_t* a, int sa, const uint32_t* b, int sb,
-                                             int k0, int k1, uint32_t p, uint64_t m) {
-    uint64_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
-    int k = k0;
-    for (; k + 1 < k1; k += 2) {
-        const uint32_t u0 = a[k * sa], v0 = b[k * sb];
-        const uint32_t u1 = a[(k + 1) * sa], v1 = b[(k + 1) * sb];
-        lo0 += (uint64_t)u0 * (v0 & 0xFFFFu);
-        hi0 += (uint64_t)u0 * (v0 >> 16);
-        lo1 += (uint64_t)u1 * (v1 & 0xFFFFu);
-        hi1 += (uint64_t)u1 * (v1 >> 16);
+constexpr int INV_THREADS = 512;  // threads of k_neg_inverse
+constexpr int INV_BYTES = (KB * (KB + 1) + KB * KB / 4) * (int)sizeof(uint32_t);
+
+// One doubling level of k_neg_inverse: the 2 SZ x 2 SZ diagonal blocks
+// [[A^-1, B], [0, C^-1]] get -A^-1 B C^-1 in place of B.  A thread owns R rows
+// by CW columns of a block's product; lanes run over the columns, so the left
+// factor's entries are broadcasts.
+template <class F, int SZ>
+__device__ __forceinline__ void inverse_level(uint32_t (*V)[KB + 1], uint32_t* T, const F& f) {
+    constexpr int CW = SZ > 32 ? 2 : 1, LN = SZ / CW;       // columns of a thread, lanes of a row
+    constexpr int R = SZ * KB / 2 / (INV_THREADS * CW);     // rows of a thread
+    constexpr int GROUPS = SZ / R;                          // threads of a column
+    const int j = threadIdx.x % LN, g = threadIdx.x / LN;
+    const int pr = g / GROUPS, i0 = g % GROUPS * R, b0 = pr * 2 * SZ;
+    uint64_t acc[R][CW];
+    auto clear = [&]() {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int w = 0; w < CW; ++w) acc[r][w] = 0;
+    };
+    // T = B C^-1 (C^-1 is upper triangular: column j needs k <= j)
+    clear();
+#pragma unroll
+    for (int w0 = 0; w0 < CW; ++w0)
+#pragma unroll 8
+        for (int k = w0 * LN; k < (w0 + 1) * LN; ++k) {
+            uint32_t v[CW];
+#pragma unroll
+            for (int w = w0; w < CW; ++w) v[w] = V[b0 + SZ + k][b0 + SZ + j + w * LN];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const uint32_t u = V[b0 + i0 + r][b0 + SZ + k];
+#pragma unroll
+                for (int w = w0; w < CW; ++w) acc[r][w] = f.lazy_add(acc[r][w], u, v[w]);
+            }
+        }
+    uint32_t* Tp = T + pr * SZ * SZ;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int w = 0; w < CW; ++w) Tp[(i0 + r) * SZ + j + w * LN] = f.lazy_mod(acc[r][w]);
+    __syncthreads();
+    // -A^-1 T (A^-1 is upper triangular: row i needs k >= i)
+    clear();
+#pragma unroll 4
+    for (int k = i0; k < SZ; ++k) {
+        uint32_t t[CW];
+#pragma unroll
+        for (int w = 0; w < CW; ++w) t[w] = Tp[k * SZ + j + w * LN];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint32_t u = V[b0 + i0 + r][b0 + k];
+#pragma unroll
+            for (int w = 0; w < CW; ++w) acc[r][w] = f.lazy_add(acc[r][w], u, t[w]);
+        }
     }
-    if (k < k1) {
-        const uint32_t u0 = a[k * sa], v0 = b[k * sb];
-        lo0 += (uint64_t)u0 * (v0 & 0xFFFFu);
-        hi0 += (uint64_t)u0 * (v0 >> 16);
-    }
-    return fold_lohi(lo0 + lo1, hi0 + hi1, p, m);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int w = 0; w < CW; ++w) {
+            const uint32_t x = f.lazy_mod(acc[r][w]);
+            V[b0 + i0 + r][b0 + SZ + j + w * LN] = x ? f.p - x : 0u;
+        }
+    __syncthreads();
 }
 
 // -U^-1 mod p for unit upper triangular blocks.  Block b is read from
 // src + b * stride_b with leading dimension ld (kb x kb, kb <= KB); the result
 // (KB x KB, identity-padded) goes to out + b * ostride with leading dimension
-// old.  One CTA per block, V = U^-1 built by doubling in shared memory: the
-// 8 x 8 diagonal blocks by back substitution, then for sz = 8, 16, 32, 64
-// every 2sz x 2sz diagonal block [[A, B], [0, C]] gets its top-right part
-// -A^-1 B C^-1 as two small products (T = B C^-1, then -A^-1 T).
+// old.  One CTA per block, V = U^-1 built in place in shared memory by
+// doubling: the 8 x 8 diagonal blocks by back substitution, a thread per
+// column, then for sz = 8, 16, 32, 64 every 2sz x 2sz diagonal block
+// [[A, B], [0, C]] gets its top-right part -A^-1 B C^-1 as two small products.
+//
+// Bound by the 64-bit multiply-adds of the sz = 64 products (4 cycles a warp
+// each).  A sum stays one 64-bit accumulator (below 2^39 for p < 2^16, folded
+// below p^2 otherwise), a thread's products share their operands' loads, and
+// 83 KB a block let two blocks share an SM: 18 us a launch of up to 296 blocks
+// (36 us for p >= 2^16); with 16-bit halves in two accumulators, an entry a
+// thread and 148 KB a block it was 55 us, and a second wave beyond 148 blocks.
 template <class F>
-__global__ void __launch_bounds__(INV_THREADS)
+__global__ void __launch_bounds__(INV_THREADS, 2)
 k_neg_inverse(const uint32_t* __restrict__ src, int64_t ld, int64_t stride_b, int32_t n_blocks,
               int32_t last_kb, uint32_t* out, int64_t ostride, int64_t old, F f) {
     extern __shared__ uint32_t inv_smem[];
-    uint32_t(*U)[KB + 1] = (uint32_t(*)[KB + 1])inv_smem;
-    uint32_t(*V)[KB + 1] = (uint32_t(*)[KB + 1])(inv_smem + KB * (KB + 1));
-    uint32_t* T = inv_smem + 2 * KB * (KB + 1);  // KB * KB / 4 entries
+    uint32_t(*V)[KB + 1] = (uint32_t(*)[KB + 1])inv_smem;
+    uint32_t* T = inv_smem + KB * (KB + 1);  // KB * KB / 4 entries
     const int b = blockIdx.x;
     const int kb = b == n_blocks - 1 ? last_kb : KB;
     const uint32_t* s = src + (size_t)b * stride_b;
     const int tid = threadIdx.x;
-    // the block: KB * KB / blockDim.x entries per thread, all loads in flight
+    // the block: KB * KB / blockDim.x entries per thread, 16 loads in flight
     constexpr int PER = KB * KB / INV_THREADS;
-    {
-        uint32_t v[PER];
+#pragma unroll 1
+    for (int q0 = 0; q0 < PER; q0 += 16) {
+        uint32_t v[16];
 #pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int t = tid + q * INV_THREADS;
+        for (int q = 0; q < 16; ++q) {
+            const int t = tid + (q0 + q) * INV_THREADS;
             const int i = t / KB, j = t % KB;
-            v[q] = (i < kb && j < kb) ? s[(size_t)i * ld + j] : (i == j ? 1u : 0u);
+            v[q] = (i < kb && j < kb && i < j) ? s[(size_t)i * ld + j] : (i == j ? 1u : 0u);
         }
 #pragma unroll
-        for (int q = 0; q < PER; ++q) {
-            const int t = tid + q * INV_THREADS;
-            const int i = t / KB, j = t % KB;
-            U[i][j] = v[q];
-            V[i][j] = i == j ? 1u : 0u;
+        for (int q = 0; q < 16; ++q) {
+            const int t = tid + (q0 + q) * INV_THREADS;
+            V[t / KB][t % KB] = v[q];
         }
     }
     __syncthreads();
-    const uint32_t p = f.p;
-    const uint64_t m = ~0ull / p;
+    // 8 x 8 diagonal blocks: V[i][j] = -sum_{i<k<=j} U[i][k] V[k][j]
+    uint32_t d[8];
+    const int b0 = tid & (KB - 8), j = tid & 7;
     if (tid < KB) {
-        // 8 x 8 diagonal blocks: V[i][j] = -sum_{i<k<=j} U[i][k] V[k][j]
-        const int b0 = tid & ~7, j = b0 + (tid & 7);
-        for (int i = j - 1; i >= b0; --i) {
-            uint64_t lo = 0, hi = 0;
-            for (int k = i + 1; k <= j; ++k) {
-                const uint32_t u = U[i][k];
-                const uint32_t v = V[k][j];
-                lo += (uint64_t)u * (v & 0xFFFFu);
-                hi += (uint64_t)u * (v >> 16);
-            }
-            const uint32_t acc = fold_lohi(lo, hi, p, m);
-            V[i][j] = acc ? p - acc : 0u;
+#pragma unroll
+        for (int i = 7; i >= 0; --i) {
+            uint64_t acc = 0;
+#pragma unroll
+            for (int k = i + 1; k < 8; ++k) acc = f.lazy_add(acc, V[b0 + i][b0 + k], d[k]);
+            const uint32_t x = f.lazy_mod(acc);
+            d[i] = i == j ? 1u : i < j && x ? f.p - x : 0u;
         }
     }
     __syncthreads();
-    for (int sz = 8; sz < KB; sz *= 2) {
-        const int per = sz * sz, total = (KB / (2 * sz)) * per;
-        // T = B C^-1 (C^-1 upper triangular: k <= j)
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int b0 = (e / per) * 2 * sz, i = (e % per) / sz, j = e % sz;
-            const uint32_t* urow = &U[b0 + i][b0 + sz];
-            const uint32_t* vcol = &V[b0 + sz][b0 + sz + j];
-            T[e] = dot_lohi(urow, 1, vcol, KB + 1, 0, j + 1, p, m);
-        }
-        __syncthreads();
-        // top-right of V = -A^-1 T (A^-1 upper triangular: k >= i)
-        for (int e = tid; e < total; e += blockDim.x) {
-            const int pr = e / per, b0 = pr * 2 * sz, i = (e % per) / sz, j = e % sz;
-            const uint32_t* Tp = T + pr * per;
-            const uint32_t acc =
-                dot_lohi(&V[b0 + i][b0], 1, Tp + j, sz, i, sz, p, m);
-            V[b0 + i][b0 + sz + j] = acc ? p - acc : 0u;
-        }
-        __syncthreads();
+    if (tid < KB) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) V[b0 + i][b0 + j] = d[i];
     }
+    __syncthreads();
+    inverse_level<F, 8>(V, T, f);
+    inverse_level<F, 16>(V, T, f);
+    inverse_level<F, 32>(V, T, f);
+    inverse_level<F, 64>(V, T, f);
     uint32_t* o = out + (size_t)b * ostride;
-    for (int t = tid; t < KB * KB; t += blockDim.x) {
+    for (int t = tid; t < KB * KB; t += INV_THREADS) {
         const int i = t / KB, jj = t % KB;
         const uint32_t v = V[i][jj];
         o[(size_t)i * old + jj] = v ? f.p - v : 0u;  // -V
@@ -928,11 +961,10 @@ static int neg_inverse_big(Ctx& c, const F& f, const uint32_t* src, int64_t lds,
     BL_LAUNCH(k_copy_blocks<<<grid_of((int64_t)n_blocks * NB * NB), 256, 0, c.s>>>(
         src, lds, stride_src, n_blocks, last_nb, NB, U));
     BL_CUDA(cudaMemsetAsync(out, 0, sizeof(uint32_t) * (size_t)n_blocks * bstride, c.s));
-    const int bytes = (2 * KB * (KB + 1) + KB * KB / 4) * (int)sizeof(uint32_t);
-    BL_CUDA(ensure_smem_limit((const void*)k_neg_inverse<F>, bytes));
+    BL_CUDA(ensure_smem_limit((const void*)k_neg_inverse<F>, INV_BYTES));
     const int32_t n_sub = n_blocks * (NB / KB);
     const int64_t dstep = (int64_t)KB * (NB + 1);  // between 128-blocks on the diagonal
-    BL_LAUNCH(k_neg_inverse<F><<<n_sub, INV_THREADS, bytes, c.s>>>(U, NB, dstep, n_sub, KB, out,
+    BL_LAUNCH(k_neg_inverse<F><<<n_sub, INV_THREADS, INV_BYTES, c.s>>>(U, NB, dstep, n_sub, KB, out,
                                                                    dstep, NB, f));
     for (int32_t sz = KB; sz < NB; sz *= 2) {
         const int32_t items = n_blocks * (NB / (2 * sz));
