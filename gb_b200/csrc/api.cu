@@ -469,6 +469,46 @@ static int plan_alloc(Plan* P) {
     return GBGPU_OK;
 }
 
+// Interreduction row by row is a chain: a row applies the pivots right of its
+// lead one after the other, 0.5 us each.  As one dense back substitution on the
+// tensor cores (interreduce_dense) it is about thirty launches and nr^2 nc
+// products.  Rows that meet kDenseHits pivots each to begin with fill up (every
+// pivot applied brings new ones), so the chains are long; rows that meet fewer
+// mostly stay sparse, and below kDenseTotal of them the launches cost more than
+// the chains.  Whole call with host rows, row form against dense, p = 32003,
+// nr x nc, entries at pivot columns a row:
+//   200 x 750, 16: 518 / 414 us      800 x 3000, 17: 1734 / 920 (p = 2^31 - 1)
+//   400 x 1500, 17: 747 / 537        800 x 3000, 5: 916 / 629
+//   1600 x 6000, 17: 5597 / 2029     3000 x 60000, 6: 99 / 91 ms
+//   150 x 562, 16: 448 / 440         800 x 3000, 2: 339 / 479
+//   300 x 1500, 3: 332 / 422         1000 x 200000, 3: 27 / 29 ms
+// Blocks past kDenseEntries keep the row form, whose memory is the block alone.
+constexpr int32_t kDenseRows = 128;  // one block of pivots
+constexpr unsigned long long kDenseHits = 4, kDenseTotal = 3000;
+constexpr int64_t kDenseEntries = (int64_t)1 << 28;
+static bool interreduce_may_be_dense(const Plan* P) {
+    return (P->p & 1) && P->p >= 3 && P->nr >= kDenseRows &&
+           (int64_t)P->nr * P->nc <= kDenseEntries &&
+           (P->requested_form == GBGPU_FORM_AUTO || P->requested_form == GBGPU_FORM_TENSOR);
+}
+
+// *hits += the entries of the rows that lie in a pivot column (leads included)
+__global__ void k_pivot_hits(int32_t nr, const int64_t* __restrict__ row_ptr,
+                             const int32_t* __restrict__ cols, int32_t nc,
+                             const int32_t* __restrict__ piv_row, unsigned long long* hits) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    unsigned n = 0;
+    for (int i = warp; i < nr; i += nwarps)
+        for (int64_t k = row_ptr[i] + lane; k < row_ptr[i + 1]; k += 32) {
+            const int32_t c = cols[k];
+            n += c >= 0 && c < nc && piv_row[c] != INT_MAX;
+        }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0 && n) atomicAdd(hits, (unsigned long long)n);
+}
+
 template <class F>
 static int run_form(Plan* P, const F& f) {
     cudaStream_t s = P->stream;
@@ -496,6 +536,15 @@ static int run_form(Plan* P, const F& f) {
                                                             P->mode == 1));
     if (P->mode == 0)
         GB_LAUNCH(k_check_pivots<<<grid_for(P->ncl, T), T, 0, s>>>(P->ncl, P->piv_row, P->err));
+    // interreduction: the entries at pivot columns decide the path below
+    const bool may_dense = P->mode == 1 && interreduce_may_be_dense(P);
+    unsigned long long hits = 0;
+    if (may_dense) {
+        GB_LAUNCH(k_pivot_hits<<<grid_for((int64_t)P->nr * 32, T), T, 0, s>>>(
+            P->nr, P->row_ptr, P->cols, P->nc, P->piv_row, (unsigned long long*)P->work_count + 1));
+        GB_CUDA(cudaMemcpyAsync(&hits, P->work_count + 1, 8, cudaMemcpyDeviceToHost, s));
+        GB_CUDA(cudaMemsetAsync(P->work_count + 1, 0, 8, s));
+    }
     GB_CUDA(cudaEventRecord(P->ev[6], s));
     if (P->tiny) {
         // the checks' verdict is read with the answer; the kernels below skip
@@ -530,6 +579,7 @@ static int run_form(Plan* P, const F& f) {
     const uint32_t* final_rows = P->D;
     int64_t rows_ld = P->ld;
     BlockedOutput bo{};
+    bool tensor = P->blocked;  // tensor-core kernels ran: their status is read at the end
     if (P->blocked) {
         BlockedInput bi{};
         bi.p = (uint32_t)P->p;
@@ -595,7 +645,26 @@ static int run_form(Plan* P, const F& f) {
     sa.queue = P->counters + 0;
     sa.work_count = P->work_count + 0;
     sa.err = P->err;
-    if (P->n_work > 0) {
+    if (may_dense && hits >= std::max(kDenseTotal, kDenseHits * (unsigned long long)P->nr)) {
+        InterreduceInput ii{};
+        ii.p = (uint32_t)P->p;
+        ii.rows = P->nr;
+        ii.ncols = P->nc;
+        ii.row_ptr = P->row_ptr;
+        ii.cols = P->cols;
+        ii.vals = P->vals;
+        ii.piv_of_col = P->piv_of_col;
+        ii.D = P->D;
+        ii.ld = P->ld;
+        ii.stream = s;
+        ii.form = GBGPU_FORM_TENSOR;
+        ii.err = P->counters + 6;
+        const int rc = interreduce_dense(ii, &launches);
+        if (rc && rc != GBGPU_ENOMEM) return rc;
+        tensor = rc == GBGPU_OK;
+        cudaGetLastError();  // without the memory for its blocks: row by row
+    }
+    if (P->n_work > 0 && !tensor) {
         if (P->pext) {
             GB_LAUNCH(k_pivot_extents<<<grid_for(sa.piv_limit, T), T, 0, s>>>(
                 sa.piv_limit, P->piv_row, P->row_ptr, P->pext));
@@ -742,7 +811,7 @@ static int run_form(Plan* P, const F& f) {
             P->out_cols, P->out_vals, 4));
     }
     GB_CUDA(cudaEventRecord(P->ev[5], s));
-    if (P->blocked) {
+    if (tensor) {
         blocked_release(&bo, s);
         int32_t tc_status = 0;
         GB_CUDA(cudaMemcpyAsync(&tc_status, P->counters + 6, 4, cudaMemcpyDeviceToHost, s));

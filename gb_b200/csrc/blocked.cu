@@ -1183,6 +1183,117 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
     return GBGPU_OK;
 }
 
+// Step 3: the echelon rows prow[0 .. r) of Dp (ascending lead, pivot columns pc,
+// h_first[q] = that of pivot q KB) to reduced echelon form, in place.
+template <class F>
+static int back_substitute(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t ncr, int32_t r,
+                           const int32_t* pc, const int32_t* prow,
+                           const std::vector<int32_t>& h_first, BlockedOutput* out) {
+    cudaStream_t s = c.s;
+    const int32_t* piv_of_col = out->piv_of_col;
+    StreamOut* so = out->stream_out;
+    int32_t* pcd = nullptr;          // pivot columns, descending (the answer's order)
+    int64_t* cnt = nullptr;          // [NB + 1] entries per row of a block
+    int64_t* loc = nullptr;          // [NB + 1] their exclusive scan
+    void* cscan = nullptr;
+    size_t cscan_bytes = 0;
+    cudaEvent_t blk_ev = nullptr;
+    if (so) {
+        pcd = c.alloc<int32_t>(r);
+        cnt = c.alloc<int64_t>(nb_for(r) + 1);
+        loc = c.alloc<int64_t>(nb_for(r) + 1);
+        cub::DeviceScan::ExclusiveSum(nullptr, cscan_bytes, cnt, loc, nb_for(r) + 1, s);
+        cscan = c.alloc<uint8_t>(cscan_bytes);
+        if (!pcd || !cnt || !loc || !cscan) return GBGPU_ENOMEM;
+        BL_LAUNCH(k_reverse_i32<<<grid_of(r), 256, 0, s>>>(r, pc, pcd));
+        BL_CUDA(cudaEventCreateWithFlags(&blk_ev, cudaEventDisableTiming));
+        so->nnz = 0;
+        so->overflow = false;
+    }
+    // block b's answer rows [r - b NB - kb, r - b NB): compacted and sent
+    auto send_block = [&](int b, int kb) -> int {
+        const int64_t out0 = (int64_t)r - ((int64_t)b * nb_for(r) + kb);
+        BL_LAUNCH(k_row_nnz<<<grid_of((int64_t)kb * 32), 256, 0, s>>>(
+            kb, pcd + out0, piv_of_col, Dp, ld, ncr, cnt));
+        BL_CUDA(cudaMemsetAsync(cnt + kb, 0, sizeof(int64_t), s));
+        size_t bytes = cscan_bytes;
+        BL_CUDA(cub::DeviceScan::ExclusiveSum(cscan, bytes, cnt, loc, kb + 1, s));
+        ++c.launches;
+        int64_t blk = 0;
+        BL_CUDA(cudaMemcpyAsync(&blk, loc + kb, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        BL_CUDA(cudaStreamSynchronize(s));
+        BL_LAUNCH(k_offs_write<<<grid_of(kb + 1), 256, 0, s>>>(kb + 1, loc, so->nnz,
+                                                               so->offs + out0));
+        if (blk > 0) {
+            int32_t* bc = nullptr;
+            uint8_t* bw = nullptr;
+            const int vb = so->val_bytes;
+            if (cudaMallocAsync((void**)&bc, sizeof(int32_t) * blk, s) != cudaSuccess ||
+                cudaMallocAsync((void**)&bw, (size_t)vb * blk, s) != cudaSuccess) {
+                set_error("answer block allocation failed");
+                return GBGPU_ENOMEM;
+            }
+            BL_LAUNCH(k_row_write<<<grid_of((int64_t)kb * 32), 256, 0, s>>>(
+                kb, pcd + out0, piv_of_col, Dp, ld, ncr, loc, so->col_shift, bc, bw, vb));
+            cudaStream_t fs = s;
+            if (!so->overflow && so->nnz + blk <= so->cap_nnz) {
+                BL_CUDA(cudaEventRecord(blk_ev, s));
+                BL_CUDA(cudaStreamWaitEvent(so->s_out, blk_ev, 0));
+                BL_CUDA(cudaMemcpyAsync(so->h_cols + so->nnz, bc, sizeof(int32_t) * blk,
+                                        cudaMemcpyDeviceToHost, so->s_out));
+                BL_CUDA(cudaMemcpyAsync((uint8_t*)so->h_vals + (size_t)so->nnz * vb, bw,
+                                        (size_t)vb * blk, cudaMemcpyDeviceToHost, so->s_out));
+                fs = so->s_out;  // freed once copied
+            } else {
+                so->overflow = true;
+            }
+            cudaFreeAsync(bc, fs);
+            cudaFreeAsync(bw, fs);
+        }
+        so->nnz += blk;
+        return GBGPU_OK;
+    };
+    const int32_t NB = nb_for(r);
+    const int64_t bstride = (int64_t)NB * (NB + 1);
+    const int32_t nb = (r + NB - 1) / NB;
+    uint32_t* Ublk = c.alloc<uint32_t>((size_t)nb * NB * NB);
+    uint32_t* Ninv = c.alloc<uint32_t>((size_t)nb * bstride);
+    uint32_t* G = c.alloc<uint32_t>((size_t)NB * std::max(r, 1));
+    if (!Ublk || !Ninv || !G) return GBGPU_ENOMEM;
+    for (int b = 0; b < nb; ++b) {
+        const int kb = std::min(NB, r - b * NB);
+        BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * kb), 256, 0, s>>>(
+            kb, kb, Dp, ld, pc + b * NB, Ublk + (size_t)b * NB * NB, NB, prow + b * NB));
+    }
+    BL_CHECK(neg_inverse_big(c, f, Ublk, NB, (int64_t)NB * NB, nb, r - (nb - 1) * NB, NB, Ninv));
+    for (int b = nb - 1; b >= 0; --b) {
+        const int kb = std::min(NB, r - b * NB);
+        const int32_t later = r - (b * NB + kb);
+        const int32_t* rows_k = prow + b * NB;
+        const int32_t c0 = h_first[b * (NB / KB)] & ~3;  // zero left of the pivot column, as below
+        if (later > 0) {
+            // E_k -= E_k[:, pc(>k)] R(>k)
+            BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * later), 256, 0, s>>>(
+                kb, later, Dp, ld, pc + b * NB + kb, G, later, rows_k));
+            const int32_t c_later = h_first[(b + 1) * (NB / KB)] & ~3;
+            TcGemmArgs g{c.p, kb, ncr - c_later, later, G, later, Dp + c_later, ld,
+                         Dp + c_later, ld};
+            g.b_rows = rows_k + kb;
+            g.d_rows = rows_k;
+            BL_CHECK(gemm_args(c, g));
+        }
+        // E_k = (E_k[:, pc(k)])^-1 E_k = -((-(U_kk)^-1) E_k), in place
+        TcGemmArgs g{c.p, kb, ncr - c0, kb, Ninv + (size_t)b * bstride, NB, Dp + c0, ld, Dp + c0,
+                     ld};
+        g.b_rows = rows_k;
+        g.d_rows = rows_k;
+        BL_CHECK(gemm_set_in_place(c, g));
+        if (so) BL_CHECK(send_block(b, kb));
+    }
+    if (blk_ev) cudaEventDestroy(blk_ev);
+    return GBGPU_OK;
+}
+
 // Steps 2 and 3 on the dense t x ncr residue matrix Dp (leading dimension
 // ld), in place: afterwards out->piv_of_col[c] is the row of Dp holding the
 // reduced pivot row of column c (-1 for non-pivot columns), out->rank is the
@@ -1351,112 +1462,55 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
     if (r > 0) {
         std::vector<int32_t> h_first;
         BL_CHECK(first_columns(c, info, pc, r, &h_first));
-        // echelon rows prow[0 .. r), ascending lead, reduced in place
-        StreamOut* so = out->stream_out;
-        int32_t* pcd = nullptr;          // pivot columns, descending (the answer's order)
-        int64_t* cnt = nullptr;          // [NB + 1] entries per row of a block
-        int64_t* loc = nullptr;          // [NB + 1] their exclusive scan
-        void* cscan = nullptr;
-        size_t cscan_bytes = 0;
-        cudaEvent_t blk_ev = nullptr;
-        if (so) {
-            pcd = c.alloc<int32_t>(r);
-            cnt = c.alloc<int64_t>(nb_for(r) + 1);
-            loc = c.alloc<int64_t>(nb_for(r) + 1);
-            cub::DeviceScan::ExclusiveSum(nullptr, cscan_bytes, cnt, loc, nb_for(r) + 1, s);
-            cscan = c.alloc<uint8_t>(cscan_bytes);
-            if (!pcd || !cnt || !loc || !cscan) return GBGPU_ENOMEM;
-            BL_LAUNCH(k_reverse_i32<<<grid_of(r), 256, 0, s>>>(r, pc, pcd));
-            BL_CUDA(cudaEventCreateWithFlags(&blk_ev, cudaEventDisableTiming));
-            so->nnz = 0;
-            so->overflow = false;
-        }
-        // block b's answer rows [r - b NB - kb, r - b NB): compacted and sent
-        auto send_block = [&](int b, int kb) -> int {
-            const int64_t out0 = (int64_t)r - ((int64_t)b * nb_for(r) + kb);
-            BL_LAUNCH(k_row_nnz<<<grid_of((int64_t)kb * 32), 256, 0, s>>>(
-                kb, pcd + out0, piv_of_col, Dp, ld, ncr, cnt));
-            BL_CUDA(cudaMemsetAsync(cnt + kb, 0, sizeof(int64_t), s));
-            size_t bytes = cscan_bytes;
-            BL_CUDA(cub::DeviceScan::ExclusiveSum(cscan, bytes, cnt, loc, kb + 1, s));
-            ++c.launches;
-            int64_t blk = 0;
-            BL_CUDA(cudaMemcpyAsync(&blk, loc + kb, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-            BL_CUDA(cudaStreamSynchronize(s));
-            BL_LAUNCH(k_offs_write<<<grid_of(kb + 1), 256, 0, s>>>(kb + 1, loc, so->nnz,
-                                                                   so->offs + out0));
-            if (blk > 0) {
-                int32_t* bc = nullptr;
-                uint8_t* bw = nullptr;
-                const int vb = so->val_bytes;
-                if (cudaMallocAsync((void**)&bc, sizeof(int32_t) * blk, s) != cudaSuccess ||
-                    cudaMallocAsync((void**)&bw, (size_t)vb * blk, s) != cudaSuccess) {
-                    set_error("answer block allocation failed");
-                    return GBGPU_ENOMEM;
-                }
-                BL_LAUNCH(k_row_write<<<grid_of((int64_t)kb * 32), 256, 0, s>>>(
-                    kb, pcd + out0, piv_of_col, Dp, ld, ncr, loc, so->col_shift, bc, bw, vb));
-                cudaStream_t fs = s;
-                if (!so->overflow && so->nnz + blk <= so->cap_nnz) {
-                    BL_CUDA(cudaEventRecord(blk_ev, s));
-                    BL_CUDA(cudaStreamWaitEvent(so->s_out, blk_ev, 0));
-                    BL_CUDA(cudaMemcpyAsync(so->h_cols + so->nnz, bc, sizeof(int32_t) * blk,
-                                            cudaMemcpyDeviceToHost, so->s_out));
-                    BL_CUDA(cudaMemcpyAsync((uint8_t*)so->h_vals + (size_t)so->nnz * vb, bw,
-                                            (size_t)vb * blk, cudaMemcpyDeviceToHost, so->s_out));
-                    fs = so->s_out;  // freed once copied
-                } else {
-                    so->overflow = true;
-                }
-                cudaFreeAsync(bc, fs);
-                cudaFreeAsync(bw, fs);
-            }
-            so->nnz += blk;
-            return GBGPU_OK;
-        };
-        const int32_t NB = nb_for(r);
-        const int64_t bstride = (int64_t)NB * (NB + 1);
-        const int32_t nb = (r + NB - 1) / NB;
-        uint32_t* Ublk = c.alloc<uint32_t>((size_t)nb * NB * NB);
-        uint32_t* Ninv = c.alloc<uint32_t>((size_t)nb * bstride);
-        uint32_t* G = c.alloc<uint32_t>((size_t)NB * std::max(r, 1));
-        if (!Ublk || !Ninv || !G) return GBGPU_ENOMEM;
-        for (int b = 0; b < nb; ++b) {
-            const int kb = std::min(NB, r - b * NB);
-            BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * kb), 256, 0, s>>>(
-                kb, kb, Dp, ld, pc + b * NB, Ublk + (size_t)b * NB * NB, NB, prow + b * NB));
-        }
-        BL_CHECK(neg_inverse_big(c, f, Ublk, NB, (int64_t)NB * NB, nb, r - (nb - 1) * NB, NB, Ninv));
-        for (int b = nb - 1; b >= 0; --b) {
-            const int kb = std::min(NB, r - b * NB);
-            const int32_t later = r - (b * NB + kb);
-            const int32_t* rows_k = prow + b * NB;
-            const int32_t c0 = h_first[b * (NB / KB)] & ~3;  // zero left of the pivot column, as below
-            if (later > 0) {
-                // E_k -= E_k[:, pc(>k)] R(>k)
-                BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)kb * later), 256, 0, s>>>(
-                    kb, later, Dp, ld, pc + b * NB + kb, G, later, rows_k));
-                const int32_t c_later = h_first[(b + 1) * (NB / KB)] & ~3;
-                TcGemmArgs g{c.p, kb, ncr - c_later, later, G, later, Dp + c_later, ld,
-                             Dp + c_later, ld};
-                g.b_rows = rows_k + kb;
-                g.d_rows = rows_k;
-                BL_CHECK(gemm_args(c, g));
-            }
-            // E_k = (E_k[:, pc(k)])^-1 E_k = -((-(U_kk)^-1) E_k), in place
-            TcGemmArgs g{c.p, kb, ncr - c0, kb, Ninv + (size_t)b * bstride, NB, Dp + c0, ld, Dp + c0,
-                         ld};
-            g.b_rows = rows_k;
-            g.d_rows = rows_k;
-            BL_CHECK(gemm_set_in_place(c, g));
-            if (so) BL_CHECK(send_block(b, kb));
-        }
-        if (blk_ev) cudaEventDestroy(blk_ev);
+        BL_CHECK(back_substitute(c, f, Dp, ld, ncr, r, pc, prow, h_first, out));
     } else if (out->stream_out) {
         out->stream_out->nnz = 0;
         BL_CUDA(cudaMemsetAsync(out->stream_out->offs, 0, sizeof(int64_t), s));
     }
     return GBGPU_OK;
+}
+
+// Rows with distinct leads, every one reduced by all others (dense: blocked.h).
+template <class F>
+static int interreduce_run(const InterreduceInput& in, Ctx& c, const F& f) {
+    cudaStream_t s = c.s;
+    BL_CUDA(ensure_smem_limit((const void*)k_densify_seg, DS_COLS * 4));
+    BL_LAUNCH(k_densify_seg<<<std::min(in.rows, 148 * 3), 512, DS_COLS * 4, s>>>(
+        in.rows, nullptr, in.row_ptr, in.cols, in.vals, in.ncols, in.ncols, 0, 0, in.D, in.ld));
+    RoundState rs{};
+    rs.ncr = in.ncols;
+    rs.piv_of_col = in.piv_of_col;
+    rs.pc = c.alloc<int32_t>(in.ncols);
+    rs.prow = c.alloc<int32_t>(in.ncols);
+    rs.n_new = c.alloc<int32_t>(1);
+    if (!rs.pc || !rs.prow || !rs.n_new) return GBGPU_ENOMEM;
+    InfoPage page(s, sizeof(RoundInfo));
+    const volatile RoundInfo* info = (const volatile RoundInfo*)page.host;
+    rs.info = (RoundInfo*)page.dev;
+    if (!info) return GBGPU_ENOMEM;
+    BL_LAUNCH(k_round_finish<<<1, RD_THREADS, 0, s>>>(rs, KB, 1));
+    BL_CUDA(cudaStreamSynchronize(s));
+    std::vector<int32_t> h_first;
+    BL_CHECK(first_columns(c, info, rs.pc, in.rows, &h_first));
+    BlockedOutput out{};
+    out.piv_of_col = in.piv_of_col;
+    return back_substitute(c, f, in.D, in.ld, in.ncols, in.rows, rs.pc, rs.prow, h_first, &out);
+}
+
+int interreduce_dense(const InterreduceInput& in, long long* launches) {
+    Ctx c;
+    c.s = in.stream;
+    c.p = in.p;
+    c.form = in.form;
+    c.err = in.err;
+    int rc;
+    if (in.p < 65536u)
+        rc = interreduce_run(in, c, FieldSmall::make(in.p));
+    else
+        rc = interreduce_run(in, c, FieldMont::make(in.p));
+    *launches += c.launches;
+    c.release();
+    return rc;
 }
 
 int blocked_reduce(const BlockedInput& in, BlockedOutput* out, long long* launches) {

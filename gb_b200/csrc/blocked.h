@@ -64,6 +64,24 @@ struct DenseRrefInput {
     int32_t* err;
 };
 int dense_rref(const DenseRrefInput& in, int32_t* rank, long long* launches);
+
+// Interreduction as one dense back substitution: CSR rows with distinct leads,
+// monic (row piv_of_col[c] has lead c), to D (rows x ncols, leading dimension ld,
+// a multiple of 4), every row reduced by all others.
+struct InterreduceInput {
+    uint32_t p;
+    int32_t rows, ncols;
+    const int64_t* row_ptr;  // device CSR
+    const int32_t* cols;
+    const uint32_t* vals;
+    int32_t* piv_of_col;     // [ncols]: row with that lead, -1
+    uint32_t* D;
+    int64_t ld;
+    cudaStream_t stream;
+    int form;
+    int32_t* err;
+};
+int interreduce_dense(const InterreduceInput& in, long long* launches);
 void blocked_release(BlockedOutput* out, cudaStream_t s);
 
 }  // namespace gbgpu
