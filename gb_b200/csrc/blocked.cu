@@ -987,10 +987,15 @@ __global__ void k_reverse_i32(int32_t n, const int32_t* __restrict__ in, int32_t
 }
 
 // offs[k] = base + loc[k]
+// *total = loc[n - 1], in mapped host memory: a copy would queue behind the
+// answer's blocks on their way to the host (0.5 to 1 ms each), and the next block
+// could not be sized before
 __global__ void k_offs_write(int32_t n, const int64_t* __restrict__ loc, int64_t base,
-                             int64_t* offs) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
+                             int64_t* offs, int64_t* total) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         offs[k] = base + loc[k];
+        if (k == n - 1) *total = loc[k];
+    }
 }
 
 // Mapped host memory for one user at a time, from the pool of internal.h.
@@ -1183,13 +1188,15 @@ static int blocked_run(const BlockedInput& in, BlockedOutput* out, Ctx& c, const
     return GBGPU_OK;
 }
 
-// Step 3: the echelon rows prow[0 .. r) of Dp (ascending lead, pivot columns pc,
-// h_first[q] = that of pivot q KB) to reduced echelon form, in place.
+// Step 3: the r echelon rows rs.prow of Dp (ascending lead, pivot columns rs.pc,
+// h_first[q] = that of pivot q KB) to reduced echelon form, in place.  info: the
+// host's view of rs.info.
 template <class F>
 static int back_substitute(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t ncr, int32_t r,
-                           const int32_t* pc, const int32_t* prow,
+                           const RoundState& rs, const volatile RoundInfo* info,
                            const std::vector<int32_t>& h_first, BlockedOutput* out) {
     cudaStream_t s = c.s;
+    const int32_t *pc = rs.pc, *prow = rs.prow;
     const int32_t* piv_of_col = out->piv_of_col;
     StreamOut* so = out->stream_out;
     int32_t* pcd = nullptr;          // pivot columns, descending (the answer's order)
@@ -1219,11 +1226,10 @@ static int back_substitute(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t
         size_t bytes = cscan_bytes;
         BL_CUDA(cub::DeviceScan::ExclusiveSum(cscan, bytes, cnt, loc, kb + 1, s));
         ++c.launches;
-        int64_t blk = 0;
-        BL_CUDA(cudaMemcpyAsync(&blk, loc + kb, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        BL_CUDA(cudaStreamSynchronize(s));
         BL_LAUNCH(k_offs_write<<<grid_of(kb + 1), 256, 0, s>>>(kb + 1, loc, so->nnz,
-                                                               so->offs + out0));
+                                                               so->offs + out0, &rs.info->entries));
+        BL_CUDA(cudaStreamSynchronize(s));
+        const int64_t blk = info->entries;
         if (blk > 0) {
             int32_t* bc = nullptr;
             uint8_t* bw = nullptr;
@@ -1462,7 +1468,7 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
     if (r > 0) {
         std::vector<int32_t> h_first;
         BL_CHECK(first_columns(c, info, pc, r, &h_first));
-        BL_CHECK(back_substitute(c, f, Dp, ld, ncr, r, pc, prow, h_first, out));
+        BL_CHECK(back_substitute(c, f, Dp, ld, ncr, r, rs, info, h_first, out));
     } else if (out->stream_out) {
         out->stream_out->nnz = 0;
         BL_CUDA(cudaMemsetAsync(out->stream_out->offs, 0, sizeof(int64_t), s));
@@ -1494,7 +1500,7 @@ static int interreduce_run(const InterreduceInput& in, Ctx& c, const F& f) {
     BL_CHECK(first_columns(c, info, rs.pc, in.rows, &h_first));
     BlockedOutput out{};
     out.piv_of_col = in.piv_of_col;
-    return back_substitute(c, f, in.D, in.ld, in.ncols, in.rows, rs.pc, rs.prow, h_first, &out);
+    return back_substitute(c, f, in.D, in.ld, in.ncols, in.rows, rs, info, h_first, &out);
 }
 
 int interreduce_dense(const InterreduceInput& in, long long* launches) {

@@ -21,6 +21,7 @@ constexpr int kInfoFirst = 16000;  // blocks of KB pivots whose first column the
 
 // mapped host memory, written by the kernels below
 struct RoundInfo {
+    int64_t entries;                                // of an answer block (k_offs_write)
     int32_t n_pend, n_dirty, first_panel, n_clean;  // k_round_plan
     int32_t n_new, n_rest;                          // k_round_finish
     int32_t first[kInfoFirst];                      // column of pivot 128 b
