@@ -39,6 +39,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/gbgpu.h"
@@ -232,23 +233,6 @@ __global__ void k_count_below(int32_t n, const int32_t* __restrict__ v, int32_t 
         }
         out[j] = lo;
     }
-}
-
-// x mod p for any 64-bit x (p < 2^31) by Barrett reduction with
-// m = floor((2^64 - 1) / p): the estimated quotient is at most 2 short.
-__device__ __forceinline__ uint32_t mod64(uint64_t x, uint32_t p, uint64_t m) {
-    const uint64_t q = __umul64hi(x, m);
-    uint64_t r = x - q * p;
-    r = r >= p ? r - p : r;
-    r = r >= p ? r - p : r;
-    return (uint32_t)r;
-}
-
-// sum of u_k v_k mod p for u_k, v_k < p < 2^31, from 16-bit halves of v
-// accumulated without reduction (each product < 2^47, at most 128 terms)
-__device__ __forceinline__ uint32_t fold_lohi(uint64_t lo, uint64_t hi, uint32_t p, uint64_t m) {
-    const uint32_t hr = mod64(hi, p, m);
-    return mod64((uint64_t)mod64(lo, p, m) + ((uint64_t)hr << 16), p, m);
 }
 
 constexpr int INV_THREADS = 512;  // threads of k_neg_inverse
@@ -517,6 +501,11 @@ __global__ void k_normalize_at(const int32_t* __restrict__ n_dev, const int32_t*
     }
 }
 
+// k_panel_apply's forms by pivots of a chunk, and the lists of their chunks: cls
+// holds PA_CLASSES counts, then a list of up to n_dirty chunks for each
+constexpr int PA_CLASSES = 3;
+__device__ __forceinline__ int pa_class(int np) { return np <= 32 ? 0 : np <= 64 ? 1 : 2; }
+
 // Reduced row echelon form of one panel (the 128 columns of panel dpanel[d], on
 // the n <= PR rows chunk_rows[d PR + i] of Dp) in the shared memory of one
 // cluster (tiny.cuh).  Its pivots are registered (piv_of_col, is_piv, wflag);
@@ -538,7 +527,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1)
 k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __restrict__ chunk_rows,
                const int32_t* __restrict__ dpanel, const int32_t* __restrict__ cursor,
                int32_t max_rows, int32_t ncr, uint32_t* F_b, int32_t* piv_rows_b, int32_t* n_piv_b,
-               int32_t* piv_of_col, uint8_t* is_piv, int32_t* wflag, F f) {
+               int32_t* piv_of_col, uint8_t* is_piv, int32_t* wflag, int32_t* cls, F f) {
     extern __shared__ __align__(16) uint32_t pf_smem[];
     const int CL = cluster_size(), rk = cluster_rank(), sh = __ffs(CL) - 1;
     const int d = blockIdx.x / CL, tid = threadIdx.x;
@@ -564,7 +553,13 @@ k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __res
     }
     __syncthreads();
     if (rk == 0) {
-        if (tid == 0) n_piv_b[d] = np;
+        if (tid == 0) {
+            n_piv_b[d] = np;
+            if (np > 0) {
+                const int q = gridDim.x == CL ? PA_CLASSES - 1 : pa_class(np);
+                cls[PA_CLASSES + q * (gridDim.x / CL) + atomicAdd(&cls[q], 1)] = d;
+            }
+        }
         for (int k = tid; k < np; k += kTinyThreads) {
             const int32_t row = rows[prow[s_col[k]]], col = pj + s_col[k];
             piv_rows_b[d * KB + k] = row;
@@ -581,216 +576,172 @@ k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __res
     }
 }
 
-// The panel transformation of every factorized chunk on CUDA cores: the pivot
-// rows of chunk d become F_d old over the columns from the first dirty panel on
-// (k_panel_factor), a small GEMM per chunk (np x np times np x width) done with
-// register tiles: a block owns tiles of 64 columns of one chunk; it stages the
-// rows of F transposed (A^T, np x 16 QC) once and, per tile, the old values of
-// the chunk's pivot rows (T, np x 64).  Every thread forms 4 pivots x QC columns,
-// one 16-byte read of A^T and QC reads of T per step of the sum; QC (1, 2 or 4)
-// is the smallest that covers the chunk's pivots in one pass (16 QC pivots), so
-// that every thread has work; chunks of more than 64 pivots take two passes.
-// 64-bit sums without reduction (p < 2^16: each product < 2^32, at most 128 of
-// them; otherwise the column value in 16-bit halves), one reduction per result.
-// A block reads all of a tile's columns before it writes any (it owns them), so
-// the update is in place.
-constexpr int PA_COLS = 64;
+// The panel transformation of every factorized chunk: the pivot rows of chunk d
+// become F_d old over the columns from the first dirty panel on (k_panel_factor),
+// np x np times np x width per chunk, in place.  A warp owns 16 columns of a chunk: it
+// reads all old values there before it writes any.
+//
+// On CUDA cores this is bound by the 64-bit multiply-adds (four issue cycles per
+// warp each: 178 us for 5000 pivot rows in chunks of 32 over 10000 columns), and
+// the chunks are too small and too many for the pipeline of tc_gemm.cu.  So the
+// products run on warp-level int8 matrix instructions straight from registers,
+// residues in L unsigned bytes as there: the old values of four rows at a column
+// are the four bytes of an operand register, and 16 columns of np rows stay in
+// registers.  What is left is reading and writing the rows (and, for four bytes,
+// the instructions' rate).  All rounds of a staircase matrix, CUDA cores before,
+// matrix instructions now: 859 -> 475 us (20000 columns, p = 65521), 295 -> 140
+// (10000, p = 251), 293 -> 264 (9001, p = 2^31 - 1); the one panel of an
+// 8192-column dense block 41 -> 13 us.
+//
+// Forms by pivots, KC blocks of 32: registers for the old values.  A block takes
+// work items (a chunk of its class, `width` columns of it) in turn: a grid over all
+// chunks launched mostly blocks without work (97 us for a round of 157 chunks).
 constexpr int PA_THREADS = 256;
-constexpr int PA_PB = 64;            // most pivots per pass (QC = 4)
-constexpr int PA_SMALL_ROWS = 32;    // chunks up to this many pivots: k_panel_apply_small
-constexpr int PA_ALD = PA_PB + 4;    // row stride of A^T (16-byte aligned rows)
-constexpr int PA_SMEM = (KB * PA_COLS + KB * PA_ALD) * (int)sizeof(uint32_t);
+constexpr int PA_COLS = 16;  // of a warp at a time
+struct PanelApply {
+    uint32_t* Dp;
+    int64_t ld;
+    int32_t ncr, j0, width, n_dirty;
+    const int32_t *cls, *dpanel, *n_piv, *piv_rows;
+    const uint32_t* F;
+};
 
-// the sums of one pass: pivots kp + 4 pg + q (q < 4, below kp + kn) times
-// columns cg + (64 / QC) u (u < QC) of the tile at c0, written to the pivots'
-// rows
-template <bool WIDE, int QC>
-__device__ __forceinline__ void pa_pass(uint32_t* Dp, int64_t ld, int32_t ncr, int c0, int n,
-                                        int kp, int kn, const uint32_t (*T)[PA_COLS],
-                                        const uint32_t (*At)[PA_ALD], const int32_t* s_rows,
-                                        uint32_t p, uint64_t m) {
-    constexpr int CG = PA_COLS / QC;  // column groups
-    const int cg = threadIdx.x % CG, pg = threadIdx.x / CG;
-    if (4 * pg >= kn) return;
-    uint64_t lo[4][QC], hi[4][QC];
+__device__ __forceinline__ void mma_u8(int32_t (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                       uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+        "{%8, %9}, {%0, %1, %2, %3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// byte l of x[0 .. 4)
+template <int L>
+__device__ __forceinline__ void pack_bytes(const uint32_t (&x)[4], uint32_t (&out)[L]) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int u = 0; u < QC; ++u) lo[q][u] = hi[q][u] = 0;
-    const bool full = 4 * pg + 4 <= kn;
-#pragma unroll 2
-    for (int j = 0; j < n; ++j) {
-        uint4 a4 = *(const uint4*)&At[j][4 * pg];
-        if (!full) {  // entries past kn are not this pass's pivots
-            const int r = kn - 4 * pg;
-            if (r < 4) a4.w = 0u;
-            if (r < 3) a4.z = 0u;
-            if (r < 2) a4.y = 0u;
-        }
-        const uint32_t a[4] = {a4.x, a4.y, a4.z, a4.w};
-        uint32_t v[QC];
-#pragma unroll
-        for (int u = 0; u < QC; ++u) v[u] = T[j][cg + CG * u];
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-            for (int u = 0; u < QC; ++u) {
-                if (WIDE) {
-                    lo[q][u] += (uint64_t)a[q] * (v[u] & 0xFFFFu);
-                    hi[q][u] += (uint64_t)a[q] * (v[u] >> 16);
-                } else {
-                    lo[q][u] += (uint64_t)a[q] * v[u];
-                }
-            }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int k = kp + 4 * pg + q;
-        if (k >= kp + kn) break;
-        uint32_t* out = Dp + (size_t)s_rows[k] * ld;
-#pragma unroll
-        for (int u = 0; u < QC; ++u) {
-            const int col = c0 + cg + CG * u;
-            if (col < ncr)
-                out[col] = WIDE ? fold_lohi(lo[q][u], hi[q][u], p, m) : mod64(lo[q][u], p, m);
-        }
+    for (int l = 0; l < L; ++l) {
+        const uint32_t sel = (uint32_t)(l | ((4 + l) << 4));
+        out[l] = __byte_perm(__byte_perm(x[0], x[1], sel), __byte_perm(x[2], x[3], sel), 0x5410u);
     }
 }
 
-// Chunks of at most 32 pivots: a warp per 32-column strip, the strip's old
-// values of the pivot rows in registers (one independent load each), the rows of
-// F broadcast from shared memory.  No barrier after the staging.  NJ >= np is
-// the unrolled row count.
-template <bool WIDE, int NJ>
-__device__ __forceinline__ void pa_small(uint32_t* Dp, int64_t ld, int32_t ncr, int c_lo,
-                                         int c_hi, int np, const uint32_t* Es,
-                                         const int32_t* s_rows, uint32_t p, uint64_t m) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int s0 = c_lo + 32 * warp; s0 < c_hi; s0 += 32 * (PA_THREADS / 32)) {
-        const int col = s0 + lane;
-        const bool ok = col < c_hi && col < ncr;
-        uint32_t v[NJ];
+// sum_w s[w] 2^(8 w) mod p, s[w] <= min(w + 1, 2 L - 1 - w) 128 255^2 < 2^25
+template <int L, class F>
+__device__ __forceinline__ uint32_t fold_weights(const int32_t (&s)[2 * L - 1], const F& f) {
+    uint64_t t = (uint32_t)s[0];
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) v[j] = (ok && j < np) ? Dp[(size_t)s_rows[j] * ld + col] : 0u;
-        for (int k = 0; k < np; ++k) {
-            const uint32_t* e = Es + k * 32;
-            uint64_t lo = 0, hi = 0;
-#pragma unroll
-            for (int j = 0; j < NJ; ++j) {
-                const uint32_t a = e[j];  // zero for j >= np
-                if (WIDE) {
-                    lo += (uint64_t)a * (v[j] & 0xFFFFu);
-                    hi += (uint64_t)a * (v[j] >> 16);
-                } else {
-                    lo += (uint64_t)a * v[j];
-                }
-            }
-            if (ok) Dp[(size_t)s_rows[k] * ld + col] = WIDE ? fold_lohi(lo, hi, p, m) : mod64(lo, p, m);
-        }
+    for (int w = 1; w < (L < 4 ? 2 * L - 1 : 4); ++w) t += (uint64_t)(uint32_t)s[w] << (8 * w);
+    // L = 2: t < 2^41; L = 4: t < 2^50 and t <= 128 p^2, one of them below p 2^32
+    uint32_t r = f.lazy_mod(t);
+    if constexpr (L == 4) {
+        uint64_t h = (uint32_t)s[4];
+        h += (uint64_t)(uint32_t)s[5] << 8;
+        h += (uint64_t)(uint32_t)s[6] << 16;
+        r += f.prep(f.lazy_mod(h));  // prep: times 2^32
+        r = r >= f.p ? r - f.p : r;
     }
+    return r;
 }
 
-template <bool WIDE>
-__global__ void __launch_bounds__(PA_THREADS)
-k_panel_apply(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_per_block,
-              const int32_t* __restrict__ dpanel, const uint32_t* __restrict__ F_b,
-              const int32_t* __restrict__ n_piv_b, const int32_t* __restrict__ piv_rows_b,
-              uint32_t p) {
-    extern __shared__ __align__(16) uint32_t pa_smem[];
-    uint32_t(*T)[PA_COLS] = (uint32_t(*)[PA_COLS])pa_smem;
-    uint32_t(*At)[PA_ALD] = (uint32_t(*)[PA_ALD])(pa_smem + KB * PA_COLS);
-    __shared__ int32_t s_rows[KB];
-    const int d = blockIdx.y;
-    const int np = n_piv_b[d];
-    const int pj = dpanel[d] * KB;
-    // the block's tiles: [tile0, tile1), the first one right of the chunk's
-    // panel start (the chunk rows are zero left of it)
-    const int ntiles = (ncr - j0 + PA_COLS - 1) / PA_COLS;
-    int tile0 = blockIdx.x * tiles_per_block;
-    const int tile1 = min(ntiles, tile0 + tiles_per_block);
-    tile0 = max(tile0, pj > j0 ? (pj - j0) / PA_COLS : 0);
-    // uniform: nothing to do, or a chunk for k_panel_apply_small
-    if (tile0 >= tile1 || np <= PA_SMALL_ROWS) return;
-    for (int t = threadIdx.x; t < np; t += PA_THREADS) s_rows[t] = piv_rows_b[(size_t)d * KB + t];
-    __syncthreads();
-    const uint32_t* F = F_b + (size_t)d * KB * KB;
-    const uint64_t m = ~0ull / p;
-    // pivots per pass (uniform over the block): np > 32 here
-    constexpr int pb = PA_PB;
-    // A^T of pivots [kp, kp + kn)
-    auto stage_a = [&](int kp, int kn) {
-        for (int t = threadIdx.x; t < kn * np; t += PA_THREADS) {
-            const int k = t / np, j = t % np;
-            At[j][k] = F[(size_t)(kp + k) * KB + j];
+// bytes of a row of F's planes (a step of 16 beyond it: no bank conflicts)
+constexpr int pa_row(int kc) { return 32 * kc + 16; }
+// blocks per SM (registers)
+constexpr int pa_blocks(int l, int kc) { return l == 4 ? (kc == 4 ? 1 : 2) : (kc == 1 ? 3 : 2); }
+template <int L, int KC, class F>
+__global__ void __launch_bounds__(PA_THREADS, pa_blocks(L, KC))
+k_panel_apply(const PanelApply a, F f) {
+    constexpr int ROW = pa_row(KC), PLANE = 32 * KC * ROW;
+    constexpr int NT = PA_COLS / 8, NW = 2 * L - 1, CLS = KC == 1 ? 0 : KC == 2 ? 1 : 2;
+    extern __shared__ __align__(16) uint8_t s_f[];  // planes of F
+    __shared__ int32_t s_rows[32 * KC];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane / 4, t = lane % 4;
+    const int n = a.cls[CLS];
+    const int items = n * ((a.ncr - a.j0 + a.width - 1) / a.width);
+    for (int i = blockIdx.x; i < items; i += gridDim.x) {
+        const int d = a.cls[PA_CLASSES + CLS * a.n_dirty + i % n];
+        // its rows are zero left of the chunk's panel
+        const int c_lo = max(a.j0 + i / n * a.width, a.dpanel[d] * KB);
+        const int c_hi = min(a.ncr, a.j0 + (i / n + 1) * a.width);
+        if (c_lo >= c_hi) continue;  // uniform
+        const int np = a.n_piv[d], mt = (np + 15) / 16;
+        __syncthreads();  // the last item's readers are done
+        for (int q = tid; q < 32 * KC; q += PA_THREADS)
+            s_rows[q] = q < np ? a.piv_rows[(size_t)d * KB + q] : -1;
+        const uint32_t* Fd = a.F + (size_t)d * KB * KB;
+#pragma unroll 4
+        for (int q = tid; q < mt * 16 * 8 * KC; q += PA_THREADS) {
+            const int k = q / (8 * KC), j = 4 * (q % (8 * KC));
+            uint4 e = make_uint4(0u, 0u, 0u, 0u);  // (past np: whatever is there)
+            if (k < np && j < np) e = *(const uint4*)(Fd + k * KB + j);
+            const uint32_t x[4] = {e.x, j + 1 < np ? e.y : 0u, j + 2 < np ? e.z : 0u,
+                                   j + 3 < np ? e.w : 0u};
+            uint32_t y[L];
+            pack_bytes<L>(x, y);
+#pragma unroll
+            for (int l = 0; l < L; ++l) *(uint32_t*)&s_f[l * PLANE + k * ROW + j] = y[l];
         }
-    };
-    const bool one_pass = np <= pb;
-    if (one_pass) stage_a(0, np);  // once for all tiles
-    for (int tile = tile0; tile < tile1; ++tile) {
-        const int c0 = j0 + tile * PA_COLS;
-        __syncthreads();  // the last tile's readers of T are done
-        {
-            // np x 64 old values, eight independent loads per thread at a time
-            const int total = np * PA_COLS;
-            for (int t0 = threadIdx.x; t0 < total; t0 += 8 * PA_THREADS) {
-                uint32_t v[8];
+        __syncthreads();
+        for (int c0 = c_lo + PA_COLS * warp; c0 < c_hi; c0 += PA_COLS * (PA_THREADS / 32)) {
+            // old values: register (kc, h, nt) of a lane holds rows 32 kc + 16 h + 4 t
+            // .. + 3 at column c0 + 8 nt + g
+            uint32_t bv[L][KC][2][NT];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int t = t0 + q * PA_THREADS;
-                    const int j = t / PA_COLS, col = c0 + t % PA_COLS;
-                    v[q] = (t < total && col < ncr) ? Dp[(size_t)s_rows[j] * ld + col] : 0u;
-                }
+            for (int kc = 0; kc < KC; ++kc)
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int t = t0 + q * PA_THREADS;
-                    if (t < total) T[t / PA_COLS][t % PA_COLS] = v[q];
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        const int col = c0 + 8 * nt + g;
+                        uint32_t x[4], y[L];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int32_t r = s_rows[32 * kc + 16 * h + 4 * t + u];
+                            x[u] = r >= 0 && col < c_hi ? a.Dp[(size_t)r * a.ld + col] : 0u;
+                        }
+                        pack_bytes<L>(x, y);
+#pragma unroll
+                        for (int l = 0; l < L; ++l) bv[l][kc][h][nt] = y[l];
+                    }
+            __syncwarp();  // every lane has read before any writes
+            for (int m = 0; m < mt; ++m) {
+                int32_t acc[NT][NW][4];
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int w = 0; w < NW; ++w)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) acc[nt][w][q] = 0;
+#pragma unroll
+                for (int kc = 0; kc < KC; ++kc)
+#pragma unroll
+                    for (int la = 0; la < L; ++la) {
+                        const uint8_t* p0 = &s_f[la * PLANE + (16 * m + g) * ROW + 32 * kc + 4 * t];
+                        const uint32_t af[4] = {*(const uint32_t*)p0, *(const uint32_t*)(p0 + 8 * ROW),
+                                                *(const uint32_t*)(p0 + 16),
+                                                *(const uint32_t*)(p0 + 8 * ROW + 16)};
+#pragma unroll
+                        for (int lb = 0; lb < L; ++lb)
+#pragma unroll
+                            for (int nt = 0; nt < NT; ++nt)
+                                mma_u8(acc[nt][la + lb], af, bv[lb][kc][0][nt], bv[lb][kc][1][nt]);
+                    }
+                // entry q: pivot 16 m + g + 8 (q / 2), column c0 + 8 nt + 2 t + q % 2
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int32_t r = s_rows[16 * m + g + 8 * (q / 2)];
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        int32_t sw[NW];
+#pragma unroll
+                        for (int w = 0; w < NW; ++w) sw[w] = acc[nt][w][q];
+                        const int col = c0 + 8 * nt + 2 * t + q % 2;
+                        const uint32_t v = fold_weights<L>(sw, f);
+                        if (r >= 0 && col < c_hi) a.Dp[(size_t)r * a.ld + col] = v;
+                    }
                 }
             }
-        }
-        for (int kp = 0; kp < np; kp += pb) {
-            const int kn = min(pb, np - kp);
-            if (!one_pass) {
-                __syncthreads();  // the last pass's readers of A^T are done
-                stage_a(kp, kn);
-            }
-            __syncthreads();  // T and A^T are in place
-            pa_pass<WIDE, 4>(Dp, ld, ncr, c0, np, kp, kn, T, At, s_rows, p, m);
         }
     }
-}
-
-// the chunks of k_panel_apply with at most PA_SMALL_ROWS pivots
-template <bool WIDE>
-__global__ void __launch_bounds__(PA_THREADS)
-k_panel_apply_small(uint32_t* Dp, int64_t ld, int32_t ncr, int32_t j0, int32_t tiles_per_block,
-                    const int32_t* __restrict__ dpanel, const uint32_t* __restrict__ F_b,
-                    const int32_t* __restrict__ n_piv_b, const int32_t* __restrict__ piv_rows_b,
-                    uint32_t p) {
-    __shared__ uint32_t Es[PA_SMALL_ROWS * 32];
-    __shared__ int32_t s_rows[PA_SMALL_ROWS];
-    const int d = blockIdx.y;
-    const int np = n_piv_b[d];
-    const int pj = dpanel[d] * KB;
-    const int ntiles = (ncr - j0 + PA_COLS - 1) / PA_COLS;
-    int tile0 = blockIdx.x * tiles_per_block;
-    const int tile1 = min(ntiles, tile0 + tiles_per_block);
-    tile0 = max(tile0, pj > j0 ? (pj - j0) / PA_COLS : 0);
-    if (np == 0 || tile0 >= tile1 || np > PA_SMALL_ROWS) return;  // uniform
-    for (int t = threadIdx.x; t < PA_SMALL_ROWS; t += PA_THREADS)
-        s_rows[t] = t < np ? piv_rows_b[(size_t)d * KB + t] : 0;
-    // the rows of F, 32 entries each (zero past np)
-    const uint32_t* F = F_b + (size_t)d * KB * KB;
-    for (int t = threadIdx.x; t < np * 32; t += PA_THREADS)
-        Es[t] = t % 32 < np ? F[(size_t)(t / 32) * KB + t % 32] : 0u;
-    __syncthreads();
-    const uint64_t m = ~0ull / p;
-    const int c_lo = j0 + tile0 * PA_COLS, c_hi = min(ncr, j0 + tile1 * PA_COLS);
-    if (np <= 8)
-        pa_small<WIDE, 8>(Dp, ld, ncr, c_lo, c_hi, np, Es, s_rows, p, m);
-    else if (np <= 16)
-        pa_small<WIDE, 16>(Dp, ld, ncr, c_lo, c_hi, np, Es, s_rows, p, m);
-    else
-        pa_small<WIDE, 32>(Dp, ld, ncr, c_lo, c_hi, np, Es, s_rows, p, m);
 }
 
 // dst block b (NB x NB, leading dimension NB, block stride NB (NB + 1)) =
@@ -933,6 +884,23 @@ static int gemm_set_batched(Ctx& c, uint32_t* D, int64_t ldd, int64_t sD, const 
     g.sB = sB;
     g.sD = sD;
     return gemm_args(c, g);
+}
+
+template <int L, class F>
+static int panel_apply(Ctx& c, const PanelApply& a, const F& f) {
+    auto launch = [&](auto kernel, int kc) -> int {
+        const int per_sm = pa_blocks(L, kc);
+        const int bytes = L * 32 * kc * pa_row(kc);
+        BL_CUDA(ensure_smem_limit((const void*)kernel, bytes));
+        BL_LAUNCH(kernel<<<148 * per_sm, PA_THREADS, bytes, c.s>>>(a, f));
+        return GBGPU_OK;
+    };
+    if (a.n_dirty > 1) {  // one alone is in the class of 128 (k_panel_factor)
+        BL_CHECK(launch(k_panel_apply<L, 1, F>, 1));
+        BL_CHECK(launch(k_panel_apply<L, 2, F>, 2));
+    }
+    BL_CHECK(launch(k_panel_apply<L, 4, F>, 4));
+    return GBGPU_OK;
 }
 
 // elimination block size: powers of two from 128 to `cap` (1024 by default)
@@ -1346,12 +1314,13 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
     rs.prow = c.alloc<int32_t>(ncr);  // their rows
     rs.pend = c.alloc<int32_t>(t);
     rs.n_new = counters;
+    rs.cls = c.alloc<int32_t>(PA_CLASSES * (1 + (size_t)max_dirty));
     int32_t *pc = rs.pc, *prow = rs.prow, *pend = rs.pend;
     uint32_t* panF = c.alloc<uint32_t>((size_t)max_dirty * KB * KB);
     int32_t* n_piv = c.alloc<int32_t>(max_dirty);
     int32_t* piv_rows = c.alloc<int32_t>((size_t)max_dirty * KB);
     if (!lead || !is_piv || !counters || !rs.wflag || !rs.hist || !rs.pdirty || !rs.dslot ||
-        !rs.dpanel || !rs.cursor || !rs.chunk_rows || !rs.per_warp || !pc || !prow || !pend ||
+        !rs.dpanel || !rs.cursor || !rs.chunk_rows || !rs.per_warp || !rs.cls || !pc || !prow || !pend ||
         !panF || !n_piv || !piv_rows)
         return GBGPU_ENOMEM;
     // the counts the host sizes launches from
@@ -1386,36 +1355,19 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
                 int64_t ld_ = ld;
                 F fv = f;
                 void* args[] = {&Dp, &ld_, &rs.chunk_rows, &rs.dpanel, &rs.cursor, &rows_, &nc_, &panF,
-                                &piv_rows, &n_piv, &piv_of_col, &is_piv, &rs.wflag, &fv};
+                                &piv_rows, &n_piv, &piv_of_col, &is_piv, &rs.wflag, &rs.cls, &fv};
                 BL_LAUNCH(BL_CUDA(launch_cluster((const void*)k_panel_factor<F>, n_dirty * cl, cl,
                                                  kTinyThreads,
                                                  (int)tiny_layout(rows_, KB, cl).words * 4, s, args)));
             }
-            {
-                // pivot rows of every chunk <- F_d old (CUDA cores, in place), columns j0..
-                const bool wide = c.p >= 65536u;
-                // tiles per block: enough blocks for about six per SM, at most 8
-                // tiles each (a block stages the rows of F once for its tiles)
-                const int tiles = (width + PA_COLS - 1) / PA_COLS;
-                const int tpb = (int)std::max<int64_t>(
-                    1, std::min<int64_t>(8, (int64_t)tiles * n_dirty / (148 * 6)));
-                const dim3 grid((unsigned)((tiles + tpb - 1) / tpb), (unsigned)n_dirty);
-                // the chunks of more than 32 pivots are few and long: one tile per block
-                const dim3 grid1((unsigned)tiles, (unsigned)n_dirty);
-                if (wide) {
-                    BL_CUDA(ensure_smem_limit((const void*)k_panel_apply<true>, PA_SMEM));
-                    BL_LAUNCH(k_panel_apply_small<true><<<grid, PA_THREADS, 0, s>>>(
-                        Dp, ld, ncr, j0, tpb, rs.dpanel, panF, n_piv, piv_rows, c.p));
-                    BL_LAUNCH(k_panel_apply<true><<<grid1, PA_THREADS, PA_SMEM, s>>>(
-                        Dp, ld, ncr, j0, 1, rs.dpanel, panF, n_piv, piv_rows, c.p));
-                } else {
-                    BL_CUDA(ensure_smem_limit((const void*)k_panel_apply<false>, PA_SMEM));
-                    BL_LAUNCH(k_panel_apply_small<false><<<grid, PA_THREADS, 0, s>>>(
-                        Dp, ld, ncr, j0, tpb, rs.dpanel, panF, n_piv, piv_rows, c.p));
-                    BL_LAUNCH(k_panel_apply<false><<<grid1, PA_THREADS, PA_SMEM, s>>>(
-                        Dp, ld, ncr, j0, 1, rs.dpanel, panF, n_piv, piv_rows, c.p));
-                }
-            }
+            // pivot rows of every chunk <- F_d old, in place, columns j0..; one chunk
+            // alone needs the narrow items to fill the SMs
+            const PanelApply pa{Dp, ld, ncr, j0, n_dirty == 1 ? 128 : 512, n_dirty, rs.cls, rs.dpanel,
+                                n_piv, piv_rows, panF};
+            if constexpr (std::is_same<F, FieldSmall>::value)
+                BL_CHECK(c.p < 256u ? panel_apply<1>(c, pa, f) : panel_apply<2>(c, pa, f));
+            else
+                BL_CHECK(panel_apply<4>(c, pa, f));
             if (trace_rounds()) {
                 std::vector<int32_t> h_cur(n_dirty), h_np(n_dirty);
                 BL_CUDA(cudaMemcpyAsync(h_cur.data(), rs.cursor, 4 * n_dirty, cudaMemcpyDeviceToHost, s));

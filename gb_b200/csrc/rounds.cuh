@@ -40,6 +40,7 @@ struct RoundState {
     int32_t* cursor;       // [max_dirty]: rows of a chunk's panel
     int32_t* chunk_rows;   // [max_dirty][pr]
     int32_t* per_warp;     // [RD_WARPS][max_dirty]
+    int32_t* cls;          // k_panel_apply's lists, their three counts first
     int32_t *pc, *prow;    // [ncr]: pivot columns ascending, their rows
     int32_t* pend;         // [t]: rows left
     int32_t* n_new;        // device copy of info->n_new
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_round_plan(const RoundState a, i
         a.dslot[q] = -1;
     }
     if (tid == 0) s_pend = s_clean = s_dirty = 0;
+    if (tid < 3) a.cls[tid] = 0;
     __syncthreads();
     const int run = (a.t + RD_THREADS - 1) / RD_THREADS * 32;  // rows of a warp
     const int r0 = warp * run, r1 = min(a.t, r0 + run);

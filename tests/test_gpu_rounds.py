@@ -70,3 +70,28 @@ def test_dense_rref_rounds(kind, m, n, p):
     assert rank.value == len(piv)
     assert pc.cpu().numpy()[: rank.value].tolist() == piv
     assert np.array_equal(dev.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("p", [3, 251, 65521, 65537, (1 << 24) + 43, 2147483647])
+@pytest.mark.parametrize("rows,n", [
+    ((2, 33, 64), 400), ((65, 16, 128), 397), ((31, 32, 17, 127, 63), 645), ((130, 1, 129), 500)])
+def test_chunks_of_every_size(rows, n, p):
+    """panel q has rows[q] rows of its own, so its chunk finds up to that many pivots"""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n + len(rows))
+    D = np.zeros((sum(rows), n), dtype=np.int64)
+    at = 0
+    for q, r in enumerate(rows):
+        D[at:at + r, 128 * q:] = rng.integers(0, p, size=(r, n - 128 * q))
+        at += r
+    D = D[rng.permutation(at)]
+    want, piv = rref(D, p)
+    dev = torch.from_numpy(D.astype(np.int32)).cuda()
+    pc = torch.zeros(min(D.shape), dtype=torch.int32, device="cuda")
+    rank = C.c_int32()
+    opt = _lib.Options(_lib.FORM_AUTO, 0, 1, 0, torch.cuda.current_stream().cuda_stream)
+    _lib.check(_lib.load().gbgpu_dense_rref(p, *D.shape, dev.data_ptr(), n, C.byref(rank),
+                                            pc.data_ptr(), C.byref(opt)))
+    assert rank.value == len(piv)
+    assert pc.cpu().numpy()[: rank.value].tolist() == piv
+    assert np.array_equal(dev.cpu().numpy(), want)
