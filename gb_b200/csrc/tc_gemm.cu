@@ -10,7 +10,8 @@
 // of at most floor((2^31-1) / (L 255^2)) columns keeps every S_w below 2^31
 // (kPanelBytes below).  After each panel the epilogue folds the weights,
 //   v = sum_w S_w * (2^(8w) R mod p)   (Montgomery, R = 2^32; one reduction of
-//       the 64-bit sum for up to three limbs, one per two weights for four),
+//       the 64-bit sum) for two and three limbs, one Barrett step of S_0 for one,
+//       three reductions for four,
 // and updates D <- D - v mod p in place, so no partial sum ever leaves [0, p).
 // The result is bit-identical to any exact evaluation of (D - A B) mod p.
 //
@@ -210,7 +211,8 @@ struct TcParams {
     unsigned long long* steps;  // optional: K steps executed, summed over tiles
     uint32_t p, pneg_inv;
     uint32_t mu;     // floor(2^32 / p)
-    uint32_t cw[7];  // 2^(8w) R mod p
+    uint32_t cw[5];    // 2^(8w) R mod p
+    uint32_t r2, r3;   // R^2, R^3 mod p
     int32_t set;     // D <- -A B: D is not read
     int32_t* err;
     long long budget;
@@ -577,7 +579,23 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                     const int c0 = cbeg + 32 * b;
                     uint32_t(&d)[32] = dv[b % PRE];
                     uint32_t v[32];
-                    if constexpr (L <= 3) {
+                    const uint32_t acc_q = tmem + ((uint32_t)(q * 32) << 16) + acc_base + (uint32_t)c0;
+                    if constexpr (L == 1) {
+                        // S_0 < 2^31: one Barrett step (through the weights' sum
+                        // 8192 x 8192 x 128 took 190 us, 181 now)
+                        uint32_t a[2][16];
+                        tmem_ld16(acc_q, a[0]);
+                        tmem_ld16(acc_q + 16, a[1]);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            tmem_wait(a[h]);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const uint32_t r = a[h][j] - __umulhi(a[h][j], prm.mu) * p;
+                                v[16 * h + j] = r >= p ? r - p : r;
+                            }
+                        }
+                    } else if constexpr (L <= 3) {
                         // one Montgomery reduction of the weighted sum:
                         // T = sum_w S_w (2^(8w) R mod p) < (2L - 1) 2^31 p, so
                         // (T + q p) / 2^32 < 2^32, then one Barrett step; 16
@@ -587,9 +605,7 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                             uint32_t a[C::NW][16];
 #pragma unroll
                             for (int w = 0; w < C::NW; ++w)
-                                tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
-                                              (uint32_t)(w * C::BN + c0 + h),
-                                          a[w]);
+                                tmem_ld16(acc_q + (uint32_t)(w * C::BN + h), a[w]);
                             uint64_t T[16];
 #pragma unroll
                             for (int w = 0; w < C::NW; ++w) {
@@ -608,35 +624,39 @@ k_tc_submul(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CU
                             }
                         }
                     } else {
-                        // two weights per reduction: T < 2 2^31 p, so
-                        // (T + q p) / 2^32 < 2 p
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = 0;
+                        // t0 = S_0 + .. + S_3 2^24 and t1 = S_4 + .. + S_6 2^16, both
+                        // below 2^56 <= p 2^32: redc(t0) R^2 + redc(t1) R^3 < 2 p^2,
+                        // and its redc is t0 + t1 2^32 (a reduction per two weights
+                        // took 388 us for 8192 x 8192 x 128, 349 now).  The same
+                        // by shifts for two limbs needs registers in flight that the
+                        // D values have: 225 -> 233 to 296 us
+                        auto redc = [&](uint64_t T) {
+                            const uint32_t qq = (uint32_t)T * prm.pneg_inv;
+                            const uint32_t r = (uint32_t)((T + (uint64_t)qq * p) >> 32);
+                            return r >= p ? r - p : r;
+                        };
 #pragma unroll
                         for (int h = 0; h < 32; h += 16) {
+                            uint32_t a[4][16], u[16];
 #pragma unroll
-                            for (int w = 0; w < C::NW; w += 2) {
-                                uint32_t a[16], a2[16];
-                                tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
-                                              (uint32_t)(w * C::BN + c0 + h),
-                                          a);
-                                if (w + 1 < C::NW)
-                                    tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + acc_base +
-                                                  (uint32_t)((w + 1) * C::BN + c0 + h),
-                                              a2);
-                                tmem_wait(a);
-                                if (w + 1 < C::NW) tmem_wait(a2);
-                                const uint32_t cw = prm.cw[w], cw2 = prm.cw[w + 1 < C::NW ? w + 1 : w];
+                            for (int w = 0; w < 4; ++w)
+                                tmem_ld16(acc_q + (uint32_t)(w * C::BN + h), a[w]);
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) {
-                                    uint64_t T = (uint64_t)a[j] * cw;
-                                    if (w + 1 < C::NW) T += (uint64_t)a2[j] * cw2;
-                                    const uint32_t qq = (uint32_t)T * prm.pneg_inv;
-                                    uint32_t r = (uint32_t)((T + (uint64_t)qq * p) >> 32);
-                                    r = r >= p ? r - p : r;
-                                    const uint32_t sum = v[h + j] + r;
-                                    v[h + j] = sum >= p ? sum - p : sum;
-                                }
+                            for (int w = 0; w < 4; ++w) tmem_wait(a[w]);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                u[j] = redc(a[0][j] + ((uint64_t)a[1][j] << 8) +
+                                            ((uint64_t)a[2][j] << 16) + ((uint64_t)a[3][j] << 24));
+#pragma unroll
+                            for (int w = 4; w < 7; ++w)
+                                tmem_ld16(acc_q + (uint32_t)(w * C::BN + h), a[w - 4]);
+#pragma unroll
+                            for (int w = 0; w < 3; ++w) tmem_wait(a[w]);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const uint32_t y = redc(a[0][j] + ((uint64_t)a[1][j] << 8) +
+                                                        ((uint64_t)a[2][j] << 16));
+                                v[h + j] = redc((uint64_t)u[j] * prm.r2 + (uint64_t)y * prm.r3);
                             }
                         }
                     }
@@ -1109,8 +1129,10 @@ static int tc_run(const TcGemmArgs& g, uint8_t* planes, cudaStream_t s, int32_t*
     prm.pneg_inv = f.pneg_inv;
     prm.mu = (uint32_t)((((uint64_t)1) << 32) / g.p);
     const uint64_t R = ((uint64_t)1 << 32) % g.p;
+    prm.r2 = (uint32_t)(R * R % g.p);
+    prm.r3 = (uint32_t)((uint64_t)prm.r2 * R % g.p);
     uint64_t pw = 1;
-    for (int w = 0; w < 7; ++w) {
+    for (int w = 0; w < 5; ++w) {
         prm.cw[w] = (uint32_t)((pw % g.p) * R % g.p);
         pw = (pw << 8) % g.p;
     }
