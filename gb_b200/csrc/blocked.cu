@@ -518,7 +518,7 @@ __device__ __forceinline__ int pa_class(int np) { return np <= 32 ? 0 : np <= 64
 // What bounds it is the chain of pivots (sixteen at a time, tiny.cuh).  A step
 // per pivot over all of the chunk's rows, with the transformation beside the
 // panel, took 191 us for 128 rows of a full panel on one SM; here one panel takes
-// 135 us with 256 candidate rows on eight SMs, and more candidates than pivots
+// 92 us with 256 candidate rows on eight SMs, and more candidates than pivots
 // keep a dense panel from running short of independent rows (an 8192 x 8192
 // block of rank 6144 takes 48 rounds instead of 76).
 
@@ -542,12 +542,14 @@ k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __res
     const int np = tiny_echelon<true>(n, KB, pf_smem, f);
     // pivots in column order: place of column c = pivot columns left of it
     const int32_t* prow = (const int32_t*)(pf_smem + L.cols);
-    __shared__ int32_t s_col[KB];
+    __shared__ int32_t s_col[KB], s_place[KB];
     if (tid < 32) {
         int at = 0;
         for (int c = tid; c < KB; c += 32) {
             const unsigned bal = __ballot_sync(0xffffffffu, prow[c] >= 0);
-            if (prow[c] >= 0) s_col[at + __popc(bal & ((1u << tid) - 1u))] = c;
+            const int k = at + __popc(bal & ((1u << tid) - 1u));
+            s_place[c] = prow[c] >= 0 ? k : -1;
+            if (prow[c] >= 0) s_col[k] = c;
             at += __popc(bal);
         }
     }
@@ -569,11 +571,12 @@ k_panel_factor(const uint32_t* __restrict__ Dp, int64_t ld, const int32_t* __res
         }
     }
     uint32_t* Fo = F_b + (size_t)d * KB * KB;
-    for (int q = tid; q < np * np; q += kTinyThreads) {
-        const int k = q / np, c = s_col[q % np];
-        if (((c / TP) & (CL - 1)) == rk)
-            Fo[k * KB + q % np] = pf_smem[tiny_at(n, prow[s_col[k]], c, sh)];
-    }
+    // this CTA's columns of F
+    for (int t = rk; t < KB / TP; t += CL)
+        for (int q = tid; q < np * TP; q += kTinyThreads) {
+            const int k = q / TP, j = s_place[t * TP + q % TP];
+            if (j >= 0) Fo[k * KB + j] = pf_smem[((t >> sh) * n + prow[s_col[k]]) * TP + q % TP];
+        }
 }
 
 // The panel transformation of every factorized chunk: the pivot rows of chunk d

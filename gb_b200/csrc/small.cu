@@ -18,10 +18,9 @@
 //   one stream synchronisation.
 //
 // Measured on a B200, 441 x 491 matrix (141 x 191 block, p = 32003): 1425 us a
-// call with one CTA for the echelon and a launch per phase, 244 us now, of it
-// k_small 207 us (checks and diagonal blocks 22, rows 75, echelon 110; all three
-// are chains of dependent steps on a few SMs, not throughput); over 2^31 - 1,
-// 2430 and 276 us.  Matrices with more rows or a longer chain of left columns
+// call with one CTA for the echelon and a launch per phase, 220 us now, of it
+// k_small 181 us (checks and diagonal blocks 22, rows 75, echelon 84; all three
+// are chains of dependent steps on a few SMs, not throughput).  Matrices with more rows or a longer chain of left columns
 // run the three phases as launches of their own, the rows on the whole device
 // (kWideRows below).
 //

@@ -11,7 +11,7 @@
 //     copies it to every CTA, and every CTA finds the panel's pivots by itself;
 //   * the columns right of the panel are updated once per panel by their
 //     owners, with 64-bit sums of TP products and one reduction per entry.
-// One cluster barrier per panel, none per pivot.
+// One or two cluster barriers per panel, none per pivot.
 //
 // The panel's pivots come from TP rows at a time (the first row of every lead,
 // then any others): their TP x TP entries are brought to reduced echelon form,
@@ -42,6 +42,7 @@ constexpr int kTinyThreads = 512;
 constexpr int kTinyWarps = kTinyThreads / 32;
 constexpr int kTinyMaxCluster = 8;          // the portable limit
 constexpr int TP = 16;                      // panel columns
+constexpr int kRelayRows = 64;              // from here panels are passed on in two steps
 // Shared memory of one CTA for an n x m block in a cluster of cl (offsets in
 // 32-bit words): its panels [panels / cl][n][TP], two copies of the current
 // panel [n][TP], the pivots' TP x TP blocks (F, the pivot rows in the panel, and
@@ -199,17 +200,16 @@ __device__ void tiny_turn(const int n_sel, const int c0, const uint32_t* pb, int
         const uint32_t si = cur ? S.scl2[i] : s_scl[i];
         pmask |= 1u << c;
         done |= 1u << i;
-        if (q == i) {
-            if (j == c) y = scl;
-            scl = 0u;
-            pval = a;
-            my_col = c;
-        } else if (mr != 0u) {
-            const uint32_t ap = f.prep(a), mn = f.prep(f.p - mr);
-            y = j == c ? f.mulp(si, mn) : f.ffsub(y, ap, v, mn);
-            scl = f.mulp(scl, ap);
-            pval = f.mulp(pval, ap);
-        }
+        // (selects: the pivot's warp would run both sides of a branch; a row with
+        // mr = 0 is scaled by a like the others)
+        const uint32_t ap = f.prep(a), mn = f.prep(f.p - mr);
+        const uint32_t z = j == c ? f.mulp(si, mn) : f.ffsub(y, ap, v, mn);
+        const uint32_t s2 = f.mulp(scl, ap), p2 = f.mulp(pval, ap);
+        const bool pivot = q == i;
+        y = pivot ? (j == c ? scl : y) : z;
+        scl = pivot ? 0u : s2;
+        pval = pivot ? a : p2;
+        my_col = pivot ? c : my_col;
         cur ^= 1;
         buf[cur * TP * TP + tid] = y;
         if (j == 0) (cur ? S.scl2 : s_scl)[q] = scl;
@@ -384,20 +384,38 @@ __device__ int tiny_echelon(const int32_t n, const int32_t m, uint32_t* smem, co
     int32_t* prow = (int32_t*)(smem + L.cols);      // [m] pivot row of a column, -1
     __shared__ TinyTurn S;
     const int tid = threadIdx.x, lane = tid & 31;
-    // the owner's panel k to every CTA's copy for panel k
+    // Panel k from its owner to every CTA's copy for panel k, and a cluster barrier.
+    // Eight copies of 256 rows (128 KB) out of one SM take 11000 cycles with the
+    // lanes of a warp storing to different CTAs, 6800 with a warp's stores to one
+    // CTA, and 3600 when each CTA gets a part and passes it on, a barrier more.
+    const bool relay = CL > 2 && n >= kRelayRows;
+    const int quads = n * (TP / 4), part = (quads + CL - 1) >> sh;  // 16-byte groups
     auto push = [&](int k) {
+        const bool mine = (k & (CL - 1)) == rk;
         const uint4* src = (const uint4*)(T + (k >> sh) * n * TP);
         const uint32_t* dst = smem + L.pb + (k & 1) * n * TP;
-        for (int t = tid; t < n * (TP / 4) * CL; t += kTinyThreads) {
-            const int q = t >> sh, to = t & (CL - 1);
-            remote_st4(remote_smem(dst + 4 * q, to), src[q]);
+        if (relay) {
+            if (mine)
+                for (int q = tid; q < quads; q += kTinyThreads)
+                    remote_st4(remote_smem(dst + 4 * q, q / part), src[q]);
+            cluster_sync();
+            const int q1 = min(quads, (rk + 1) * part);
+            const int g = tid / 32 % CL, w = tid / 32 / CL;  // warps by destination
+            if (g != rk)
+                for (int q = rk * part + 32 * w + tid % 32; q < q1; q += kTinyThreads / CL)
+                    remote_st4(remote_smem(dst + 4 * q, g), *(const uint4*)(dst + 4 * q));
+        } else if (mine) {
+            for (int q = tid; q < quads; q += kTinyThreads) {
+                const uint4 x = src[q];
+                for (int to = 0; to < CL; ++to) remote_st4(remote_smem(dst + 4 * q, to), x);
+            }
         }
+        cluster_sync();
     };
     for (int c = tid; c < L.panels * TP; c += kTinyThreads) prow[c] = -1;
     for (int r = tid; r < n; r += kTinyThreads) pcol[r] = -1;
     cluster_sync();  // every CTA has started, its panels are in place
-    if (rk == 0) push(0);
-    cluster_sync();
+    push(0);
     constexpr uint32_t kFull = (1u << TP) - 1u;
     int found = 0;  // pivots so far (uniform over the cluster)
     for (int k = 0; k < L.panels; ++k) {
@@ -437,8 +455,7 @@ __device__ int tiny_echelon(const int32_t n, const int32_t m, uint32_t* smem, co
                 own[t] = pmask == kFull ? (pcol[t / TP] == c0 + t % TP ? 1u : 0u) : pb[t];
         }
         if (k + 1 == L.panels) break;
-        if (((k + 1) & (CL - 1)) == rk) push(k + 1);
-        cluster_sync();
+        push(k + 1);
         if (found == n) break;
     }
     cluster_sync();
