@@ -48,9 +48,6 @@ int bucket_of(int K) {
     return kBuckets - 1;
 }
 
-// the built-in rule (measured when the shapes were written)
-int default_shape(int, int) { return kShapeBig; }
-
 bool valid(int L, int, int shape) {
     return shape == kShapeBig || (shape == kShapeMid && L <= 2);
 }
@@ -96,8 +93,7 @@ __global__ void k_uniform(uint32_t* x, int64_t n, uint32_t p, uint64_t seed) {
 int tc_shape_for(int L, int K) {
     std::lock_guard<std::mutex> lock(g_mu);
     if (!g_loaded) load_locked(default_path());
-    const int t = g_table[std::min(std::max(L, 1), 4)][bucket_of(K)];
-    return t >= 0 ? t : default_shape(L, K);
+    return g_table[std::min(std::max(L, 1), 4)][bucket_of(K)];
 }
 
 }  // namespace gbgpu
@@ -165,7 +161,7 @@ extern "C" int gbgpu_autotune(int32_t device, const char* path) {
                 if (valid(L, kKmax[b], sh)) cands[nc++] = sh;
             if (nc < 2) continue;
             float best = 1e30f;
-            int best_sh = default_shape(L, K);
+            int best_sh = kShapeBig;
             for (int c = 0; c < nc; ++c) {
                 TcGemmArgs g{p, M, N, K, A, Kmax, B, N, D, N};
                 long long launches = 0;

@@ -41,3 +41,36 @@ def test_submul_edges(p, M, N, K, off, extra):
                                               dbuf.data_ptr() + 4 * off, ldd, C.byref(opt)))
     view[:, :N] = exact_submul(D, A, B, p)
     assert np.array_equal(dbuf.cpu().numpy(), buf)
+
+
+def run(p, D, A, B, torch):
+    M, K, N = A.shape[0], A.shape[1], B.shape[1]
+    dA, dB, dD = (torch.from_numpy(x.astype(np.int32)).cuda() for x in (A, B, D))
+    opt = _lib.Options(_lib.FORM_TENSOR, 0, 1, 0, torch.cuda.current_stream().cuda_stream)
+    _lib.check(_lib.load().gbgpu_dense_submul(p, M, N, K, dA.data_ptr(), K, dB.data_ptr(), N,
+                                              dD.data_ptr(), N, C.byref(opt)))
+    return dD.cpu().numpy()
+
+
+@pytest.mark.parametrize("p", [251, 65521])
+@pytest.mark.parametrize("M,N,K", [(1112, 1220, 200), (2520, 1221, 937), (2083, 799, 2200),
+                                   (1752, 2756, 500), (3032, 1476, 2000)])
+def test_submul_few_waves(p, M, N, K):
+    """sizes on both sides of the rule between the tile shapes (products below
+    2^32 K: exact in doubles)"""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(M + N + K)
+    A, B, D = (rng.integers(0, p, size=s).astype(np.float64) for s in ((M, K), (K, N), (M, N)))
+    assert np.array_equal(run(p, D, A, B, torch), ((D - A @ B) % p).astype(np.int32))
+
+
+@pytest.mark.parametrize("p,panel", [(251, 32768), (65521, 16384), (16777213, 10880),
+                                     ((1 << 24) + 43, 8192), (2147483647, 8192)])
+def test_submul_full_accumulators(p, panel):
+    """every operand p - 1, a whole panel of K and the start of the next:
+    A B = K mod p everywhere"""
+    torch = pytest.importorskip("torch")
+    K = panel + 64
+    D = np.random.default_rng(K).integers(0, p, size=(130, 70))
+    A, B = np.full((130, K), p - 1), np.full((K, 70), p - 1)
+    assert np.array_equal(run(p, D, A, B, torch), ((D - K) % p).astype(np.int32))
