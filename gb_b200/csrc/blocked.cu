@@ -16,16 +16,14 @@
 //                                                  pivots of block k touch)
 //      with X_k stored over W[:, k]; (b) D' = D - X B as one GEMM whose zero
 //      tiles (staircase X, banded B) are skipped.
-//   2. Echelon of D': one claim round first (the first row of every distinct
-//      lead becomes a pivot, all other rows are eliminated against these at
-//      once), then 128-column panels, left to right, for the rows that remain:
-//      the pending rows whose lead lies in the panel (128 at a time) are brought to echelon form
-//      inside the panel in shared memory (k_panel_factor), the recorded row
-//      transformation is applied to their trailing columns with one GEMM, the
-//      pivots found are registered, and the panel's other pending rows are
-//      eliminated against them (eliminate: gathered pivot columns, block
-//      inverses, GEMMs).
-//   3. Back substitution to reduced echelon form, blocks of 128 pivots from
+//   2. Echelon of D' by rounds over all pending rows: a 128-column panel whose
+//      rows all have leads of their own gives them as pivots; up to 256 rows of
+//      every other panel are brought to reduced echelon form inside the panel by
+//      one thread-block cluster (k_panel_factor), the row transformation it
+//      records is applied to the pivot rows' whole width (k_panel_apply), and
+//      the round's other pending rows are eliminated against all its pivots
+//      (eliminate: gathered pivot columns, block inverses, GEMMs).
+//   3. Back substitution to reduced echelon form, blocks of 1024 pivots from
 //      the last to the first: U_k -= U_k[:, piv(>k)] R_(>k) (GEMM against the
 //      already reduced later rows), then U_k = (U_k[:, piv(k)])^-1 U_k.
 //   4. Compaction into CSR rows in descending lead order (plain.cu kernels).
