@@ -394,14 +394,16 @@ __global__ void k_gather_cols(int32_t rows, int32_t n, const uint32_t* __restric
                               int64_t lds, const int32_t* __restrict__ cols, uint32_t* dst,
                               int64_t ldd, const int32_t* __restrict__ rlist = nullptr) {
     GB_WARP_ROWS(rows, n) {
-        const uint32_t* s = src + (size_t)(rlist ? rlist[i] : i) * lds;
+        const int32_t r = rlist ? rlist[i] : i;
+        const uint32_t* s = src + (size_t)max(r, 0) * lds;
         uint32_t* o = dst + (size_t)i * ldd;
         for (int j0 = jb + lane; j0 < je; j0 += 128) {
             uint32_t v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int jj = j0 + 32 * u;
-                v[u] = jj < je ? s[cols[jj]] : 0u;
+                const int32_t col = jj < je && r >= 0 ? cols[jj] : -1;
+                v[u] = col >= 0 ? s[col] : 0u;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -432,7 +434,7 @@ __global__ void k_scatter_rows_dense(int32_t nrows, const int32_t* __restrict__ 
 }
 
 // first nonzero column of every row (-1 for zero rows), one warp per row;
-// with from_prev the scan starts at the row's current lead (leads only move
+// (negative entries of list: none); with from_prev the scan starts at the row's current lead (leads only move
 // right under elimination).  A pass covers LEAD_U chunks of 32 columns whose
 // loads are in flight together.
 constexpr int LEAD_U = 8;
@@ -444,6 +446,7 @@ __global__ void k_row_leads(int32_t rows, const int32_t* __restrict__ list, int3
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int i = warp; i < rows; i += nwarps) {
         const int32_t r = list ? list[i] : i;
+        if (r < 0) continue;
         const uint32_t* row = M + (size_t)r * ld;
         int found = -1;
         const int start = from_prev && lead[r] > 0 ? lead[r] : 0;
@@ -1389,19 +1392,29 @@ static int echelon_rref(Ctx& c, const F& f, uint32_t* Dp, int64_t ld, int32_t t,
         }
         // all pivots of the round, ascending columns, and the rows left; the
         // panels' pivots are normalised already
-        BL_LAUNCH(k_round_finish<<<1, RD_THREADS, 0, s>>>(rs, KB, 0));
-        if (n_clean > 0)
-            BL_LAUNCH(k_normalize_at<F><<<std::min(t, 148 * 8), 256, 0, s>>>(counters, prow, pc, ncr,
-                                                                             Dp, ld, f));
-        BL_CUDA(cudaStreamSynchronize(s));
-        const int32_t n_new = info->n_new, n_rest = info->n_rest;
-        if (trace_rounds()) fprintf(stderr, "gbgpu echelon round %d: new pivots %d\n", rounds, n_new);
-        if (n_rest == 0) break;
-        // the first pivot column of every block of KB pivots
-        std::vector<int32_t> h_first;
-        BL_CHECK(first_columns(c, info, pc, n_new, &h_first));
-        // one panel alone: its pivot rows are reduced among themselves already
+        //
+        // One panel alone: its pivot rows are reduced among themselves already, and
+        // the elimination is one product over at most KB pivots and n_pend rows, so
+        // the host does not wait for the counts (dense RREF of 48 rounds: 14.3 -> 14.1 ms).
         const bool unit = n_dirty == 1 && n_clean == 0;
+        BL_LAUNCH(k_round_finish<<<1, RD_THREADS, 0, s>>>(rs, KB, 0, unit ? n_pend : 0));
+        int32_t n_new = std::min(KB, ncr), n_rest = n_pend;
+        std::vector<int32_t> h_first;
+        if (unit) {
+            h_first.assign(1, info->first_panel * KB);  // zero left of the panel
+        } else {
+            if (n_clean > 0)
+                BL_LAUNCH(k_normalize_at<F><<<std::min(t, 148 * 8), 256, 0, s>>>(counters, prow, pc, ncr,
+                                                                                 Dp, ld, f));
+            BL_CUDA(cudaStreamSynchronize(s));
+            n_new = info->n_new;
+            n_rest = info->n_rest;
+            if (trace_rounds())
+                fprintf(stderr, "gbgpu echelon round %d: new pivots %d\n", rounds, n_new);
+            if (n_rest == 0) break;
+            // the first pivot column of every block of KB pivots
+            BL_CHECK(first_columns(c, info, pc, n_new, &h_first));
+        }
         BL_CHECK(eliminate(c, f, Dp, ld, pend, n_rest, ncr, prow, n_new, pc, h_first, unit));
         BL_LAUNCH(k_row_leads<<<grid_of((int64_t)n_rest * 32), 256, 0, s>>>(n_rest, pend, ncr, Dp,
                                                                              ld, lead, 1));

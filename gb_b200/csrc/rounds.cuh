@@ -208,8 +208,11 @@ __global__ void __launch_bounds__(RD_THREADS) k_round_plan(const RoundState a, i
 }
 
 // The round's new pivots (`all`: every pivot) in ascending column order, and the
-// rows left, in row order.
-__global__ void __launch_bounds__(RD_THREADS) k_round_finish(const RoundState a, int32_t kb, int32_t all) {
+// rows left, in row order.  With pad_rows > 0 the lists are filled up with -1, the
+// pivots to kb (they are at most as many) and the rows to pad_rows, for a
+// host that does not wait for their lengths.
+__global__ void __launch_bounds__(RD_THREADS)
+k_round_finish(const RoundState a, int32_t kb, int32_t all, int32_t pad_rows = 0) {
     __shared__ int s_warp[RD_WARPS];
     const int tid = threadIdx.x;
     // four columns (rows) per thread and pass
@@ -249,6 +252,10 @@ __global__ void __launch_bounds__(RD_THREADS) k_round_finish(const RoundState a,
         for (int u = 0; u < 4; ++u)
             if (p[u]) a.pend[at++] = r0 + u;
         rest += total;
+    }
+    if (pad_rows > 0) {
+        for (int k = n + tid; k < min(kb, a.ncr); k += RD_THREADS) a.pc[k] = a.prow[k] = -1;
+        for (int k = rest + tid; k < pad_rows; k += RD_THREADS) a.pend[k] = -1;
     }
     if (tid == 0) {
         *a.n_new = n;
