@@ -426,6 +426,9 @@ k_small(int32_t n, const SmallItem one, const SmallItem* items, const uint8_t* i
     extern __shared__ __align__(16) uint32_t sm_smem[];
     __shared__ int s_item;
     const int CL = cluster_size(), rk = cluster_rank(), tid = threadIdx.x;
+    // the queue's first entry goes to the other CTAs' shared memory, which may be
+    // written only once all of them have started
+    if (items) cluster_sync();
     for (int pass = 0;; ++pass) {
         if (items) {
             if (rk == 0 && tid < 32) {
