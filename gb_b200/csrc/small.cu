@@ -59,7 +59,8 @@ struct SmallItem {
 
 __host__ __device__ inline int64_t rup(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
 // scratch of one matrix: pivot row of every left column [ncl] | its entries'
-// extent [ncl] | C|D rows [nr] | checks' verdict | diagonal blocks [ncl][LB]
+// extent [ncl] | C|D rows [nr] | checks' verdict, then the missing pivots' bit
+// while the checks run | diagonal blocks [ncl][LB]
 // | dense rows [n_work][ncr] of the three-launch form
 struct ScrLayout {
     int64_t piv, pext, work, err, diag, D, bytes;
@@ -137,7 +138,7 @@ __device__ uint32_t small_prep(const SmallMat& a, uint32_t* smem, int smem_words
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gw = rk * kTinyWarps + warp, ngw = CL * kTinyWarps;
     for (int c = rk * kTinyThreads + tid; c < a.ncl; c += CL * kTinyThreads) a.piv_row[c] = INT_MAX;
-    if (rk == 0 && tid == 0) *a.err = 0;
+    if (rk == 0 && tid == 0) a.err[0] = a.err[1] = 0;
     cluster_sync();
     for (int i = gw; i < a.nr; i += ngw) {
         const int64_t b = a.row_ptr[i], e = a.row_ptr[i + 1];
@@ -160,11 +161,14 @@ __device__ uint32_t small_prep(const SmallMat& a, uint32_t* smem, int smem_words
         if (lane == 0 && bad) atomicOr(a.err, bad);
     }
     cluster_sync();
-    const bool good = __ldcg(a.err) == 0;  // the rows may be walked
+    // the rows may be walked.  The block barriers below are inside this branch, so
+    // every thread has to read the same: the loop behind it reports missing pivots
+    // in a word of its own
+    const bool good = __ldcg(a.err) == 0;
     for (int c = gw; c < a.ncl; c += ngw) {
         const int32_t r = __ldcg(a.piv_row + c);
         if (r == INT_MAX) {
-            if (lane == 0) atomicOr(a.err, kErrMissingPivot);
+            if (lane == 0) atomicOr(a.err + 1, kErrMissingPivot);
             continue;
         }
         if (!good) continue;
@@ -201,7 +205,8 @@ __device__ uint32_t small_prep(const SmallMat& a, uint32_t* smem, int smem_words
         }
     }
     cluster_sync();
-    const uint32_t verdict = __ldcg(a.err);
+    const uint32_t verdict = __ldcg(a.err) | __ldcg(a.err + 1);
+    if (rk == 0 && tid == 0) a.err[0] = verdict;  // for the launches behind this one
     if (verdict == 0) {
         // a warp per block U (unit upper triangular), lane j column j of its
         // inverse V, from the last row up: V[i] = e_i - sum_(k > i) U[i][k] V[k]

@@ -7,7 +7,8 @@ import re
 import pytest
 
 import oracle
-from gb_b200 import la, synth
+from gb_b200 import _lib, la, synth
+from gb_b200.matrix import MacaulayMatrix
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "gb_b200", "csrc")
 PRIMES = [2, 251, 65521, 65537, 2147483647]
@@ -46,3 +47,46 @@ def test_batches_around_the_clusters_of_the_device(count):
         assert not any(status)
         for i, (a, w) in enumerate(zip(answers, want)):
             assert a.equals(w), (i, a.first_difference(w))
+
+
+def test_the_checks_verdict_is_uniform_where_barriers_depend_on_it():
+    """Between the read that opens the branch with block barriers and the next
+    cluster barrier nothing writes the word that was read."""
+    body = body_of("small.cu", "small_prep")
+    part = body[body.index("const bool good"):]
+    part = part[:part.index("cluster_sync()")]
+    assert "__syncthreads()" in part and "__ldcg(a.err) == 0" in part
+    assert not re.search(r"atomic\w+\(\s*a\.err\s*,|\*a\.err\s*=|a\.err\[0\]\s*=", part)
+
+
+def without_pivots(m, columns):
+    """`m` with the rows of the given left columns' pivots led by column 0 instead:
+    every row is valid, the columns have no pivot."""
+    cols = m.cols.copy()
+    for i in range(m.nr):
+        b, e = m.row_ptr[i], m.row_ptr[i + 1]
+        if cols[b] in columns:
+            assert 0 not in cols[b:e]
+            cols[b] = 0
+    return MacaulayMatrix(m.p, m.ncl, m.ncr, m.row_ptr, cols, m.vals)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", [251, 65521, 2147483647])
+@pytest.mark.parametrize("nru,nrl,ncr", [(3, 1, 2), (130, 40, 60), (900, 30, 90), (1400, 20, 50),
+                                         (300, 200, 50)])
+def test_missing_pivots_of_valid_rows(nru, nrl, ncr, p):
+    """One launch and three, alone and beside valid matrices: the call is refused
+    with that reason, and the next one is answered."""
+    m = synth.random_macaulay(nru, nrl, ncr, p, density=0.05, seed=nru + nrl)
+    want, _ = oracle.oracle_la(m)
+    for columns in ({nru - 1}, set(range(1, nru))):
+        bad = without_pivots(m, columns)
+        with pytest.raises(_lib.GbgpuError) as ei:
+            la.linear_algebra(bad)
+        assert ei.value.code == _lib.GBGPU_EINVAL and "pivot" in str(ei.value)
+        assert la.linear_algebra(m).equals(want)
+        answers, status = la.reduce_batch([bad, m] * 5)
+        assert list(status) == [_lib.GBGPU_EINVAL, 0] * 5
+        assert all(a is None for a in answers[::2])
+        assert all(a.equals(want) for a in answers[1::2])
