@@ -793,13 +793,25 @@ struct Ctx {
         tmp.push_back(q);
         return (T*)q;
     }
+    // frees, in stream order, what was allocated since tmp held n buffers
+    void release_to(size_t n) {
+        for (; tmp.size() > n; tmp.pop_back()) cudaFreeAsync(tmp.back(), s);
+    }
     void release() {
-        for (void* q : tmp) cudaFreeAsync(q, s);
-        tmp.clear();
+        release_to(0);
         if (ws) cudaFreeAsync(ws, s);
         ws = nullptr;
         ws_bytes = 0;
     }
+};
+
+// Buffers of one step, freed behind it: the rounds of an echelon would otherwise
+// hold them all until it ends (rows x 512 bytes a round, and more).
+struct Scratch {
+    Ctx& c;
+    size_t n;
+    explicit Scratch(Ctx& c_) : c(c_), n(c_.tmp.size()) {}
+    ~Scratch() { c.release_to(n); }
 };
 
 #define BL_CHECK(expr)                                                   \
@@ -862,6 +874,7 @@ static int gemm_set_in_place(Ctx& c, TcGemmArgs g) {
     uint32_t* D = g.D;
     const int64_t ldd = g.ldd;
     const int32_t* rows = g.d_rows;
+    const Scratch scratch(c);
     uint32_t* T = c.alloc<uint32_t>((size_t)g.M * g.N);
     if (!T) return GBGPU_ENOMEM;
     g.D = T;
@@ -926,6 +939,7 @@ static int neg_inverse_big(Ctx& c, const F& f, const uint32_t* src, int64_t lds,
                            int64_t stride_src, int32_t n_blocks, int32_t last_nb, int32_t NB,
                            uint32_t* out) {
     if (n_blocks <= 0) return GBGPU_OK;
+    const Scratch scratch(c);
     const int64_t bstride = (int64_t)NB * (NB + 1);
     uint32_t* U = c.alloc<uint32_t>((size_t)n_blocks * bstride);
     uint32_t* T = c.alloc<uint32_t>((size_t)n_blocks * NB * NB / 4 + 1);
@@ -1016,6 +1030,7 @@ static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t*
                      int32_t rows, int32_t ncols, const int32_t* u_rows, int32_t n_p,
                      const int32_t* d_pc, const std::vector<int32_t>& h_first, bool unit) {
     if (rows <= 0 || n_p <= 0) return GBGPU_OK;
+    const Scratch scratch(c);
     if (unit) {  // U[:, pc] is the identity (at most KB pivots): T -= T[:, pc] U
         uint32_t* G = c.alloc<uint32_t>((size_t)rows * KB);
         if (!G) return GBGPU_ENOMEM;
