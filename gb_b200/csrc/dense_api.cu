@@ -35,20 +35,20 @@ int run_dense(int32_t p, int32_t M, int32_t N, int32_t K, const uint32_t* A, int
         return GBGPU_EINVAL;
     }
     if (tensor) {
+        // the status word behind the workspace: one allocation (5 us where a
+        // finished plan's stream is parked, see StreamKit)
         void* ws = nullptr;
-        int32_t* err = nullptr;
-        const size_t bytes = tc_workspace_bytes((uint32_t)p, M, N, K);
-        if (cudaMallocAsync(&ws, bytes > 0 ? bytes : 1, s) != cudaSuccess ||
-            cudaMallocAsync((void**)&err, sizeof(int32_t), s) != cudaSuccess) {
+        const size_t bytes = (tc_workspace_bytes((uint32_t)p, M, N, K) + 255) & ~(size_t)255;
+        if (cudaMallocAsync(&ws, bytes + sizeof(int32_t), s) != cudaSuccess) {
             set_error("dense GEMM workspace allocation failed");
             return GBGPU_ENOMEM;
         }
+        int32_t* err = (int32_t*)((uint8_t*)ws + bytes);
         cudaMemsetAsync(err, 0, sizeof(int32_t), s);
         rc = tc_submul(g, ws, s, err, &launches);
         int32_t herr = 0;
         cudaMemcpyAsync(&herr, err, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
         cudaFreeAsync(ws, s);
-        cudaFreeAsync(err, s);
         cudaError_t e = cudaStreamSynchronize(s);
         if (!rc && e != cudaSuccess) {
             set_error(std::string("dense GEMM: ") + cudaGetErrorString(e));
