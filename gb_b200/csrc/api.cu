@@ -308,7 +308,7 @@ struct Plan {
     // small matrices: one-cluster echelon + compaction, no host round trip in a
     // run; its checks, counts and timings are read when the answer is taken
     bool tiny = false;
-    int tiny_cl = 0;  // CTAs of its cluster
+    int32_t tiny_cap = 0;  // rows its cluster holds at a time
     int64_t* tiny_counts = nullptr;  // [3]: rows, entries of the answer, verdict
     bool pending = false;            // a tiny run whose results are not read yet
     // answer streamed to host arrays during the run (gbgpu_plan_run_into_v)
@@ -427,8 +427,8 @@ static int plan_alloc(Plan* P) {
     // small blocks; larger ones show the sparse-row form's own echelon
     if (P->mode == 0 && !P->blocked && P->n_work > 0 && P->ncr > 0 &&
         (int64_t)P->n_work * P->ncr <= kTinyPlanBlock)
-        P->tiny_cl = tiny_cluster(P->n_work, P->ncr, P->dev.smem_optin);
-    P->tiny = P->tiny_cl > 0;
+        P->tiny_cap = tiny_capacity(P->n_work, P->ncr, P->dev.smem_optin);
+    P->tiny = P->tiny_cap > 0;
     if (P->tiny) {
         // the answer has at most n_work rows of ncr entries
         const size_t cap = (size_t)P->n_work * P->ncr;
@@ -680,10 +680,10 @@ static int run_form(Plan* P, const F& f) {
     GB_CUDA(cudaEventRecord(P->ev[2], s));
 
     if (P->tiny) {
-        // ---- small right block: echelon form and compaction in one CTA ------
+        // ---- small right block: echelon form and compaction in one cluster --
         GB_CALL(launch_tiny_rref(P->n_work, P->ncr, P->D, P->ld, P->err, P->ncl,
                                  P->offs, P->out_cols, P->out_vals, P->piv_of_col,
-                                 P->tiny_counts, P->tiny_cl, s, f));
+                                 P->tiny_counts, P->tiny_cap, s, f));
         P->stats.echelon_rounds = 0;
         GB_CUDA(cudaEventRecord(P->ev[3], s));
         GB_CUDA(cudaEventRecord(P->ev[4], s));

@@ -85,15 +85,16 @@ cudaError_t launch_promote(int grid, int threads, cudaStream_t s, const int32_t*
                            int32_t* piv_of_col, uint32_t* rows, int64_t ld, int32_t ncr,
                            int32_t* losers, int32_t* n_losers, const F& f);
 
-// one-CTA reduced row echelon form of a small dense block (see plain.cu)
-int tiny_cluster(int32_t n, int32_t m, int smem_optin);
+// reduced row echelon form of a small dense block in one cluster (see plain.cu),
+// cap = tiny_capacity rows at a time
+int tiny_capacity(int32_t n, int32_t m, int smem_optin);
 // a launch of grid CTAs in clusters of cl
 cudaError_t launch_cluster(const void* kernel, int grid, int cl, int threads, int bytes,
                            cudaStream_t s, void** args);
 template <class F>
 cudaError_t launch_tiny_rref(int32_t n, int32_t m, const uint32_t* D, int64_t ld,
                              const uint32_t* err, int32_t col_shift, int64_t* offs, int32_t* cols,
-                             int32_t* vals, int32_t* piv_of_col, int64_t* counts, int cl,
+                             int32_t* vals, int32_t* piv_of_col, int64_t* counts, int32_t cap,
                              cudaStream_t s, const F& f);
 
 __global__ void k_claim(const int32_t* cand, const int32_t* n_cand, const int32_t* lead,

@@ -690,9 +690,12 @@ cudaError_t launch_promote(int grid, int threads, cudaStream_t s, const int32_t*
 // rows in descending pivot-column order as CSR (columns + col_shift), their
 // offsets, piv_of_col, and counts[0..1] = rows, entries.  When the input
 // checks flagged an error nothing is read and the answer is empty.
+//
+// A block with more rows than the cluster holds (cap) comes in turns: the pivot
+// rows so far stay, the free places take the next rows.
 template <class F>
 __global__ void __launch_bounds__(kTinyThreads, 1)
-k_tiny_rref(int32_t n, int32_t m, const uint32_t* __restrict__ D, int64_t ld,
+k_tiny_rref(int32_t n, int32_t cap, int32_t m, const uint32_t* __restrict__ D, int64_t ld,
             const uint32_t* err, TinyOut out, F f) {
     extern __shared__ __align__(16) uint32_t tiny_smem[];
     const int CL = cluster_size(), rk = cluster_rank();
@@ -710,20 +713,30 @@ k_tiny_rref(int32_t n, int32_t m, const uint32_t* __restrict__ D, int64_t ld,
         return;
     }
     if (rk == 0 && threadIdx.x == 0) out.counts[2] = 0;
-    for (int t = rk; t * TP < m; t += CL)
-        for (int q = threadIdx.x; q < n * TP; q += kTinyThreads) {
-            const int r = q / TP, j = t * TP + q % TP;
-            tiny_smem[(t / CL) * n * TP + q] = j < m ? D[(size_t)r * ld + j] : 0u;
-        }
-    tiny_rref_body(n, m, tiny_smem, out, f);
+    for (int r0 = 0, kept = 0;;) {
+        const int take = min(n - r0, cap - kept);
+        for (int t = rk; t * TP < m; t += CL)
+            for (int q = threadIdx.x; q < (cap - kept) * TP; q += kTinyThreads) {
+                const int r = q / TP, j = t * TP + q % TP;
+                tiny_smem[((t / CL) * cap + kept) * TP + q] =
+                    r < take && j < m ? D[(size_t)(r0 + r) * ld + j] : 0u;
+            }
+        r0 += take;
+        if (r0 >= n) break;
+        tiny_echelon<false>(cap, m, tiny_smem, f);
+        kept = tiny_keep(cap, m, tiny_smem);
+    }
+    tiny_rref_body(cap, m, tiny_smem, out, f);
 }
 
-// CTAs of k_tiny_rref's cluster for an n x m block (0: too large)
-int tiny_cluster(int32_t n, int32_t m, int smem_optin) {
-    const int64_t room = smem_optin - 4096;
-    return tiny_layout(n, m, kTinyMaxCluster).words * 4 <= room ? kTinyMaxCluster : 0;
+// Rows of an n x m block that k_tiny_rref's cluster holds at a time (n: all of
+// them; 0: the block is not for it).
+int tiny_capacity(int32_t n, int32_t m, int smem_optin) {
+    const int64_t words = (smem_optin - 4096) / 4;
+    if (tiny_layout(n, m, kTinyMaxCluster).words <= words) return n;
+    const int64_t cap = tiny_rows(m, kTinyMaxCluster, words);
+    return m <= kTinyTallCols && n <= kTinyTallTurns * (cap - m) ? (int)cap : 0;
 }
-
 cudaError_t launch_cluster(const void* kernel, int grid, int cl, int threads, int bytes,
                            cudaStream_t s, void** args) {
     cudaError_t e = ensure_smem_limit(kernel, bytes);
@@ -746,13 +759,14 @@ cudaError_t launch_cluster(const void* kernel, int grid, int cl, int threads, in
 template <class F>
 cudaError_t launch_tiny_rref(int32_t n, int32_t m, const uint32_t* D, int64_t ld,
                              const uint32_t* err, int32_t col_shift, int64_t* offs, int32_t* cols,
-                             int32_t* vals, int32_t* piv_of_col, int64_t* counts, int cl,
+                             int32_t* vals, int32_t* piv_of_col, int64_t* counts, int32_t cap,
                              cudaStream_t s, const F& f) {
     TinyOut o{col_shift, offs, cols, vals, piv_of_col, counts};
     F fv = f;
-    void* args[] = {&n, &m, &D, &ld, &err, &o, &fv};
+    constexpr int cl = kTinyMaxCluster;
+    void* args[] = {&n, &cap, &m, &D, &ld, &err, &o, &fv};
     return launch_cluster((const void*)k_tiny_rref<F>, cl, cl, kTinyThreads,
-                          (int)(tiny_layout(n, m, cl).words * 4), s, args);
+                          (int)(tiny_layout(cap, m, cl).words * 4), s, args);
 }
 
 #define GBGPU_INSTANTIATE(F)                                                                   \

@@ -618,7 +618,7 @@ int64_t small_words(int32_t nr, int32_t ncl, int32_t ncr, int cl, int smem_optin
 // The three-launch form takes matrices whose echelon fits a cluster and four of
 // whose accumulators fit an SM.
 bool small_wide(int32_t nr, int32_t ncl, int32_t ncr, int smem_optin) {
-    return nr > ncl && tiny_cluster(nr - ncl, ncr, smem_optin) > 0 &&
+    return nr > ncl && tiny_capacity(nr - ncl, ncr, smem_optin) > 0 &&
            small_warps(4, ncl + ncr, (smem_optin - 2048) / 4) == 4;
 }
 
@@ -725,7 +725,7 @@ int small_reduce(const SmallInput& in, SmallAnswer* ans) {
             if (e == cudaSuccess)
                 e = launch_tiny_rref(n_work, ncr, D, ld, a.err, ncl, (int64_t*)(hd + O.offs),
                                      (int32_t*)(hd + O.cols), (int32_t*)(hd + O.vals), nullptr,
-                                     (int64_t*)hd, tiny_cluster(n_work, ncr, optin), s, f);
+                                     (int64_t*)hd, tiny_capacity(n_work, ncr, optin), s, f);
         };
         if ((uint32_t)in.p < 65536u) run(it.fs);
         else run(it.fm);

@@ -42,6 +42,14 @@ constexpr int kTinyThreads = 512;
 constexpr int kTinyWarps = kTinyThreads / 32;
 constexpr int kTinyMaxCluster = 8;          // the portable limit
 constexpr int TP = 16;                      // panel columns
+// Tall blocks that come in turns (k_tiny_rref): a row takes 49 words of every CTA
+// however few columns it has, so 1111 rows fit.  With a launch of one CTA, whose rows
+// took a word a column, blocks of up to 7130 rows had this path; all of those and the
+// wider ones up to 48 columns are faster here than by the echelon rounds of a plan
+// (a call, 100 left columns, p = 2^31 - 1, in turns / rounds): 1200 x 1 151 / 494 us,
+// 7000 x 1 428 / 1002, 1200 x 48 236 / 2188, 4000 x 48 468 / 2423, 7000 x 20 643 /
+// 1498.  Only a plan's run alone gains little with one column: 7000 x 1 862 / 854.
+constexpr int kTinyTallCols = 48, kTinyTallTurns = 7;
 constexpr int kRelayRows = 64;              // from here panels are passed on in two steps
 // Shared memory of one CTA for an n x m block in a cluster of cl (offsets in
 // 32-bit words): its panels [panels / cl][n][TP], two copies of the current
@@ -60,6 +68,11 @@ __host__ __device__ inline TinyLayout tiny_layout(int32_t n, int32_t m, int32_t 
     L.cols = L.rows + (int64_t)n;
     L.words = (L.cols + 3 * (int64_t)L.panels * TP + 3) & ~(int64_t)3;
     return L;
+}
+// rows of a block of m columns that `words` of shared memory hold (< 0: none)
+__host__ __device__ inline int64_t tiny_rows(int32_t m, int32_t cl, int64_t words) {
+    const int64_t none = tiny_layout(0, m, cl).words, one = tiny_layout(64, m, cl).words;
+    return 64 * (words - none - 4) / (one - none);
 }
 // word offset of entry (r, j) in the CTA that owns it, (j / TP) % CL
 __device__ __forceinline__ int tiny_at(int n, int r, int j, int cl_shift) {
@@ -460,6 +473,32 @@ __device__ int tiny_echelon(const int32_t n, const int32_t m, uint32_t* smem, co
     }
     cluster_sync();
     return found;
+}
+
+// The pivot rows of an n-row block to its first rows, in column order; their
+// number.  Through the two copies of the current panel, which are free between
+// echelons and hold 2 n rows of one panel (the callers' m is at most a panel a CTA
+// and at most n).  Reached by every thread of every CTA, behind tiny_echelon.
+__device__ inline int tiny_keep(const int32_t n, const int32_t m, uint32_t* smem) {
+    const int CL = cluster_size(), rk = cluster_rank(), tid = threadIdx.x;
+    const TinyLayout L = tiny_layout(n, m, CL);
+    const int32_t* prow = (const int32_t*)(smem + L.cols);
+    int32_t* place = (int32_t*)(smem + L.cols) + L.panels * TP;  // [m] pivots left of a column
+    __shared__ int s_part[kTinyWarps];
+    for (int c = tid; c < m; c += kTinyThreads) place[c] = prow[c] >= 0 ? 1 : 0;
+    __syncthreads();
+    const int np = tiny_exscan(place, m, s_part);
+    const int mine = (L.panels - rk + CL - 1) / CL;  // panels of this CTA
+    uint32_t* copy = smem + L.pb;
+    for (int q = tid; q < mine * m * TP; q += kTinyThreads) {
+        const int g = q / (m * TP), c = q / TP % m;
+        if (prow[c] >= 0)
+            copy[(g * np + place[c]) * TP + q % TP] = smem[((size_t)g * n + prow[c]) * TP + q % TP];
+    }
+    __syncthreads();
+    for (int q = tid; q < mine * np * TP; q += kTinyThreads)
+        smem[(size_t)(q / (np * TP)) * n * TP + q % (np * TP)] = copy[q];
+    return np;
 }
 
 // tiny_echelon and the compaction of its pivot rows.
