@@ -615,11 +615,16 @@ int64_t small_words(int32_t nr, int32_t ncl, int32_t ncr, int cl, int smem_optin
     return std::max<int64_t>(least, L.words + w * 2 * (int64_t)nc);
 }
 
-// The three-launch form takes matrices whose echelon fits a cluster and four of
-// whose accumulators fit an SM.
+// The three-launch form takes matrices whose echelon fits a cluster (or comes to it
+// in turns) and two of whose accumulators fit an SM (14400 columns).  With fewer
+// than four (from 7200 columns on) a block that a plan reduces in the blocked form
+// is faster there: 8000 left columns, blocks of 100 x 200, 300 x 200 and 1000 x 40,
+// here / by a plan: 1777 / 5411, 1853 / 1369 and 2678 / 8239 us; 12000: 2763 / 8628,
+// 2852 / 1875 and 5124 / 14713.
 bool small_wide(int32_t nr, int32_t ncl, int32_t ncr, int smem_optin) {
-    return nr > ncl && tiny_capacity(nr - ncl, ncr, smem_optin) > 0 &&
-           small_warps(4, ncl + ncr, (smem_optin - 2048) / 4) == 4;
+    if (nr <= ncl || !tiny_capacity(nr - ncl, ncr, smem_optin)) return false;
+    const int warps = small_warps(4, ncl + ncr, (smem_optin - 2048) / 4);
+    return warps == 4 || (warps >= 2 && (nr - ncl < 128 || ncr < 128));
 }
 
 // The three-launch form is the faster one where the cluster would take its rows
