@@ -93,8 +93,9 @@ struct FieldSmall {
         const uint32_t r = t - __umulhi(t, mu) * p;
         return r >= p ? r - p : r;
     }
-    // a residue with up to 2^14 products m v (m, v < p) added, not reduced
-    // (below 2^46), and its value
+    // a residue with fewer than kLazyTerms products m v (m, v < p) added, not
+    // reduced (below 2^46, the bound of sum_mod), and its value
+    static constexpr int kLazyTerms = 1 << 14;
     __device__ __forceinline__ uint64_t lazy_add(uint64_t t, uint32_t m, uint32_t v) const {
         return t + (uint64_t)m * v;
     }

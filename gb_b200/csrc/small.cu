@@ -45,7 +45,10 @@
 
 namespace gbgpu {
 
-constexpr int kSmallMaxLeft = 12288;  // left columns
+// Left columns.  The row phase adds a product per known pivot to a sum before it
+// reduces it, so the field's bound on such sums is one on the left columns.
+constexpr int kSmallMaxLeft = 12288;
+static_assert(kSmallMaxLeft < FieldSmall::kLazyTerms, "sums of the row phase");
 constexpr int LB = 32;                // left columns of a diagonal block (one per lane)
 
 struct SmallItem {
