@@ -606,10 +606,12 @@ SmallItem small_item(int32_t p, int32_t nr, int32_t ncl, int32_t ncr) {
 // 32-bit words of shared memory a CTA of a cluster of cl needs for a matrix of
 // this shape: the echelon's, and an accumulator for every row of the CTA up to
 // one per warp (at least four, or one per row), or four blocks of the prep
-// phase; 0: does not fit
+// phase; 0: does not fit.  A matrix of known pivots alone is only checked; it
+// comes here up to the columns of two accumulators, as those of small_wide, because
+// its whole input would pass through the session's pinned staging.
 int64_t small_words(int32_t nr, int32_t ncl, int32_t ncr, int cl, int smem_optin) {
     const int64_t room = (smem_optin - 2048) / 4, least = 4 * 2 * LB * LB;
-    if (nr <= ncl) return least;
+    if (nr <= ncl) return 4 * ((int64_t)ncl + ncr) <= room ? least : 0;
     const TinyLayout L = tiny_layout(nr - ncl, ncr, cl);
     const int32_t nc = ncl + ncr;
     const int nloc = (nr - ncl + cl - 1) / cl;

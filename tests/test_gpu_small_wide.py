@@ -65,3 +65,18 @@ def test_other_matrices_leave_it(nru, nrl, ncr):
     got, n = launches(m)
     assert n > 3
     assert got.equals(want), got.first_difference(want)
+
+
+@pytest.mark.parametrize("ncr,small", [(1, True), (COLUMNS - 700, True), (COLUMNS - 699, False),
+                                       (300000, False)])
+def test_known_pivots_alone(ncr, small):
+    """Nothing to reduce: an empty answer, and only the checks of the general path
+    (no copy through pinned memory) once the rows are long."""
+    m = banded(700, 0, ncr, 65521, seed=ncr)
+    got, n = launches(m)
+    assert (n == 1) == small
+    assert got.np == 0 and got.nnz == 0
+    m.vals[m.row_ptr[699]] = 2
+    with pytest.raises(_lib.GbgpuError) as ei:
+        la.linear_algebra(m)
+    assert ei.value.code == _lib.GBGPU_EINVAL
