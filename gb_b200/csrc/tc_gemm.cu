@@ -47,6 +47,7 @@
 #include "field.cuh"
 #include "internal.h"
 #include "tc_gemm.h"
+#include "tc_shape.h"
 
 namespace gbgpu {
 
@@ -148,12 +149,8 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 //            L = 2, 128 x 64 for L = 3, 4.  One limb keeps its accumulators twice
 //            (the next tile's MMAs run while the epilogue drains the last);
 //            2 x NW x BN does not fit the 512 TMEM columns of the others;
-//   TC_MID   one or two limbs, 128 x 64 tiles, accumulators twice: for products
-//            with fewer tiles than SMs, where a wide tile only lengthens the one
-//            tile of its SM (measured, L = 2: 512 x 512 x 128 6.4 us against 8.4,
-//            1024 x 1024 x 1024 11.7 against 14.0), and for those of few waves and
-//            short K (few_waves_mid).
-constexpr int TC_BIG = 0, TC_MID = 2;
+//   TC_MID   one or two limbs, 128 x 64 tiles, accumulators twice.
+// tc_shape.h has the rule that picks one.
 
 template <int L, int SHAPE = TC_BIG>
 struct TcCfg {
@@ -1190,25 +1187,6 @@ size_t tc_workspace_bytes(uint32_t p, int32_t M, int32_t N, int32_t K, int32_t b
     return nb * L * (Mp + Np) * Kp + ((flags + 255) & ~(size_t)255);
 }
 
-// The narrow shape for a product of up to three waves of wide tiles: a wave costs
-// a fixed part (the epilogue, which the next tile's MMAs do not overlap in the wide
-// shapes with one accumulator set) and a part per 128 columns of K, in 10 ns,
-// fitted to the times of both shapes over 1 to 3 waves and K = 200 .. 4000:
-//   two limbs, 2520 x 1220: K = 200 66 / 54 us wide / narrow, 937 80 / 67,
-//   2000 101 / 89, 4000 125 / 135; 3032 x 1476: 937 81 / 79, 2000 90 / 104;
-//   one limb, 2520 x 2500: 200 68 / 61, 937 82 / 72, 2000 78 / 94.
-// A single wave of wide tiles leaves SMs idle that the narrow ones use (the larger
-// allowance).  With more waves the wide shape's fetches overlap its epilogue, and
-// it wins at every K (5000 x 20000 x 256, two limbs: 302 against 316 us).
-static bool few_waves_mid(int L, int K, int64_t wide, int64_t narrow) {
-    const int64_t sms = num_sms(), steps = (K + 127) / 128;
-    const int64_t ww = (wide + sms - 1) / sms, wn = (narrow + sms - 1) / sms;
-    if (ww > 3) return false;
-    const int64_t cost_w = ww * (L == 1 ? 55 * steps + 1100 : 95 * steps + 750);
-    const int64_t cost_n = wn * (L == 1 ? 46 * steps + 170 : 81 * steps + 190);
-    return 100 * cost_n < (ww == 1 ? 131 : 108) * cost_w;
-}
-
 int tc_submul(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err,
               long long* launches) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.batch <= 0) return GBGPU_OK;
@@ -1221,11 +1199,7 @@ int tc_submul(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err
         return GBGPU_EINVAL;
     }
     const int L = limbs_for(g.p);
-    const int64_t rows = (g.M + 127) / 128;
-    const int64_t narrow = rows * ((g.N + 63) / 64) * g.batch;
-    const int64_t wide = rows * ((g.N + (L == 1 ? 255 : 127)) / (L == 1 ? 256 : 128)) * g.batch;
-    int shape = narrow <= num_sms() ? TC_MID : tc_shape_for(L, g.K);
-    if (shape < 0) shape = L <= 2 && few_waves_mid(L, g.K, wide, narrow) ? TC_MID : TC_BIG;
+    const int shape = tc_shape(L, g.M, g.N, g.K, g.batch, num_sms(), tc_shape_for(L, g.K));
     return tc_submul_shape(g, workspace, s, err, launches, shape);
 }
 

@@ -65,8 +65,7 @@ int tc_submul(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err
 // the same with an explicit tile shape (0 big, 2 mid; tune.cu)
 int tc_submul_shape(const TcGemmArgs& g, void* workspace, cudaStream_t s, int32_t* err,
                     long long* launches, int shape);
-// the tile shape the autotuner's cache picks for L, K; -1: none, the built-in
-// rule of tc_submul
+// the tile shape the autotuner's cache holds for L, K; -1: none (tc_shape.h)
 int tc_shape_for(int L, int K);
 // CUDA-core path (any p)
 int plain_submul(const TcGemmArgs& g, cudaStream_t s, long long* launches);

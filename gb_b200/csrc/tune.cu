@@ -1,8 +1,8 @@
 // tune.cu -- the autotuner of the tensor-core GEMM's tile shape.
 //
 // k_tc_submul has up to two tile shapes per limb count L (tc_gemm.cu: big and
-// mid); products with fewer tiles than SMs always take the mid one, the others
-// what is tuned here for their reduction depth K.
+// mid).  Products of more than three waves of tiles take what is tuned here for
+// their reduction depth K; smaller ones keep the rule of tc_shape.h.
 // gbgpu_autotune times every candidate shape on this device for every
 // (L, K bucket) -- exact modular GEMMs on uniform residues, CUDA events, best
 // of three after a warm-up -- and writes the winners to a cache file:
@@ -48,7 +48,7 @@ int bucket_of(int K) {
     return kBuckets - 1;
 }
 
-bool valid(int L, int, int shape) {
+bool valid(int L, int shape) {
     return shape == kShapeBig || (shape == kShapeMid && L <= 2);
 }
 
@@ -72,7 +72,7 @@ void load_locked(const std::string& path) {
         if (sscanf(line, "%d %d %d", &L, &kmax, &shape) != 3) continue;
         if (L < 1 || L > 4) continue;
         const int b = bucket_of(kmax);
-        if (kKmax[b] != kmax || !valid(L, kmax, shape)) continue;
+        if (kKmax[b] != kmax || !valid(L, shape)) continue;
         g_table[L][b] = shape;
     }
     fclose(f);
@@ -158,7 +158,7 @@ extern "C" int gbgpu_autotune(int32_t device, const char* path) {
             const int K = std::min(kKmax[b], Kmax);
             int cands[3], nc = 0;
             for (int sh : {kShapeBig, kShapeMid})
-                if (valid(L, kKmax[b], sh)) cands[nc++] = sh;
+                if (valid(L, sh)) cands[nc++] = sh;
             if (nc < 2) continue;
             float best = 1e30f;
             int best_sh = kShapeBig;
