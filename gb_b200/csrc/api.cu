@@ -257,6 +257,7 @@ struct Plan {
     int requested_form = GBGPU_FORM_AUTO;
     int profile = 0;
     unsigned long long* gemm_steps = nullptr;
+    bool dense_interreduced = false;  // the last run's path of an interreduction
     bool blocked = false;  // blocked (dense block) algorithm instead of sparse rows
     int check = 1;
     int32_t p = 0, nr = 0, ncl = 0, ncr = 0, nc = 0, n_work = 0;
@@ -489,12 +490,16 @@ static int plan_alloc(Plan* P) {
 //   1600 x 6000, 17: 5597 / 2029     3000 x 60000, 6: 99 / 91 ms
 //   150 x 562, 16: 448 / 440         800 x 3000, 2: 339 / 479
 //   300 x 1500, 3: 332 / 422         1000 x 200000, 3: 27 / 29 ms
+// Three and four limbs make the dense form's few blocks dearer, so it begins later:
+//   150 x 375, 30: 401 / 424 (p = 2^31 - 1), 404 / 415 (65537), 430 / 385 (251)
+//   200 x 500, 24: 459 / 432 (p = 2^31 - 1), 457 / 422 (65537), 489 / 392 (251)
 // Blocks past kDenseEntries keep the row form, whose memory is the block alone.
-constexpr int32_t kDenseRows = 128;  // one block of pivots
+constexpr int32_t kDenseRows = 128, kDenseRows3 = 160;  // one and two limbs; three and four
 constexpr unsigned long long kDenseHits = 4, kDenseTotal = 3000;
 constexpr int64_t kDenseEntries = (int64_t)1 << 28;
 static bool interreduce_may_be_dense(const Plan* P) {
-    return (P->p & 1) && P->p >= 3 && P->nr >= kDenseRows &&
+    return (P->p & 1) && P->p >= 3 &&
+           P->nr >= (limbs_for((uint32_t)P->p) <= 2 ? kDenseRows : kDenseRows3) &&
            (int64_t)P->nr * P->nc <= kDenseEntries &&
            (P->requested_form == GBGPU_FORM_AUTO || P->requested_form == GBGPU_FORM_TENSOR);
 }
@@ -546,6 +551,7 @@ static int run_form(Plan* P, const F& f) {
     // interreduction: the entries at pivot columns decide the path below
     const bool may_dense = P->mode == 1 && interreduce_may_be_dense(P);
     unsigned long long hits = 0;
+    P->dense_interreduced = false;
     if (may_dense) {
         GB_LAUNCH(k_pivot_hits<<<grid_for((int64_t)P->nr * 32, T), T, 0, s>>>(
             P->nr, P->row_ptr, P->cols, P->nc, P->piv_row, (unsigned long long*)P->work_count + 1));
@@ -668,7 +674,7 @@ static int run_form(Plan* P, const F& f) {
         ii.err = P->counters + 6;
         const int rc = interreduce_dense(ii, &launches);
         if (rc && rc != GBGPU_ENOMEM) return rc;
-        tensor = rc == GBGPU_OK;
+        tensor = P->dense_interreduced = rc == GBGPU_OK;
         cudaGetLastError();  // without the memory for its blocks: row by row
     }
     if (P->n_work > 0 && !tensor) {
@@ -938,7 +944,8 @@ int finish_stats(Plan* P) {
     P->stats.rows_reduced = P->n_work;
     P->stats.rank = P->np;
     P->stats.kernel_launches = P->launches;
-    P->stats.form_used = !P->blocked ? GBGPU_FORM_PLAIN
+    P->stats.form_used = P->dense_interreduced ? GBGPU_FORM_TENSOR
+                         : !P->blocked         ? GBGPU_FORM_PLAIN
                          : (P->form == GBGPU_FORM_TENSOR ? GBGPU_FORM_TENSOR
                                                          : GBGPU_FORM_BLOCKED_PLAIN);
     return GBGPU_OK;
