@@ -20,9 +20,9 @@
 // Measured on a B200, 441 x 491 matrix (141 x 191 block, p = 32003): 1425 us a
 // call with one CTA for the echelon and a launch per phase, 220 us now, of it
 // k_small 181 us (checks and diagonal blocks 22, rows 75, echelon 84; all three
-// are chains of dependent steps on a few SMs, not throughput).  Matrices with more rows or a longer chain of left columns
-// run the three phases as launches of their own, the rows on the whole device
-// (kWideRows below).
+// are chains of dependent steps on a few SMs, not throughput).  Matrices with more
+// rows or a longer chain of left columns run the three phases as launches of their
+// own, the rows on the whole device (kWideRows below).
 //
 // A batch's small matrices share one launch: the clusters take matrices from a
 // work queue.  The answer is the canonical one of every other path (descending
@@ -428,7 +428,7 @@ k_small_rows(const SmallMat a, int32_t n_work, uint32_t* D, int64_t ld, F f) {
 }
 
 // n matrices, items[0 .. n) from the queue, or the one in `one` (items null)
-__global__ void __launch_bounds__(kTinyThreads)
+__global__ void __launch_bounds__(kTinyThreads, 1)
 k_small(int32_t n, const SmallItem one, const SmallItem* items, const uint8_t* in, uint8_t* scr,
         uint8_t* out, int32_t* queue, int32_t smem_words) {
     extern __shared__ __align__(16) uint32_t sm_smem[];
@@ -535,8 +535,9 @@ int grow_host(uint8_t** buf, size_t* capv, size_t need, unsigned flags, cudaStre
     return GBGPU_OK;
 }
 
-// A session keeps at most this much of each buffer between calls; what one call
-// needed beyond it is given back when the call ends.
+// A batch leaves at most this much of each buffer in the session; what it needed
+// beyond that is given back when the call ends.  (Single matrices grow the buffers to
+// a high-water mark: their answer lies in them when the call returns.)
 constexpr size_t kKeepHost = (size_t)64 << 20, kKeepDevice = (size_t)256 << 20;
 
 void trim(Session& S) {
@@ -834,9 +835,9 @@ int small_batch(int32_t n, const gbgpu_csr* const* ms, int device, gbgpu_rows* o
     int32_t* d_queue = (int32_t*)(d_in + o_queue);
     cudaError_t e = cudaMemcpyAsync(d_in, h_in, (size_t)o_scr, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        // as many clusters as the device holds at two CTAs per SM where they fit
-        const int per_sm = words * 4 + 1024 <= (dev.smem_optin - 1024) / 2 ? 2 : 1;
-        const int grid = cl * std::max(1, std::min(n, dev.sms * per_sm / cl));
+        // as many clusters as the device has SMs for: the registers of k_small (128
+        // for 512 threads) leave an SM one CTA
+        const int grid = cl * std::max(1, std::min(n, dev.sms / cl));
         SmallItem none{};
         const SmallItem* its = d_items;
         uint8_t* scr = d_in + o_scr;
