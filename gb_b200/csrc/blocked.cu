@@ -433,10 +433,10 @@ __global__ void k_scatter_rows_dense(int32_t nrows, const int32_t* __restrict__ 
     }
 }
 
-// first nonzero column of every row (-1 for zero rows), one warp per row;
-// (negative entries of list: none); with from_prev the scan starts at the row's current lead (leads only move
-// right under elimination).  A pass covers LEAD_U chunks of 32 columns whose
-// loads are in flight together.
+// First nonzero column of every row (-1 for zero rows), one warp per row; entries of
+// list below 0 stand for no row.  With from_prev the scan starts at the row's current
+// lead (leads only move right under elimination).  A pass covers LEAD_U chunks of 32
+// columns whose loads are in flight together.
 constexpr int LEAD_U = 8;
 __global__ void k_row_leads(int32_t rows, const int32_t* __restrict__ list, int32_t ncols,
                             const uint32_t* __restrict__ M, int64_t ld, int32_t* lead,

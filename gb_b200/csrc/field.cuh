@@ -100,10 +100,6 @@ struct FieldSmall {
         return t + (uint64_t)m * v;
     }
     __device__ __forceinline__ uint32_t lazy_mod(uint64_t t) const { return sum_mod(t); }
-    __device__ __forceinline__ uint64_t lazy_add2(uint64_t t, uint32_t m, uint32_t v, uint32_t n,
-                                                  uint32_t w) const {
-        return t + (uint64_t)m * v + (uint64_t)n * w;
-    }
     // a^-1 = a^(p-2) mod p (0 < a < p), square and multiply
     __device__ __forceinline__ uint32_t inv(uint32_t a) const {
         uint32_t r = 1u, b = a;
@@ -185,14 +181,6 @@ struct FieldMont {
         return t >= p2 ? t - p2 : t;
     }
     __device__ __forceinline__ uint32_t lazy_mod(uint64_t t) const { return prep(redc(t)); }
-    // the same with two products at a time, kept below 2 p^2 < p 2^32 (the sum
-    // before the subtraction stays below 4 p^2 < 2^64)
-    __device__ __forceinline__ uint64_t lazy_add2(uint64_t t, uint32_t m, uint32_t v, uint32_t n,
-                                                  uint32_t w) const {
-        const uint64_t p2 = 2 * (uint64_t)p * p;
-        t += (uint64_t)m * v + (uint64_t)n * w;
-        return t >= p2 ? t - p2 : t;
-    }
     // a^-1 = a^(p-2) mod p (0 < a < p), square and multiply in Montgomery form
     __device__ __forceinline__ uint32_t inv(uint32_t a) const {
         uint32_t r = prep(1u), b = prep(a);

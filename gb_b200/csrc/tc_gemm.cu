@@ -31,8 +31,9 @@
 // 8192^3, p = 251: 879 -> 613 us; 5000 x 8000 x 1024: 359 -> 159 us (p = 251),
 // 340 -> 301 us (p = 65521), 1013 -> 717 us (p = 2^31 - 1); 5000 x 20000 x 256:
 // 410 -> 327, 471 -> 350, 1418 -> 679 us.  CTA pairs (cta_group::2, 256-row tiles)
-// move a third less per flop but run their MMAs no faster: 914 us against 1048
-// on 8192^3, p = 251, before that epilogue, and equal or slower elsewhere.
+// were tried before that epilogue only: 914 us against 1048 on 8192^3, p = 251, and
+// equal or slower elsewhere.  They move a third less per flop, and shared memory's
+// bandwidth bounds that product now (235 cycles an MMA), so this is open.
 // Every mbarrier wait is bounded (clock64 budget); on expiry the CTA records
 // GBGPU_ETIMEDOUT in *err, drains its in-flight copies and frees its TMEM.
 // No cluster multicast is used anywhere.
