@@ -793,25 +793,40 @@ struct Ctx {
         tmp.push_back(q);
         return (T*)q;
     }
-    // frees, in stream order, what was allocated since tmp held n buffers
-    void release_to(size_t n) {
-        for (; tmp.size() > n; tmp.pop_back()) cudaFreeAsync(tmp.back(), s);
+    // Buffers of one step each, for every round's step in turn: n entries of slot
+    // `which`, whatever the last step left in it.  They stay until the end: freed behind
+    // every step instead, each of a plan's runs waits in the pool for its largest
+    // buffers, which no longer find the place of the run before (20000 x 5000 staircase:
+    // 10 to 50 ms a reduction instead of 7.8).
+    enum { kU, kT, kBlocks, kInverses, kGathered, kSolved, kProduct, kSlots };
+    void* slot[kSlots] = {};
+    size_t slot_bytes[kSlots] = {};
+    uint32_t* step(int which, size_t n) {
+        const size_t bytes = std::max<size_t>(n, 1) * sizeof(uint32_t);
+        if (bytes > slot_bytes[which]) {
+            if (slot[which]) cudaFreeAsync(slot[which], s);
+            slot[which] = nullptr;
+            slot_bytes[which] = 0;
+            if (cudaMallocAsync(&slot[which], bytes, s) != cudaSuccess) {
+                slot[which] = nullptr;
+                return nullptr;
+            }
+            slot_bytes[which] = bytes;
+        }
+        return (uint32_t*)slot[which];
     }
     void release() {
-        release_to(0);
+        for (void* q : tmp) cudaFreeAsync(q, s);
+        tmp.clear();
+        for (int k = 0; k < kSlots; ++k) {
+            if (slot[k]) cudaFreeAsync(slot[k], s);
+            slot[k] = nullptr;
+            slot_bytes[k] = 0;
+        }
         if (ws) cudaFreeAsync(ws, s);
         ws = nullptr;
         ws_bytes = 0;
     }
-};
-
-// Buffers of one step, freed behind it: the rounds of an echelon would otherwise
-// hold them all until it ends (rows x 512 bytes a round, and more).
-struct Scratch {
-    Ctx& c;
-    size_t n;
-    explicit Scratch(Ctx& c_) : c(c_), n(c_.tmp.size()) {}
-    ~Scratch() { c.release_to(n); }
 };
 
 #define BL_CHECK(expr)                                                   \
@@ -874,8 +889,7 @@ static int gemm_set_in_place(Ctx& c, TcGemmArgs g) {
     uint32_t* D = g.D;
     const int64_t ldd = g.ldd;
     const int32_t* rows = g.d_rows;
-    const Scratch scratch(c);
-    uint32_t* T = c.alloc<uint32_t>((size_t)g.M * g.N);
+    uint32_t* T = c.step(Ctx::kProduct, (size_t)g.M * g.N);
     if (!T) return GBGPU_ENOMEM;
     g.D = T;
     g.ldd = g.N;
@@ -939,10 +953,9 @@ static int neg_inverse_big(Ctx& c, const F& f, const uint32_t* src, int64_t lds,
                            int64_t stride_src, int32_t n_blocks, int32_t last_nb, int32_t NB,
                            uint32_t* out) {
     if (n_blocks <= 0) return GBGPU_OK;
-    const Scratch scratch(c);
     const int64_t bstride = (int64_t)NB * (NB + 1);
-    uint32_t* U = c.alloc<uint32_t>((size_t)n_blocks * bstride);
-    uint32_t* T = c.alloc<uint32_t>((size_t)n_blocks * NB * NB / 4 + 1);
+    uint32_t* U = c.step(Ctx::kU, (size_t)n_blocks * bstride);
+    uint32_t* T = c.step(Ctx::kT, (size_t)n_blocks * NB * NB / 4 + 1);
     if (!U || !T) return GBGPU_ENOMEM;
     BL_LAUNCH(k_copy_blocks<<<grid_of((int64_t)n_blocks * NB * NB), 256, 0, c.s>>>(
         src, lds, stride_src, n_blocks, last_nb, NB, U));
@@ -1030,9 +1043,8 @@ static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t*
                      int32_t rows, int32_t ncols, const int32_t* u_rows, int32_t n_p,
                      const int32_t* d_pc, const std::vector<int32_t>& h_first, bool unit) {
     if (rows <= 0 || n_p <= 0) return GBGPU_OK;
-    const Scratch scratch(c);
     if (unit) {  // U[:, pc] is the identity (at most KB pivots): T -= T[:, pc] U
-        uint32_t* G = c.alloc<uint32_t>((size_t)rows * KB);
+        uint32_t* G = c.step(Ctx::kGathered, (size_t)rows * KB);
         if (!G) return GBGPU_ENOMEM;
         const int32_t first_col = h_first[0] & ~3;
         BL_LAUNCH(k_gather_cols<<<grid_of((int64_t)rows * n_p), 256, 0, c.s>>>(rows, n_p, M, ld, d_pc,
@@ -1045,10 +1057,10 @@ static int eliminate(Ctx& c, const F& f, uint32_t* M, int64_t ld, const int32_t*
     const int32_t NB = nb_for(n_p);
     const int32_t nb = (n_p + NB - 1) / NB;
     const int64_t bstride = (int64_t)NB * (NB + 1);
-    uint32_t* Ublk = c.alloc<uint32_t>((size_t)nb * NB * NB);   // U[:, pc] diagonal blocks
-    uint32_t* Ninv = c.alloc<uint32_t>((size_t)nb * bstride);
-    uint32_t* G = c.alloc<uint32_t>((size_t)rows * NB);         // T[:, pc_k]
-    uint32_t* X = c.alloc<uint32_t>((size_t)rows * NB);
+    uint32_t* Ublk = c.step(Ctx::kBlocks, (size_t)nb * NB * NB);  // U[:, pc] diagonal blocks
+    uint32_t* Ninv = c.step(Ctx::kInverses, (size_t)nb * bstride);
+    uint32_t* G = c.step(Ctx::kGathered, (size_t)rows * NB);      // T[:, pc_k]
+    uint32_t* X = c.step(Ctx::kSolved, (size_t)rows * NB);
     if (!Ublk || !Ninv || !G || !X) return GBGPU_ENOMEM;
     for (int b = 0; b < nb; ++b) {
         const int kb = std::min(NB, n_p - b * NB);
@@ -1514,6 +1526,8 @@ int blocked_reduce(const BlockedInput& in, BlockedOutput* out, long long* launch
     *launches += c.launches;
     out->keep = new std::vector<void*>(c.tmp);
     if (c.ws) out->keep->push_back(c.ws);
+    for (void* q : c.slot)
+        if (q) out->keep->push_back(q);
     return rc;
 }
 

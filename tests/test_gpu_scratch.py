@@ -1,4 +1,4 @@
-"""Device memory of the echelon: what a round uses is free for the next one, so the
+"""Device memory of the echelon: what a round uses serves the next one, so the
 scratch of a block does not grow with its number of rounds."""
 import ctypes as C
 
