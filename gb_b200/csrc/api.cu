@@ -147,21 +147,24 @@ int device_init(int device, DeviceInfo* info) {
 }
 
 // ---------------------------------------------------------------------------
-// Stream and events of a finished plan, kept for the next one: creating and
-// destroying a stream takes 0.12 ms, a quarter of the reduction of a small
-// matrix.  One per device waits here (the rest are destroyed), because a stream
-// that has used the stream-ordered pool makes every later allocation dearer: the
-// pool asks each living one whether its freed blocks are done, 2.7 us apiece.
-// With the four streams of a batch's workers parked, a 1295 x 1892 x 144 product
-// took 74 us instead of 57 and an interreduction of 67 rows 590 instead of 388.
-// A plan holds its kit alone from plan_setup to its destructor, which returns it
-// with no work of its own pending.
+// Streams and events of finished plans, kept for the next ones: creating and
+// destroying a stream takes 0.12 ms, a quarter of the reduction of a small matrix,
+// and longer beside running work (eight matrices of 8040 x 8200 over a batch's four
+// workers: 11.4 ms a batch, 21.8 with a stream per matrix).  At most kMaxKits per
+// device wait here (the rest are destroyed); a plan holds its kit alone from
+// plan_setup to its destructor, which returns it with no work of its own pending.
+//
+// A parked stream must not have freed blocks of the stream-ordered pool: every later
+// allocation, by anyone, asks each living stream that has whether they are done, 2.7
+// us apiece (four streams of a batch's workers: a 1295 x 1892 x 144 product 74 us
+// instead of 49, an interreduction of 67 rows 590 instead of 360).  So a plan waits
+// for its stream and gives its memory back with pool_free.
 constexpr int kPlanEvents = 8;
 struct StreamKit {
     cudaStream_t s = nullptr;
     cudaEvent_t ev[kPlanEvents] = {};
 };
-constexpr int kMaxKits = 1;
+constexpr int kMaxKits = 8;
 static std::mutex g_kit_mu;
 static std::vector<StreamKit>& kits_of(int device) {
     static auto* kits = new std::map<int, std::vector<StreamKit>>();  // outlives every plan
@@ -203,6 +206,14 @@ static void kit_return(int device, StreamKit& k) {
         }
     }
     kit_destroy(k);
+}
+
+void pool_free(void* const* q, size_t n) {
+    // another thread's stream capture in global mode forbids cudaFree, not this use
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    for (size_t k = 0; k < n; ++k) cudaFree(q[k]);
+    cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 // mapped pages (internal.h): pinning one takes longer than a round of the echelon
@@ -344,8 +355,8 @@ struct Plan {
             cudaStreamSynchronize(s_out);
             cudaStreamDestroy(s_out);
         }
-        for (void* q : bufs) cudaFreeAsync(q, stream);
         if (stream) cudaStreamSynchronize(stream);
+        pool_free(bufs.data(), bufs.size());
         kit_return(device, kit);
     }
 };
@@ -592,6 +603,11 @@ static int run_form(Plan* P, const F& f) {
     const uint32_t* final_rows = P->D;
     int64_t rows_ld = P->ld;
     BlockedOutput bo{};
+    struct Release {  // on every way out
+        BlockedOutput& bo;
+        cudaStream_t s;
+        ~Release() { blocked_release(&bo, s); }
+    } release{bo, s};
     bool tensor = P->blocked;  // tensor-core kernels ran: their status is read at the end
     if (P->blocked) {
         BlockedInput bi{};
@@ -612,10 +628,7 @@ static int run_form(Plan* P, const F& f) {
         bo.ms_event_echelon = P->ev[3];
         bo.stream_out = P->stream_req;
         const int rc = blocked_reduce(bi, &bo, &launches);
-        if (rc) {
-            blocked_release(&bo, s);
-            return rc;
-        }
+        if (rc) return rc;
         final_rows = bo.rows;
         rows_ld = bo.ld;
         P->np = (int32_t)bo.rank;
@@ -672,7 +685,8 @@ static int run_form(Plan* P, const F& f) {
         ii.stream = s;
         ii.form = GBGPU_FORM_TENSOR;
         ii.err = P->counters + 6;
-        const int rc = interreduce_dense(ii, &launches);
+        const int rc = interreduce_dense(ii, &bo, &launches);
+        if (rc) blocked_release(&bo, s);
         if (rc && rc != GBGPU_ENOMEM) return rc;
         tensor = P->dense_interreduced = rc == GBGPU_OK;
         cudaGetLastError();  // without the memory for its blocks: row by row
@@ -825,10 +839,10 @@ static int run_form(Plan* P, const F& f) {
     }
     GB_CUDA(cudaEventRecord(P->ev[5], s));
     if (tensor) {
-        blocked_release(&bo, s);
         int32_t tc_status = 0;
         GB_CUDA(cudaMemcpyAsync(&tc_status, P->counters + 6, 4, cudaMemcpyDeviceToHost, s));
         GB_CUDA(cudaStreamSynchronize(s));
+        blocked_release(&bo, s);
         if (tc_status) {
             set_error("tensor-core kernel: a bounded wait expired");
             return tc_status;

@@ -815,6 +815,14 @@ struct Ctx {
         }
         return (uint32_t*)slot[which];
     }
+    // all buffers, for blocked_release
+    std::vector<void*>* hand_over() {
+        auto* keep = new std::vector<void*>(tmp);
+        if (ws) keep->push_back(ws);
+        for (void* q : slot)
+            if (q) keep->push_back(q);
+        return keep;
+    }
     void release() {
         for (void* q : tmp) cudaFreeAsync(q, s);
         tmp.clear();
@@ -1496,7 +1504,7 @@ static int interreduce_run(const InterreduceInput& in, Ctx& c, const F& f) {
     return back_substitute(c, f, in.D, in.ld, in.ncols, in.rows, rs, info, h_first, &out);
 }
 
-int interreduce_dense(const InterreduceInput& in, long long* launches) {
+int interreduce_dense(const InterreduceInput& in, BlockedOutput* out, long long* launches) {
     Ctx c;
     c.s = in.stream;
     c.p = in.p;
@@ -1508,7 +1516,7 @@ int interreduce_dense(const InterreduceInput& in, long long* launches) {
     else
         rc = interreduce_run(in, c, FieldMont::make(in.p));
     *launches += c.launches;
-    c.release();
+    out->keep = c.hand_over();
     return rc;
 }
 
@@ -1524,10 +1532,7 @@ int blocked_reduce(const BlockedInput& in, BlockedOutput* out, long long* launch
     else
         rc = blocked_run(in, out, c, FieldMont::make(in.p));
     *launches += c.launches;
-    out->keep = new std::vector<void*>(c.tmp);
-    if (c.ws) out->keep->push_back(c.ws);
-    for (void* q : c.slot)
-        if (q) out->keep->push_back(q);
+    out->keep = c.hand_over();
     return rc;
 }
 
@@ -1584,7 +1589,8 @@ int dense_rref(const DenseRrefInput& in, int32_t* rank, long long* launches) {
 
 void blocked_release(BlockedOutput* out, cudaStream_t s) {
     if (!out->keep) return;
-    for (void* q : *out->keep) cudaFreeAsync(q, s);
+    cudaStreamSynchronize(s);
+    pool_free(out->keep->data(), out->keep->size());
     delete out->keep;
     out->keep = nullptr;
 }

@@ -81,7 +81,9 @@ struct InterreduceInput {
     int form;
     int32_t* err;
 };
-int interreduce_dense(const InterreduceInput& in, long long* launches);
+// out->keep receives its buffers
+int interreduce_dense(const InterreduceInput& in, BlockedOutput* out, long long* launches);
+// waits for s and gives the kept buffers back
 void blocked_release(BlockedOutput* out, cudaStream_t s);
 
 }  // namespace gbgpu

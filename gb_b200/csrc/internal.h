@@ -22,6 +22,9 @@ void count_launch(long long n);
 // so a launch in one host thread never sees another thread lower it.
 cudaError_t ensure_smem_limit(const void* kernel, int bytes);
 int device_init(int device, DeviceInfo* info);
+// Gives n stream-ordered allocations back whose uses are over (their stream has been
+// waited for): cudaFree takes no time for these and ties them to no stream.
+void pool_free(void* const* q, size_t n);
 // Small pages of mapped host memory on the current device, for kernels that
 // report counts to the host: a bounded pool shared by all threads (api.cu).  The
 // user returns the page with no kernel left that writes it.
